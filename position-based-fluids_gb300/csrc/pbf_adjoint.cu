@@ -11,9 +11,8 @@
 //   v2 = (p^I - x)/dt,  v3 = v2 + c POLY6 sum (v2_j - v2_i) W,
 //   omega_i = -G sum (v2_j - v2_i) x k,  eta_i = -G sum |omega_j| k,
 //   v4 = v3 + dt eps_v (eta/|eta|) x omega_i.
-// Each kernel below walks the same friends as its forward kernel (the flat
-// rows the substep recorded: friend t of particle i at list[t * N + i]) and
-// scatters neighbour terms with atomics, so the sums are not ordered: these
+// Each kernel below walks the same friends as its forward kernel (the rows
+// the substep recorded, walk_friends) and scatters neighbour terms with atomics, so the sums are not ordered: these
 // are FP32 gradients, not bit-reproducible ones.  The derivation is the same
 // as the FP64 adjoint the tests compare against.
 
@@ -42,7 +41,7 @@ __device__ __forceinline__ float len(F3 a) { return sqrtf(dot(a, a)); }
 __device__ __forceinline__ void add3(float4* a, F3 v) { atomicAdd(a, make_float4(v.x, v.y, v.z, 0.0f)); }
 
 // A friend's records as the walks below load them, four friends in flight
-// (gather_flat): its index and one or two float4 records.
+// (walk_friends): its index and one or two float4 records.
 struct Friend1 {
     uint32_t j;
     float4 a;
@@ -51,7 +50,6 @@ struct Friend2 {
     uint32_t j;
     float4 a, b;
 };
-constexpr int kAdjU = 4;
 
 // k(r) and the adjoint of its argument: d/dr [k . kb] = f kb + f'(|r|)(kb.r) r/|r|
 // with f = (h-|r|)^2/|r|, f' = -(h-|r|)(h+|r|)/|r|^2.  y is 1/|r| within an
@@ -91,7 +89,7 @@ template <typename T> __device__ __forceinline__ T block_sum(T v) {
 // v4 = v3 + dt*vort*(N x omega_i): adjoints of omega (omb) and of p^I (pb).
 __global__ void __launch_bounds__(kAdjBlock)
 adj_vorticity_kernel(DevConsts c, const float4* __restrict__ pI, const float4* __restrict__ omega,
-                     const uint32_t* __restrict__ list, const uint2* __restrict__ meta,
+                     const uint4* __restrict__ rows, const uint2* __restrict__ meta,
                      const float4* __restrict__ vb, float4* __restrict__ omb, float4* __restrict__ pb) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = c.n;
@@ -105,7 +103,7 @@ adj_vorticity_kernel(DevConsts c, const float4* __restrict__ pI, const float4* _
         j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex);
         return Friend2{j, pI[j], omega[j]};
     };
-    gather_flat<kAdjU>(list, n, i, f1.total, loadPO, [&](const Friend2& f) {
+    walk_friends(rows, n, i, f1.total, loadPO, [&](const Friend2& f) {
         const F3 r = pi - f3(f.a);
         const float r2 = dot(r, r);
         if (!xsph_pair(c, r2, f.a.w)) return;
@@ -124,7 +122,7 @@ adj_vorticity_kernel(DevConsts c, const float4* __restrict__ pI, const float4* _
     const F3 etab = (1.0f / l) * (Nb - dot(N, Nb) * N);
     FlatFriends f2(mt, kept_other(mt));
     F3 pbi = {0.0f, 0.0f, 0.0f};  // particle i's own terms, added once
-    gather_flat<kAdjU>(list, n, i, f2.total, loadPO, [&](const Friend2& f) {
+    walk_friends(rows, n, i, f2.total, loadPO, [&](const Friend2& f) {
         const F3 r = pi - f3(f.a);
         const float r2 = dot(r, r);
         if (!xsph_pair(c, r2, f.a.w)) return;
@@ -145,7 +143,7 @@ adj_vorticity_kernel(DevConsts c, const float4* __restrict__ pI, const float4* _
 // adjoints of v2 (v2b), p^I (pb) and of the XSPH factor (cbar).
 __global__ void __launch_bounds__(kAdjBlock)
 adj_viscosity_kernel(DevConsts c, const float4* __restrict__ pI, const float4* __restrict__ v2,
-                     const float4* __restrict__ omb, const float4* __restrict__ vb, const uint32_t* __restrict__ list,
+                     const float4* __restrict__ omb, const float4* __restrict__ vb, const uint4* __restrict__ rows,
                      const uint2* __restrict__ meta, float4* __restrict__ v2b, float4* __restrict__ pb,
                      float* __restrict__ cbar) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -161,7 +159,7 @@ adj_viscosity_kernel(DevConsts c, const float4* __restrict__ pI, const float4* _
             j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex);
             return Friend2{j, pI[j], v2[j]};
         };
-        gather_flat<kAdjU>(list, n, i, fr.total, loadPV, [&](const Friend2& f) {
+        walk_friends(rows, n, i, fr.total, loadPV, [&](const Friend2& f) {
             const uint32_t j = f.j;
             const F3 r = pi - f3(f.a);
             const float r2 = dot(r, r);
@@ -203,7 +201,7 @@ __global__ void adj_velocity_kernel(DevConsts c, const float4* __restrict__ xb, 
 // lambda^t (lb) from that of p^{t+1} (pbn).  q = (p^t, lambda^t).
 __global__ void __launch_bounds__(kAdjBlock)
 adj_delta_kernel(DevConsts c, const float4* __restrict__ q, const uint8_t* __restrict__ mask,
-                 const float4* __restrict__ pbn, const uint32_t* __restrict__ list, const uint2* __restrict__ meta,
+                 const float4* __restrict__ pbn, const uint4* __restrict__ rows, const uint2* __restrict__ meta,
                  float4* __restrict__ pbt, float* __restrict__ lb) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = c.n;
@@ -226,7 +224,7 @@ adj_delta_kernel(DevConsts c, const float4* __restrict__ q, const uint8_t* __res
         j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex);
         return Friend1{j, q[j]};
     };
-    gather_flat<kAdjU>(list, n, i, fr.total, loadQ, [&](const Friend1& f) {
+    walk_friends(rows, n, i, fr.total, loadQ, [&](const Friend1& f) {
         const uint32_t j = f.j;
         const float4 qj = f.a;
         const F3 r = pi - f3(qj);
@@ -253,7 +251,7 @@ adj_delta_kernel(DevConsts c, const float4* __restrict__ q, const uint8_t* __res
 // lambda^t from p^t: adjoint of p^t (pbt) from that of lambda^t (lb).
 __global__ void __launch_bounds__(kAdjBlock)
 adj_scaling_kernel(DevConsts c, const float4* __restrict__ q, const float* __restrict__ lb,
-                   const uint32_t* __restrict__ list, const uint2* __restrict__ meta, float4* __restrict__ pbt) {
+                   const uint4* __restrict__ rows, const uint2* __restrict__ meta, float4* __restrict__ pbt) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = c.n;
     if (i >= n) return;
@@ -269,7 +267,7 @@ adj_scaling_kernel(DevConsts c, const float4* __restrict__ q, const float* __res
         j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex);
         return Friend1{j, q[j]};
     };
-    gather_flat<kAdjU>(list, n, i, f1.total, loadQ, [&](const Friend1& f) {
+    walk_friends(rows, n, i, f1.total, loadQ, [&](const Friend1& f) {
         const F3 r = pi - f3(f.a);
         const float r2 = dot(r, r);
         if (!in_support(c, r2)) return;
@@ -287,7 +285,7 @@ adj_scaling_kernel(DevConsts c, const float4* __restrict__ q, const float* __res
     const float Db = lbar * Cc / (den * den) / c.rho0sq;
     FlatFriends f2(mt, kept_density(mt));
     F3 pbi = {0.0f, 0.0f, 0.0f};  // particle i's own terms, added once
-    gather_flat<kAdjU>(list, n, i, f2.total, loadQ, [&](const Friend1& f) {
+    walk_friends(rows, n, i, f2.total, loadQ, [&](const Friend1& f) {
         const uint32_t j = f.j;
         const F3 r = pi - f3(f.a);
         const float r2 = dot(r, r);
@@ -353,16 +351,16 @@ void adjoint_substep(const DevConsts& c, const AdjointTape& tp, AdjointBuffers& 
     cudaMemsetAsync(ab.omb, 0, v4, s);
     cudaMemsetAsync(ab.pb, 0, v4, s);
     cudaMemsetAsync(ab.v2b, 0, v4, s);
-    adj_vorticity_kernel<<<grid_for(n), kAdjBlock, 0, s>>>(c, tp.pI, tp.omega, tp.list, tp.meta, ab.vb, ab.omb, ab.pb);
-    adj_viscosity_kernel<<<grid_for(n), kAdjBlock, 0, s>>>(c, tp.pI, tp.v2, ab.omb, ab.vb, tp.list, tp.meta, ab.v2b,
+    adj_vorticity_kernel<<<grid_for(n), kAdjBlock, 0, s>>>(c, tp.pI, tp.omega, tp.rows, tp.meta, ab.vb, ab.omb, ab.pb);
+    adj_viscosity_kernel<<<grid_for(n), kAdjBlock, 0, s>>>(c, tp.pI, tp.v2, ab.omb, ab.vb, tp.rows, tp.meta, ab.v2b,
                                                            ab.pb, ab.scalars);
     adj_velocity_kernel<<<grid_for(n), kAdjBlock, 0, s>>>(c, ab.xb, ab.v2b, ab.pb, ab.xsb);
     for (int t = tp.iterations - 1; t >= 0; --t) {
         cudaMemsetAsync(ab.pbt, 0, v4, s);
         cudaMemsetAsync(ab.lb, 0, 4 * (size_t)n, s);
         adj_delta_kernel<<<grid_for(n), kAdjBlock, 0, s>>>(c, tp.q[t], tp.mask ? tp.mask + (size_t)t * n : nullptr,
-                                                           ab.pb, tp.list, tp.meta, ab.pbt, ab.lb);
-        adj_scaling_kernel<<<grid_for(n), kAdjBlock, 0, s>>>(c, tp.q[t], ab.lb, tp.list, tp.meta, ab.pbt);
+                                                           ab.pb, tp.rows, tp.meta, ab.pbt, ab.lb);
+        adj_scaling_kernel<<<grid_for(n), kAdjBlock, 0, s>>>(c, tp.q[t], ab.lb, tp.rows, tp.meta, ab.pbt);
         float4* tmp = ab.pb;
         ab.pb = ab.pbt;
         ab.pbt = tmp;

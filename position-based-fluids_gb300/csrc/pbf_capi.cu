@@ -49,7 +49,7 @@ struct pbf_ctx {
     uint32_t* hist = nullptr;
     uint32_t* cells = nullptr;
     uint32_t* list = nullptr;
-    uint32_t* flat = nullptr;    // the friends of the substep in order, one flat row per position (see enqueue_substep)
+    uint4* rows = nullptr;       // the friends of the substep in order, four per entry (see enqueue_substep)
     uint2* meta = nullptr;       // per-particle friend counts per circle + kept circles
     uint32_t* taint = nullptr;          // per particle: the substep that tainted it (pbf::DevConsts::taint)
     int4* cellXYZ = nullptr;            // per particle: its cell at the friends build and the scene's first key
@@ -251,6 +251,7 @@ DevConsts make_consts(const PbfParameters& p, int n) {
     c.recipPoly6q = 1.0f / c.poly6q;
     c.quotientPoly6q = (std::isnormal(c.poly6q) && std::isnormal(c.recipPoly6q) && c.h2 >= std::ldexp(1.0f, -8) &&
                         c.h2 <= 1.0f && (double)c.h2 * c.h2 * c.h2 / c.poly6q < 1e30) ? 1 : 0;
+    c.negZero2 = 0x8000000080000000ull;
     c.circles = (int)p.friendsCircles;
     c.perCircle = (int)p.particlesPerCircle;
     c.grid = p.gridBufSize;
@@ -526,12 +527,11 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
     }
     const uint32_t* keys = ctx->keys[ctx->keysIdx];
     const size_t v4 = 16 * (size_t)c.n;
-    // With a tape, the friends (flat rows), the packed (p, lambda) of every
+    // With a tape, the friends (rows), the packed (p, lambda) of every
     // iteration and omega are written straight into the tape's buffers.  The
-    // circle rows (friends builds 1 and 2), or the staged build's scratch,
-    // stay in ctx->list.
+    // circle rows stay in ctx->list.
     uint32_t* list = ctx->list;
-    uint32_t* flat = tape ? tape->list : ctx->flat;
+    uint4* rows = tape ? tape->rows : ctx->rows;
     uint2* meta = tape ? tape->meta : ctx->meta;
     float4* omega = tape ? tape->omega : ctx->omega;
     if (tape) PBF_CUDA(ctx, cudaMemcpyAsync(tape->perm, ctx->perm[ctx->keysIdx], 4 * (size_t)c.n, cudaMemcpyDeviceToDevice, s));
@@ -540,10 +540,10 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
     c.keys = keys;  // the taint of irregular positions finds a cell's particles in them
     pbf::launch_update_cells(c.n, keys, ctx->cells, tableKeys, ctx->errWord, s, ctx->cellStart);
     mark("buildFriendsList");
-    // the flat rows of the kept friends: written by the staged build, else
-    // recorded by the first density pass (or flattened when there is none)
-    bool haveFlat = pbf::launch_build_friends(c, b, ctx->pred[sortedPred], ctx->cells, list, flat, meta, ctx->errWord,
-                                              ls.friends, ls.friendsAlgorithm, s);
+    // the rows of the kept friends are recorded by the first density pass (or
+    // flattened when there is none)
+    pbf::launch_build_friends(c, b, ctx->pred[sortedPred], ctx->cells, list, meta, ctx->errWord, ls.friends,
+                              ls.friendsAlgorithm, s);
     mark("resetPartList");
     pbf::launch_reset_cells(c.n, keys, ctx->cells, tableKeys, ctx->errWord, s);
     launched += 3;
@@ -552,18 +552,16 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
     for (unsigned it = 0; it < iters; ++it) {
         float4* packed = tape ? tape->q[it] : ctx->pred[a ^ 1];
         mark("computeScaling", (int)it);
-        // the first density pass records the flat rows from circle rows when the build wrote those
-        pbf::launch_compute_scaling(c, ctx->pred[a], packed, ctx->density, list, meta, haveFlat ? flat : nullptr,
-                                    haveFlat ? nullptr : flat, ls.scaling, ls.balance, tiles(1), s);
-        haveFlat = true;
+        pbf::launch_compute_scaling(c, ctx->pred[a], packed, ctx->density, list, meta, it > 0 ? rows : nullptr,
+                                    it > 0 ? nullptr : rows, ls.scaling, ls.balance, tiles(1), s);
         mark("computeDelta", (int)it);
-        pbf::launch_compute_delta(c, b, packed, ctx->pos[sortedPos], ctx->pred[a], ctx->density, list, meta,
+        pbf::launch_compute_delta(c, b, packed, ctx->pos[sortedPos], ctx->pred[a], ctx->density, meta,
                                   it + 1 == iters, tape && tape->mask ? tape->mask + (size_t)it * c.n : nullptr,
-                                  flat, ls.delta, ls.balance, tiles(2), s);
+                                  rows, ls.delta, ls.balance, tiles(2), s);
         launched += 2;
     }
-    if (!haveFlat) {
-        pbf::launch_flatten_friends(c, list, meta, flat, s);
+    if (iters == 0) {
+        pbf::launch_flatten_friends(c, list, meta, rows, s);
         ++launched;
     }
     if (iters == 0) {  // packData with the density buffer as it stands (src/Simulation.cpp:591)
@@ -583,7 +581,7 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
     }
     if (tape) PBF_CUDA(ctx, cudaMemcpyAsync(tape->v2, ctx->vel[V], v4, cudaMemcpyDeviceToDevice, s));
     mark("applyViscosity");
-    pbf::launch_apply_viscosity(c, b, ctx->pred[a], ctx->vel[V], ctx->vel[V ^ 1], omega, list, meta, flat, ls.viscosity,
+    pbf::launch_apply_viscosity(c, b, ctx->pred[a], ctx->vel[V], ctx->vel[V ^ 1], omega, meta, rows, ls.viscosity,
                                 ls.balance, tiles(3), s);
     mark("applyVorticity");
     const int vortTiles = (c.n + ls.vorticity - 1) / ls.vorticity;
@@ -591,13 +589,13 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
         // the first half of the particles' velocities copy out while the second half runs
         const int half = vortTiles / 2;
         const size_t headBytes = 16 * (size_t)half * (size_t)ls.vorticity;
-        pbf::launch_apply_vorticity(c, ctx->pred[a], omega, ctx->vel[V ^ 1], ctx->vel[V], list, meta, flat,
+        pbf::launch_apply_vorticity(c, ctx->pred[a], omega, ctx->vel[V ^ 1], ctx->vel[V], meta, rows,
                                     ls.vorticity, ls.balance, nullptr, s, 0, half);
         PBF_CUDA(ctx, cudaEventRecord(ctx->evVelHead, s));
         PBF_CUDA(ctx, cudaStreamWaitEvent(ctx->copyStream, ctx->evVelHead, 0));
         PBF_CUDA(ctx, cudaMemcpyAsync(ctx->readVel, ctx->vel[V], headBytes, cudaMemcpyDeviceToHost, ctx->copyStream));
         PBF_CUDA(ctx, cudaEventRecord(ctx->evCopyDone, ctx->copyStream));
-        pbf::launch_apply_vorticity(c, ctx->pred[a], omega, ctx->vel[V ^ 1], ctx->vel[V], list, meta, flat,
+        pbf::launch_apply_vorticity(c, ctx->pred[a], omega, ctx->vel[V ^ 1], ctx->vel[V], meta, rows,
                                     ls.vorticity, ls.balance, nullptr, s, half, vortTiles - half);
         PBF_CUDA(ctx, cudaMemcpyAsync(reinterpret_cast<char*>(ctx->readVel) + headBytes,
                                       reinterpret_cast<const char*>(ctx->vel[V]) + headBytes, v4 - headBytes,
@@ -605,7 +603,7 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
         velCopied = true;
         ++launched;
     } else {
-        pbf::launch_apply_vorticity(c, ctx->pred[a], omega, ctx->vel[V ^ 1], ctx->vel[V], list, meta, flat,
+        pbf::launch_apply_vorticity(c, ctx->pred[a], omega, ctx->vel[V ^ 1], ctx->vel[V], meta, rows,
                                     ls.vorticity, ls.balance, tiles(4), s);
     }
     launched += 3;
@@ -740,7 +738,7 @@ int ensure_tape(pbf_ctx* ctx) {
     for (pbf::AdjointTape& t : ctx->tapes) {
         t.iterations = iters;
         t.perm = (uint32_t*)take(4 * (size_t)n);
-        t.list = (uint32_t*)take(4 * (size_t)ctx->listSlots * n);
+        t.rows = (uint4*)take(16 * pbf::row_entries(ctx->listSlots) * n);
         t.meta = (uint2*)take(8 * (size_t)n);
         for (int it = 0; it < iters; ++it) t.q[it] = (float4*)take(v4);
         t.mask = clamp ? (uint8_t*)take((size_t)iters * n) : nullptr;
@@ -913,7 +911,7 @@ int pbf_destroy(pbf_ctx* ctx) {
         dev_free(ctx->keys[k]); dev_free(ctx->perm[k]);
     }
     dev_free(ctx->omega); dev_free(ctx->density); dev_free(ctx->hist); dev_free(ctx->cells);
-    dev_free(ctx->list); dev_free(ctx->flat); dev_free(ctx->meta); dev_free(ctx->errWord); dev_free(ctx->tileCounters);
+    dev_free(ctx->list); dev_free(ctx->rows); dev_free(ctx->meta); dev_free(ctx->errWord); dev_free(ctx->tileCounters);
     dev_free(ctx->taint); dev_free(ctx->cellXYZ); dev_free(ctx->cellStart);
     dev_free(ctx->scenes); dev_free(ctx->sceneOf); dev_free(ctx->ids); dev_free(ctx->idsTmp);
     dev_free(ctx->quadsDev); dev_free(ctx->maskDev); dev_free(ctx->waveDev);
@@ -1010,7 +1008,7 @@ int pbf_init_cells(pbf_ctx* ctx) {
     ctx->cellsN = ctx->n;
     ++ctx->epoch;
     if ((rc = dev_alloc(ctx, &ctx->list, (size_t)ctx->listSlots * ctx->n)) ||
-        (rc = dev_alloc(ctx, &ctx->flat, (size_t)ctx->listSlots * ctx->n)) || (rc = dev_alloc(ctx, &ctx->meta, ctx->n)) ||
+        (rc = dev_alloc(ctx, &ctx->rows, pbf::row_entries(ctx->listSlots) * ctx->n)) || (rc = dev_alloc(ctx, &ctx->meta, ctx->n)) ||
         (rc = dev_alloc(ctx, &ctx->taint, ctx->n)) || (rc = dev_alloc(ctx, &ctx->cellXYZ, ctx->n)) ||
         (rc = dev_alloc(ctx, &ctx->cellStart, tableWords)))
         return rc;
@@ -1537,11 +1535,11 @@ int pbf_read_friends(pbf_ctx* ctx, uint32_t* counts, uint32_t* list, int list_sl
     const int n = ctx->n;
     std::vector<uint2> meta(n);
     PBF_CUDA(ctx, cudaMemcpyAsync(meta.data(), ctx->meta, 8 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
-    // the kept friends of every particle in order: the flat rows the passes walk
+    // the kept friends of every particle in order: the rows the passes walk
     const int slots = list ? std::min(list_slots, ctx->listSlots) : 0;
-    std::vector<uint32_t> rows((size_t)std::max(slots, 0) * n);
+    std::vector<uint4> rows(pbf::row_entries(std::max(slots, 0)) * n);
     if (slots > 0)
-        PBF_CUDA(ctx, cudaMemcpyAsync(rows.data(), ctx->flat, 4 * rows.size(), cudaMemcpyDeviceToHost, ctx->stream));
+        PBF_CUDA(ctx, cudaMemcpyAsync(rows.data(), ctx->rows, 16 * rows.size(), cudaMemcpyDeviceToHost, ctx->stream));
     PBF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     for (int i = 0; i < n; ++i) {
         const uint64_t m = (uint64_t)meta[i].x | ((uint64_t)meta[i].y << 32);
@@ -1552,7 +1550,7 @@ int pbf_read_friends(pbf_ctx* ctx, uint32_t* counts, uint32_t* list, int list_sl
             nl += cnt;
             if (k < keptD) nd += cnt;
         }
-        for (int t = 0; t < slots && t < (int)nl; ++t) list[(size_t)t * n + i] = rows[(size_t)t * n + i];
+        for (int t = 0; t < slots && t < (int)nl; ++t) list[(size_t)t * n + i] = (&rows[(size_t)(t / 4) * n + i].x)[t % 4];
         if (counts) { counts[2 * i] = nl; counts[2 * i + 1] = nd; }
     }
     return PBF_OK;

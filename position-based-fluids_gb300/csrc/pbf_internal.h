@@ -58,6 +58,7 @@ struct DevConsts {
                                  // (NULL in relaxed mode: nothing is tainted)
     const uint32_t* cellStart;   // per cell key: its first particle, when the substep's keys confirm it
     const uint32_t* keys;        // the substep's sorted cell keys (set per substep)
+    unsigned long long negZero2; // two floats -0 (product2 in pbf_device.cuh)
     int circles, perCircle;
     uint32_t grid;
     int n;
@@ -120,35 +121,36 @@ void launch_reset_cells(int n, const uint32_t* keys, uint32_t* cells, uint32_t k
 // per tile of particles): the solver passes' persistent grid, whose
 // blocks take the tiles from it (LaunchShape::persistent).
 // algorithm: LaunchShape::friendsAlgorithm.  Every build writes the circle
-// rows into `list`; none writes the flat rows (the first density pass
-// records them), so the return value, whether `flat` was written, is false.
-bool launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const uint32_t* cells, uint32_t* list,
-                          uint32_t* flat, uint2* meta, int* errorWord, int block, int algorithm, cudaStream_t s);
-// The flat rows from the circle rows, when no density pass records them.
-void launch_flatten_friends(const DevConsts& c, const uint32_t* list, const uint2* meta, uint32_t* flat, cudaStream_t s);
-// flatIn / flatOut (may be NULL): the friends recorded in order as flat rows
-// flat[t * N + i] by the first density pass of a substep (flatOut) and read
-// from there by the passes after it (flatIn) instead of the circle rows.
+// rows into `list`; the first density pass records the rows from them.
+void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const uint32_t* cells, uint32_t* list,
+                          uint2* meta, int* errorWord, int block, int algorithm, cudaStream_t s);
+// uint4 words per particle of the rows (walk_pairs in pbf_device.cuh) for
+// `slots` friends.
+inline size_t row_entries(int slots) { return ((size_t)slots + 3) / 4; }
+// The rows from the circle rows, when no density pass records them.
+void launch_flatten_friends(const DevConsts& c, const uint32_t* list, const uint2* meta, uint4* rows, cudaStream_t s);
+// rowsOut (may be NULL): the rows recorded by the first density pass of a
+// substep; rowsIn: the rows, walked by the passes after it.
 void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* predPacked, float* density,
-                            const uint32_t* list, const uint2* meta, const uint32_t* flatIn, uint32_t* flatOut,
+                            const uint32_t* list, const uint2* meta, const uint4* rowsIn, uint4* rowsOut,
                             int block, int balance, int* tileCounter, cudaStream_t s);
 // posPrev: the sorted positions, read only by the force planes.
 void launch_compute_delta(const DevConsts& c, Batch b, const float4* predPacked, const float4* posPrev,
-                          float4* predOut, const float* density, const uint32_t* list, const uint2* meta,
-                          int lastIteration, uint8_t* clampMask, const uint32_t* flatIn, int block, int balance,
-                          int* tileCounter, cudaStream_t s);
+                          float4* predOut, const float* density, const uint2* meta, int lastIteration,
+                          uint8_t* clampMask, const uint4* rows, int block, int balance, int* tileCounter,
+                          cudaStream_t s);
 void launch_update_velocities(const DevConsts& c, const float4* pred, const float4* posIn, float4* posOut,
                               float4* vel, const uint32_t* idsIn, uint32_t* idsOut, cudaStream_t s);
 void launch_apply_viscosity(const DevConsts& c, Batch b, const float4* pred, const float4* velIn, float4* velOut,
-                            float4* omega, const uint32_t* list, const uint2* meta, const uint32_t* flatIn, int block,
-                            int balance, int* tileCounter, cudaStream_t s);
+                            float4* omega, const uint2* meta, const uint4* rows, int block, int balance,
+                            int* tileCounter, cudaStream_t s);
 // tileCount > 0: only the particle tiles [firstTile, firstTile + tileCount)
 // of `block` particles, one block per tile (a frame's read-back splits the
 // last vorticity pass so that the first part's velocities copy out while the
 // rest runs).
 void launch_apply_vorticity(const DevConsts& c, const float4* pred, const float4* omega, const float4* velIn,
-                            float4* velOut, const uint32_t* list, const uint2* meta, const uint32_t* flatIn, int block,
-                            int balance, int* tileCounter, cudaStream_t s, int firstTile = 0, int tileCount = 0);
+                            float4* velOut, const uint2* meta, const uint4* rows, int block, int balance,
+                            int* tileCounter, cudaStream_t s, int firstTile = 0, int tileCount = 0);
 
 // ---- radix sort (pbf_sort.cu) ----
 struct SortPlan {
@@ -174,7 +176,7 @@ int radix_sort_launches(const SortPlan& plan);
 struct AdjointTape {
     int iterations = 0;
     uint32_t* perm = nullptr;      // sorted index k came from perm[k]
-    uint32_t* list = nullptr;      // the substep's kept friends as flat rows (friend t of i at t * N + i)
+    uint4* rows = nullptr;         // the substep's kept friends in order, four per entry (walk_pairs)
     uint2* meta = nullptr;
     float4* q[64] = {};            // (p^t, lambda^t), t < iterations
     uint8_t* mask = nullptr;       // iterations x N box-clamp decisions (NULL: no clamp)

@@ -19,8 +19,8 @@
 //                           reference's friends layout, build_friends_list.cl:
 //                           1-21); a warp of consecutive particles reads one
 //                           row coalesced.
-//   flat                  : uint32[circles * perCircle][N]: particle i's
-//                           friends in summation order, the t-th in row t;
+//   rows                  : uint4[ceil(circles * perCircle / 4)][N]: particle
+//                           i's friends in summation order, four per entry;
 //                           recorded by the first density pass of a substep
 //                           and walked by the passes after it.
 //   meta                  : uint2[N] per particle: 7-bit friend count of each
@@ -607,68 +607,99 @@ __device__ __forceinline__ void for_tiles(int tiles, int* counter, F body) {
 // root w = 1/|r| replaces sqrt(r^2) and the divisions by |r|, and sums are
 // fused multiply-adds: the reference's kernels as its own
 // -cl-fast-relaxed-math -cl-mad-enable build may evaluate them.
-// Spiky gradient magnitude over |r|: (h - |r|)^2 / |r| with |r| = r^2 w.
-__device__ __forceinline__ float spiky_over_r(const DevConsts& c, float r2, float& w) {
-    w = rsqrtf(r2);
-    const float hr = fmaf(-r2, w, c.h);
-    return hr * hr * w;
+// Spiky gradient magnitude over |r|: (h - |r|)^2 / |r| with |r| = r^2 w.  The
+// scalar operations of each friend are those named here, packed for two.
+__device__ __forceinline__ F2 spiky_over_r2(const DevConsts& c, F2 r2, F2& w) {
+    const float2 r = unpack2(r2);
+    w = pack2(rsqrtf(r.x), rsqrtf(r.y));
+    const F2 hr = fma2(neg2(r2), w, both(c.h));
+    return mul2(mul2(hr, hr), w);
 }
 
 // compute_scaling.cl:27-112 followed by pack_data.cl (w = lambda).  Q: the
-// exact quotients by |r| through one reciprocal (quotient_rn).
-template <bool R, bool B, int W, bool Q>
+// exact quotients by |r| through one reciprocal (quotient_rn).  Rec: the
+// friends come from the circle rows, and the rows are recorded.
+template <bool R, bool Rec, bool Q>
 __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const float4* __restrict__ pred,
                                                      float4* __restrict__ predPacked, float* __restrict__ density,
-                                                     const uint32_t* __restrict__ list, const uint2* __restrict__ meta,
-                                                     const uint32_t* __restrict__ flatIn, uint32_t* __restrict__ flatOut,
-                                                     int i, const float4 pi, uint64_t mt) {
+                                                     const uint32_t* __restrict__ list, const uint4* __restrict__ rowsIn,
+                                                     uint4* __restrict__ rowsOut, int i, const float4 pi, uint64_t mt) {
     const int n = c.n;
     // complete neighbour sets count the particle itself first: d = h^2 - 0
     float ds = c.complete ? c.h2 * c.h2 * c.h2 : 0.0f, gsk = 0.0f, gx = 0.0f, gy = 0.0f, gz = 0.0f;
-    constexpr int U = 4;  // friends in flight: the passes wait on their neighbour gathers (long scoreboard)
-    gather_walk<W, U, true>(list, flatIn, flatOut, n, i, FriendRows(mt, kept_density(mt), c.perCircle),
-                      [&](uint32_t j) { return __ldg(pred + checked_index(j, (uint32_t)n, c.err, kErrFriendIndex)); }, [&](const float4 pj) {
-        const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
+    auto load = [&](uint32_t j) { return __ldg(pred + checked_index(j, (uint32_t)n, c.err, kErrFriendIndex)); };
+    auto one = [&](float rx, float ry, float rz, float r2) {  // a friend in support, divided the IEEE way
+        const float rl = sqrtf(r2);
+        const float hr = c.h - rl;
+        const float sc = c.gradSpiky * hr * hr;
+        const float g0 = (sc * rx) / rl, g1 = (sc * ry) / rl, g2 = (sc * rz) / rl;
+        const float d = c.h2 - r2;
+        ds = ds + d * d * d;
+        gsk = gsk + dot3(g0, g1, g2, g0, g1, g2);
+        gx = gx + g0;
+        gy = gy + g1;
+        gz = gz + g2;
+    };
+    auto pair = [&](const float4& pa, const float4& pb, bool va, bool vb) {
+        const F2 rx = pack2(pi.x - pa.x, pi.x - pb.x), ry = pack2(pi.y - pa.y, pi.y - pb.y),
+                 rz = pack2(pi.z - pa.z, pi.z - pb.z);
+        const F2 r2 = R ? fma2(rz, rz, fma2(ry, ry, mul2(rx, rx))) : dot2(c, rx, ry, rz, rx, ry, rz);
+        const float2 s2 = unpack2(r2);
+        va = va && in_support(c, s2.x);
+        vb = vb && in_support(c, s2.y);
+        if (!R && !Q) {
+            const float2 x = unpack2(rx), y = unpack2(ry), z = unpack2(rz);
+            if (va) one(x.x, y.x, z.x, s2.x);
+            if (vb) one(x.y, y.y, z.y, s2.y);
+            return;
+        }
+        F2 g0, g1, g2;
         if (R) {
-            const float r2 = fmaf(rz, rz, fmaf(ry, ry, rx * rx));
-            if (in_support(c, r2)) {
-                float w;
-                const float s = c.gradSpiky * spiky_over_r(c, r2, w);
-                const float g0 = s * rx, g1 = s * ry, g2 = s * rz;
-                const float d = c.h2 - r2;
-                ds = fmaf(d * d, d, ds);
-                gsk = fmaf(g2, g2, fmaf(g1, g1, fmaf(g0, g0, gsk)));
-                gx += g0;
-                gy += g1;
-                gz += g2;
+            F2 w;
+            const F2 s = mul2(both(c.gradSpiky), spiky_over_r2(c, r2, w));
+            g0 = mul2(s, rx);
+            g1 = mul2(s, ry);
+            g2 = mul2(s, rz);
+        } else {
+            F2 nrl, y;
+            sqrt_recip_rn2(r2, nrl, y);
+            const F2 hr = add2(both(c.h), nrl);
+            const F2 sc = mul2(mul2(both(c.gradSpiky), hr), hr);
+            g0 = quotient_rn2(mul2(sc, rx), nrl, y);
+            g1 = quotient_rn2(mul2(sc, ry), nrl, y);
+            g2 = quotient_rn2(mul2(sc, rz), nrl, y);
+        }
+        const F2 d = sub2(both(c.h2), r2);
+        const float2 x = unpack2(g0), y = unpack2(g1), z = unpack2(g2);
+        if (R) {
+            const float2 dd = unpack2(mul2(d, d)), d1 = unpack2(d);
+            if (va) {
+                ds = fmaf(dd.x, d1.x, ds);
+                gsk = fmaf(z.x, z.x, fmaf(y.x, y.x, fmaf(x.x, x.x, gsk)));
+                gx += x.x; gy += y.x; gz += z.x;
+            }
+            if (vb) {
+                ds = fmaf(dd.y, d1.y, ds);
+                gsk = fmaf(z.y, z.y, fmaf(y.y, y.y, fmaf(x.y, x.y, gsk)));
+                gx += x.y; gy += y.y; gz += z.y;
             }
         } else {
-            const float r2 = dot3(rx, ry, rz, rx, ry, rz);
-            if (in_support(c, r2)) {
-                float rl, y;
-                if (Q) sqrt_recip_rn(r2, rl, y);
-                else rl = sqrtf(r2);
-                const float hr = c.h - rl;
-                const float sc = c.gradSpiky * hr * hr;
-                float g0, g1, g2;
-                if (Q) {
-                    g0 = quotient_rn(sc * rx, rl, y);
-                    g1 = quotient_rn(sc * ry, rl, y);
-                    g2 = quotient_rn(sc * rz, rl, y);
-                } else {
-                    g0 = (sc * rx) / rl;
-                    g1 = (sc * ry) / rl;
-                    g2 = (sc * rz) / rl;
-                }
-                const float d = c.h2 - r2;
-                ds = ds + d * d * d;
-                gsk = gsk + dot3(g0, g1, g2, g0, g1, g2);
-                gx = gx + g0;
-                gy = gy + g1;
-                gz = gz + g2;
+            const float2 d3 = unpack2(mul2(mul2(d, d), d)), gg = unpack2(dot2(c, g0, g1, g2, g0, g1, g2));
+            if (va) {
+                ds = ds + d3.x;
+                gsk = gsk + gg.x;
+                gx = gx + x.x; gy = gy + y.x; gz = gz + z.x;
+            }
+            if (vb) {
+                ds = ds + d3.y;
+                gsk = gsk + gg.y;
+                gx = gx + x.y; gy = gy + y.y; gz = gz + z.y;
             }
         }
-    });
+    };
+    const FriendRows fr(mt, kept_density(mt), c.perCircle);
+    if (Rec) walk_pairs_recording(list, rowsOut, n, i, fr, load, pair);
+    else walk_pairs(rowsIn, n, i, fr.total, load, pair);
     ds = ds * c.poly6;
     density[i] = ds;
     gsk = gsk + dot3(gx, gy, gz, gx, gy, gz);
@@ -677,22 +708,20 @@ __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const f
     predPacked[i] = make_float4(pi.x, pi.y, pi.z, lambda);
 }
 
-// The exact recording pass is held to 40 registers (three 512-thread blocks
-// per SM): 11 % faster than its natural 60, spills and all.
-template <bool R, bool B, int W>
-__global__ void __launch_bounds__(kMaxBlock, (!R && W == kWalkRecord) ? 3 : 0)
+template <bool R, bool B, bool Rec>
+__global__ void __launch_bounds__(kMaxBlock)
 compute_scaling_kernel(DevConsts c, const float4* __restrict__ pred, float4* __restrict__ predPacked,
                        float* __restrict__ density, const uint32_t* __restrict__ list,
-                       const uint2* __restrict__ meta, const uint32_t* __restrict__ flatIn,
-                       uint32_t* __restrict__ flatOut, int tiles, int* tileCounter) {
+                       const uint2* __restrict__ meta, const uint4* __restrict__ rowsIn,
+                       uint4* __restrict__ rowsOut, int tiles, int* tileCounter) {
     for_tiles(tiles, tileCounter, [&](int tile) {
         const int i = B ? balanced_particle(meta, c.n, true, tile) : tile * (int)blockDim.x + (int)threadIdx.x;
         if (i < 0 || i >= c.n) return;
         const float4 pi = pred[i];
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) compute_scaling_body<R, B, W, true>(c, pred, predPacked, density, list, meta, flatIn, flatOut, i, pi, mt);
-        else compute_scaling_body<R, B, W, false>(c, pred, predPacked, density, list, meta, flatIn, flatOut, i, pi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) compute_scaling_body<R, Rec, true>(c, pred, predPacked, density, list, rowsIn, rowsOut, i, pi, mt);
+        else compute_scaling_body<R, Rec, false>(c, pred, predPacked, density, list, rowsIn, rowsOut, i, pi, mt);
     });
 }
 
@@ -701,58 +730,70 @@ compute_scaling_kernel(DevConsts c, const float4* __restrict__ pred, float4* __r
 // the optional box clamp on `future`, then update_predicted.cl.  After the
 // last iteration w carries the density (pack_data.cl with the density source,
 // src/Simulation.cpp:591).
-template <bool R, bool B, int W, bool Q>
+template <bool R, bool Q>
 __device__ __forceinline__ void compute_delta_body(const DevConsts& c, const Batch& b, const float4* __restrict__ pp,
                                                    const float4* __restrict__ posPrev, float4* __restrict__ predOut,
-                                                   const float* __restrict__ density, const uint32_t* __restrict__ list,
-                                                   const uint2* __restrict__ meta, int lastIteration,
-                                                   uint8_t* __restrict__ clampMask, const uint32_t* __restrict__ flatIn,
+                                                   const float* __restrict__ density, int lastIteration,
+                                                   uint8_t* __restrict__ clampMask, const uint4* __restrict__ rows,
                                                    int i, const float4 pi, uint64_t mt) {
     const int n = c.n;
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-    constexpr int U = 4;  // friends in flight: the passes wait on their neighbour gathers (long scoreboard)
-    gather_walk<W, U, true>(list, flatIn, nullptr, n, i, FriendRows(mt, kept_other(mt), c.perCircle),
-                      [&](uint32_t j) { return __ldg(pp + checked_index(j, (uint32_t)n, c.err, kErrFriendIndex)); }, [&](const float4 pj) {
-        const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
+    auto load = [&](uint32_t j) { return __ldg(pp + checked_index(j, (uint32_t)n, c.err, kErrFriendIndex)); };
+    auto one = [&](float rx, float ry, float rz, float r2, float wj) {  // a friend in support, divided the IEEE way
+        const float rl = sqrtf(r2);
+        const float hr = c.h - rl;
+        const float g0 = (rx / rl) * hr * hr, g1 = (ry / rl) * hr * hr, g2 = (rz / rl) * hr * hr;
+        const float d = c.h2 - r2;
+        const float p6 = d * d * d;
+        const float rq = p6 / c.poly6q;
+        const float scorr = c.K * rq * rq * rq * rq;
+        const float a = pi.w + wj + scorr;
+        sx = sx + a * g0;
+        sy = sy + a * g1;
+        sz = sz + a * g2;
+    };
+    walk_pairs(rows, n, i, FlatFriends(mt, kept_other(mt)).total, load, [&](const float4& pa, const float4& pb, bool va, bool vb) {
+        const F2 rx = pack2(pi.x - pa.x, pi.x - pb.x), ry = pack2(pi.y - pa.y, pi.y - pb.y),
+                 rz = pack2(pi.z - pa.z, pi.z - pb.z);
+        const F2 r2 = R ? fma2(rz, rz, fma2(ry, ry, mul2(rx, rx))) : dot2(c, rx, ry, rz, rx, ry, rz);
+        const float2 s2 = unpack2(r2);
+        va = va && in_support(c, s2.x);
+        vb = vb && in_support(c, s2.y);
+        if (!R && !Q) {
+            const float2 x = unpack2(rx), y = unpack2(ry), z = unpack2(rz);
+            if (va) one(x.x, y.x, z.x, s2.x, pa.w);
+            if (vb) one(x.y, y.y, z.y, s2.y, pb.w);
+            return;
+        }
+        const F2 d = sub2(both(c.h2), r2);
+        const F2 p6 = mul2(mul2(d, d), d);
+        const F2 wij = pack2(pi.w + pa.w, pi.w + pb.w);
         if (R) {
-            const float r2 = fmaf(rz, rz, fmaf(ry, ry, rx * rx));
-            if (in_support(c, r2)) {
-                float w;
-                const float k = spiky_over_r(c, r2, w);
-                const float d = c.h2 - r2;
-                const float rq = d * d * d * c.invPoly6q;
-                const float rq2 = rq * rq;
-                const float a = fmaf(c.K * rq2, rq2, pi.w + pj.w) * k;
-                sx = fmaf(a, rx, sx);
-                sy = fmaf(a, ry, sy);
-                sz = fmaf(a, rz, sz);
-            }
+            F2 w;
+            const F2 k = spiky_over_r2(c, r2, w);
+            const F2 rq = mul2(p6, both(c.invPoly6q));
+            const F2 rq2 = mul2(rq, rq);
+            const float2 a = unpack2(mul2(fma2(mul2(both(c.K), rq2), rq2, wij), k));
+            const float2 x = unpack2(rx), y = unpack2(ry), z = unpack2(rz);
+            if (va) { sx = fmaf(a.x, x.x, sx); sy = fmaf(a.x, y.x, sy); sz = fmaf(a.x, z.x, sz); }
+            if (vb) { sx = fmaf(a.y, x.y, sx); sy = fmaf(a.y, y.y, sy); sz = fmaf(a.y, z.y, sz); }
         } else {
-            const float r2 = dot3(rx, ry, rz, rx, ry, rz);
-            if (in_support(c, r2)) {
-                float rl, y;
-                if (Q) sqrt_recip_rn(r2, rl, y);
-                else rl = sqrtf(r2);
-                const float hr = c.h - rl;
-                float g0, g1, g2;
-                if (Q) {
-                    g0 = quotient_rn(rx, rl, y) * hr * hr;
-                    g1 = quotient_rn(ry, rl, y) * hr * hr;
-                    g2 = quotient_rn(rz, rl, y) * hr * hr;
-                } else {
-                    g0 = (rx / rl) * hr * hr;
-                    g1 = (ry / rl) * hr * hr;
-                    g2 = (rz / rl) * hr * hr;
-                }
-                const float d = c.h2 - r2;
-                const float p6 = d * d * d;
-                const float rq = c.quotientPoly6q ? quotient_rn(p6, c.poly6q, c.recipPoly6q) : p6 / c.poly6q;
-                const float scorr = c.K * rq * rq * rq * rq;
-                const float a = pi.w + pj.w + scorr;
-                sx = sx + a * g0;
-                sy = sy + a * g1;
-                sz = sz + a * g2;
+            F2 nrl, y;
+            sqrt_recip_rn2(r2, nrl, y);
+            const F2 hr = add2(both(c.h), nrl);
+            const F2 g0 = mul2(mul2(quotient_rn2(rx, nrl, y), hr), hr), g1 = mul2(mul2(quotient_rn2(ry, nrl, y), hr), hr),
+                     g2 = mul2(mul2(quotient_rn2(rz, nrl, y), hr), hr);
+            F2 rq;
+            if (c.quotientPoly6q) {
+                rq = quotient_rn2(p6, both(-c.poly6q), both(c.recipPoly6q));
+            } else {
+                const float2 p = unpack2(p6);
+                rq = pack2(p.x / c.poly6q, p.y / c.poly6q);
             }
+            const F2 a = add2(wij, product2(c, mul2(mul2(mul2(both(c.K), rq), rq), rq), rq));
+            const float2 x = unpack2(mul2(a, g0)), v = unpack2(mul2(a, g1)), z = unpack2(mul2(a, g2));
+            if (va) { sx = sx + x.x; sy = sy + v.x; sz = sz + z.x; }
+            if (vb) { sx = sx + x.y; sy = sy + v.y; sz = sz + z.y; }
         }
     });
     float fx, fy, fz;
@@ -795,21 +836,20 @@ __device__ __forceinline__ void compute_delta_body(const DevConsts& c, const Bat
     if (!R) note_position(c, i, out.x, out.y, out.z);
 }
 
-// The exact position pass is held to 40 registers (from 46): 1.3 % faster.
-template <bool R, bool B, int W>
-__global__ void __launch_bounds__(kMaxBlock, R ? 0 : 3)
+template <bool R, bool B>
+__global__ void __launch_bounds__(kMaxBlock)
 compute_delta_kernel(DevConsts c, Batch b, const float4* __restrict__ pp, const float4* __restrict__ posPrev,
-                     float4* __restrict__ predOut, const float* __restrict__ density, const uint32_t* __restrict__ list,
+                     float4* __restrict__ predOut, const float* __restrict__ density,
                      const uint2* __restrict__ meta, int lastIteration, uint8_t* __restrict__ clampMask,
-                     const uint32_t* __restrict__ flatIn, int tiles, int* tileCounter) {
+                     const uint4* __restrict__ rows, int tiles, int* tileCounter) {
     for_tiles(tiles, tileCounter, [&](int tile) {
         const int i = B ? balanced_particle(meta, c.n, false, tile) : tile * (int)blockDim.x + (int)threadIdx.x;
         if (i < 0 || i >= c.n) return;
         const float4 pi = pp[i];
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) compute_delta_body<R, B, W, true>(c, b, pp, posPrev, predOut, density, list, meta, lastIteration, clampMask, flatIn, i, pi, mt);
-        else compute_delta_body<R, B, W, false>(c, b, pp, posPrev, predOut, density, list, meta, lastIteration, clampMask, flatIn, i, pi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) compute_delta_body<R, true>(c, b, pp, posPrev, predOut, density, lastIteration, clampMask, rows, i, pi, mt);
+        else compute_delta_body<R, false>(c, b, pp, posPrev, predOut, density, lastIteration, clampMask, rows, i, pi, mt);
     });
 }
 
@@ -836,57 +876,71 @@ __global__ void update_velocities_kernel(DevConsts c, const float4* __restrict__
 // velocities (Jacobi).  omega.w receives |omega| (sqrt of its dot product, as
 // apply_vorticity.cl:55 forms it for each neighbour), so that the vorticity
 // pass reads it instead of recomputing it per pair.
-template <bool R, bool B, int W, bool Q>
+template <bool R, bool Q>
 __device__ __forceinline__ void apply_viscosity_body(const DevConsts& c, const Batch& b, const float4* __restrict__ pred,
                                                      const float4* __restrict__ velIn, float4* __restrict__ velOut,
-                                                     float4* __restrict__ omega, const uint32_t* __restrict__ list,
-                                                     const uint2* __restrict__ meta, const uint32_t* __restrict__ flatIn,
-                                                     int i, const float4 pi, const float4 vi, uint64_t mt) {
+                                                     float4* __restrict__ omega, const uint4* __restrict__ rows, int i,
+                                                     const float4 pi, const float4 vi, uint64_t mt) {
     const int n = c.n;
     float vsx = 0.0f, vsy = 0.0f, vsz = 0.0f, ox = 0.0f, oy = 0.0f, oz = 0.0f;
-    constexpr int U = 4;  // friends in flight: the passes wait on their neighbour gathers (long scoreboard)
-    gather_walk<W, U>(list, flatIn, nullptr, n, i, FriendRows(mt, kept_other(mt), c.perCircle),
-                      [&](uint32_t j) { j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex); return PairRec{__ldg(pred + j), __ldg(velIn + j)}; }, [&](const PairRec& q) {
-        const float4 pj = q.a;
-        const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
-        const float r2 = rx * rx + ry * ry + rz * rz;
-        if (in_support(c, r2) && fabsf(pj.w) > 1e-8f) {
-            const float4 vj = q.b;
-            const float ux = vj.x - vi.x, uy = vj.y - vi.y, uz = vj.z - vi.z;
-            const float d = c.h2 - r2;
-            if (R) {
-                float w;
-                const float k = spiky_over_r(c, r2, w);
-                const float g0 = k * rx, g1 = k * ry, g2 = k * rz;
-                ox += fmaf(uy, g2, -uz * g1);
-                oy += fmaf(uz, g0, -ux * g2);
-                oz += fmaf(ux, g1, -uy * g0);
-                const float d3 = d * d * d;
-                vsx = fmaf(ux, d3, vsx);
-                vsy = fmaf(uy, d3, vsy);
-                vsz = fmaf(uz, d3, vsz);
-            } else {
-                float rl, y;
-                if (Q) sqrt_recip_rn(r2, rl, y);
-                else rl = sqrtf(r2);
-                const float hr = c.h - rl;
-                float g0, g1, g2;
-                if (Q) {
-                    g0 = quotient_rn(rx, rl, y) * hr * hr;
-                    g1 = quotient_rn(ry, rl, y) * hr * hr;
-                    g2 = quotient_rn(rz, rl, y) * hr * hr;
-                } else {
-                    g0 = (rx / rl) * hr * hr;
-                    g1 = (ry / rl) * hr * hr;
-                    g2 = (rz / rl) * hr * hr;
-                }
-                ox = ox + (uy * g2 - uz * g1);
-                oy = oy + (uz * g0 - ux * g2);
-                oz = oz + (ux * g1 - uy * g0);
-                const float d3 = d * d * d;
-                vsx = vsx + ux * d3;
-                vsy = vsy + uy * d3;
-                vsz = vsz + uz * d3;
+    auto load = [&](uint32_t j) { j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex); return PairRec{__ldg(pred + j), __ldg(velIn + j)}; };
+    walk_pairs(rows, n, i, FlatFriends(mt, kept_other(mt)).total, load, [&](const PairRec& qa, const PairRec& qb, bool va, bool vb) {
+        const float4 pa = qa.a, pb = qb.a;
+        const F2 rx = pack2(pi.x - pa.x, pi.x - pb.x), ry = pack2(pi.y - pa.y, pi.y - pb.y),
+                 rz = pack2(pi.z - pa.z, pi.z - pb.z);
+        const F2 r2 = dot2(c, rx, ry, rz, rx, ry, rz);
+        const float2 s2 = unpack2(r2);
+        va = va && in_support(c, s2.x) && fabsf(pa.w) > 1e-8f;
+        vb = vb && in_support(c, s2.y) && fabsf(pb.w) > 1e-8f;
+        const F2 ux = pack2(qa.b.x - vi.x, qb.b.x - vi.x), uy = pack2(qa.b.y - vi.y, qb.b.y - vi.y),
+                 uz = pack2(qa.b.z - vi.z, qb.b.z - vi.z);
+        F2 g0, g1, g2;
+        if (R) {
+            F2 w;
+            const F2 k = spiky_over_r2(c, r2, w);
+            g0 = mul2(k, rx);
+            g1 = mul2(k, ry);
+            g2 = mul2(k, rz);
+        } else if (Q) {
+            F2 nrl, y;
+            sqrt_recip_rn2(r2, nrl, y);
+            const F2 hr = add2(both(c.h), nrl);
+            g0 = mul2(mul2(quotient_rn2(rx, nrl, y), hr), hr);
+            g1 = mul2(mul2(quotient_rn2(ry, nrl, y), hr), hr);
+            g2 = mul2(mul2(quotient_rn2(rz, nrl, y), hr), hr);
+        } else {
+            const float la = sqrtf(s2.x), lb = sqrtf(s2.y);
+            const F2 hr = pack2(c.h - la, c.h - lb);
+            const float2 x = unpack2(rx), y = unpack2(ry), z = unpack2(rz);
+            g0 = mul2(mul2(pack2(x.x / la, x.y / lb), hr), hr);
+            g1 = mul2(mul2(pack2(y.x / la, y.y / lb), hr), hr);
+            g2 = mul2(mul2(pack2(z.x / la, z.y / lb), hr), hr);
+        }
+        const F2 d = sub2(both(c.h2), r2);
+        const F2 d3 = mul2(mul2(d, d), d);
+        if (R) {
+            const float2 x = unpack2(fma2(uy, g2, neg2(mul2(uz, g1)))), y = unpack2(fma2(uz, g0, neg2(mul2(ux, g2)))),
+                         z = unpack2(fma2(ux, g1, neg2(mul2(uy, g0)))), t = unpack2(d3), a0 = unpack2(ux),
+                         a1 = unpack2(uy), a2 = unpack2(uz);
+            if (va) {
+                ox += x.x; oy += y.x; oz += z.x;
+                vsx = fmaf(a0.x, t.x, vsx); vsy = fmaf(a1.x, t.x, vsy); vsz = fmaf(a2.x, t.x, vsz);
+            }
+            if (vb) {
+                ox += x.y; oy += y.y; oz += z.y;
+                vsx = fmaf(a0.y, t.y, vsx); vsy = fmaf(a1.y, t.y, vsy); vsz = fmaf(a2.y, t.y, vsz);
+            }
+        } else {
+            const float2 p0 = unpack2(mul2(uy, g2)), p1 = unpack2(mul2(uz, g0)), p2 = unpack2(mul2(ux, g1)),
+                         q0 = unpack2(mul2(uz, g1)), q1 = unpack2(mul2(ux, g2)), q2 = unpack2(mul2(uy, g0)),
+                         a0 = unpack2(mul2(ux, d3)), a1 = unpack2(mul2(uy, d3)), a2 = unpack2(mul2(uz, d3));
+            if (va) {
+                ox = ox + (p0.x - q0.x); oy = oy + (p1.x - q1.x); oz = oz + (p2.x - q2.x);
+                vsx = vsx + a0.x; vsy = vsy + a1.x; vsz = vsz + a2.x;
+            }
+            if (vb) {
+                ox = ox + (p0.y - q0.y); oy = oy + (p1.y - q1.y); oz = oz + (p2.y - q2.y);
+                vsx = vsx + a0.y; vsy = vsy + a1.y; vsz = vsz + a2.y;
             }
         }
     });
@@ -899,68 +953,73 @@ __device__ __forceinline__ void apply_viscosity_body(const DevConsts& c, const B
     omega[i] = make_float4(wx, wy, wz, sqrtf(dot3(wx, wy, wz, wx, wy, wz)));
 }
 
-template <bool R, bool B, int W>
+template <bool R, bool B>
 __global__ void __launch_bounds__(kMaxBlock)
 apply_viscosity_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, const float4* __restrict__ velIn,
-                       float4* __restrict__ velOut, float4* __restrict__ omega,
-                       const uint32_t* __restrict__ list, const uint2* __restrict__ meta,
-                       const uint32_t* __restrict__ flatIn, int tiles, int* tileCounter) {
+                       float4* __restrict__ velOut, float4* __restrict__ omega, const uint2* __restrict__ meta,
+                       const uint4* __restrict__ rows, int tiles, int* tileCounter) {
     for_tiles(tiles, tileCounter, [&](int tile) {
         const int i = B ? balanced_particle(meta, c.n, false, tile) : tile * (int)blockDim.x + (int)threadIdx.x;
         if (i < 0 || i >= c.n) return;
         const float4 pi = pred[i], vi = velIn[i];
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) apply_viscosity_body<R, B, W, true>(c, b, pred, velIn, velOut, omega, list, meta, flatIn, i, pi, vi, mt);
-        else apply_viscosity_body<R, B, W, false>(c, b, pred, velIn, velOut, omega, list, meta, flatIn, i, pi, vi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) apply_viscosity_body<R, true>(c, b, pred, velIn, velOut, omega, rows, i, pi, vi, mt);
+        else apply_viscosity_body<R, false>(c, b, pred, velIn, velOut, omega, rows, i, pi, vi, mt);
     });
 }
 
 // apply_vorticity.cl:12-86; |omega_j| is read from omega.w (apply_viscosity).
-template <bool R, bool B, int W, bool Q>
+template <bool R, bool Q>
 __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const float4* __restrict__ pred,
                                                      const float4* __restrict__ omega, const float4* __restrict__ velIn,
-                                                     float4* __restrict__ velOut, const uint32_t* __restrict__ list,
-                                                     const uint2* __restrict__ meta, const uint32_t* __restrict__ flatIn,
-                                                     int i, const float4 pi, uint64_t mt) {
+                                                     float4* __restrict__ velOut, const uint4* __restrict__ rows, int i,
+                                                     const float4 pi, uint64_t mt) {
     const int n = c.n;
     float ex = 0.0f, ey = 0.0f, ez = 0.0f;
-    constexpr int U = 4;  // friends in flight: the passes wait on their neighbour gathers (long scoreboard)
-    gather_walk<W, U>(list, flatIn, nullptr, n, i, FriendRows(mt, kept_other(mt), c.perCircle),
-                      [&](uint32_t j) { j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex); return PairRec{__ldg(pred + j), __ldg(omega + j)}; }, [&](const PairRec& q) {
-        const float4 pj = q.a;
-        const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
-        const float r2 = rx * rx + ry * ry + rz * rz;
-        if (in_support(c, r2) && fabsf(pj.w) > 1e-8f) {
-            const float4 oj = q.b;
-            if (R) {
-                float w;
-                const float k = spiky_over_r(c, r2, w);
+    auto load = [&](uint32_t j) { j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex); return PairRec{__ldg(pred + j), __ldg(omega + j)}; };
+    walk_pairs(rows, n, i, FlatFriends(mt, kept_other(mt)).total, load, [&](const PairRec& qa, const PairRec& qb, bool va, bool vb) {
+        const float4 pa = qa.a, pb = qb.a;
+        const F2 rx = pack2(pi.x - pa.x, pi.x - pb.x), ry = pack2(pi.y - pa.y, pi.y - pb.y),
+                 rz = pack2(pi.z - pa.z, pi.z - pb.z);
+        const F2 r2 = dot2(c, rx, ry, rz, rx, ry, rz);
+        const float2 s2 = unpack2(r2);
+        va = va && in_support(c, s2.x) && fabsf(pa.w) > 1e-8f;
+        vb = vb && in_support(c, s2.y) && fabsf(pb.w) > 1e-8f;
+        if (R) {
+            F2 w;
+            const float2 k = unpack2(spiky_over_r2(c, r2, w)), x = unpack2(rx), y = unpack2(ry), z = unpack2(rz);
+            auto add = [&](const float4& oj, float kj, float x1, float y1, float z1) {
                 const float o2 = fmaf(oj.z, oj.z, fmaf(oj.y, oj.y, oj.x * oj.x));
-                const float s = o2 > 0.0f ? o2 * rsqrtf(o2) * k : 0.0f;
-                ex = fmaf(s, rx, ex);
-                ey = fmaf(s, ry, ey);
-                ez = fmaf(s, rz, ez);
+                const float s = o2 > 0.0f ? o2 * rsqrtf(o2) * kj : 0.0f;
+                ex = fmaf(s, x1, ex);
+                ey = fmaf(s, y1, ey);
+                ez = fmaf(s, z1, ez);
+            };
+            if (va) add(qa.b, k.x, x.x, y.x, z.x);
+            if (vb) add(qb.b, k.y, x.y, y.y, z.y);
+        } else {
+            F2 g0, g1, g2;
+            if (Q) {
+                F2 nrl, y;
+                sqrt_recip_rn2(r2, nrl, y);
+                const F2 hr = add2(both(c.h), nrl);
+                g0 = mul2(mul2(quotient_rn2(rx, nrl, y), hr), hr);
+                g1 = mul2(mul2(quotient_rn2(ry, nrl, y), hr), hr);
+                g2 = mul2(mul2(quotient_rn2(rz, nrl, y), hr), hr);
             } else {
-                float rl, y;
-                if (Q) sqrt_recip_rn(r2, rl, y);
-                else rl = sqrtf(r2);
-                const float hr = c.h - rl;
-                float g0, g1, g2;
-                if (Q) {
-                    g0 = quotient_rn(rx, rl, y) * hr * hr;
-                    g1 = quotient_rn(ry, rl, y) * hr * hr;
-                    g2 = quotient_rn(rz, rl, y) * hr * hr;
-                } else {
-                    g0 = (rx / rl) * hr * hr;
-                    g1 = (ry / rl) * hr * hr;
-                    g2 = (rz / rl) * hr * hr;
-                }
-                const float ol = oj.w;  // sqrt(dot(omega_j, omega_j)), formed once by apply_viscosity
-                ex = ex + ol * g0;
-                ey = ey + ol * g1;
-                ez = ez + ol * g2;
+                const float la = sqrtf(s2.x), lb = sqrtf(s2.y);
+                const F2 hr = pack2(c.h - la, c.h - lb);
+                const float2 x = unpack2(rx), y = unpack2(ry), z = unpack2(rz);
+                g0 = mul2(mul2(pack2(x.x / la, x.y / lb), hr), hr);
+                g1 = mul2(mul2(pack2(y.x / la, y.y / lb), hr), hr);
+                g2 = mul2(mul2(pack2(z.x / la, z.y / lb), hr), hr);
             }
+            // |omega_j| is sqrt(dot(omega_j, omega_j)), formed once by apply_viscosity
+            const F2 ol = pack2(qa.b.w, qb.b.w);
+            const float2 x = unpack2(mul2(ol, g0)), y = unpack2(mul2(ol, g1)), z = unpack2(mul2(ol, g2));
+            if (va) { ex = ex + x.x; ey = ey + y.x; ez = ez + z.x; }
+            if (vb) { ex = ex + x.y; ey = ey + y.y; ez = ez + z.y; }
         }
     });
     ex = ex * c.negGradSpiky;
@@ -990,12 +1049,11 @@ __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const f
     velOut[i] = make_float4(v.x + fx * c.dt, v.y + fy * c.dt, v.z + fz * c.dt, v.w + 0.0f);
 }
 
-template <bool R, bool B, int W>
+template <bool R, bool B>
 __global__ void __launch_bounds__(kMaxBlock)
 apply_vorticity_kernel(DevConsts c, const float4* __restrict__ pred, const float4* __restrict__ omega,
-                       const float4* __restrict__ velIn, float4* __restrict__ velOut,
-                       const uint32_t* __restrict__ list, const uint2* __restrict__ meta,
-                       const uint32_t* __restrict__ flatIn, int tiles, int* tileCounter, int tileOffset) {
+                       const float4* __restrict__ velIn, float4* __restrict__ velOut, const uint2* __restrict__ meta,
+                       const uint4* __restrict__ rows, int tiles, int* tileCounter, int tileOffset) {
     for_tiles(tiles, tileCounter, [&](int tile) {
         tile += tileOffset;  // a launch over part of the tiles (one block per tile)
         const int i = B ? balanced_particle(meta, c.n, false, tile) : tile * (int)blockDim.x + (int)threadIdx.x;
@@ -1003,8 +1061,8 @@ apply_vorticity_kernel(DevConsts c, const float4* __restrict__ pred, const float
         const float4 pi = pred[i];
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) apply_vorticity_body<R, B, W, true>(c, pred, omega, velIn, velOut, list, meta, flatIn, i, pi, mt);
-        else apply_vorticity_body<R, B, W, false>(c, pred, omega, velIn, velOut, list, meta, flatIn, i, pi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) apply_vorticity_body<R, true>(c, pred, omega, velIn, velOut, rows, i, pi, mt);
+        else apply_vorticity_body<R, false>(c, pred, omega, velIn, velOut, rows, i, pi, mt);
     });
 }
 
@@ -1062,8 +1120,8 @@ unsigned grid_for_tiles(K kernel, int n, int block, bool persistent, int* tiles)
     return cap;
 }
 
-bool launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const uint32_t* cells, uint32_t* list,
-                          uint32_t* flat, uint2* meta, int* errorWord, int block, int algorithm, cudaStream_t s) {
+void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const uint32_t* cells, uint32_t* list,
+                          uint2* meta, int* errorWord, int block, int algorithm, cudaStream_t s) {
     const bool pow2 = (c.grid & (c.grid - 1)) == 0;
     const uint32_t keys = c.grid * (uint32_t)(b.scenes ? b.nscenes : 1);
     const uint2* cellPairs = reinterpret_cast<const uint2*>(cells);
@@ -1072,62 +1130,61 @@ bool launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const
     if (algorithm == 2 && pow2 && c.grid >= 64) {  // one block per 4x4x4-cell brick over all scenes
         auto kb = narrow ? build_friends_brick_kernel<4, true> : build_friends_brick_kernel<4, false>;
         kb<<<keys / 64u, BrickShape<4>::threads, 0, s>>>(c, pred, cellPairs, list, meta, errorWord);
-        return false;
+        return;
     }
     if (algorithm == 1) {
         build_friends_warp_kernel<<<blocks_for(c.n, block), block, 0, s>>>(c, b, pred, cellPairs, list, meta, errorWord);
-        return false;
+        return;
     }
     // one block per tile: the tile loop of a persistent grid costs this kernel
     // spilled registers in its candidate loop, and the grid gains nothing
     auto k = narrow ? build_friends_kernel<2, true> : build_friends_kernel<2, false>;
     k<<<blocks_for(c.n, block), block, 0, s>>>(c, b, pred, cellPairs, list, meta, errorWord);
-    return false;
 }
 
 namespace {
-// The kept circles' friends as flat rows, in order, from the circle rows,
-// when no density pass records them (zero solver iterations).
+// The kept circles' friends as rows, in order, from the circle rows, when no
+// density pass records them (zero solver iterations).
 __global__ void flatten_friends_kernel(int n, int perCircle, const uint32_t* __restrict__ list,
-                                       const uint2* __restrict__ meta, uint32_t* __restrict__ flat) {
+                                       const uint2* __restrict__ meta, uint4* __restrict__ rows) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint64_t mt = load_meta(meta, i);
-    FriendRows fr(mt, kept_density(mt), perCircle);
-    for (int t = 0; t < fr.total; ++t) flat[(size_t)t * n + i] = list[(size_t)fr.row(t) * n + i];
+    walk_pairs_recording(list, rows, n, i, FriendRows(mt, kept_density(mt), perCircle), [](uint32_t) { return 0; },
+                         [](int, int, bool, bool) {});
 }
 }  // namespace
 
-void launch_flatten_friends(const DevConsts& c, const uint32_t* list, const uint2* meta, uint32_t* flat, cudaStream_t s) {
-    flatten_friends_kernel<<<blocks_for(c.n), kBlock, 0, s>>>(c.n, c.perCircle, list, meta, flat);
+void launch_flatten_friends(const DevConsts& c, const uint32_t* list, const uint2* meta, uint4* rows, cudaStream_t s) {
+    flatten_friends_kernel<<<blocks_for(c.n), kBlock, 0, s>>>(c.n, c.perCircle, list, meta, rows);
 }
 
-// The first density pass of a substep records the flat rows from the circle
-// rows (flatOut); the other passes walk the flat rows (flatIn).
+// The first density pass of a substep records the rows from the circle rows
+// (rowsOut); the other passes walk them (rowsIn).
 void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* predPacked, float* density,
-                            const uint32_t* list, const uint2* meta, const uint32_t* flatIn, uint32_t* flatOut,
+                            const uint32_t* list, const uint2* meta, const uint4* rowsIn, uint4* rowsOut,
                             int block, int balance, int* tileCounter, cudaStream_t s) {
-    const bool record = flatOut != nullptr;
-    auto pick = [record](auto rec, auto flat) { return record ? rec : flat; };
-    auto k = c.relaxed ? (balance ? pick(compute_scaling_kernel<true, true, kWalkRecord>, compute_scaling_kernel<true, true, kWalkFlat>)
-                                  : pick(compute_scaling_kernel<true, false, kWalkRecord>, compute_scaling_kernel<true, false, kWalkFlat>))
-                       : (balance ? pick(compute_scaling_kernel<false, true, kWalkRecord>, compute_scaling_kernel<false, true, kWalkFlat>)
-                                  : pick(compute_scaling_kernel<false, false, kWalkRecord>, compute_scaling_kernel<false, false, kWalkFlat>));
+    const bool record = rowsOut != nullptr;
+    auto pick = [record](auto rec, auto walk) { return record ? rec : walk; };
+    auto k = c.relaxed ? (balance ? pick(compute_scaling_kernel<true, true, true>, compute_scaling_kernel<true, true, false>)
+                                  : pick(compute_scaling_kernel<true, false, true>, compute_scaling_kernel<true, false, false>))
+                       : (balance ? pick(compute_scaling_kernel<false, true, true>, compute_scaling_kernel<false, true, false>)
+                                  : pick(compute_scaling_kernel<false, false, true>, compute_scaling_kernel<false, false, false>));
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
-    k<<<grid, block, 0, s>>>(c, pred, predPacked, density, list, meta, flatIn, flatOut, tiles, tileCounter);
+    k<<<grid, block, 0, s>>>(c, pred, predPacked, density, list, meta, rowsIn, rowsOut, tiles, tileCounter);
 }
 
 void launch_compute_delta(const DevConsts& c, Batch b, const float4* predPacked, const float4* posPrev,
-                          float4* predOut, const float* density, const uint32_t* list, const uint2* meta,
-                          int lastIteration, uint8_t* clampMask, const uint32_t* flatIn, int block, int balance,
-                          int* tileCounter, cudaStream_t s) {
-    auto k = c.relaxed ? (balance ? compute_delta_kernel<true, true, kWalkFlat> : compute_delta_kernel<true, false, kWalkFlat>)
-                       : (balance ? compute_delta_kernel<false, true, kWalkFlat> : compute_delta_kernel<false, false, kWalkFlat>);
+                          float4* predOut, const float* density, const uint2* meta, int lastIteration,
+                          uint8_t* clampMask, const uint4* rows, int block, int balance, int* tileCounter,
+                          cudaStream_t s) {
+    auto k = c.relaxed ? (balance ? compute_delta_kernel<true, true> : compute_delta_kernel<true, false>)
+                       : (balance ? compute_delta_kernel<false, true> : compute_delta_kernel<false, false>);
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
-    k<<<grid, block, 0, s>>>(c, b, predPacked, posPrev, predOut, density, list, meta, lastIteration, clampMask, flatIn,
-                             tiles, tileCounter);
+    k<<<grid, block, 0, s>>>(c, b, predPacked, posPrev, predOut, density, meta, lastIteration, clampMask, rows, tiles,
+                             tileCounter);
 }
 
 void launch_update_velocities(const DevConsts& c, const float4* pred, const float4* posIn, float4* posOut,
@@ -1136,27 +1193,27 @@ void launch_update_velocities(const DevConsts& c, const float4* pred, const floa
 }
 
 void launch_apply_viscosity(const DevConsts& c, Batch b, const float4* pred, const float4* velIn, float4* velOut,
-                            float4* omega, const uint32_t* list, const uint2* meta, const uint32_t* flatIn, int block,
-                            int balance, int* tileCounter, cudaStream_t s) {
-    auto k = c.relaxed ? (balance ? apply_viscosity_kernel<true, true, kWalkFlat> : apply_viscosity_kernel<true, false, kWalkFlat>)
-                       : (balance ? apply_viscosity_kernel<false, true, kWalkFlat> : apply_viscosity_kernel<false, false, kWalkFlat>);
+                            float4* omega, const uint2* meta, const uint4* rows, int block, int balance,
+                            int* tileCounter, cudaStream_t s) {
+    auto k = c.relaxed ? (balance ? apply_viscosity_kernel<true, true> : apply_viscosity_kernel<true, false>)
+                       : (balance ? apply_viscosity_kernel<false, true> : apply_viscosity_kernel<false, false>);
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
-    k<<<grid, block, 0, s>>>(c, b, pred, velIn, velOut, omega, list, meta, flatIn, tiles, tileCounter);
+    k<<<grid, block, 0, s>>>(c, b, pred, velIn, velOut, omega, meta, rows, tiles, tileCounter);
 }
 
 void launch_apply_vorticity(const DevConsts& c, const float4* pred, const float4* omega, const float4* velIn,
-                            float4* velOut, const uint32_t* list, const uint2* meta, const uint32_t* flatIn, int block,
-                            int balance, int* tileCounter, cudaStream_t s, int firstTile, int tileCount) {
-    auto k = c.relaxed ? (balance ? apply_vorticity_kernel<true, true, kWalkFlat> : apply_vorticity_kernel<true, false, kWalkFlat>)
-                       : (balance ? apply_vorticity_kernel<false, true, kWalkFlat> : apply_vorticity_kernel<false, false, kWalkFlat>);
+                            float4* velOut, const uint2* meta, const uint4* rows, int block, int balance,
+                            int* tileCounter, cudaStream_t s, int firstTile, int tileCount) {
+    auto k = c.relaxed ? (balance ? apply_vorticity_kernel<true, true> : apply_vorticity_kernel<true, false>)
+                       : (balance ? apply_vorticity_kernel<false, true> : apply_vorticity_kernel<false, false>);
     if (tileCount > 0) {  // tiles [firstTile, firstTile + tileCount), one block each
-        k<<<(unsigned)tileCount, block, 0, s>>>(c, pred, omega, velIn, velOut, list, meta, flatIn, 0, nullptr, firstTile);
+        k<<<(unsigned)tileCount, block, 0, s>>>(c, pred, omega, velIn, velOut, meta, rows, 0, nullptr, firstTile);
         return;
     }
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
-    k<<<grid, block, 0, s>>>(c, pred, omega, velIn, velOut, list, meta, flatIn, tiles, tileCounter, 0);
+    k<<<grid, block, 0, s>>>(c, pred, omega, velIn, velOut, meta, rows, tiles, tileCounter, 0);
 }
 
 }  // namespace pbf
