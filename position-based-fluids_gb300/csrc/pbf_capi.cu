@@ -10,8 +10,8 @@
 //   friends      pred[1] cells            -> list, counts; cells reset
 //   iterations   pred[1] -> pred[0] (lambda packed in w) -> pred[1]
 //   velocities   pred[1] pos[P^1]         -> pos[P], vel[V]
-//   viscosity    pred[1] vel[V]           -> vel[V^1], omega
-//   vorticity    vel[V^1] omega           -> vel[V]
+//   viscosity    pred[1] vel[V]           -> vel[V^1], omega, pred[0] (neighbour records)
+//   vorticity    vel[V^1] omega pred[0]   -> vel[V]
 // so an unpaused substep starts and ends with the same roles and one
 // captured CUDA graph replays every substep.
 
@@ -581,7 +581,8 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
     }
     if (tape) PBF_CUDA(ctx, cudaMemcpyAsync(tape->v2, ctx->vel[V], v4, cudaMemcpyDeviceToDevice, s));
     mark("applyViscosity");
-    pbf::launch_apply_viscosity(c, b, ctx->pred[a], ctx->vel[V], ctx->vel[V ^ 1], omega, meta, rows, ls.viscosity,
+    float4* near = ctx->pred[a ^ 1];  // free: the iterations are done, and the next substep writes its predictions there
+    pbf::launch_apply_viscosity(c, b, ctx->pred[a], ctx->vel[V], ctx->vel[V ^ 1], omega, near, meta, rows, ls.viscosity,
                                 ls.balance, tiles(3), s);
     mark("applyVorticity");
     const int vortTiles = (c.n + ls.vorticity - 1) / ls.vorticity;
@@ -589,13 +590,13 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
         // the first half of the particles' velocities copy out while the second half runs
         const int half = vortTiles / 2;
         const size_t headBytes = 16 * (size_t)half * (size_t)ls.vorticity;
-        pbf::launch_apply_vorticity(c, ctx->pred[a], omega, ctx->vel[V ^ 1], ctx->vel[V], meta, rows,
+        pbf::launch_apply_vorticity(c, ctx->pred[a], near, omega, ctx->vel[V ^ 1], ctx->vel[V], meta, rows,
                                     ls.vorticity, ls.balance, nullptr, s, 0, half);
         PBF_CUDA(ctx, cudaEventRecord(ctx->evVelHead, s));
         PBF_CUDA(ctx, cudaStreamWaitEvent(ctx->copyStream, ctx->evVelHead, 0));
         PBF_CUDA(ctx, cudaMemcpyAsync(ctx->readVel, ctx->vel[V], headBytes, cudaMemcpyDeviceToHost, ctx->copyStream));
         PBF_CUDA(ctx, cudaEventRecord(ctx->evCopyDone, ctx->copyStream));
-        pbf::launch_apply_vorticity(c, ctx->pred[a], omega, ctx->vel[V ^ 1], ctx->vel[V], meta, rows,
+        pbf::launch_apply_vorticity(c, ctx->pred[a], near, omega, ctx->vel[V ^ 1], ctx->vel[V], meta, rows,
                                     ls.vorticity, ls.balance, nullptr, s, half, vortTiles - half);
         PBF_CUDA(ctx, cudaMemcpyAsync(reinterpret_cast<char*>(ctx->readVel) + headBytes,
                                       reinterpret_cast<const char*>(ctx->vel[V]) + headBytes, v4 - headBytes,
@@ -603,7 +604,7 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
         velCopied = true;
         ++launched;
     } else {
-        pbf::launch_apply_vorticity(c, ctx->pred[a], omega, ctx->vel[V ^ 1], ctx->vel[V], meta, rows,
+        pbf::launch_apply_vorticity(c, ctx->pred[a], near, omega, ctx->vel[V ^ 1], ctx->vel[V], meta, rows,
                                     ls.vorticity, ls.balance, tiles(4), s);
     }
     launched += 3;

@@ -141,15 +141,16 @@ void launch_compute_delta(const DevConsts& c, Batch b, const float4* predPacked,
                           cudaStream_t s);
 void launch_update_velocities(const DevConsts& c, const float4* pred, const float4* posIn, float4* posOut,
                               float4* vel, const uint32_t* idsIn, uint32_t* idsOut, cudaStream_t s);
+// near: the neighbour records that launch_apply_vorticity reads.
 void launch_apply_viscosity(const DevConsts& c, Batch b, const float4* pred, const float4* velIn, float4* velOut,
-                            float4* omega, const uint2* meta, const uint4* rows, int block, int balance,
+                            float4* omega, float4* near, const uint2* meta, const uint4* rows, int block, int balance,
                             int* tileCounter, cudaStream_t s);
 // tileCount > 0: only the particle tiles [firstTile, firstTile + tileCount)
 // of `block` particles, one block per tile (a frame's read-back splits the
 // last vorticity pass so that the first part's velocities copy out while the
 // rest runs).
-void launch_apply_vorticity(const DevConsts& c, const float4* pred, const float4* omega, const float4* velIn,
-                            float4* velOut, const uint2* meta, const uint4* rows, int block, int balance,
+void launch_apply_vorticity(const DevConsts& c, const float4* pred, const float4* near, const float4* omega,
+                            const float4* velIn, float4* velOut, const uint2* meta, const uint4* rows, int block, int balance,
                             int* tileCounter, cudaStream_t s, int firstTile = 0, int tileCount = 0);
 
 // ---- radix sort (pbf_sort.cu) ----

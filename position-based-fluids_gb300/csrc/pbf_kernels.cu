@@ -873,18 +873,23 @@ __global__ void update_velocities_kernel(DevConsts c, const float4* __restrict__
 }
 
 // apply_viscosity.cl:12-86, every neighbour read from the pre-pass
-// velocities (Jacobi).  omega.w receives |omega| (sqrt of its dot product, as
-// apply_vorticity.cl:55 forms it for each neighbour), so that the vorticity
-// pass reads it instead of recomputing it per pair.
+// velocities (Jacobi).  near receives the one record that the vorticity pass
+// reads of a neighbour: its position and |omega| (as apply_vorticity.cl:55
+// forms it for each neighbour), with x = infinity, which is out of every
+// support, where the neighbour's density is too small to count
+// (apply_vorticity.cl:44).  The vorticity pass was bound by the L1 wavefronts
+// of its two gathers per friend (79 %); with one it takes 0.191 ms instead of
+// 0.214 (1M particles, mid-collapse, two substeps).
 template <bool R, bool Q>
 __device__ __forceinline__ void apply_viscosity_body(const DevConsts& c, const Batch& b, const float4* __restrict__ pred,
                                                      const float4* __restrict__ velIn, float4* __restrict__ velOut,
-                                                     float4* __restrict__ omega, const uint4* __restrict__ rows, int i,
-                                                     const float4 pi, const float4 vi, uint64_t mt) {
+                                                     float4* __restrict__ omega, float4* __restrict__ near,
+                                                     const uint4* __restrict__ rows, int i, const float4 pi,
+                                                     const float4 vi, uint64_t mt) {
     const int n = c.n;
     float vsx = 0.0f, vsy = 0.0f, vsz = 0.0f, ox = 0.0f, oy = 0.0f, oz = 0.0f;
     auto load = [&](uint32_t j) { j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex); return PairRec{__ldg(pred + j), __ldg(velIn + j)}; };
-    walk_pairs(rows, n, i, FlatFriends(mt, kept_other(mt)).total, load, [&](const PairRec& qa, const PairRec& qb, bool va, bool vb) {
+    walk_pairs<true>(rows, n, i, FlatFriends(mt, kept_other(mt)).total, load, [&](const PairRec& qa, const PairRec& qb, bool va, bool vb) {
         const float4 pa = qa.a, pb = qb.a;
         const F2 rx = pack2(pi.x - pa.x, pi.x - pb.x), ry = pack2(pi.y - pa.y, pi.y - pb.y),
                  rz = pack2(pi.z - pa.z, pi.z - pb.z);
@@ -950,54 +955,60 @@ __device__ __forceinline__ void apply_viscosity_body(const DevConsts& c, const B
     const float visc = b.scenes ? b.scenes[b.sceneOf[i]].visc : c.visc;
     velOut[i] = make_float4(vi.x + visc * vsx, vi.y + visc * vsy, vi.z + visc * vsz, vi.w + visc * 0.0f);
     const float wx = ox * c.negGradSpiky, wy = oy * c.negGradSpiky, wz = oz * c.negGradSpiky;
-    omega[i] = make_float4(wx, wy, wz, sqrtf(dot3(wx, wy, wz, wx, wy, wz)));
+    float size;
+    if (R) {
+        const float o2 = fmaf(wz, wz, fmaf(wy, wy, wx * wx));
+        size = o2 > 0.0f ? o2 * rsqrtf(o2) : 0.0f;
+    } else {
+        size = sqrtf(dot3(wx, wy, wz, wx, wy, wz));
+    }
+    omega[i] = make_float4(wx, wy, wz, size);
+    near[i] = make_float4(fabsf(pi.w) > 1e-8f ? pi.x : __int_as_float(0x7F800000), pi.y, pi.z, size);
 }
 
 template <bool R, bool B>
 __global__ void __launch_bounds__(kMaxBlock)
 apply_viscosity_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, const float4* __restrict__ velIn,
-                       float4* __restrict__ velOut, float4* __restrict__ omega, const uint2* __restrict__ meta,
-                       const uint4* __restrict__ rows, int tiles, int* tileCounter) {
+                       float4* __restrict__ velOut, float4* __restrict__ omega, float4* __restrict__ near,
+                       const uint2* __restrict__ meta, const uint4* __restrict__ rows, int tiles, int* tileCounter) {
     for_tiles(tiles, tileCounter, [&](int tile) {
         const int i = B ? balanced_particle(meta, c.n, false, tile) : tile * (int)blockDim.x + (int)threadIdx.x;
         if (i < 0 || i >= c.n) return;
         const float4 pi = pred[i], vi = velIn[i];
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) apply_viscosity_body<R, true>(c, b, pred, velIn, velOut, omega, rows, i, pi, vi, mt);
-        else apply_viscosity_body<R, false>(c, b, pred, velIn, velOut, omega, rows, i, pi, vi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) apply_viscosity_body<R, true>(c, b, pred, velIn, velOut, omega, near, rows, i, pi, vi, mt);
+        else apply_viscosity_body<R, false>(c, b, pred, velIn, velOut, omega, near, rows, i, pi, vi, mt);
     });
 }
 
-// apply_vorticity.cl:12-86; |omega_j| is read from omega.w (apply_viscosity).
+// apply_vorticity.cl:12-86; neighbours are read from near (apply_viscosity).
 template <bool R, bool Q>
-__device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const float4* __restrict__ pred,
-                                                     const float4* __restrict__ omega, const float4* __restrict__ velIn,
-                                                     float4* __restrict__ velOut, const uint4* __restrict__ rows, int i,
-                                                     const float4 pi, uint64_t mt) {
+__device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const float4* __restrict__ near,
+                                                     const float4* __restrict__ omega,
+                                                     const float4* __restrict__ velIn, float4* __restrict__ velOut,
+                                                     const uint4* __restrict__ rows, int i, const float4 pi, uint64_t mt) {
     const int n = c.n;
     float ex = 0.0f, ey = 0.0f, ez = 0.0f;
-    auto load = [&](uint32_t j) { j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex); return PairRec{__ldg(pred + j), __ldg(omega + j)}; };
-    walk_pairs(rows, n, i, FlatFriends(mt, kept_other(mt)).total, load, [&](const PairRec& qa, const PairRec& qb, bool va, bool vb) {
-        const float4 pa = qa.a, pb = qb.a;
+    auto load = [&](uint32_t j) { return __ldg(near + checked_index(j, (uint32_t)n, c.err, kErrFriendIndex)); };
+    walk_pairs(rows, n, i, FlatFriends(mt, kept_other(mt)).total, load, [&](const float4& pa, const float4& pb, bool va, bool vb) {
         const F2 rx = pack2(pi.x - pa.x, pi.x - pb.x), ry = pack2(pi.y - pa.y, pi.y - pb.y),
                  rz = pack2(pi.z - pa.z, pi.z - pb.z);
         const F2 r2 = dot2(c, rx, ry, rz, rx, ry, rz);
         const float2 s2 = unpack2(r2);
-        va = va && in_support(c, s2.x) && fabsf(pa.w) > 1e-8f;
-        vb = vb && in_support(c, s2.y) && fabsf(pb.w) > 1e-8f;
+        va = va && in_support(c, s2.x);
+        vb = vb && in_support(c, s2.y);
         if (R) {
             F2 w;
             const float2 k = unpack2(spiky_over_r2(c, r2, w)), x = unpack2(rx), y = unpack2(ry), z = unpack2(rz);
-            auto add = [&](const float4& oj, float kj, float x1, float y1, float z1) {
-                const float o2 = fmaf(oj.z, oj.z, fmaf(oj.y, oj.y, oj.x * oj.x));
-                const float s = o2 > 0.0f ? o2 * rsqrtf(o2) * kj : 0.0f;
+            auto add = [&](float ol, float kj, float x1, float y1, float z1) {
+                const float s = ol > 0.0f ? ol * kj : 0.0f;
                 ex = fmaf(s, x1, ex);
                 ey = fmaf(s, y1, ey);
                 ez = fmaf(s, z1, ez);
             };
-            if (va) add(qa.b, k.x, x.x, y.x, z.x);
-            if (vb) add(qb.b, k.y, x.y, y.y, z.y);
+            if (va) add(pa.w, k.x, x.x, y.x, z.x);
+            if (vb) add(pb.w, k.y, x.y, y.y, z.y);
         } else {
             F2 g0, g1, g2;
             if (Q) {
@@ -1015,8 +1026,7 @@ __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const f
                 g1 = mul2(mul2(pack2(y.x / la, y.y / lb), hr), hr);
                 g2 = mul2(mul2(pack2(z.x / la, z.y / lb), hr), hr);
             }
-            // |omega_j| is sqrt(dot(omega_j, omega_j)), formed once by apply_viscosity
-            const F2 ol = pack2(qa.b.w, qb.b.w);
+            const F2 ol = pack2(pa.w, pb.w);
             const float2 x = unpack2(mul2(ol, g0)), y = unpack2(mul2(ol, g1)), z = unpack2(mul2(ol, g2));
             if (va) { ex = ex + x.x; ey = ey + y.x; ez = ez + z.x; }
             if (vb) { ex = ex + x.y; ey = ey + y.y; ez = ez + z.y; }
@@ -1051,8 +1061,8 @@ __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const f
 
 template <bool R, bool B>
 __global__ void __launch_bounds__(kMaxBlock)
-apply_vorticity_kernel(DevConsts c, const float4* __restrict__ pred, const float4* __restrict__ omega,
-                       const float4* __restrict__ velIn, float4* __restrict__ velOut, const uint2* __restrict__ meta,
+apply_vorticity_kernel(DevConsts c, const float4* __restrict__ pred, const float4* __restrict__ near,
+                       const float4* __restrict__ omega, const float4* __restrict__ velIn, float4* __restrict__ velOut, const uint2* __restrict__ meta,
                        const uint4* __restrict__ rows, int tiles, int* tileCounter, int tileOffset) {
     for_tiles(tiles, tileCounter, [&](int tile) {
         tile += tileOffset;  // a launch over part of the tiles (one block per tile)
@@ -1061,8 +1071,8 @@ apply_vorticity_kernel(DevConsts c, const float4* __restrict__ pred, const float
         const float4 pi = pred[i];
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) apply_vorticity_body<R, true>(c, pred, omega, velIn, velOut, rows, i, pi, mt);
-        else apply_vorticity_body<R, false>(c, pred, omega, velIn, velOut, rows, i, pi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) apply_vorticity_body<R, true>(c, near, omega, velIn, velOut, rows, i, pi, mt);
+        else apply_vorticity_body<R, false>(c, near, omega, velIn, velOut, rows, i, pi, mt);
     });
 }
 
@@ -1193,27 +1203,27 @@ void launch_update_velocities(const DevConsts& c, const float4* pred, const floa
 }
 
 void launch_apply_viscosity(const DevConsts& c, Batch b, const float4* pred, const float4* velIn, float4* velOut,
-                            float4* omega, const uint2* meta, const uint4* rows, int block, int balance,
+                            float4* omega, float4* near, const uint2* meta, const uint4* rows, int block, int balance,
                             int* tileCounter, cudaStream_t s) {
     auto k = c.relaxed ? (balance ? apply_viscosity_kernel<true, true> : apply_viscosity_kernel<true, false>)
                        : (balance ? apply_viscosity_kernel<false, true> : apply_viscosity_kernel<false, false>);
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
-    k<<<grid, block, 0, s>>>(c, b, pred, velIn, velOut, omega, meta, rows, tiles, tileCounter);
+    k<<<grid, block, 0, s>>>(c, b, pred, velIn, velOut, omega, near, meta, rows, tiles, tileCounter);
 }
 
-void launch_apply_vorticity(const DevConsts& c, const float4* pred, const float4* omega, const float4* velIn,
-                            float4* velOut, const uint2* meta, const uint4* rows, int block, int balance,
+void launch_apply_vorticity(const DevConsts& c, const float4* pred, const float4* near, const float4* omega,
+                            const float4* velIn, float4* velOut, const uint2* meta, const uint4* rows, int block, int balance,
                             int* tileCounter, cudaStream_t s, int firstTile, int tileCount) {
     auto k = c.relaxed ? (balance ? apply_vorticity_kernel<true, true> : apply_vorticity_kernel<true, false>)
                        : (balance ? apply_vorticity_kernel<false, true> : apply_vorticity_kernel<false, false>);
     if (tileCount > 0) {  // tiles [firstTile, firstTile + tileCount), one block each
-        k<<<(unsigned)tileCount, block, 0, s>>>(c, pred, omega, velIn, velOut, meta, rows, 0, nullptr, firstTile);
+        k<<<(unsigned)tileCount, block, 0, s>>>(c, pred, near, omega, velIn, velOut, meta, rows, 0, nullptr, firstTile);
         return;
     }
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
-    k<<<grid, block, 0, s>>>(c, pred, omega, velIn, velOut, meta, rows, tiles, tileCounter, 0);
+    k<<<grid, block, 0, s>>>(c, pred, near, omega, velIn, velOut, meta, rows, tiles, tileCounter, 0);
 }
 
 }  // namespace pbf
