@@ -417,10 +417,9 @@ int pbf_render_read(pbf_ctx* ctx, int which, float* rgba);
 /* The launch shape, PBF_LAUNCH_SHAPE_FIELDS ints: threads per block of the
    five neighbour kernels in the order friends, density (scaling), delta,
    viscosity, vorticity (multiples of 32 in [32, 512]), then the friends
-   algorithm (0: one thread scans the 27 cells per particle; 1: a warp scans
-   the cells of each run of same-cell particles together; 2: a block stages
-   the 6x6x6-cell halo of a 4x4x4-cell brick in shared memory and its threads
-   scan from there, for power-of-two GridBufferSize >= 64, else 0), then the balance
+   algorithm (0, and 2 as well: warps test the candidates of each run of
+   same-cell particles together, in blocks of 128 threads whatever the friends
+   block size; 1: one thread scans the 27 cells per particle), then the balance
    flag (1: the four solver passes hand each block's particles to its threads
    in decreasing order of friend count, so warps walk lists of similar
    length), then the persistent flag (1: the four solver passes launch at
@@ -432,7 +431,7 @@ int pbf_get_launch_shape(pbf_ctx* ctx, int* blocks);
 int pbf_set_launch_shape(pbf_ctx* ctx, const int* blocks);
 
 /* Time `trial_substeps` substeps from the current state for each candidate
-   block size (64, 128, 256, 512), the three friends algorithms and both balance
+   block size (64, 128, 256, 512), friends algorithms 0 and 1 and both balance
    settings, keep the fastest per kernel (the balance setting by the sum of
    the solver passes), then time that shape with and without persistent
    grids and keep the faster, restore the state (positions, velocities, particle ids

@@ -7,7 +7,7 @@
 //   sort         keys/perm ping-pong      -> keys[k], perm[k]
 //   gather       pos[P] pred[0]           -> pos[P^1], pred[1]   (sortParticles)
 //   cells        keys[k]                  -> cells
-//   friends      pred[1] cells            -> list, counts; cells reset
+//   friends      pred[1] cells            -> rows, meta; cells reset
 //   iterations   pred[1] -> pred[0] (lambda packed in w) -> pred[1]
 //   velocities   pred[1] pos[P^1]         -> pos[P], vel[V]
 //   viscosity    pred[1] vel[V]           -> vel[V^1], omega, pred[0] (neighbour records)
@@ -48,7 +48,6 @@ struct pbf_ctx {
     uint32_t* perm[2] = {nullptr, nullptr};
     uint32_t* hist = nullptr;
     uint32_t* cells = nullptr;
-    uint32_t* list = nullptr;
     uint4* rows = nullptr;       // the friends of the substep in order, four per entry (see enqueue_substep)
     uint2* meta = nullptr;       // per-particle friend counts per circle + kept circles
     uint32_t* taint = nullptr;          // per particle: the substep that tainted it (pbf::DevConsts::taint)
@@ -528,9 +527,7 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
     const uint32_t* keys = ctx->keys[ctx->keysIdx];
     const size_t v4 = 16 * (size_t)c.n;
     // With a tape, the friends (rows), the packed (p, lambda) of every
-    // iteration and omega are written straight into the tape's buffers.  The
-    // circle rows stay in ctx->list.
-    uint32_t* list = ctx->list;
+    // iteration and omega are written straight into the tape's buffers.
     uint4* rows = tape ? tape->rows : ctx->rows;
     uint2* meta = tape ? tape->meta : ctx->meta;
     float4* omega = tape ? tape->omega : ctx->omega;
@@ -540,9 +537,7 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
     c.keys = keys;  // the taint of irregular positions finds a cell's particles in them
     pbf::launch_update_cells(c.n, keys, ctx->cells, tableKeys, ctx->errWord, s, ctx->cellStart);
     mark("buildFriendsList");
-    // the rows of the kept friends are recorded by the first density pass (or
-    // flattened when there is none)
-    pbf::launch_build_friends(c, b, ctx->pred[sortedPred], ctx->cells, list, meta, ctx->errWord, ls.friends,
+    pbf::launch_build_friends(c, b, ctx->pred[sortedPred], ctx->cells, rows, meta, ctx->errWord, ls.friends,
                               ls.friendsAlgorithm, s);
     mark("resetPartList");
     pbf::launch_reset_cells(c.n, keys, ctx->cells, tableKeys, ctx->errWord, s);
@@ -552,17 +547,12 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
     for (unsigned it = 0; it < iters; ++it) {
         float4* packed = tape ? tape->q[it] : ctx->pred[a ^ 1];
         mark("computeScaling", (int)it);
-        pbf::launch_compute_scaling(c, ctx->pred[a], packed, ctx->density, list, meta, it > 0 ? rows : nullptr,
-                                    it > 0 ? nullptr : rows, ls.scaling, ls.balance, tiles(1), s);
+        pbf::launch_compute_scaling(c, ctx->pred[a], packed, ctx->density, meta, rows, ls.scaling, ls.balance, tiles(1), s);
         mark("computeDelta", (int)it);
         pbf::launch_compute_delta(c, b, packed, ctx->pos[sortedPos], ctx->pred[a], ctx->density, meta,
                                   it + 1 == iters, tape && tape->mask ? tape->mask + (size_t)it * c.n : nullptr,
                                   rows, ls.delta, ls.balance, tiles(2), s);
         launched += 2;
-    }
-    if (iters == 0) {
-        pbf::launch_flatten_friends(c, list, meta, rows, s);
-        ++launched;
     }
     if (iters == 0) {  // packData with the density buffer as it stands (src/Simulation.cpp:591)
         mark("packData");
@@ -912,7 +902,7 @@ int pbf_destroy(pbf_ctx* ctx) {
         dev_free(ctx->keys[k]); dev_free(ctx->perm[k]);
     }
     dev_free(ctx->omega); dev_free(ctx->density); dev_free(ctx->hist); dev_free(ctx->cells);
-    dev_free(ctx->list); dev_free(ctx->rows); dev_free(ctx->meta); dev_free(ctx->errWord); dev_free(ctx->tileCounters);
+    dev_free(ctx->rows); dev_free(ctx->meta); dev_free(ctx->errWord); dev_free(ctx->tileCounters);
     dev_free(ctx->taint); dev_free(ctx->cellXYZ); dev_free(ctx->cellStart);
     dev_free(ctx->scenes); dev_free(ctx->sceneOf); dev_free(ctx->ids); dev_free(ctx->idsTmp);
     dev_free(ctx->quadsDev); dev_free(ctx->maskDev); dev_free(ctx->waveDev);
@@ -1008,8 +998,7 @@ int pbf_init_cells(pbf_ctx* ctx) {
     ctx->listSlots = (int)(p.friendsCircles * p.particlesPerCircle);
     ctx->cellsN = ctx->n;
     ++ctx->epoch;
-    if ((rc = dev_alloc(ctx, &ctx->list, (size_t)ctx->listSlots * ctx->n)) ||
-        (rc = dev_alloc(ctx, &ctx->rows, pbf::row_entries(ctx->listSlots) * ctx->n)) || (rc = dev_alloc(ctx, &ctx->meta, ctx->n)) ||
+    if ((rc = dev_alloc(ctx, &ctx->rows, pbf::row_entries(ctx->listSlots) * ctx->n)) || (rc = dev_alloc(ctx, &ctx->meta, ctx->n)) ||
         (rc = dev_alloc(ctx, &ctx->taint, ctx->n)) || (rc = dev_alloc(ctx, &ctx->cellXYZ, ctx->n)) ||
         (rc = dev_alloc(ctx, &ctx->cellStart, tableWords)))
         return rc;
@@ -1721,9 +1710,9 @@ int pbf_autotune(pbf_ctx* ctx, int trial_substeps, int* blocks_out) {
     for (int bal = 0; bal < 2; ++bal)
         for (int q = 0; q < 4; ++q) { solverMs[bal][q] = 1e30f; solverBlock[bal][q] = 256; }
     ctx->stageTiming = true;
-    for (int trial = 0; trial < 24; ++trial) {
-        // block size x friends algorithm (3) x balanced thread map (2)
-        const int cand = candidates[trial % 4], algo = (trial / 4) % 3, bal = trial / 12;
+    for (int trial = 0; trial < 16; ++trial) {
+        // block size x friends algorithm (2) x balanced thread map (2)
+        const int cand = candidates[trial % 4], algo = (trial / 4) % 2, bal = trial / 8;
         ctx->shape = pbf::LaunchShape{cand, cand, cand, cand, cand, algo, bal, 0};
         ctx->stageNames.clear();
         ctx->stageMs.clear();

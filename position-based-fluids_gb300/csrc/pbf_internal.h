@@ -96,8 +96,7 @@ SceneParams make_scene_params(const PbfParameters& p, uint32_t keyBase);
 // Threads per block of the kernels whose block size the autotuner chooses.
 struct LaunchShape {
     int friends = 256, scaling = 256, delta = 256, viscosity = 256, vorticity = 256;
-    int friendsAlgorithm = 0;  // 0: one thread scans per particle; 1: warp-cooperative runs;
-                               // 2: 4x4x4-cell bricks streamed through shared memory
+    int friendsAlgorithm = 0;  // 1: one thread scans per particle; else: built by warps, run by run
     int balance = 0;           // solver passes: threads take the block's particles by friend count
     int persistent = 0;        // the four solver passes: a grid of the resident blocks takes
                                // the particle tiles from a counter (no waits between blocks)
@@ -120,20 +119,15 @@ void launch_reset_cells(int n, const uint32_t* keys, uint32_t* cells, uint32_t k
 // tileCounter (two device words, zero between launches; NULL for one block
 // per tile of particles): the solver passes' persistent grid, whose
 // blocks take the tiles from it (LaunchShape::persistent).
-// algorithm: LaunchShape::friendsAlgorithm.  Every build writes the circle
-// rows into `list`; the first density pass records the rows from them.
-void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const uint32_t* cells, uint32_t* list,
+// Writes the rows (walk_pairs in pbf_device.cuh) and meta.  algorithm:
+// LaunchShape::friendsAlgorithm; block is the scan's.
+void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const uint32_t* cells, uint4* rows,
                           uint2* meta, int* errorWord, int block, int algorithm, cudaStream_t s);
-// uint4 words per particle of the rows (walk_pairs in pbf_device.cuh) for
-// `slots` friends.
+// uint4 entries per particle of the rows for `slots` friends.
 inline size_t row_entries(int slots) { return ((size_t)slots + 3) / 4; }
-// The rows from the circle rows, when no density pass records them.
-void launch_flatten_friends(const DevConsts& c, const uint32_t* list, const uint2* meta, uint4* rows, cudaStream_t s);
-// rowsOut (may be NULL): the rows recorded by the first density pass of a
-// substep; rowsIn: the rows, walked by the passes after it.
 void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* predPacked, float* density,
-                            const uint32_t* list, const uint2* meta, const uint4* rowsIn, uint4* rowsOut,
-                            int block, int balance, int* tileCounter, cudaStream_t s);
+                            const uint2* meta, const uint4* rows, int block, int balance, int* tileCounter,
+                            cudaStream_t s);
 // posPrev: the sorted positions, read only by the force planes.
 void launch_compute_delta(const DevConsts& c, Batch b, const float4* predPacked, const float4* posPrev,
                           float4* predOut, const float* density, const uint2* meta, int lastIteration,

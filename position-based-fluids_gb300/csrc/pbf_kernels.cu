@@ -14,15 +14,10 @@
 //   pos, pred, vel, omega : float4[N]  (16-byte records, coalesced 128-bit I/O)
 //   keys, perm            : uint32[N]
 //   cells                 : uint2[gridBufSize]  (start, inclusive end)
-//   list                  : uint32[circles * perCircle][N]: friend s of circle
-//                           c of particle i at row c*perCircle + s (the
-//                           reference's friends layout, build_friends_list.cl:
-//                           1-21); a warp of consecutive particles reads one
-//                           row coalesced.
 //   rows                  : uint4[ceil(circles * perCircle / 4)][N]: particle
-//                           i's friends in summation order, four per entry;
-//                           recorded by the first density pass of a substep
-//                           and walked by the passes after it.
+//                           i's friends that the density pass keeps, in
+//                           summation order, four per entry; written by the
+//                           friends build and walked by the passes after it.
 //   meta                  : uint2[N] per particle: 7-bit friend count of each
 //                           of up to 8 circles (bits 0-55), the circles the
 //                           density pass keeps (bits 56-59) and the circles
@@ -138,107 +133,94 @@ __global__ void reset_cells_kernel(int n, const uint32_t* __restrict__ keys, uin
 // Number of leading circles a pass keeps: circles are visited in order and
 // skipped once processed/total exceeds the threshold (compute_scaling.cl:47-54
 // with 0.6f; compute_delta.cl:97-104, apply_viscosity.cl:25-32 and
-// apply_vorticity.cl:23-30 with 0.5f).
-__device__ __forceinline__ int circles_kept(uint64_t cnt, int C, int total, float threshold) {
-    int processed = 0, kept = 0;
-    for (int k = 0; k < C; ++k) {
-        if (((float)processed) / total > threshold) continue;
-        processed += (int)byte_of(cnt, k);
-        kept = k + 1;
-    }
-    return kept;
+// apply_vorticity.cl:23-30 with 0.5f).  The rounded quotient of two counts of
+// at most 512 exceeds 0.6f exactly when 5 processed > 3 total, and 0.5f when
+// 2 processed > total: 0.6f is the float nearest 3/5, and a quotient that is
+// not 3/5 differs from it by at least 1/2560.
+__device__ __forceinline__ bool density_keeps(const DevConsts& c, int processed, int total) {
+    return c.complete || 5 * processed <= 3 * total;
+}
+__device__ __forceinline__ bool others_keep(const DevConsts& c, int processed, int total) {
+    return c.complete || 2 * processed <= total;
 }
 
-// One particle's friend circles as the candidates arrive (build_friends_list.cl:
-// 58-95): r^2 < h^2, binned into circles by min(int(adj^3 * C), C-1) with
-// adj = max(0, (r - 0.3h) / 0.7h), at most perCircle per circle (later ones
-// are dropped, :79-83).  The circle is read off precomputed r^2 thresholds
-// (DevConsts::circT): the same integer the sqrt / divide / cube / truncate
-// sequence gives, without computing it.
-//
-// Narrow (at most 5 circles of at most 63): the counters are 6-bit fields of
-// one word, so a candidate's slot, the test "inside and its circle not full",
-// the store and the increment are a few 32-bit operations with no branch
-// (the wide form's 64-bit counter arithmetic is longer).  Either form writes
-// the same entries in the same order.
-template <bool Narrow>
-struct FriendCircles {
-    const DevConsts& c;
-    uint32_t* row0;     // this particle's entry of list row 0; row r is row0 + r * n
-    uint32_t rowBytes;  // 4 n
-    int n, i;
-    float4 pi;
-    uint64_t cnt = 0;   // wide: 8 circles x 8-bit counters
-    uint32_t cnt6 = 0;  // narrow: 5 circles x 6-bit counters
-    __device__ __forceinline__ FriendCircles(const DevConsts& cc, uint32_t* l, int i_, float4 p)
-        : c(cc), row0(l + i_), rowBytes(4u * (uint32_t)cc.n), n(cc.n), i(i_), pi(p) {}
-    __device__ __forceinline__ uint32_t count(int k) const {
-        return Narrow ? (cnt6 >> (6 * k)) & 63u : byte_of(cnt, k);
+// The meta words (see the head of this file) of a particle whose circles'
+// counts are the bytes of cnt; *dense receives the friends the density pass
+// keeps.
+__device__ __forceinline__ uint2 make_meta(const DevConsts& c, uint64_t cnt, int* dense) {
+    const int C = c.circles;
+    int total = 0;
+    for (int k = 0; k < C; ++k) total += (int)byte_of(cnt, k);
+    uint64_t mt = 0;
+    int before = 0, keptL = 0, keptO = 0;
+    *dense = 0;
+    for (int k = 0; k < C; ++k) {
+        const int nk = (int)byte_of(cnt, k);
+        mt |= (uint64_t)nk << (7 * k);
+        const bool d = density_keeps(c, before, total), o = others_keep(c, before, total);
+        before += nk;
+        if (d) { keptL = k + 1; *dense = before; }
+        if (o) keptO = k + 1;
     }
-    __device__ __forceinline__ void consider(uint32_t j, const float4 pj) {
-        const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
-        const float r2 = dot3(rx, ry, rz, rx, ry, rz);
-        // thresholds past C-1 are +inf, so only the first C-1 decide
-        int circ = (r2 >= c.circT[0]) + (r2 >= c.circT[1]) + (r2 >= c.circT[2]) + (r2 >= c.circT[3]);
-        if (Narrow) {
-            const uint32_t sh = 6u * (uint32_t)circ;
-            const uint32_t k = (cnt6 >> sh) & 63u;
-            const bool take = !(r2 >= c.h2) && (int)k < c.perCircle;  // NaN distances are taken, as in the scan
-            const uint32_t row = (uint32_t)circ * (uint32_t)c.perCircle + k;
-            if (take) *reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(row0) + (size_t)row * rowBytes) = j;
-            cnt6 += take ? 1u << sh : 0u;
-        } else {
-            if (r2 >= c.h2) return;
-            if (c.circles > 5) circ += (r2 >= c.circT[4]) + (r2 >= c.circT[5]) + (r2 >= c.circT[6]);
-            const uint32_t k = byte_of(cnt, circ);
-            if ((int)k >= c.perCircle) return;
-            row0[(size_t)(circ * c.perCircle + (int)k) * n] = j;
-            cnt += 1ull << (8 * circ);
-        }
+    mt |= (uint64_t)keptL << 56 | (uint64_t)keptO << 60;
+    return make_uint2((uint32_t)mt, (uint32_t)(mt >> 32));
+}
+
+// Friend `pos` of particle i in the rows.
+__device__ __forceinline__ void put_friend(uint4* __restrict__ rows, int n, int i, int pos, uint32_t j) {
+    char* entry = reinterpret_cast<char*>(rows + i) + (uint64_t)((uint32_t)pos >> 2) * (16u * (uint32_t)n);
+    *reinterpret_cast<uint32_t*>(entry + 4u * ((uint32_t)pos & 3u)) = j;
+}
+
+// The friend circle of r^2 < h^2: min(int(adj^3 * C), C-1) with
+// adj = max(0, (r - 0.3h) / 0.7h) (build_friends_list.cl:58-95), read off
+// precomputed r^2 thresholds (DevConsts::circT): the same integer the sqrt /
+// divide / cube / truncate sequence gives, without computing it.  Thresholds
+// past C-1 are +inf.
+__device__ __forceinline__ int circle_of(const DevConsts& c, float r2) {
+    int circ = 0;  // the thresholds do not decrease: the last one reached counts
+    if (r2 >= c.circT[0]) circ = 1;
+    if (r2 >= c.circT[1]) circ = 2;
+    if (r2 >= c.circT[2]) circ = 3;
+    if (r2 >= c.circT[3]) circ = 4;
+    if (c.circles > 5) {
+        if (r2 >= c.circT[4]) circ = 5;
+        if (r2 >= c.circT[5]) circ = 6;
+        if (r2 >= c.circT[6]) circ = 7;
     }
-    __device__ __forceinline__ void finish(uint2* meta) const {
-        const int C = c.circles;
-        int total = 0;
-        uint64_t mt = 0, bytes = 0;
-        for (int k = 0; k < C; ++k) {
-            total += (int)count(k);
-            mt |= (uint64_t)count(k) << (7 * k);
-            bytes |= (uint64_t)count(k) << (8 * k);
-        }
-        mt |= (uint64_t)(c.complete ? C : circles_kept(bytes, C, total, 0.6f)) << 56;
-        mt |= (uint64_t)(c.complete ? C : circles_kept(bytes, C, total, 0.5f)) << 60;
-        meta[i] = make_uint2((uint32_t)mt, (uint32_t)(mt >> 32));
-    }
-};
+    return circ;
+}
 
 // build_friends_list.cl:29-102 for particle i: one scan of the 27 neighbour
 // cells in the reference's order (x, then y, then z offsets; particles of a
-// cell in sorted order), self excluded, candidates read through L1 with U
-// loads in flight.  The 27 hashes are formed from the three spread
-// coordinates of each axis.
-template <int U, typename FC>
-__device__ __forceinline__ void friends_scan_global(const DevConsts& c, uint32_t base, const float4* __restrict__ pred,
-                                                   const uint2* __restrict__ cells, int* __restrict__ err, FC& fc) {
-    const int i = fc.i, n = c.n;
-    const float4 pi = fc.pi;
-    const int cx = __float2int_rz(pi.x / c.h), cy = __float2int_rz(pi.y / c.h), cz = __float2int_rz(pi.z / c.h);
+// cell in sorted order), self excluded, candidates read through L1 with two
+// loads in flight: consider(j, r^2) for every candidate that is not out of
+// reach (a NaN distance is taken, as in the reference's test).  The 27 hashes
+// are formed from the three spread coordinates of each axis.
+template <typename F>
+__device__ __forceinline__ void scan_neighbours(const DevConsts& c, uint32_t base, const float4* __restrict__ pred,
+                                                const uint2* __restrict__ cells, int* __restrict__ err, int i,
+                                                const float4 pi, int cx, int cy, int cz, F consider) {
+    const int n = c.n;
     const bool pow2 = (c.grid & (c.grid - 1)) == 0;
     const uint32_t mask = c.grid - 1;
     const uint32_t exm = expand_bits(cx - 1), ex0 = expand_bits(cx), exp_ = expand_bits(cx + 1);
     const uint32_t eym = expand_bits(cy - 1) << 1, ey0 = expand_bits(cy) << 1, eyp = expand_bits(cy + 1) << 1;
     const uint32_t ezm = expand_bits(cz - 1) << 2, ez0 = expand_bits(cz) << 2, ezp = expand_bits(cz + 1) << 2;
     const uint32_t selfHash = pow2 ? ((ex0 | ey0 | ez0) & mask) : ((ex0 | ey0 | ez0) % c.grid);
-    record_cell(c, i, pi, cx, cy, cz, base);
+    auto test = [&](uint32_t j, const float4 pj) {
+        const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
+        const float r2 = dot3(rx, ry, rz, rx, ry, rz);
+        if (!(r2 >= c.h2)) consider(j, r2);
+    };
     auto scan = [&](uint32_t lo, uint32_t hi) {
         uint32_t j = lo;
-        for (; j + (U - 1) <= hi; j += U) {
-            float4 p[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) p[u] = __ldg(pred + j + u);
-#pragma unroll
-            for (int u = 0; u < U; ++u) fc.consider(j + u, p[u]);
+        for (; j + 1 <= hi; j += 2) {
+            const float4 p0 = __ldg(pred + j), p1 = __ldg(pred + j + 1);
+            test(j, p0);
+            test(j + 1, p1);
         }
-        for (; j <= hi; ++j) fc.consider(j, __ldg(pred + j));
+        if (j <= hi) test(j, __ldg(pred + j));
     };
     for (int x = -1; x <= 1; ++x) {
         const uint32_t ex = x < 0 ? exm : (x > 0 ? exp_ : ex0);
@@ -263,167 +245,148 @@ __device__ __forceinline__ void friends_scan_global(const DevConsts& c, uint32_t
     }
 }
 
-// One thread per particle, candidates through L1.
-template <int U, bool Narrow>
+// Particle i's friends by one thread: the circles are counted in one scan, and
+// each friend is put in its place in a second.  Circle counts saturate at
+// perCircle (later candidates are dropped, build_friends_list.cl:79-83).
+__device__ __noinline__ void friends_of_one(const DevConsts& c, uint32_t base, const float4* __restrict__ pred,
+                                            const uint2* __restrict__ cells, uint4* __restrict__ rows,
+                                            uint2* __restrict__ meta, int* __restrict__ err, int i, const float4 pi,
+                                            int cx, int cy, int cz) {
+    uint64_t cnt = 0;  // 8 circles x 8-bit counters
+    scan_neighbours(c, base, pred, cells, err, i, pi, cx, cy, cz, [&](uint32_t, float r2) {
+        const int k = circle_of(c, r2);
+        if ((int)byte_of(cnt, k) < c.perCircle) cnt += 1ull << (8 * k);
+    });
+    int dense;
+    const uint2 m = make_meta(c, cnt, &dense);
+    meta[i] = m;
+    uint64_t left = cnt;  // places not taken yet
+    scan_neighbours(c, base, pred, cells, err, i, pi, cx, cy, cz, [&](uint32_t j, float r2) {
+        const int k = circle_of(c, r2);
+        const int free = (int)byte_of(left, k);
+        if (free == 0) return;
+        left -= 1ull << (8 * k);
+        int pos = -free;
+        for (int q = 0; q <= k; ++q) pos += (int)byte_of(cnt, q);
+        if (pos < dense) put_friend(rows, c.n, i, pos, j);
+    });
+    for (int t = dense; t & 3; ++t) put_friend(rows, c.n, i, t, (uint32_t)i);
+}
+
 __global__ void __launch_bounds__(kMaxBlock)
-build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, const uint2* __restrict__ cells,
-                     uint32_t* __restrict__ list, uint2* __restrict__ meta, int* __restrict__ err) {
+build_friends_scan_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, const uint2* __restrict__ cells,
+                          uint4* __restrict__ rows, uint2* __restrict__ meta, int* __restrict__ err) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
-    FriendCircles<Narrow> fc(c, list, i, pred[i]);
-    friends_scan_global<U>(c, key_base(b, i), pred, cells, err, fc);
-    fc.finish(meta);
+    const float4 pi = pred[i];
+    const int cx = __float2int_rz(pi.x / c.h), cy = __float2int_rz(pi.y / c.h), cz = __float2int_rz(pi.z / c.h);
+    const uint32_t base = key_base(b, i);
+    record_cell(c, i, pi, cx, cy, cz, base);
+    friends_of_one(c, base, pred, cells, rows, meta, err, i, pi, cx, cy, cz);
 }
 
-// The same lists with the candidates streamed through shared memory, one
-// block per brick of B x B x B cells (B^3 consecutive Morton numbers, so the
-// brick's particles are one range of the sorted order).  The block stages the
-// brick's (B+2)^3 halo of cells into shared memory with coalesced float4
-// loads (every particle's 27 neighbour cells lie in it), then each thread
-// scans its particle's 27 cells from there in the reference's order.  A
-// particle whose cell is not the brick's (a key that aliases through the hash
-// modulo), or a halo too large for the buffer, takes the per-particle scan
-// through L1.  Needs a power-of-two GridBufferSize of at least B^3.
-template <int B> struct BrickShape;
-template <> struct BrickShape<4> { static constexpr int threads = 256, capacity = 2816; };  // 44 KB of float4
-
-__device__ __forceinline__ uint32_t compact_bits(uint32_t x) {
-    x &= 0x09249249u;
-    x = (x ^ (x >> 2)) & 0x030C30C3u;
-    x = (x ^ (x >> 4)) & 0x0300F00Fu;
-    x = (x ^ (x >> 8)) & 0x030000FFu;
-    x = (x ^ (x >> 16)) & 0x000003FFu;
-    return x;
+// Least and largest value of a warp's lanes, NaN if any lane holds one.
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm volatile("redux.sync.min.NaN.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm volatile("redux.sync.max.NaN.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+// The larger one, NaN if either is.
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
 }
 
-template <int B, bool Narrow>
-__global__ void __launch_bounds__(BrickShape<B>::threads)
-build_friends_brick_kernel(DevConsts c, const float4* __restrict__ pred, const uint2* __restrict__ cells,
-                           uint32_t* __restrict__ list, uint2* __restrict__ meta, int* __restrict__ err) {
-    constexpr int T = BrickShape<B>::threads, kCap = BrickShape<B>::capacity;
-    constexpr int E = B + 2, kHalo = E * E * E, kCodes = B * B * B, kPerLane = (kHalo + 31) / 32;
-    __shared__ uint32_t hStart[kHalo], hCount[kHalo], hOff[kHalo];
-    __shared__ float4 staged[kCap];
-    __shared__ uint32_t firstP, lastP, haloTotal;
-    const int t = threadIdx.x, n = c.n;
-    const uint32_t key0 = blockIdx.x * (uint32_t)kCodes;   // first key of the brick
-    const uint32_t base = (key0 / c.grid) * c.grid;        // the scene's key offset
-    const uint32_t m0 = key0 - base;                       // its Morton number
-    const int bx = (int)compact_bits(m0), by = (int)compact_bits(m0 >> 1), bz = (int)compact_bits(m0 >> 2);
-    if (t == 0) { firstP = 0xFFFFFFFFu; lastP = 0u; }
-    __syncthreads();
-    for (int q = t; q < kCodes; q += T) {  // the brick's particle range
-        const uint2 r = cells[key0 + q];
-        if (r.x != kEmpty) {
-            atomicMin(&firstP, r.x);
-            atomicMax(&lastP, min(r.y, (uint32_t)(n - 1)));
-        }
-    }
-    const uint32_t mask = c.grid - 1;
-    for (int h = t; h < kHalo; h += T) {
-        const int hx = bx - 1 + h / (E * E), hy = by - 1 + (h / E) % E, hz = bz - 1 + h % E;
-        const uint32_t m = expand_bits(hx) | (expand_bits(hy) << 1) | (expand_bits(hz) << 2);
-        const uint2 range = cells[base + (m & mask)];
-        uint32_t count = 0;
-        if (range.x != kEmpty) {
-            const uint32_t last = min(range.y, (uint32_t)(n - 1));
-            if (range.x <= last) count = last - range.x + 1u;
-            else atomicOr(err, kErrCellTable);
-        }
-        hStart[h] = range.x;
-        hCount[h] = count;
-    }
-    __syncthreads();
-    if (firstP == 0xFFFFFFFFu) return;  // an empty brick
-    if (t < 32) {  // exclusive scan of the halo counts
-        uint32_t v[kPerLane], s = 0;
-#pragma unroll
-        for (int k = 0; k < kPerLane; ++k) {
-            const int h = kPerLane * t + k;
-            v[k] = h < kHalo ? hCount[h] : 0u;
-            s += v[k];
-        }
-        uint32_t incl = s;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-            if (t >= d) incl += u;
-        }
-        uint32_t run = incl - s;
-#pragma unroll
-        for (int k = 0; k < kPerLane; ++k) {
-            const int h = kPerLane * t + k;
-            if (h < kHalo) hOff[h] = run;
-            run += v[k];
-        }
-        if (t == 31) haloTotal = incl;
-    }
-    __syncthreads();
-    const uint32_t total = haloTotal;
-    const bool useSmem = total <= (uint32_t)kCap;
-    if (useSmem) {
-        for (uint32_t e = t; e < total; e += T) {
-            int lo = 0;  // the halo cell holding staged entry e: the last with hOff <= e
-#pragma unroll
-            for (int s = 128; s > 0; s >>= 1)
-                if (lo + s < kHalo && hOff[lo + s] <= e) lo += s;
-            while (lo < kHalo - 1 && (hCount[lo] == 0 || hOff[lo] + hCount[lo] <= e)) ++lo;
-            staged[e] = pred[hStart[lo] + (e - hOff[lo])];
-        }
-    }
-    __syncthreads();
-    for (uint32_t p = firstP + t; p <= lastP; p += T) {
-        const int i = (int)p;
-        FriendCircles<Narrow> fc(c, list, i, pred[i]);
-        const int cx = __float2int_rz(fc.pi.x / c.h), cy = __float2int_rz(fc.pi.y / c.h), cz = __float2int_rz(fc.pi.z / c.h);
-        const int lx = cx - bx, ly = cy - by, lz = cz - bz;
-        if (useSmem && (unsigned)lx < (unsigned)B && (unsigned)ly < (unsigned)B && (unsigned)lz < (unsigned)B) {
-            record_cell(c, i, fc.pi, cx, cy, cz, base);
-            // staged entries [a, b) of one cell, candidates st + (k - off), two in flight, self skipped
-            auto scanStaged = [&](uint32_t a, uint32_t b, uint32_t jOfA) {
-                uint32_t k = a;
-                for (; k + 1 < b; k += 2) {
-                    const float4 p0 = staged[k], p1 = staged[k + 1];
-                    fc.consider(jOfA + (k - a), p0);
-                    fc.consider(jOfA + (k + 1 - a), p1);
-                }
-                if (k < b) fc.consider(jOfA + (k - a), staged[k]);
-            };
-#pragma unroll 1
-            for (int x = 0; x < 3; ++x)
-#pragma unroll 1
-                for (int y = 0; y < 3; ++y)
-#pragma unroll
-                    for (int z = 0; z < 3; ++z) {
-                        const int h = (lx + x) * (E * E) + (ly + y) * E + (lz + z);
-                        const uint32_t cnt = hCount[h], off = hOff[h], st = hStart[h];
-                        if ((uint32_t)i - st < cnt) {  // the particle's own range: skip itself
-                            const uint32_t self = off + ((uint32_t)i - st);
-                            scanStaged(off, self, st);
-                            scanStaged(self + 1, off + cnt, (uint32_t)i + 1);
-                        } else {
-                            scanStaged(off, off + cnt, st);
-                        }
-                    }
-        } else {
-            friends_scan_global<2>(c, base, pred, cells, err, fc);
-        }
-        fc.finish(meta);
-    }
-}
+// The same rows, built by warps.  A warp takes its 32 particles run by run (a
+// run: consecutive particles in one cell of one scene, which share the 27-cell
+// candidate sequence).  The sequence goes to shared memory once per run, in
+// order, without the candidates farther than h from the box around the run's
+// members (their r^2 to every member is at least their r^2 to the box, which
+// the same rounded operations form).  Then all lanes test the candidates
+// against one member after another, 64 at a time, and append the accepted ones
+// to a list, in order; then they sort the list by circle, which ballots over
+// the thresholds of r^2 do stably, and write the member's rows.
+//
+// What bounds it is instruction issue.  A scan by one thread per particle
+// tests 424 candidates in lockstep for each, at about 49 instructions, and
+// stores friends 4 bytes at a time into rows N apart; here a member costs about
+// 4 steps of 64 candidates and the sorting of its list, and its friends are
+// stored 16 bytes together.  1M particles, mid-collapse: 641M -> 453M warp
+// instructions, 649 -> 462 us at 81 % issue active, DRAM writes 489 -> 160 MB,
+// and the density pass that used to copy the friends into rows (149 us) is one
+// of the others (100 us).  Per particle the candidate sequence takes about 100
+// instructions, the tests 160 and the sorting 170.  Against the scan below, which
+// has to run twice to write the rows: faster from one particle to a cell on
+// (500,000 particles: 0.21 against 0.25 ms there, 0.17 against 0.46 at four), 13 %
+// slower at one particle to two cells.  Runs whose candidates do not fit are taken
+// member by member; a member with more than kMostFriends accepted candidates and
+// runs with coordinates that are not finite take the scan.
+constexpr int kFriendWarps = 4, kCandidates = 384, kMostFriends = 128;
+struct FriendShared {
+    float x[kCandidates], y[kCandidates], z[kCandidates];
+    uint32_t j[kCandidates];
+    uint2 list[kMostFriends + 64];  // candidate, bits of r^2
+};
 
-// The same lists, built warp-cooperatively.  A warp takes its 32 particles
-// run by run (a run: consecutive particles in one cell of one scene, which
-// share the 27-cell candidate sequence).  Lanes take 32 candidates of the
-// run's sequence at a time, in order (the candidate of lane L follows that of
-// lane L-1), and every run member tests all 32: its accepted candidates are
-// appended to their circles in sequence order, with ranks from the circle
-// counts and match_any, so the lists equal those of the per-particle scan
-// while every lane stays busy.  Circle counts saturate at perCircle.
-__global__ void __launch_bounds__(kMaxBlock)
-build_friends_warp_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, const uint2* __restrict__ cells,
-                          uint32_t* __restrict__ list, uint2* __restrict__ meta, int* __restrict__ err) {
+// Sorts the cnt <= 32 NR entries of the list by circle, at most perCircle to a
+// circle (later candidates are dropped, build_friends_list.cl:79-83), and
+// writes the rows of particle ip.  Returns the circles' counts, one byte each.
+// The counts stay below 256, so that four bytes of a word are added, and
+// summed up to each circle by one multiplication, at once.
+template <int NR>
+__device__ __forceinline__ uint64_t sort_friends(const DevConsts& c, const FriendShared& sh, int lane, uint32_t ltMask,
+                                                 int cnt, int ip, uint4* __restrict__ rows) {
     constexpr unsigned kFull = 0xFFFFFFFFu;
+    constexpr uint32_t kOnes = 0x01010101u;
+    uint32_t j[NR], circ[NR], rank[NR];
+    uint32_t lo = 0, hi = 0;  // counts of circles 0-3 and 4-7
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        const int e = 32 * r + lane;
+        const uint2 entry = sh.list[e];
+        j[r] = sh.j[e < cnt ? entry.x : 0u];
+        const bool valid = e < cnt && (int)j[r] != ip;  // not itself (build_friends_list.cl:62)
+        circ[r] = valid ? (uint32_t)circle_of(c, __uint_as_float(entry.y)) : 8u;
+        const uint32_t peers = __match_any_sync(kFull, circ[r]);
+        const uint32_t one = valid ? 1u << (8u * (circ[r] & 3u)) : 0u, one0 = circ[r] < 4u ? one : 0u;
+        rank[r] = (uint32_t)__popc(peers & ltMask) + (r ? __byte_perm(lo, hi, circ[r] & 7u) & 0xFFu : 0u);
+        lo += __reduce_add_sync(kFull, one0);
+        hi += __reduce_add_sync(kFull, one - one0);
+    }
+    const uint32_t over = (127u - (uint32_t)c.perCircle) * kOnes;
+    if (((lo + over) | (hi + over)) & 0x80808080u) {  // a circle is over its limit
+        auto clip = [&](uint32_t w) {
+            uint32_t v = 0;
+            for (int k = 0; k < 4; ++k) v |= min((w >> (8 * k)) & 0xFFu, (uint32_t)c.perCircle) << (8 * k);
+            return v;
+        };
+        lo = clip(lo);
+        hi = clip(hi);
+    }
+    const uint32_t ends = lo * kOnes, upTo3 = ends >> 24, endsHi = (hi + upTo3) * kOnes;
+    const uint32_t begins = ends << 8, beginsHi = (endsHi << 8) | upTo3;
+    const int total = (int)(endsHi >> 24);
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        const int first = (int)__byte_perm(begins, beginsHi, circ[r] & 7u);  // the zero byte 0 fills the other bytes
+        if (circ[r] < 8u && (int)rank[r] < c.perCircle && density_keeps(c, first, total))
+            put_friend(rows, c.n, ip, first + (int)rank[r], j[r]);
+    }
+    return (uint64_t)lo | ((uint64_t)hi << 32);
+}
+
+__global__ void __launch_bounds__(32 * kFriendWarps)
+build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, const uint2* __restrict__ cells,
+                     uint4* __restrict__ rows, uint2* __restrict__ meta, int* __restrict__ err) {
+    constexpr unsigned kFull = 0xFFFFFFFFu;
+    __shared__ FriendShared shared[kFriendWarps];
+    FriendShared& sh = shared[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int warpBase = i - lane;
@@ -433,7 +396,6 @@ build_friends_warp_kernel(DevConsts c, Batch b, const float4* __restrict__ pred,
     const float4 pi = valid ? pred[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const int cx = __float2int_rz(pi.x / c.h), cy = __float2int_rz(pi.y / c.h), cz = __float2int_rz(pi.z / c.h);
     const uint32_t base = valid ? key_base(b, i) : 0u;
-    const int C = c.circles, P = c.perCircle;
     if (valid) record_cell(c, i, pi, cx, cy, cz, base);
     const bool pow2 = (c.grid & (c.grid - 1)) == 0;
     const uint32_t gmask = c.grid - 1;
@@ -443,14 +405,22 @@ build_friends_warp_kernel(DevConsts c, Batch b, const float4* __restrict__ pred,
     uint32_t heads = __ballot_sync(kFull, head);
     const uint32_t validMask = __ballot_sync(kFull, valid);
     const uint32_t ltMask = (1u << lane) - 1u;
-    const uint32_t capP = (uint32_t)P * 0x01010101u;
-    uint32_t cntLo = 0, cntHi = 0;  // this lane's particle: 8 circles x 8-bit counters
+    const float inf = __int_as_float(0x7F800000);
+    uint32_t scan = 0;   // lanes whose particles take the scan
+    uint64_t counts = 0; // this lane's particle: its circles' counts
     while (heads) {
         const int h0 = __ffs(heads) - 1;
         heads &= heads - 1;
-        const int h1 = heads ? __ffs(heads) - 1 : 32;
-        const uint32_t upTo = h1 == 32 ? kFull : ((1u << h1) - 1u);
+        const uint32_t upTo = heads ? (heads & (0u - heads)) - 1u : kFull;
         const uint32_t runMask = validMask & upTo & ~((1u << h0) - 1u);
+        const bool member = (runMask >> lane) & 1u;
+        const float lx = warp_min(member ? pi.x : inf), ly = warp_min(member ? pi.y : inf), lz = warp_min(member ? pi.z : inf);
+        const float hx = warp_max(member ? pi.x : -inf), hy = warp_max(member ? pi.y : -inf), hz = warp_max(member ? pi.z : -inf);
+        const float sum = (lx + hx) + (ly + hy) + (lz + hz);
+        if (!(fabsf(sum) < inf)) {
+            scan |= runMask;
+            continue;
+        }
         const int rx0 = __shfl_sync(kFull, cx, h0), ry0 = __shfl_sync(kFull, cy, h0), rz0 = __shfl_sync(kFull, cz, h0);
         const uint32_t rbase = __shfl_sync(kFull, base, h0);
         // lane q < 27: neighbour cell q in the scan order (x, then y, then z offsets)
@@ -472,59 +442,83 @@ build_friends_warp_kernel(DevConsts c, Batch b, const float4* __restrict__ pred,
             if (lane >= d) end += v;
         }
         const uint32_t total = __shfl_sync(kFull, end, 31);
+        // the cells that hold any, in order: candidate t of the q-th is particle t + shift
+        const uint32_t occupied = __ballot_sync(kFull, count > 0u);
+        if (count > 0u) sh.list[__popc(occupied & ltMask)] = make_uint2(end, start - (end - count));
+        __syncwarp();
+        const uint2 cell = sh.list[lane];
+        end = lane < __popc(occupied) ? cell.x : 0xFFFFFFFFu;
+        const uint32_t shift = cell.y;
+        __syncwarp();
+        uint32_t kept = 0;
+        int firstCell = 0;  // of candidate t0
         for (uint32_t t0 = 0; t0 < total; t0 += 32) {
             const uint32_t t = t0 + (uint32_t)lane;
-            const bool tv = t < total;
-            int q = 0;  // the first cell with end > t
-#pragma unroll
-            for (int s = 16; s > 0; s >>= 1) {
-                const uint32_t e = __shfl_sync(kFull, end, q + s - 1);
-                if (e <= t) q += s;
+            // bit l: a cell ends at candidate t0 + l
+            const uint32_t ending = __reduce_or_sync(kFull, end - t0 < 32u ? 1u << (end - t0) : 0u);
+            const int q = firstCell + __popc(ending & (ltMask | (1u << lane)));
+            firstCell += __popc(ending);
+            const uint32_t j = t + __shfl_sync(kFull, shift, q);
+            const float4 pj = t < total ? __ldg(pred + j) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float dx = max_nan(max_nan(lx - pj.x, pj.x - hx), 0.0f), dy = max_nan(max_nan(ly - pj.y, pj.y - hy), 0.0f),
+                        dz = max_nan(max_nan(lz - pj.z, pj.z - hz), 0.0f);
+            const bool keep = t < total && !(dot3(dx, dy, dz, dx, dy, dz) >= c.h2);
+            const uint32_t km = __ballot_sync(kFull, keep);
+            const uint32_t pos = kept + (uint32_t)__popc(km & ltMask);
+            if (keep && pos < (uint32_t)kCandidates) {
+                sh.x[pos] = pj.x;
+                sh.y[pos] = pj.y;
+                sh.z[pos] = pj.z;
+                sh.j[pos] = j;
             }
-            const uint32_t qs = __shfl_sync(kFull, start, q), qe = __shfl_sync(kFull, end, q);
-            const uint32_t qc = __shfl_sync(kFull, count, q);
-            const uint32_t j = qs + (t - (qe - qc));
-            const float4 pj = tv ? __ldg(pred + j) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            for (uint32_t rm = runMask; rm; rm &= rm - 1u) {
-                const int pl = __ffs(rm) - 1;
-                const int ip = warpBase + pl;
-                const float px = __shfl_sync(kFull, pi.x, pl), py = __shfl_sync(kFull, pi.y, pl);
-                const float pz = __shfl_sync(kFull, pi.z, pl);
-                const float rx = px - pj.x, ry = py - pj.y, rz = pz - pj.z;
-                const float r2 = dot3(rx, ry, rz, rx, ry, rz);
-                const bool acc = tv && (int)j != ip && !(r2 >= c.h2);  // NaN distances are kept, as in the scan
-                const uint32_t am = __ballot_sync(kFull, acc);
-                if (!am) continue;
-                int circ = (r2 >= c.circT[0]) + (r2 >= c.circT[1]) + (r2 >= c.circT[2]) + (r2 >= c.circT[3]);
-                if (C > 5) circ += (r2 >= c.circT[4]) + (r2 >= c.circT[5]) + (r2 >= c.circT[6]);
-                const uint32_t plo = __shfl_sync(kFull, cntLo, pl), phi = __shfl_sync(kFull, cntHi, pl);
-                if (acc) {
-                    const uint32_t peers = __match_any_sync(am, circ);
-                    const uint32_t have = circ < 4 ? (plo >> (8 * circ)) & 0xFFu : (phi >> (8 * (circ - 4))) & 0xFFu;
-                    const uint32_t rank = have + (uint32_t)__popc(peers & ltMask);
-                    if ((int)rank < P) list[(size_t)(circ * P + (int)rank) * n + ip] = j;
-                }
-                const uint32_t incLo = (acc && circ < 4) ? 1u << (8 * circ) : 0u;
-                const uint32_t incHi = (acc && circ >= 4) ? 1u << (8 * (circ - 4)) : 0u;
-                const uint32_t sLo = __reduce_add_sync(kFull, incLo), sHi = __reduce_add_sync(kFull, incHi);
-                if (lane == pl) {  // bytes stay below 256 (<= 64 + 32), then saturate at perCircle
-                    cntLo = __vminu4(plo + sLo, capP);
-                    cntHi = __vminu4(phi + sHi, capP);
-                }
+            kept += (uint32_t)__popc(km);
+        }
+        if (kept > (uint32_t)kCandidates) {
+            if (runMask & (runMask - 1u)) heads |= runMask;  // one member at a time
+            else scan |= runMask;
+            continue;
+        }
+        for (uint32_t e = kept + (uint32_t)lane; e < ((kept + 63u) & ~63u); e += 32) {  // up to a step of 64: out of reach
+            sh.x[e] = inf;
+            sh.y[e] = sh.z[e] = 0.0f;
+        }
+        __syncwarp();
+        for (uint32_t rm = runMask; rm; rm &= rm - 1u) {
+            const int pl = __ffs(rm) - 1;
+            const F2 px = both(__shfl_sync(kFull, pi.x, pl)), py = both(__shfl_sync(kFull, pi.y, pl)),
+                     pz = both(__shfl_sync(kFull, pi.z, pl));
+            int cnt = 0;
+            for (uint32_t k = 0; k < kept && cnt <= kMostFriends; k += 64) {
+                const uint32_t e = k + 2u * (uint32_t)lane;
+                const F2 rx = sub2(px, load2(sh.x + e)), ry = sub2(py, load2(sh.y + e)), rz = sub2(pz, load2(sh.z + e));
+                const float2 r2 = unpack2(dot2(c, rx, ry, rz, rx, ry, rz));
+                const bool a0 = !(r2.x >= c.h2), a1 = !(r2.y >= c.h2);  // a NaN distance is taken, as in the scan
+                const uint32_t m0 = __ballot_sync(kFull, a0), m1 = __ballot_sync(kFull, a1);
+                const int pos = cnt + __popc(m0 & ltMask) + __popc(m1 & ltMask);
+                if (a0) sh.list[pos] = make_uint2(e, __float_as_uint(r2.x));
+                if (a1) sh.list[pos + (a0 ? 1 : 0)] = make_uint2(e + 1u, __float_as_uint(r2.y));
+                cnt += __popc(m0) + __popc(m1);
             }
+            __syncwarp();
+            const int ip = warpBase + pl;
+            uint64_t mine = 0;
+            if (cnt <= 32) mine = sort_friends<1>(c, sh, lane, ltMask, cnt, ip, rows);
+            else if (cnt <= 64) mine = sort_friends<2>(c, sh, lane, ltMask, cnt, ip, rows);
+            else if (cnt <= 96) mine = sort_friends<3>(c, sh, lane, ltMask, cnt, ip, rows);
+            else if (cnt <= kMostFriends) mine = sort_friends<4>(c, sh, lane, ltMask, cnt, ip, rows);
+            else scan |= 1u << pl;
+            if (lane == pl) counts = mine;
+            __syncwarp();  // the list is read before the next member's is written
         }
     }
     if (!valid) return;
-    const uint64_t cnt = (uint64_t)cntLo | ((uint64_t)cntHi << 32);
-    int total = 0;
-    uint64_t mt = 0;
-    for (int k = 0; k < C; ++k) {
-        total += (int)byte_of(cnt, k);
-        mt |= (uint64_t)byte_of(cnt, k) << (7 * k);
+    if ((scan >> lane) & 1u) {
+        friends_of_one(c, base, pred, cells, rows, meta, err, i, pi, cx, cy, cz);
+        return;
     }
-    mt |= (uint64_t)(c.complete ? C : circles_kept(cnt, C, total, 0.6f)) << 56;
-    mt |= (uint64_t)(c.complete ? C : circles_kept(cnt, C, total, 0.5f)) << 60;
-    meta[i] = make_uint2((uint32_t)mt, (uint32_t)(mt >> 32));
+    int dense;
+    meta[i] = make_meta(c, counts, &dense);
+    for (int t = dense; t & 3; ++t) put_friend(rows, n, i, t, (uint32_t)i);
 }
 
 // ------------------------------------------------- balanced thread map --
@@ -617,13 +611,11 @@ __device__ __forceinline__ F2 spiky_over_r2(const DevConsts& c, F2 r2, F2& w) {
 }
 
 // compute_scaling.cl:27-112 followed by pack_data.cl (w = lambda).  Q: the
-// exact quotients by |r| through one reciprocal (quotient_rn).  Rec: the
-// friends come from the circle rows, and the rows are recorded.
-template <bool R, bool Rec, bool Q>
+// exact quotients by |r| through one reciprocal (quotient_rn).
+template <bool R, bool Q>
 __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const float4* __restrict__ pred,
                                                      float4* __restrict__ predPacked, float* __restrict__ density,
-                                                     const uint32_t* __restrict__ list, const uint4* __restrict__ rowsIn,
-                                                     uint4* __restrict__ rowsOut, int i, const float4 pi, uint64_t mt) {
+                                                     const uint4* __restrict__ rows, int i, const float4 pi, uint64_t mt) {
     const int n = c.n;
     // complete neighbour sets count the particle itself first: d = h^2 - 0
     float ds = c.complete ? c.h2 * c.h2 * c.h2 : 0.0f, gsk = 0.0f, gx = 0.0f, gy = 0.0f, gz = 0.0f;
@@ -640,7 +632,7 @@ __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const f
         gy = gy + g1;
         gz = gz + g2;
     };
-    auto pair = [&](const float4& pa, const float4& pb, bool va, bool vb) {
+    walk_pairs(rows, n, i, FlatFriends(mt, kept_density(mt)).total, load, [&](const float4& pa, const float4& pb, bool va, bool vb) {
         const F2 rx = pack2(pi.x - pa.x, pi.x - pb.x), ry = pack2(pi.y - pa.y, pi.y - pb.y),
                  rz = pack2(pi.z - pa.z, pi.z - pb.z);
         const F2 r2 = R ? fma2(rz, rz, fma2(ry, ry, mul2(rx, rx))) : dot2(c, rx, ry, rz, rx, ry, rz);
@@ -696,10 +688,7 @@ __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const f
                 gx = gx + x.y; gy = gy + y.y; gz = gz + z.y;
             }
         }
-    };
-    const FriendRows fr(mt, kept_density(mt), c.perCircle);
-    if (Rec) walk_pairs_recording(list, rowsOut, n, i, fr, load, pair);
-    else walk_pairs(rowsIn, n, i, fr.total, load, pair);
+    });
     ds = ds * c.poly6;
     density[i] = ds;
     gsk = gsk + dot3(gx, gy, gz, gx, gy, gz);
@@ -708,20 +697,19 @@ __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const f
     predPacked[i] = make_float4(pi.x, pi.y, pi.z, lambda);
 }
 
-template <bool R, bool B, bool Rec>
+template <bool R, bool B>
 __global__ void __launch_bounds__(kMaxBlock)
 compute_scaling_kernel(DevConsts c, const float4* __restrict__ pred, float4* __restrict__ predPacked,
-                       float* __restrict__ density, const uint32_t* __restrict__ list,
-                       const uint2* __restrict__ meta, const uint4* __restrict__ rowsIn,
-                       uint4* __restrict__ rowsOut, int tiles, int* tileCounter) {
+                       float* __restrict__ density, const uint2* __restrict__ meta, const uint4* __restrict__ rows,
+                       int tiles, int* tileCounter) {
     for_tiles(tiles, tileCounter, [&](int tile) {
         const int i = B ? balanced_particle(meta, c.n, true, tile) : tile * (int)blockDim.x + (int)threadIdx.x;
         if (i < 0 || i >= c.n) return;
         const float4 pi = pred[i];
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) compute_scaling_body<R, Rec, true>(c, pred, predPacked, density, list, rowsIn, rowsOut, i, pi, mt);
-        else compute_scaling_body<R, Rec, false>(c, pred, predPacked, density, list, rowsIn, rowsOut, i, pi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) compute_scaling_body<R, true>(c, pred, predPacked, density, rows, i, pi, mt);
+        else compute_scaling_body<R, false>(c, pred, predPacked, density, rows, i, pi, mt);
     });
 }
 
@@ -1130,59 +1118,25 @@ unsigned grid_for_tiles(K kernel, int n, int block, bool persistent, int* tiles)
     return cap;
 }
 
-void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const uint32_t* cells, uint32_t* list,
+void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const uint32_t* cells, uint4* rows,
                           uint2* meta, int* errorWord, int block, int algorithm, cudaStream_t s) {
-    const bool pow2 = (c.grid & (c.grid - 1)) == 0;
-    const uint32_t keys = c.grid * (uint32_t)(b.scenes ? b.nscenes : 1);
     const uint2* cellPairs = reinterpret_cast<const uint2*>(cells);
-    // narrow counters: at most 5 circles of at most 63 friends
-    const bool narrow = c.circles <= 5 && c.perCircle <= 63;
-    if (algorithm == 2 && pow2 && c.grid >= 64) {  // one block per 4x4x4-cell brick over all scenes
-        auto kb = narrow ? build_friends_brick_kernel<4, true> : build_friends_brick_kernel<4, false>;
-        kb<<<keys / 64u, BrickShape<4>::threads, 0, s>>>(c, pred, cellPairs, list, meta, errorWord);
-        return;
-    }
     if (algorithm == 1) {
-        build_friends_warp_kernel<<<blocks_for(c.n, block), block, 0, s>>>(c, b, pred, cellPairs, list, meta, errorWord);
+        build_friends_scan_kernel<<<blocks_for(c.n, block), block, 0, s>>>(c, b, pred, cellPairs, rows, meta, errorWord);
         return;
     }
-    // one block per tile: the tile loop of a persistent grid costs this kernel
-    // spilled registers in its candidate loop, and the grid gains nothing
-    auto k = narrow ? build_friends_kernel<2, true> : build_friends_kernel<2, false>;
-    k<<<blocks_for(c.n, block), block, 0, s>>>(c, b, pred, cellPairs, list, meta, errorWord);
+    constexpr int threads = 32 * kFriendWarps;
+    build_friends_kernel<<<blocks_for(c.n, threads), threads, 0, s>>>(c, b, pred, cellPairs, rows, meta, errorWord);
 }
 
-namespace {
-// The kept circles' friends as rows, in order, from the circle rows, when no
-// density pass records them (zero solver iterations).
-__global__ void flatten_friends_kernel(int n, int perCircle, const uint32_t* __restrict__ list,
-                                       const uint2* __restrict__ meta, uint4* __restrict__ rows) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint64_t mt = load_meta(meta, i);
-    walk_pairs_recording(list, rows, n, i, FriendRows(mt, kept_density(mt), perCircle), [](uint32_t) { return 0; },
-                         [](int, int, bool, bool) {});
-}
-}  // namespace
-
-void launch_flatten_friends(const DevConsts& c, const uint32_t* list, const uint2* meta, uint4* rows, cudaStream_t s) {
-    flatten_friends_kernel<<<blocks_for(c.n), kBlock, 0, s>>>(c.n, c.perCircle, list, meta, rows);
-}
-
-// The first density pass of a substep records the rows from the circle rows
-// (rowsOut); the other passes walk them (rowsIn).
 void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* predPacked, float* density,
-                            const uint32_t* list, const uint2* meta, const uint4* rowsIn, uint4* rowsOut,
-                            int block, int balance, int* tileCounter, cudaStream_t s) {
-    const bool record = rowsOut != nullptr;
-    auto pick = [record](auto rec, auto walk) { return record ? rec : walk; };
-    auto k = c.relaxed ? (balance ? pick(compute_scaling_kernel<true, true, true>, compute_scaling_kernel<true, true, false>)
-                                  : pick(compute_scaling_kernel<true, false, true>, compute_scaling_kernel<true, false, false>))
-                       : (balance ? pick(compute_scaling_kernel<false, true, true>, compute_scaling_kernel<false, true, false>)
-                                  : pick(compute_scaling_kernel<false, false, true>, compute_scaling_kernel<false, false, false>));
+                            const uint2* meta, const uint4* rows, int block, int balance, int* tileCounter,
+                            cudaStream_t s) {
+    auto k = c.relaxed ? (balance ? compute_scaling_kernel<true, true> : compute_scaling_kernel<true, false>)
+                       : (balance ? compute_scaling_kernel<false, true> : compute_scaling_kernel<false, false>);
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
-    k<<<grid, block, 0, s>>>(c, pred, predPacked, density, list, meta, rowsIn, rowsOut, tiles, tileCounter);
+    k<<<grid, block, 0, s>>>(c, pred, predPacked, density, meta, rows, tiles, tileCounter);
 }
 
 void launch_compute_delta(const DevConsts& c, Batch b, const float4* predPacked, const float4* posPrev,
