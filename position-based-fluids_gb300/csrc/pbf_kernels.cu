@@ -324,9 +324,12 @@ __device__ __forceinline__ float max_nan(float a, float b) {
 // instructions, the tests 160 and the sorting 170.  Against the scan below, which
 // has to run twice to write the rows: faster from one particle to a cell on
 // (500,000 particles: 0.21 against 0.25 ms there, 0.17 against 0.46 at four), 13 %
-// slower at one particle to two cells.  Runs whose candidates do not fit are taken
-// member by member; a member with more than kMostFriends accepted candidates and
-// runs with coordinates that are not finite take the scan.
+// slower at one particle to two cells.  A run whose candidates do not fit is split
+// across the longest side of its box; a member that alone has too many, and runs
+// with coordinates that are not finite, take the scan.
+// 384 candidates leave room for 7 blocks per SM: 320 is 2 % faster on the scene
+// above and 10 % slower where 560 candidates are common (262,144 particles in two
+// colliding columns: 0.300 against 0.273 ms), 448 is 5 % slower on the former.
 constexpr int kFriendWarps = 4, kCandidates = 384, kMostFriends = 128;
 struct FriendShared {
     float x[kCandidates], y[kCandidates], z[kCandidates];
@@ -381,6 +384,42 @@ __device__ __forceinline__ uint64_t sort_friends(const DevConsts& c, const Frien
     return (uint64_t)lo | ((uint64_t)hi << 32);
 }
 
+// The same for a particle with more than kMostFriends accepted candidates: the
+// shared candidates are walked twice, to count the circles and to put each
+// friend in its place.
+__device__ __noinline__ uint64_t sort_many_friends(const DevConsts& c, const FriendShared& sh, int lane, uint32_t ltMask,
+                                                   uint32_t kept, float px, float py, float pz, int ip,
+                                                   uint4* __restrict__ rows) {
+    constexpr unsigned kFull = 0xFFFFFFFFu;
+    const uint32_t limit = (uint32_t)c.perCircle * 0x01010101u;
+    uint32_t lo = 0, hi = 0;  // counts of circles 0-3 and 4-7, a byte each, at most perCircle
+    int total = 0;
+    for (int pass = 0; pass < 2; ++pass) {
+        const uint64_t all = (uint64_t)lo | ((uint64_t)hi << 32);
+        for (int k = 0; k < 8; ++k) total += (int)byte_of(all, k);
+        lo = hi = 0;
+        for (uint32_t k = 0; k < kept; k += 32) {
+            const uint32_t e = k + (uint32_t)lane;
+            const float rx = px - sh.x[e], ry = py - sh.y[e], rz = pz - sh.z[e];
+            const float r2 = dot3(rx, ry, rz, rx, ry, rz);
+            const uint32_t j = sh.j[e];
+            const bool valid = e < kept && !(r2 >= c.h2) && (int)j != ip;
+            const uint32_t circ = valid ? (uint32_t)circle_of(c, r2) : 8u;
+            const uint32_t peers = __match_any_sync(kFull, circ);
+            const int rank = __popc(peers & ltMask) + (int)(__byte_perm(lo, hi, circ & 7u) & 0xFFu);
+            if (pass == 1 && valid && rank < c.perCircle) {
+                int first = 0;
+                for (int q = 0; q < (int)circ; ++q) first += (int)byte_of(all, q);
+                if (density_keeps(c, first, total)) put_friend(rows, c.n, ip, first + rank, j);
+            }
+            const uint32_t one = valid ? 1u << (8u * (circ & 3u)) : 0u, one0 = circ < 4u ? one : 0u;
+            lo = __vminu4(lo + __reduce_add_sync(kFull, one0), limit);
+            hi = __vminu4(hi + __reduce_add_sync(kFull, one - one0), limit);
+        }
+    }
+    return (uint64_t)lo | ((uint64_t)hi << 32);
+}
+
 __global__ void __launch_bounds__(32 * kFriendWarps)
 build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, const uint2* __restrict__ cells,
                      uint4* __restrict__ rows, uint2* __restrict__ meta, int* __restrict__ err) {
@@ -408,11 +447,19 @@ build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, cons
     const float inf = __int_as_float(0x7F800000);
     uint32_t scan = 0;   // lanes whose particles take the scan
     uint64_t counts = 0; // this lane's particle: its circles' counts
-    while (heads) {
-        const int h0 = __ffs(heads) - 1;
-        heads &= heads - 1;
-        const uint32_t upTo = heads ? (heads & (0u - heads)) - 1u : kFull;
-        const uint32_t runMask = validMask & upTo & ~((1u << h0) - 1u);
+    uint32_t now = 0, later = 0;  // the parts of a split run: the one to do next, and the rest
+    while (heads | now | later) {
+        uint32_t runMask = now;
+        if (now == 0 && later == 0) {
+            const uint32_t first = heads & (0u - heads);
+            heads ^= first;
+            runMask = validMask & (heads ? (heads & (0u - heads)) - 1u : kFull) & ~(first - 1u);
+        } else if (now == 0) {
+            runMask = later;
+            later = 0;
+        }
+        now = 0;
+        const int h0 = __ffs(runMask) - 1;
         const bool member = (runMask >> lane) & 1u;
         const float lx = warp_min(member ? pi.x : inf), ly = warp_min(member ? pi.y : inf), lz = warp_min(member ? pi.z : inf);
         const float hx = warp_max(member ? pi.x : -inf), hy = warp_max(member ? pi.y : -inf), hz = warp_max(member ? pi.z : -inf);
@@ -473,9 +520,13 @@ build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, cons
             }
             kept += (uint32_t)__popc(km);
         }
-        if (kept > (uint32_t)kCandidates) {
-            if (runMask & (runMask - 1u)) heads |= runMask;  // one member at a time
-            else scan |= runMask;
+        if (kept > (uint32_t)kCandidates) {  // the members on one side of the box's middle first, across its longest side
+            const float ex = hx - lx, ey = hy - ly, ez = hz - lz;
+            const bool low = ex >= ey && ex >= ez ? pi.x < lx + 0.5f * ex : ey >= ez ? pi.y < ly + 0.5f * ey : pi.z < lz + 0.5f * ez;
+            uint32_t part = __ballot_sync(kFull, member && low);
+            if (part == 0u || part == runMask) part = runMask & (0u - runMask);
+            if (part == runMask) scan |= runMask;  // a single member
+            else { now = part; later |= runMask & ~part; }
             continue;
         }
         for (uint32_t e = kept + (uint32_t)lane; e < ((kept + 63u) & ~63u); e += 32) {  // up to a step of 64: out of reach
@@ -506,7 +557,7 @@ build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, cons
             else if (cnt <= 64) mine = sort_friends<2>(c, sh, lane, ltMask, cnt, ip, rows);
             else if (cnt <= 96) mine = sort_friends<3>(c, sh, lane, ltMask, cnt, ip, rows);
             else if (cnt <= kMostFriends) mine = sort_friends<4>(c, sh, lane, ltMask, cnt, ip, rows);
-            else scan |= 1u << pl;
+            else mine = sort_many_friends(c, sh, lane, ltMask, kept, unpack2(px).x, unpack2(py).x, unpack2(pz).x, ip, rows);
             if (lane == pl) counts = mine;
             __syncwarp();  // the list is read before the next member's is written
         }
