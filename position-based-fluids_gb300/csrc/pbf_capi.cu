@@ -4,7 +4,7 @@
 //
 // Buffer roles within one substep (N particles; index in brackets):
 //   predict      pos[P] vel[V]            -> pred[0], keys[0], perm[0]
-//   sort         keys/perm ping-pong      -> keys[k], perm[k]
+//   sort         keys/perm ping-pong      -> keys[k], perm[k] (or by counting, with the cells' first indices)
 //   gather       pos[P] pred[0]           -> pos[P^1], pred[1]   (sortParticles)
 //   cells        keys[k]                  -> cells
 //   friends      pred[1] cells            -> rows, meta; cells reset
@@ -53,6 +53,9 @@ struct pbf_ctx {
     uint32_t* taint = nullptr;          // per particle: the substep that tainted it (pbf::DevConsts::taint)
     int4* cellXYZ = nullptr;            // per particle: its cell at the friends build and the scene's first key
     uint32_t* cellStart = nullptr;      // per cell key: its first particle (pbf::DevConsts::cellStart)
+    uint32_t* cellCounts = nullptr;     // counting sort: per cell key its particles, zero between substeps
+    uint32_t* scanSums = nullptr;       // counting sort: the scan's block sums
+    pbf::CountingPlan counting;         // blocks == 0: the radix sort
     int* errWord = nullptr;
     int* tileCounters = nullptr;  // 2 words per neighbour kernel: its persistent grid's tile counter
     size_t histWords = 0;
@@ -481,6 +484,9 @@ __global__ void pack_density_kernel(int n, float4* pred, const float* density) {
 }
 
 
+// The keys / perm buffers that hold an unpaused substep's sorted order.
+int sorted_index(const pbf_ctx* ctx) { return ctx->counting.blocks > 0 ? 1 : ctx->plan.passes & 1; }
+
 // Enqueue one Simulation::Step on the context's stream; with a tape, also
 // copy out what the reverse pass needs.
 int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tape = nullptr) {
@@ -509,17 +515,33 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
     const pbf::LaunchShape& ls = ctx->shape;
     // persistent grids: each neighbour kernel's pair of tile-counter words
     auto tiles = [&](int kernel) { return ls.persistent ? ctx->tileCounters + 2 * kernel : nullptr; };
-    pbf::launch_predict_keys(c, b, ctx->pos[P], ctx->vel[V], ctx->pred[0], ctx->keys[0], ctx->perm[0], paused, s);
+    // a paused substep keeps the last sort's keys, and takes its cells from them
+    const bool counting = ctx->counting.blocks > 0 && !paused;
+    uint32_t* order = reinterpret_cast<uint32_t*>(ctx->vel[V ^ 1]);  // free until XSPH
+    pbf::launch_predict_keys(c, b, ctx->pos[P], ctx->vel[V], ctx->pred[0], ctx->keys[0], ctx->perm[0],
+                             counting ? ctx->cellCounts : nullptr, paused, s);
     ++launched;
     int sortedPos = P, sortedPred = 0;
     if (!paused) {
         mark("radixsort");
-        ctx->keysIdx = pbf::launch_radix_sort(ctx->plan, ctx->keys, ctx->perm, ctx->hist, nullptr, nullptr, nullptr,
-                                              nullptr, s);
-        launched += pbf::radix_sort_launches(ctx->plan);
+        if (counting) {
+            pbf::launch_counting_sort(ctx->counting, c.n, ctx->cellCounts, ctx->scanSums, ctx->cellStart, ctx->keys[0],
+                                      ctx->perm[0], order, ctx->errWord, s);
+            launched += 3;
+        } else {
+            ctx->keysIdx = pbf::launch_radix_sort(ctx->plan, ctx->keys, ctx->perm, ctx->hist, nullptr, nullptr, nullptr,
+                                                  nullptr, s);
+            launched += pbf::radix_sort_launches(ctx->plan);
+        }
         mark("sortParticles");
-        pbf::launch_gather_sorted(c.n, ctx->perm[ctx->keysIdx], ctx->pos[P], ctx->pred[0], ctx->ids, ctx->pos[P ^ 1],
-                                  ctx->pred[1], ctx->idsTmp, ctx->errWord, s);
+        if (counting) {
+            ctx->keysIdx = 1;
+            pbf::launch_cell_gather(c.n, ctx->keys[0], ctx->cellStart, order, ctx->keys[1], ctx->perm[1], ctx->pos[P],
+                                    ctx->pred[0], ctx->ids, ctx->pos[P ^ 1], ctx->pred[1], ctx->idsTmp, ctx->errWord, s);
+        } else {
+            pbf::launch_gather_sorted(c.n, ctx->perm[ctx->keysIdx], ctx->pos[P], ctx->pred[0], ctx->ids, ctx->pos[P ^ 1],
+                                      ctx->pred[1], ctx->idsTmp, ctx->errWord, s);
+        }
         ++launched;
         sortedPos = P ^ 1;
         sortedPred = 1;
@@ -535,13 +557,19 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
     mark("updateCells");
     const uint32_t tableKeys = ctx->cellsWords * (uint32_t)(is_batch(ctx) ? ctx->sceneParams.size() : 1);
     c.keys = keys;  // the taint of irregular positions finds a cell's particles in them
-    pbf::launch_update_cells(c.n, keys, ctx->cells, tableKeys, ctx->errWord, s, ctx->cellStart);
+    if (!counting) {
+        pbf::launch_update_cells(c.n, keys, ctx->cells, tableKeys, ctx->errWord, s, ctx->cellStart);
+        ++launched;
+    }
     mark("buildFriendsList");
-    pbf::launch_build_friends(c, b, ctx->pred[sortedPred], ctx->cells, rows, meta, ctx->errWord, ls.friends,
-                              ls.friendsAlgorithm, s);
+    pbf::launch_build_friends(c, b, ctx->pred[sortedPred], ctx->cells, counting ? ctx->cellStart : nullptr, rows, meta,
+                              ctx->errWord, ls.friends, ls.friendsAlgorithm, s);
+    ++launched;
     mark("resetPartList");
-    pbf::launch_reset_cells(c.n, keys, ctx->cells, tableKeys, ctx->errWord, s);
-    launched += 3;
+    if (!counting) {
+        pbf::launch_reset_cells(c.n, keys, ctx->cells, tableKeys, ctx->errWord, s);
+        ++launched;
+    }
     int a = sortedPred;
     const unsigned iters = ctx->params.simIterations;
     for (unsigned it = 0; it < iters; ++it) {
@@ -817,7 +845,7 @@ int run_segment_graph(pbf_ctx* ctx, int len, pbf::AdjointBuffers& ab) {
     // substep keeps the position role and ends with the sorted keys and
     // predictions in their second buffers
     if (len > 0) {
-        ctx->keysIdx = ctx->plan.passes & 1;
+        ctx->keysIdx = sorted_index(ctx);
         ctx->curPred = 1;
     }
     return PBF_OK;
@@ -904,6 +932,7 @@ int pbf_destroy(pbf_ctx* ctx) {
     dev_free(ctx->omega); dev_free(ctx->density); dev_free(ctx->hist); dev_free(ctx->cells);
     dev_free(ctx->rows); dev_free(ctx->meta); dev_free(ctx->errWord); dev_free(ctx->tileCounters);
     dev_free(ctx->taint); dev_free(ctx->cellXYZ); dev_free(ctx->cellStart);
+    dev_free(ctx->cellCounts); dev_free(ctx->scanSums);
     dev_free(ctx->scenes); dev_free(ctx->sceneOf); dev_free(ctx->ids); dev_free(ctx->idsTmp);
     dev_free(ctx->quadsDev); dev_free(ctx->maskDev); dev_free(ctx->waveDev);
     if (ctx->timingAnchor) cudaEventDestroy(ctx->timingAnchor);
@@ -994,14 +1023,23 @@ int pbf_init_cells(pbf_ctx* ctx) {
     const size_t tableWords = (size_t)p.gridBufSize * (is_batch(ctx) ? ctx->sceneParams.size() : 1);
     if ((rc = dev_alloc(ctx, &ctx->cells, 2 * tableWords))) return rc;
     PBF_CUDA(ctx, cudaMemset(ctx->cells, 0xFF, 8 * tableWords));
+    const pbf::CountingPlan counting = pbf::make_counting_plan(ctx->n, tableWords);
+    ctx->counting = pbf::CountingPlan{};
     ctx->cellsWords = p.gridBufSize;
     ctx->listSlots = (int)(p.friendsCircles * p.particlesPerCircle);
     ctx->cellsN = ctx->n;
     ++ctx->epoch;
     if ((rc = dev_alloc(ctx, &ctx->rows, pbf::row_entries(ctx->listSlots) * ctx->n)) || (rc = dev_alloc(ctx, &ctx->meta, ctx->n)) ||
         (rc = dev_alloc(ctx, &ctx->taint, ctx->n)) || (rc = dev_alloc(ctx, &ctx->cellXYZ, ctx->n)) ||
-        (rc = dev_alloc(ctx, &ctx->cellStart, tableWords)))
+        (rc = dev_alloc(ctx, &ctx->cellStart, std::max(tableWords, counting.words))))
         return rc;
+    dev_free(ctx->cellCounts);
+    if (counting.blocks > 0) {
+        if ((rc = dev_alloc(ctx, &ctx->cellCounts, counting.words)) || (rc = dev_alloc(ctx, &ctx->scanSums, counting.blocks)))
+            return rc;
+        PBF_CUDA(ctx, cudaMemset(ctx->cellCounts, 0, 4 * counting.words));
+    }
+    ctx->counting = counting;
     PBF_CUDA(ctx, cudaMemset(ctx->meta, 0, 8 * (size_t)ctx->n));
     // taint marks are substep numbers from 1 on (the counter restarts with them); no cell start yet
     PBF_CUDA(ctx, cudaMemset(ctx->taint, 0, 4 * (size_t)ctx->n));
@@ -1319,7 +1357,7 @@ int pbf_step_async(pbf_ctx* ctx, int substeps) {
                 if ((rc = capture_graph(ctx, false))) return rc;
             PBF_CUDA(ctx, cudaGraphLaunch(ctx->graph.exec, ctx->stream));
             // the replayed substep has the captured buffer roles
-            ctx->keysIdx = ctx->plan.passes & 1;
+            ctx->keysIdx = sorted_index(ctx);
             ctx->curPred = 1;
             ctx->launches += ctx->graph.kernels;
         } else {
@@ -1360,7 +1398,7 @@ int pbf_step_read_async(pbf_ctx* ctx, int substeps, float* pos, float* vel) {
             if (e != cudaSuccess) rc = fail(ctx, PBF_ERR_CUDA, std::string("graph launch: ") + cudaGetErrorString(e));
         }
         if (rc == PBF_OK) {  // the replayed substep has the captured buffer roles, as in pbf_step_async
-            ctx->keysIdx = ctx->plan.passes & 1;
+            ctx->keysIdx = sorted_index(ctx);
             ctx->curPred = 1;
             ctx->launches += g.kernels;
         }

@@ -104,8 +104,11 @@ struct LaunchShape {
 constexpr int kMaxBlock = 512;
 
 // ---- kernels (pbf_kernels.cu) ----
+// counts (may be NULL): the number of particles of each key is added up there,
+// and perm receives each particle's place of arrival among them instead of its
+// own index.
 void launch_predict_keys(const DevConsts& c, Batch b, const float4* pos, float4* vel, float4* pred,
-                         uint32_t* keys, uint32_t* perm, int paused, cudaStream_t s);
+                         uint32_t* keys, uint32_t* perm, uint32_t* counts, int paused, cudaStream_t s);
 void launch_compute_keys(const DevConsts& c, Batch b, const float4* pred, uint32_t* keys, uint32_t* perm,
                          cudaStream_t s);
 // err (may be NULL): the error word that bounds-checked builds report bad
@@ -121,8 +124,11 @@ void launch_reset_cells(int n, const uint32_t* keys, uint32_t* cells, uint32_t k
 // blocks take the tiles from it (LaunchShape::persistent).
 // Writes the rows (walk_pairs in pbf_device.cuh) and meta.  algorithm:
 // LaunchShape::friendsAlgorithm; block is the scan's.
-void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const uint32_t* cells, uint4* rows,
-                          uint2* meta, int* errorWord, int block, int algorithm, cudaStream_t s);
+// The cells come as ranges (launch_update_cells) or, where starts is given, as
+// the first index of every key and one beyond the last.
+void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const uint32_t* cells,
+                          const uint32_t* starts, uint4* rows, uint2* meta, int* errorWord, int block, int algorithm,
+                          cudaStream_t s);
 // uint4 entries per particle of the rows for `slots` friends.
 inline size_t row_entries(int slots) { return ((size_t)slots + 3) / 4; }
 void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* predPacked, float* density,
@@ -165,6 +171,29 @@ int launch_radix_sort(const SortPlan& plan, uint32_t* keys[2], uint32_t* perm[2]
                       cudaStream_t s);
 // Kernels launched by one launch_radix_sort call.
 int radix_sort_launches(const SortPlan& plan);
+
+// ---- counting sort (pbf_sort.cu) ----
+// Taken by a substep whose keys are at most kCountingRatio times its particles
+// (or at most kCountingSmall), so that the scan over the key range (12 bytes a
+// key: 35 us for 2^24 keys at the measured copy rate) stays below the radix
+// passes that it replaces (65 us at 1M particles and three passes); the radix
+// sort above takes the others.
+constexpr uint64_t kCountingSmall = 1u << 20, kCountingRatio = 16;
+struct CountingPlan {
+    uint32_t blocks = 0;          // of the scan; 0: the radix sort
+    uint32_t chunks = 0, chunksPerBlock = 0;
+    size_t words = 0;             // counters, and first indices, as allocated
+};
+CountingPlan make_counting_plan(int n, uint64_t keys);
+// From the counts and the particles' places of arrival (launch_predict_keys):
+// the first index of every key into `starts`, and the particles grouped by key,
+// in any order within a key, into `order`.  Zeroes the counts.
+void launch_counting_sort(const CountingPlan& plan, int n, uint32_t* counts, uint32_t* sums, uint32_t* starts,
+                          const uint32_t* keys, const uint32_t* place, uint32_t* order, int* err, cudaStream_t s);
+// The stable order from it, with the records gathered (launch_gather_sorted).
+void launch_cell_gather(int n, const uint32_t* keys, const uint32_t* starts, const uint32_t* order, uint32_t* keysOut,
+                        uint32_t* permOut, const float4* pos, const float4* pred, const uint32_t* ids, float4* posOut,
+                        float4* predOut, uint32_t* idsOut, int* err, cudaStream_t s);
 
 // ---- adjoint (pbf_adjoint.cu) ----
 // What one substep of a rollout leaves for its reverse pass.

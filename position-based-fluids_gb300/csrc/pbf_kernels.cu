@@ -46,8 +46,9 @@ __device__ __forceinline__ uint32_t key_base(const Batch& b, int i) {
 // predict_positions.cl:8-17 fused with computeKeys (radixsort.cl:7-19).
 __global__ void predict_keys_kernel(DevConsts c, Batch b, const float4* __restrict__ pos, float4* __restrict__ vel,
                                     float4* __restrict__ pred, uint32_t* __restrict__ keys,
-                                    uint32_t* __restrict__ perm, int paused) {
+                                    uint32_t* __restrict__ perm, uint32_t* __restrict__ counts, int paused) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned valid = __ballot_sync(0xFFFFFFFFu, i < c.n);
     if (i >= c.n) return;
     float4 v = vel[i];
     float gx = c.gx, gy = c.gy, gz = c.gz;
@@ -68,8 +69,18 @@ __global__ void predict_keys_kernel(DevConsts c, Batch b, const float4* __restri
     pred[i] = q;
     if (i == 0) *c.epoch += 1u;  // a new substep: earlier taint marks lapse
     if (!paused) {
-        keys[i] = base + grid_hash(__float2int_rz(q.x / c.h), __float2int_rz(q.y / c.h), __float2int_rz(q.z / c.h), c.grid);
-        perm[i] = (uint32_t)i;
+        const uint32_t key = base + grid_hash(__float2int_rz(q.x / c.h), __float2int_rz(q.y / c.h), __float2int_rz(q.z / c.h), c.grid);
+        keys[i] = key;
+        if (!counts) {
+            perm[i] = (uint32_t)i;
+            return;
+        }
+        // the particles come nearly sorted, a few keys to a warp: one atomic per key and warp
+        const unsigned peers = __match_any_sync(valid, key);
+        const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
+        uint32_t place = 0;
+        if (lane == leader) place = atomicAdd(&counts[key], (uint32_t)__popc(peers));
+        perm[i] = __shfl_sync(valid, place, leader) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
     }
 }
 
@@ -166,6 +177,31 @@ __device__ __forceinline__ uint2 make_meta(const DevConsts& c, uint64_t cnt, int
     return make_uint2((uint32_t)mt, (uint32_t)(mt >> 32));
 }
 
+// The particles of a cell, from either form of the cell table (CellTable).
+struct CellTable {
+    const uint2* ranges;     // first and last particle, kEmpty for none (update_cells.cl)
+    const uint32_t* starts;  // or the first particle of every key, and one beyond the last
+};
+__device__ __forceinline__ void cell_range(const CellTable& cells, uint32_t key, int n, int* __restrict__ err,
+                                           uint32_t& first, uint32_t& count) {
+    uint32_t last;
+    count = 0;
+    if (cells.starts) {
+        first = cells.starts[key];
+        last = cells.starts[key + 1];  // one beyond
+        if (first == last) return;
+        --last;
+    } else {
+        const uint2 range = cells.ranges[key];
+        first = range.x;
+        last = range.y;
+        if (first == kEmpty) return;
+    }
+    last = min(last, (uint32_t)(n - 1));
+    if (first > last) atomicOr(err, kErrCellTable);
+    else count = last - first + 1u;
+}
+
 // Friend `pos` of particle i in the rows.
 __device__ __forceinline__ void put_friend(uint4* __restrict__ rows, int n, int i, int pos, uint32_t j) {
     char* entry = reinterpret_cast<char*>(rows + i) + (uint64_t)((uint32_t)pos >> 2) * (16u * (uint32_t)n);
@@ -199,7 +235,7 @@ __device__ __forceinline__ int circle_of(const DevConsts& c, float r2) {
 // are formed from the three spread coordinates of each axis.
 template <typename F>
 __device__ __forceinline__ void scan_neighbours(const DevConsts& c, uint32_t base, const float4* __restrict__ pred,
-                                                const uint2* __restrict__ cells, int* __restrict__ err, int i,
+                                                const CellTable& cells, int* __restrict__ err, int i,
                                                 const float4 pi, int cx, int cy, int cz, F consider) {
     const int n = c.n;
     const bool pow2 = (c.grid & (c.grid - 1)) == 0;
@@ -229,16 +265,16 @@ __device__ __forceinline__ void scan_neighbours(const DevConsts& c, uint32_t bas
             for (int z = -1; z <= 1; ++z) {
                 const uint32_t m = exy | (z < 0 ? ezm : (z > 0 ? ezp : ez0));
                 const uint32_t hm = pow2 ? (m & mask) : (m % c.grid);
-                const uint2 range = cells[base + hm];
-                if (range.x == kEmpty) continue;
-                const uint32_t last = min(range.y, (uint32_t)(n - 1));
-                if (range.x > last) { atomicOr(err, kErrCellTable); continue; }
-                if (hm == selfHash && range.x <= (uint32_t)i && (uint32_t)i <= last) {
+                uint32_t first, count;
+                cell_range(cells, base + hm, n, err, first, count);
+                if (count == 0u) continue;
+                const uint32_t last = first + count - 1u;
+                if (hm == selfHash && first <= (uint32_t)i && (uint32_t)i <= last) {
                     // the particle's own table entry: skip itself (build_friends_list.cl:62)
-                    if ((uint32_t)i > range.x) scan(range.x, (uint32_t)i - 1);
+                    if ((uint32_t)i > first) scan(first, (uint32_t)i - 1);
                     if ((uint32_t)i < last) scan((uint32_t)i + 1, last);
                 } else {
-                    scan(range.x, last);
+                    scan(first, last);
                 }
             }
         }
@@ -249,7 +285,7 @@ __device__ __forceinline__ void scan_neighbours(const DevConsts& c, uint32_t bas
 // each friend is put in its place in a second.  Circle counts saturate at
 // perCircle (later candidates are dropped, build_friends_list.cl:79-83).
 __device__ __noinline__ void friends_of_one(const DevConsts& c, uint32_t base, const float4* __restrict__ pred,
-                                            const uint2* __restrict__ cells, uint4* __restrict__ rows,
+                                            const CellTable& cells, uint4* __restrict__ rows,
                                             uint2* __restrict__ meta, int* __restrict__ err, int i, const float4 pi,
                                             int cx, int cy, int cz) {
     uint64_t cnt = 0;  // 8 circles x 8-bit counters
@@ -274,7 +310,7 @@ __device__ __noinline__ void friends_of_one(const DevConsts& c, uint32_t base, c
 }
 
 __global__ void __launch_bounds__(kMaxBlock)
-build_friends_scan_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, const uint2* __restrict__ cells,
+build_friends_scan_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, CellTable cells,
                           uint4* __restrict__ rows, uint2* __restrict__ meta, int* __restrict__ err) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
@@ -421,7 +457,7 @@ __device__ __noinline__ uint64_t sort_many_friends(const DevConsts& c, const Fri
 }
 
 __global__ void __launch_bounds__(32 * kFriendWarps)
-build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, const uint2* __restrict__ cells,
+build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, CellTable cells,
                      uint4* __restrict__ rows, uint2* __restrict__ meta, int* __restrict__ err) {
     constexpr unsigned kFull = 0xFFFFFFFFu;
     __shared__ FriendShared shared[kFriendWarps];
@@ -475,12 +511,7 @@ build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, cons
         if (lane < 27) {
             const int x = lane / 9 - 1, y = (lane / 3) % 3 - 1, z = lane % 3 - 1;
             const uint32_t m = expand_bits(rx0 + x) | (expand_bits(ry0 + y) << 1) | (expand_bits(rz0 + z) << 2);
-            const uint2 range = cells[rbase + (pow2 ? (m & gmask) : (m % c.grid))];
-            if (range.x != kEmpty) {
-                const uint32_t last = min(range.y, (uint32_t)(n - 1));
-                if (range.x > last) atomicOr(err, kErrCellTable);
-                else { start = range.x; count = last - range.x + 1u; }
-            }
+            cell_range(cells, rbase + (pow2 ? (m & gmask) : (m % c.grid)), n, err, start, count);
         }
         uint32_t end = count;  // inclusive scan: candidates up to and including cell q
 #pragma unroll
@@ -1119,8 +1150,8 @@ apply_vorticity_kernel(DevConsts c, const float4* __restrict__ pred, const float
 
 // ------------------------------------------------------------- launchers --
 void launch_predict_keys(const DevConsts& c, Batch b, const float4* pos, float4* vel, float4* pred, uint32_t* keys,
-                         uint32_t* perm, int paused, cudaStream_t s) {
-    predict_keys_kernel<<<blocks_for(c.n), kBlock, 0, s>>>(c, b, pos, vel, pred, keys, perm, paused);
+                         uint32_t* perm, uint32_t* counts, int paused, cudaStream_t s) {
+    predict_keys_kernel<<<blocks_for(c.n), kBlock, 0, s>>>(c, b, pos, vel, pred, keys, perm, counts, paused);
 }
 
 void launch_compute_keys(const DevConsts& c, Batch b, const float4* pred, uint32_t* keys, uint32_t* perm,
@@ -1169,15 +1200,16 @@ unsigned grid_for_tiles(K kernel, int n, int block, bool persistent, int* tiles)
     return cap;
 }
 
-void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const uint32_t* cells, uint4* rows,
-                          uint2* meta, int* errorWord, int block, int algorithm, cudaStream_t s) {
-    const uint2* cellPairs = reinterpret_cast<const uint2*>(cells);
+void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const uint32_t* cells,
+                          const uint32_t* starts, uint4* rows, uint2* meta, int* errorWord, int block, int algorithm,
+                          cudaStream_t s) {
+    const CellTable table{reinterpret_cast<const uint2*>(cells), starts};
     if (algorithm == 1) {
-        build_friends_scan_kernel<<<blocks_for(c.n, block), block, 0, s>>>(c, b, pred, cellPairs, rows, meta, errorWord);
+        build_friends_scan_kernel<<<blocks_for(c.n, block), block, 0, s>>>(c, b, pred, table, rows, meta, errorWord);
         return;
     }
     constexpr int threads = 32 * kFriendWarps;
-    build_friends_kernel<<<blocks_for(c.n, threads), threads, 0, s>>>(c, b, pred, cellPairs, rows, meta, errorWord);
+    build_friends_kernel<<<blocks_for(c.n, threads), threads, 0, s>>>(c, b, pred, table, rows, meta, errorWord);
 }
 
 void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* predPacked, float* density,

@@ -18,10 +18,19 @@
 // smaller sorts still spread over the SMs (at 2^20 keys, 512 tiles sort
 // 12 % faster than 256).  Each warp owns consecutive keys taken round by
 // round, so (warp, round, lane) order is input order.
+//
+// A substep whose key range is not much larger than its particle count sorts
+// by counting instead (counting_scan_*, cell_scatter, cell_gather): predict
+// counts each key's particles and keeps each particle's place of arrival among
+// them, one scan over the key range turns the counts into first indices (which
+// are the cell table as well), and the particles of a cell, few and in any
+// order after the scatter, are put in input order by counting the smaller
+// indices among them.
 
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "pbf_device.cuh"
 #include "pbf_internal.h"
 
 namespace pbf {
@@ -158,7 +167,138 @@ radix_downsweep_kernel(const uint32_t* __restrict__ keysIn, const uint32_t* __re
     }
 }
 
+// ---- counting sort ----
+constexpr int kScanChunk = 4 * kThreads;  // counters a block takes at a time
+
+// Sum of each block's tile of counters.
+__global__ void __launch_bounds__(kThreads)
+counting_sums_kernel(const uint4* __restrict__ counts, uint32_t chunks, uint32_t chunksPerBlock,
+                     uint32_t* __restrict__ sums) {
+    __shared__ uint32_t warpSums[kWarps];
+    const uint32_t first = blockIdx.x * chunksPerBlock, last = min(first + chunksPerBlock, chunks);
+    uint32_t sum = 0;
+    for (uint32_t k = first; k < last; ++k) {
+        const uint4 v = counts[(size_t)k * kThreads + threadIdx.x];
+        sum += (v.x + v.y) + (v.z + v.w);
+    }
+    sum = __reduce_add_sync(0xFFFFFFFFu, sum);
+    if ((threadIdx.x & 31) == 0) warpSums[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t all = 0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) all += warpSums[w];
+        sums[blockIdx.x] = all;
+    }
+}
+
+// starts[k] = number of particles with a smaller key than k, for every key and
+// one beyond the last; the counters are left at zero for the next substep.
+// Every block adds up the sums of the blocks before it (at most kMaxScanBlocks
+// of them), so no block waits for another.
+constexpr uint32_t kMaxScanBlocks = 1024;
+__global__ void __launch_bounds__(kThreads)
+counting_scan_kernel(uint4* __restrict__ counts, uint32_t chunks, uint32_t chunksPerBlock,
+                     const uint32_t* __restrict__ sums, uint4* __restrict__ starts) {
+    __shared__ uint32_t warpSums[kWarps];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    uint32_t before = 0;
+    for (uint32_t b = t; b < blockIdx.x; b += kThreads) before += sums[b];
+    before = __reduce_add_sync(0xFFFFFFFFu, before);
+    if (lane == 0) warpSums[warp] = before;
+    __syncthreads();
+    uint32_t carry = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) carry += warpSums[w];
+    const uint32_t first = blockIdx.x * chunksPerBlock, last = min(first + chunksPerBlock, chunks);
+    for (uint32_t k = first; k < last; ++k) {
+        const size_t at = (size_t)k * kThreads + t;
+        const uint4 v = counts[at];
+        counts[at] = make_uint4(0u, 0u, 0u, 0u);
+        const uint32_t sum = (v.x + v.y) + (v.z + v.w);
+        uint32_t incl = sum;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+            if (lane >= d) incl += u;
+        }
+        __syncthreads();  // warpSums is read by all before it is written again
+        if (lane == 31) warpSums[warp] = incl;
+        __syncthreads();
+        uint32_t base = carry, all = 0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            const uint32_t ws = warpSums[w];
+            base += w < warp ? ws : 0u;
+            all += ws;
+        }
+        base += incl - sum;
+        starts[at] = make_uint4(base, base + v.x, base + v.x + v.y, base + v.x + v.y + v.z);
+        carry += all;
+    }
+}
+
+// order[first index of the key + place of arrival] = particle
+__global__ void __launch_bounds__(kThreads)
+cell_scatter_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ place,
+                    const uint32_t* __restrict__ starts, uint32_t* __restrict__ order, int* __restrict__ err) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) order[checked_index(starts[keys[i]] + place[i], (uint32_t)n, err, kErrSortIndex)] = (uint32_t)i;
+}
+
+// The particle in slot s of the scattered order goes to its cell's first index
+// plus the number of smaller indices in the cell: the stable order.  With it go
+// its key, index, position, prediction and id (radixsort.cl:22-37; velocities
+// are not permuted, they are recomputed before any read, update_velocities.cl:13).
+__global__ void __launch_bounds__(kThreads)
+cell_gather_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ starts,
+                   const uint32_t* __restrict__ order, uint32_t* __restrict__ keysOut, uint32_t* __restrict__ permOut,
+                   const float4* __restrict__ pos, const float4* __restrict__ pred, const uint32_t* __restrict__ ids,
+                   float4* __restrict__ posOut, float4* __restrict__ predOut, uint32_t* __restrict__ idsOut,
+                   int* __restrict__ err) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    const uint32_t i = checked_index(order[s], (uint32_t)n, err, kErrSortIndex);
+    const float4 x = pos[i], p = pred[i];
+    const uint32_t id = ids[i], key = keys[i];
+    const uint32_t first = starts[key], end = starts[key + 1];
+    uint32_t to = first;
+    for (uint32_t q = first; q < end; ++q) to += order[q] < i;
+    to = checked_index(to, (uint32_t)n, err, kErrSortIndex);
+    keysOut[to] = key;
+    permOut[to] = i;
+    posOut[to] = x;
+    predOut[to] = p;
+    idsOut[to] = id;
+}
+
 }  // namespace
+
+CountingPlan make_counting_plan(int n, uint64_t keys) {
+    CountingPlan p;
+    if (keys > kCountingSmall && keys > kCountingRatio * (uint64_t)n) return p;
+    p.chunks = (uint32_t)((keys + 1 + kScanChunk - 1) / kScanChunk);  // one start beyond the last key
+    p.chunksPerBlock = (p.chunks + kMaxScanBlocks - 1) / kMaxScanBlocks;
+    p.blocks = (p.chunks + p.chunksPerBlock - 1) / p.chunksPerBlock;
+    p.words = (size_t)p.chunks * kScanChunk;
+    return p;
+}
+
+void launch_counting_sort(const CountingPlan& plan, int n, uint32_t* counts, uint32_t* sums, uint32_t* starts,
+                          const uint32_t* keys, const uint32_t* place, uint32_t* order, int* err, cudaStream_t s) {
+    uint4* c4 = reinterpret_cast<uint4*>(counts);
+    counting_sums_kernel<<<plan.blocks, kThreads, 0, s>>>(c4, plan.chunks, plan.chunksPerBlock, sums);
+    counting_scan_kernel<<<plan.blocks, kThreads, 0, s>>>(c4, plan.chunks, plan.chunksPerBlock, sums,
+                                                          reinterpret_cast<uint4*>(starts));
+    cell_scatter_kernel<<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(n, keys, place, starts, order, err);
+}
+
+void launch_cell_gather(int n, const uint32_t* keys, const uint32_t* starts, const uint32_t* order, uint32_t* keysOut,
+                        uint32_t* permOut, const float4* pos, const float4* pred, const uint32_t* ids, float4* posOut,
+                        float4* predOut, uint32_t* idsOut, int* err, cudaStream_t s) {
+    cell_gather_kernel<<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(n, keys, starts, order, keysOut, permOut, pos,
+                                                                          pred, ids, posOut, predOut, idsOut, err);
+}
 
 SortPlan make_sort_plan(int n, uint32_t gridBufSize) {
     SortPlan p;
