@@ -527,7 +527,7 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
         if (counting) {
             pbf::launch_counting_sort(ctx->counting, c.n, ctx->cellCounts, ctx->scanSums, ctx->cellStart, ctx->keys[0],
                                       ctx->perm[0], order, ctx->errWord, s);
-            launched += 3;
+            launched += ctx->counting.blocks > 1 ? 3 : 2;
         } else {
             ctx->keysIdx = pbf::launch_radix_sort(ctx->plan, ctx->keys, ctx->perm, ctx->hist, nullptr, nullptr, nullptr,
                                                   nullptr, s);
@@ -572,12 +572,13 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
     }
     int a = sortedPred;
     const unsigned iters = ctx->params.simIterations;
+    const pbf::StepEnd end{ctx->pos[sortedPos ^ 1], ctx->vel[V], paused ? nullptr : ctx->idsTmp, ctx->ids};
     for (unsigned it = 0; it < iters; ++it) {
         float4* packed = tape ? tape->q[it] : ctx->pred[a ^ 1];
         mark("computeScaling", (int)it);
         pbf::launch_compute_scaling(c, ctx->pred[a], packed, ctx->density, meta, rows, ls.scaling, ls.balance, tiles(1), s);
         mark("computeDelta", (int)it);
-        pbf::launch_compute_delta(c, b, packed, ctx->pos[sortedPos], ctx->pred[a], ctx->density, meta,
+        pbf::launch_compute_delta(c, b, packed, ctx->pos[sortedPos], it + 1 == iters ? end : pbf::StepEnd{}, ctx->pred[a], ctx->density, meta,
                                   it + 1 == iters, tape && tape->mask ? tape->mask + (size_t)it * c.n : nullptr,
                                   rows, ls.delta, ls.balance, tiles(2), s);
         launched += 2;
@@ -589,8 +590,10 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
     }
     if (tape) PBF_CUDA(ctx, cudaMemcpyAsync(tape->pI, ctx->pred[a], v4, cudaMemcpyDeviceToDevice, s));
     mark("updateVelocities");
-    pbf::launch_update_velocities(c, ctx->pred[a], ctx->pos[sortedPos], ctx->pos[sortedPos ^ 1], ctx->vel[V],
-                                  paused ? nullptr : ctx->idsTmp, ctx->ids, s);
+    if (iters == 0) {  // else by the last position pass
+        pbf::launch_update_velocities(c, end, ctx->pred[a], ctx->pos[sortedPos], s);
+        ++launched;
+    }
     if (ctx->readPos) {  // the positions are final: copy them out while XSPH and vorticity run
         PBF_CUDA(ctx, cudaEventRecord(ctx->evPosReady, s));
         PBF_CUDA(ctx, cudaStreamWaitEvent(ctx->copyStream, ctx->evPosReady, 0));
@@ -625,7 +628,7 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
         pbf::launch_apply_vorticity(c, ctx->pred[a], near, omega, ctx->vel[V ^ 1], ctx->vel[V], meta, rows,
                                     ls.vorticity, ls.balance, tiles(4), s);
     }
-    launched += 3;
+    launched += 2;
     if (rangeOpen) nvtxRangePop();
     if (ctx->readVel && !velCopied) PBF_CUDA(ctx, cudaMemcpyAsync(ctx->readVel, ctx->vel[V], v4, cudaMemcpyDeviceToHost, s));
     if (ctx->readPos) PBF_CUDA(ctx, cudaStreamWaitEvent(s, ctx->evCopyDone, 0));  // later work waits for the copy

@@ -134,13 +134,22 @@ inline size_t row_entries(int slots) { return ((size_t)slots + 3) / 4; }
 void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* predPacked, float* density,
                             const uint2* meta, const uint4* rows, int block, int balance, int* tileCounter,
                             cudaStream_t s);
-// posPrev: the sorted positions, read only by the force planes.
+// What the last position pass of a substep also writes: the new positions and
+// velocities, and the particle ids (idsIn NULL: they stay).  posOut NULL: not
+// the last pass.
+struct StepEnd {
+    float4* posOut = nullptr;
+    float4* vel = nullptr;
+    const uint32_t* idsIn = nullptr;
+    uint32_t* idsOut = nullptr;
+};
+// posPrev: the sorted positions, read by the force planes and the step's end.
 void launch_compute_delta(const DevConsts& c, Batch b, const float4* predPacked, const float4* posPrev,
-                          float4* predOut, const float* density, const uint2* meta, int lastIteration,
+                          const StepEnd& end, float4* predOut, const float* density, const uint2* meta, int lastIteration,
                           uint8_t* clampMask, const uint4* rows, int block, int balance, int* tileCounter,
                           cudaStream_t s);
-void launch_update_velocities(const DevConsts& c, const float4* pred, const float4* posIn, float4* posOut,
-                              float4* vel, const uint32_t* idsIn, uint32_t* idsOut, cudaStream_t s);
+void launch_update_velocities(const DevConsts& c, const StepEnd& end, const float4* pred, const float4* posIn,
+                              cudaStream_t s);
 // near: the neighbour records that launch_apply_vorticity reads.
 void launch_apply_viscosity(const DevConsts& c, Batch b, const float4* pred, const float4* velIn, float4* velOut,
                             float4* omega, float4* near, const uint2* meta, const uint4* rows, int block, int balance,

@@ -456,6 +456,9 @@ __device__ __noinline__ uint64_t sort_many_friends(const DevConsts& c, const Fri
     return (uint64_t)lo | ((uint64_t)hi << 32);
 }
 
+// W particles to a warp: 32, or fewer where that leaves the chip without warps
+// (a warp takes its members one after another).
+template <int W>
 __global__ void __launch_bounds__(32 * kFriendWarps)
 build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, CellTable cells,
                      uint4* __restrict__ rows, uint2* __restrict__ meta, int* __restrict__ err) {
@@ -463,11 +466,11 @@ build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, Cell
     __shared__ FriendShared shared[kFriendWarps];
     FriendShared& sh = shared[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int warpBase = i - lane;
+    const int warpBase = (int)(blockIdx.x * kFriendWarps + (threadIdx.x >> 5)) * W;
+    const int i = warpBase + lane;
     const int n = c.n;
     if (warpBase >= n) return;  // whole warp idle
-    const bool valid = i < n;
+    const bool valid = lane < W && i < n;
     const float4 pi = valid ? pred[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const int cx = __float2int_rz(pi.x / c.h), cy = __float2int_rz(pi.y / c.h), cz = __float2int_rz(pi.z / c.h);
     const uint32_t base = valid ? key_base(b, i) : 0u;
@@ -795,14 +798,29 @@ compute_scaling_kernel(DevConsts c, const float4* __restrict__ pred, float4* __r
     });
 }
 
+// update_velocities.cl:11-14 (the GL texture write is dropped) for particle i
+// at its final prediction p, from its position q.  Also moves the sorted
+// particle ids back to their fixed buffer.
+__device__ __forceinline__ void end_of_step(const DevConsts& c, const StepEnd& end, int i, const float4& p, const float4& q) {
+    if (end.idsIn) end.idsOut[i] = end.idsIn[i];
+    float4 v = end.vel[i];
+    v.x = (p.x - q.x) / c.dt;
+    v.y = (p.y - q.y) / c.dt;
+    v.z = (p.z - q.z) / c.dt;
+    end.vel[i] = v;
+    end.posOut[i] = make_float4(p.x, p.y, p.z, sqrtf(dot3(v.x, v.y, v.z, v.x, v.y, v.z)));
+}
+
 // ---------------------------------------------------------------- delta --
 // compute_delta.cl:54-185 (force planes: identity for an all-zero mask) with
 // the optional box clamp on `future`, then update_predicted.cl.  After the
 // last iteration w carries the density (pack_data.cl with the density source,
-// src/Simulation.cpp:591).
+// src/Simulation.cpp:591), and the velocities are updated there as well
+// (end.posOut), which saves a launch and the prediction's way through memory.
 template <bool R, bool Q>
 __device__ __forceinline__ void compute_delta_body(const DevConsts& c, const Batch& b, const float4* __restrict__ pp,
-                                                   const float4* __restrict__ posPrev, float4* __restrict__ predOut,
+                                                   const float4* __restrict__ posPrev, const StepEnd& end,
+                                                   float4* __restrict__ predOut,
                                                    const float* __restrict__ density, int lastIteration,
                                                    uint8_t* __restrict__ clampMask, const uint4* __restrict__ rows,
                                                    int i, const float4 pi, uint64_t mt) {
@@ -904,12 +922,13 @@ __device__ __forceinline__ void compute_delta_body(const DevConsts& c, const Bat
     const float4 out = make_float4(pi.x + dx, pi.y + dy, pi.z + dz, lastIteration ? density[i] : pi.w + 0.0f);
     predOut[i] = out;
     if (!R) note_position(c, i, out.x, out.y, out.z);
+    if (end.posOut) end_of_step(c, end, i, out, posPrev[i]);
 }
 
 template <bool R, bool B>
 __global__ void __launch_bounds__(kMaxBlock)
 compute_delta_kernel(DevConsts c, Batch b, const float4* __restrict__ pp, const float4* __restrict__ posPrev,
-                     float4* __restrict__ predOut, const float* __restrict__ density,
+                     StepEnd end, float4* __restrict__ predOut, const float* __restrict__ density,
                      const uint2* __restrict__ meta, int lastIteration, uint8_t* __restrict__ clampMask,
                      const uint4* __restrict__ rows, int tiles, int* tileCounter) {
     for_tiles(tiles, tileCounter, [&](int tile) {
@@ -918,28 +937,17 @@ compute_delta_kernel(DevConsts c, Batch b, const float4* __restrict__ pp, const 
         const float4 pi = pp[i];
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) compute_delta_body<R, true>(c, b, pp, posPrev, predOut, density, lastIteration, clampMask, rows, i, pi, mt);
-        else compute_delta_body<R, false>(c, b, pp, posPrev, predOut, density, lastIteration, clampMask, rows, i, pi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) compute_delta_body<R, true>(c, b, pp, posPrev, end, predOut, density, lastIteration, clampMask, rows, i, pi, mt);
+        else compute_delta_body<R, false>(c, b, pp, posPrev, end, predOut, density, lastIteration, clampMask, rows, i, pi, mt);
     });
 }
 
 // ----------------------------------------------------------- velocities --
-// update_velocities.cl:11-14 (the GL texture write is dropped).
-// Also moves the sorted particle ids back to their fixed buffer.
-__global__ void update_velocities_kernel(DevConsts c, const float4* __restrict__ pred,
-                                         const float4* __restrict__ posIn, float4* __restrict__ posOut,
-                                         float4* __restrict__ vel, const uint32_t* __restrict__ idsIn,
-                                         uint32_t* __restrict__ idsOut) {
+// The end of a step without solver iterations.
+__global__ void update_velocities_kernel(DevConsts c, StepEnd end, const float4* __restrict__ pred,
+                                         const float4* __restrict__ posIn) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
-    if (idsIn) idsOut[i] = idsIn[i];
-    const float4 p = pred[i], q = posIn[i];
-    float4 v = vel[i];
-    v.x = (p.x - q.x) / c.dt;
-    v.y = (p.y - q.y) / c.dt;
-    v.z = (p.z - q.z) / c.dt;
-    vel[i] = v;
-    posOut[i] = make_float4(p.x, p.y, p.z, sqrtf(dot3(v.x, v.y, v.z, v.x, v.y, v.z)));
+    if (i < c.n) end_of_step(c, end, i, pred[i], posIn[i]);
 }
 
 // apply_viscosity.cl:12-86, every neighbour read from the pre-pass
@@ -1208,8 +1216,11 @@ void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const
         build_friends_scan_kernel<<<blocks_for(c.n, block), block, 0, s>>>(c, b, pred, table, rows, meta, errorWord);
         return;
     }
-    constexpr int threads = 32 * kFriendWarps;
-    build_friends_kernel<<<blocks_for(c.n, threads), threads, 0, s>>>(c, b, pred, table, rows, meta, errorWord);
+    // friends of 2,048 / 16,384 / 65,536 / 131,072 / 262,144 particles, us: 13 / 20 / 45 / 81 / 152 with 4 to a
+    // warp, 17 / 23 / 38 / 65 / 120 with 8, 22 / 32 / 38 / 58 / 105 with 16, 34 / 41 / 47 / 63 / 104 with 32
+    const int w = c.n <= 16384 ? 4 : c.n <= 49152 ? 8 : c.n <= 196608 ? 16 : 32;
+    auto k = w == 4 ? build_friends_kernel<4> : w == 8 ? build_friends_kernel<8> : w == 16 ? build_friends_kernel<16> : build_friends_kernel<32>;
+    k<<<blocks_for(c.n, w * kFriendWarps), 32 * kFriendWarps, 0, s>>>(c, b, pred, table, rows, meta, errorWord);
 }
 
 void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* predPacked, float* density,
@@ -1223,20 +1234,20 @@ void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* pred
 }
 
 void launch_compute_delta(const DevConsts& c, Batch b, const float4* predPacked, const float4* posPrev,
-                          float4* predOut, const float* density, const uint2* meta, int lastIteration,
+                          const StepEnd& end, float4* predOut, const float* density, const uint2* meta, int lastIteration,
                           uint8_t* clampMask, const uint4* rows, int block, int balance, int* tileCounter,
                           cudaStream_t s) {
     auto k = c.relaxed ? (balance ? compute_delta_kernel<true, true> : compute_delta_kernel<true, false>)
                        : (balance ? compute_delta_kernel<false, true> : compute_delta_kernel<false, false>);
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
-    k<<<grid, block, 0, s>>>(c, b, predPacked, posPrev, predOut, density, meta, lastIteration, clampMask, rows, tiles,
+    k<<<grid, block, 0, s>>>(c, b, predPacked, posPrev, end, predOut, density, meta, lastIteration, clampMask, rows, tiles,
                              tileCounter);
 }
 
-void launch_update_velocities(const DevConsts& c, const float4* pred, const float4* posIn, float4* posOut,
-                              float4* vel, const uint32_t* idsIn, uint32_t* idsOut, cudaStream_t s) {
-    update_velocities_kernel<<<blocks_for(c.n), kBlock, 0, s>>>(c, pred, posIn, posOut, vel, idsIn, idsOut);
+void launch_update_velocities(const DevConsts& c, const StepEnd& end, const float4* pred, const float4* posIn,
+                              cudaStream_t s) {
+    update_velocities_kernel<<<blocks_for(c.n), kBlock, 0, s>>>(c, end, pred, posIn);
 }
 
 void launch_apply_viscosity(const DevConsts& c, Batch b, const float4* pred, const float4* velIn, float4* velOut,

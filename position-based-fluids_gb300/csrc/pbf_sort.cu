@@ -196,7 +196,7 @@ counting_sums_kernel(const uint4* __restrict__ counts, uint32_t chunks, uint32_t
 // one beyond the last; the counters are left at zero for the next substep.
 // Every block adds up the sums of the blocks before it (at most kMaxScanBlocks
 // of them), so no block waits for another.
-constexpr uint32_t kMaxScanBlocks = 1024;
+constexpr uint32_t kMaxScanBlocks = 1024, kOneBlockChunks = 16;
 __global__ void __launch_bounds__(kThreads)
 counting_scan_kernel(uint4* __restrict__ counts, uint32_t chunks, uint32_t chunksPerBlock,
                      const uint32_t* __restrict__ sums, uint4* __restrict__ starts) {
@@ -278,7 +278,8 @@ CountingPlan make_counting_plan(int n, uint64_t keys) {
     CountingPlan p;
     if (keys > kCountingSmall && keys > kCountingRatio * (uint64_t)n) return p;
     p.chunks = (uint32_t)((keys + 1 + kScanChunk - 1) / kScanChunk);  // one start beyond the last key
-    p.chunksPerBlock = (p.chunks + kMaxScanBlocks - 1) / kMaxScanBlocks;
+    // a key range of a few chunks is scanned by one block, which needs no sums of others before it
+    p.chunksPerBlock = p.chunks <= kOneBlockChunks ? p.chunks : (p.chunks + kMaxScanBlocks - 1) / kMaxScanBlocks;
     p.blocks = (p.chunks + p.chunksPerBlock - 1) / p.chunksPerBlock;
     p.words = (size_t)p.chunks * kScanChunk;
     return p;
@@ -287,7 +288,9 @@ CountingPlan make_counting_plan(int n, uint64_t keys) {
 void launch_counting_sort(const CountingPlan& plan, int n, uint32_t* counts, uint32_t* sums, uint32_t* starts,
                           const uint32_t* keys, const uint32_t* place, uint32_t* order, int* err, cudaStream_t s) {
     uint4* c4 = reinterpret_cast<uint4*>(counts);
-    counting_sums_kernel<<<plan.blocks, kThreads, 0, s>>>(c4, plan.chunks, plan.chunksPerBlock, sums);
+    if (plan.blocks > 1)
+        counting_sums_kernel<<<plan.blocks, kThreads, 0, s>>>(c4, plan.chunks, plan.chunksPerBlock,
+                                                                      sums);
     counting_scan_kernel<<<plan.blocks, kThreads, 0, s>>>(c4, plan.chunks, plan.chunksPerBlock, sums,
                                                           reinterpret_cast<uint4*>(starts));
     cell_scatter_kernel<<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(n, keys, place, starts, order, err);
