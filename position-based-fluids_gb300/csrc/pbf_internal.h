@@ -103,6 +103,23 @@ struct LaunchShape {
 };
 constexpr int kMaxBlock = 512;
 
+// Launches a kernel of the substep's chain: it may start before the kernel
+// before it on the stream has ended, and waits for that one's end itself
+// (chain_wait in pbf_device.cuh) before it touches memory.
+template <typename... P, typename... A>
+inline void launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t s, A&&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ---- kernels (pbf_kernels.cu) ----
 // counts (may be NULL): the number of particles of each key is added up there,
 // and perm receives each particle's place of arrival among them instead of its

@@ -47,6 +47,7 @@ __device__ __forceinline__ uint32_t key_base(const Batch& b, int i) {
 __global__ void predict_keys_kernel(DevConsts c, Batch b, const float4* __restrict__ pos, float4* __restrict__ vel,
                                     float4* __restrict__ pred, uint32_t* __restrict__ keys,
                                     uint32_t* __restrict__ perm, uint32_t* __restrict__ counts, int paused) {
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned valid = __ballot_sync(0xFFFFFFFFu, i < c.n);
     if (i >= c.n) return;
@@ -102,6 +103,7 @@ __global__ void gather_sorted_kernel(int n, const uint32_t* __restrict__ perm, c
                                      const float4* __restrict__ pred, const uint32_t* __restrict__ ids,
                                      float4* __restrict__ posOut, float4* __restrict__ predOut,
                                      uint32_t* __restrict__ idsOut, int* err) {
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t j = checked_index(perm[i], (uint32_t)n, err, kErrSortIndex);
@@ -312,6 +314,7 @@ __device__ __noinline__ void friends_of_one(const DevConsts& c, uint32_t base, c
 __global__ void __launch_bounds__(kMaxBlock)
 build_friends_scan_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, CellTable cells,
                           uint4* __restrict__ rows, uint2* __restrict__ meta, int* __restrict__ err) {
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
     const float4 pi = pred[i];
@@ -462,6 +465,7 @@ template <int W>
 __global__ void __launch_bounds__(32 * kFriendWarps)
 build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, CellTable cells,
                      uint4* __restrict__ rows, uint2* __restrict__ meta, int* __restrict__ err) {
+    chain_wait();
     constexpr unsigned kFull = 0xFFFFFFFFu;
     __shared__ FriendShared shared[kFriendWarps];
     FriendShared& sh = shared[threadIdx.x >> 5];
@@ -787,6 +791,7 @@ __global__ void __launch_bounds__(kMaxBlock)
 compute_scaling_kernel(DevConsts c, const float4* __restrict__ pred, float4* __restrict__ predPacked,
                        float* __restrict__ density, const uint2* __restrict__ meta, const uint4* __restrict__ rows,
                        int tiles, int* tileCounter) {
+    chain_wait();
     for_tiles(tiles, tileCounter, [&](int tile) {
         const int i = B ? balanced_particle(meta, c.n, true, tile) : tile * (int)blockDim.x + (int)threadIdx.x;
         if (i < 0 || i >= c.n) return;
@@ -931,6 +936,7 @@ compute_delta_kernel(DevConsts c, Batch b, const float4* __restrict__ pp, const 
                      StepEnd end, float4* __restrict__ predOut, const float* __restrict__ density,
                      const uint2* __restrict__ meta, int lastIteration, uint8_t* __restrict__ clampMask,
                      const uint4* __restrict__ rows, int tiles, int* tileCounter) {
+    chain_wait();
     for_tiles(tiles, tileCounter, [&](int tile) {
         const int i = B ? balanced_particle(meta, c.n, false, tile) : tile * (int)blockDim.x + (int)threadIdx.x;
         if (i < 0 || i >= c.n) return;
@@ -1049,6 +1055,7 @@ __global__ void __launch_bounds__(kMaxBlock)
 apply_viscosity_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, const float4* __restrict__ velIn,
                        float4* __restrict__ velOut, float4* __restrict__ omega, float4* __restrict__ near,
                        const uint2* __restrict__ meta, const uint4* __restrict__ rows, int tiles, int* tileCounter) {
+    chain_wait();
     for_tiles(tiles, tileCounter, [&](int tile) {
         const int i = B ? balanced_particle(meta, c.n, false, tile) : tile * (int)blockDim.x + (int)threadIdx.x;
         if (i < 0 || i >= c.n) return;
@@ -1142,6 +1149,7 @@ __global__ void __launch_bounds__(kMaxBlock)
 apply_vorticity_kernel(DevConsts c, const float4* __restrict__ pred, const float4* __restrict__ near,
                        const float4* __restrict__ omega, const float4* __restrict__ velIn, float4* __restrict__ velOut, const uint2* __restrict__ meta,
                        const uint4* __restrict__ rows, int tiles, int* tileCounter, int tileOffset) {
+    chain_wait();
     for_tiles(tiles, tileCounter, [&](int tile) {
         tile += tileOffset;  // a launch over part of the tiles (one block per tile)
         const int i = B ? balanced_particle(meta, c.n, false, tile) : tile * (int)blockDim.x + (int)threadIdx.x;
@@ -1159,7 +1167,7 @@ apply_vorticity_kernel(DevConsts c, const float4* __restrict__ pred, const float
 // ------------------------------------------------------------- launchers --
 void launch_predict_keys(const DevConsts& c, Batch b, const float4* pos, float4* vel, float4* pred, uint32_t* keys,
                          uint32_t* perm, uint32_t* counts, int paused, cudaStream_t s) {
-    predict_keys_kernel<<<blocks_for(c.n), kBlock, 0, s>>>(c, b, pos, vel, pred, keys, perm, counts, paused);
+    launch_chained(predict_keys_kernel, blocks_for(c.n), kBlock, s, c, b, pos, vel, pred, keys, perm, counts, paused);
 }
 
 void launch_compute_keys(const DevConsts& c, Batch b, const float4* pred, uint32_t* keys, uint32_t* perm,
@@ -1169,7 +1177,7 @@ void launch_compute_keys(const DevConsts& c, Batch b, const float4* pred, uint32
 
 void launch_gather_sorted(int n, const uint32_t* perm, const float4* pos, const float4* pred, const uint32_t* ids,
                           float4* posOut, float4* predOut, uint32_t* idsOut, int* err, cudaStream_t s) {
-    gather_sorted_kernel<<<blocks_for(n), kBlock, 0, s>>>(n, perm, pos, pred, ids, posOut, predOut, idsOut, err);
+    launch_chained(gather_sorted_kernel, blocks_for(n), kBlock, s, n, perm, pos, pred, ids, posOut, predOut, idsOut, err);
 }
 
 void launch_update_cells(int n, const uint32_t* keys, uint32_t* cells, uint32_t keyLimit, int* err, cudaStream_t s,
@@ -1213,14 +1221,14 @@ void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const
                           cudaStream_t s) {
     const CellTable table{reinterpret_cast<const uint2*>(cells), starts};
     if (algorithm == 1) {
-        build_friends_scan_kernel<<<blocks_for(c.n, block), block, 0, s>>>(c, b, pred, table, rows, meta, errorWord);
+        launch_chained(build_friends_scan_kernel, blocks_for(c.n, block), block, s, c, b, pred, table, rows, meta, errorWord);
         return;
     }
     // friends of 2,048 / 16,384 / 65,536 / 131,072 / 262,144 particles, us: 13 / 20 / 45 / 81 / 152 with 4 to a
     // warp, 17 / 23 / 38 / 65 / 120 with 8, 22 / 32 / 38 / 58 / 105 with 16, 34 / 41 / 47 / 63 / 104 with 32
     const int w = c.n <= 16384 ? 4 : c.n <= 49152 ? 8 : c.n <= 196608 ? 16 : 32;
     auto k = w == 4 ? build_friends_kernel<4> : w == 8 ? build_friends_kernel<8> : w == 16 ? build_friends_kernel<16> : build_friends_kernel<32>;
-    k<<<blocks_for(c.n, w * kFriendWarps), 32 * kFriendWarps, 0, s>>>(c, b, pred, table, rows, meta, errorWord);
+    launch_chained(k, blocks_for(c.n, w * kFriendWarps), 32 * kFriendWarps, s, c, b, pred, table, rows, meta, errorWord);
 }
 
 void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* predPacked, float* density,
@@ -1230,7 +1238,7 @@ void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* pred
                        : (balance ? compute_scaling_kernel<false, true> : compute_scaling_kernel<false, false>);
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
-    k<<<grid, block, 0, s>>>(c, pred, predPacked, density, meta, rows, tiles, tileCounter);
+    launch_chained(k, grid, block, s, c, pred, predPacked, density, meta, rows, tiles, tileCounter);
 }
 
 void launch_compute_delta(const DevConsts& c, Batch b, const float4* predPacked, const float4* posPrev,
@@ -1241,7 +1249,7 @@ void launch_compute_delta(const DevConsts& c, Batch b, const float4* predPacked,
                        : (balance ? compute_delta_kernel<false, true> : compute_delta_kernel<false, false>);
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
-    k<<<grid, block, 0, s>>>(c, b, predPacked, posPrev, end, predOut, density, meta, lastIteration, clampMask, rows, tiles,
+    launch_chained(k, grid, block, s, c, b, predPacked, posPrev, end, predOut, density, meta, lastIteration, clampMask, rows, tiles,
                              tileCounter);
 }
 
@@ -1257,7 +1265,7 @@ void launch_apply_viscosity(const DevConsts& c, Batch b, const float4* pred, con
                        : (balance ? apply_viscosity_kernel<false, true> : apply_viscosity_kernel<false, false>);
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
-    k<<<grid, block, 0, s>>>(c, b, pred, velIn, velOut, omega, near, meta, rows, tiles, tileCounter);
+    launch_chained(k, grid, block, s, c, b, pred, velIn, velOut, omega, near, meta, rows, tiles, tileCounter);
 }
 
 void launch_apply_vorticity(const DevConsts& c, const float4* pred, const float4* near, const float4* omega,
@@ -1266,12 +1274,12 @@ void launch_apply_vorticity(const DevConsts& c, const float4* pred, const float4
     auto k = c.relaxed ? (balance ? apply_vorticity_kernel<true, true> : apply_vorticity_kernel<true, false>)
                        : (balance ? apply_vorticity_kernel<false, true> : apply_vorticity_kernel<false, false>);
     if (tileCount > 0) {  // tiles [firstTile, firstTile + tileCount), one block each
-        k<<<(unsigned)tileCount, block, 0, s>>>(c, pred, near, omega, velIn, velOut, meta, rows, 0, nullptr, firstTile);
+        launch_chained(k, (unsigned)tileCount, block, s, c, pred, near, omega, velIn, velOut, meta, rows, 0, nullptr, firstTile);
         return;
     }
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
-    k<<<grid, block, 0, s>>>(c, pred, near, omega, velIn, velOut, meta, rows, tiles, tileCounter, 0);
+    launch_chained(k, grid, block, s, c, pred, near, omega, velIn, velOut, meta, rows, tiles, tileCounter, 0);
 }
 
 }  // namespace pbf

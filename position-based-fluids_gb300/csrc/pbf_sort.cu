@@ -174,6 +174,7 @@ constexpr int kScanChunk = 4 * kThreads;  // counters a block takes at a time
 __global__ void __launch_bounds__(kThreads)
 counting_sums_kernel(const uint4* __restrict__ counts, uint32_t chunks, uint32_t chunksPerBlock,
                      uint32_t* __restrict__ sums) {
+    chain_wait();
     __shared__ uint32_t warpSums[kWarps];
     const uint32_t first = blockIdx.x * chunksPerBlock, last = min(first + chunksPerBlock, chunks);
     uint32_t sum = 0;
@@ -200,6 +201,7 @@ constexpr uint32_t kMaxScanBlocks = 1024, kOneBlockChunks = 16;
 __global__ void __launch_bounds__(kThreads)
 counting_scan_kernel(uint4* __restrict__ counts, uint32_t chunks, uint32_t chunksPerBlock,
                      const uint32_t* __restrict__ sums, uint4* __restrict__ starts) {
+    chain_wait();
     __shared__ uint32_t warpSums[kWarps];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     uint32_t before = 0;
@@ -242,6 +244,7 @@ counting_scan_kernel(uint4* __restrict__ counts, uint32_t chunks, uint32_t chunk
 __global__ void __launch_bounds__(kThreads)
 cell_scatter_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ place,
                     const uint32_t* __restrict__ starts, uint32_t* __restrict__ order, int* __restrict__ err) {
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) order[checked_index(starts[keys[i]] + place[i], (uint32_t)n, err, kErrSortIndex)] = (uint32_t)i;
 }
@@ -256,6 +259,7 @@ cell_gather_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __r
                    const float4* __restrict__ pos, const float4* __restrict__ pred, const uint32_t* __restrict__ ids,
                    float4* __restrict__ posOut, float4* __restrict__ predOut, uint32_t* __restrict__ idsOut,
                    int* __restrict__ err) {
+    chain_wait();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const uint32_t i = checked_index(order[s], (uint32_t)n, err, kErrSortIndex);
@@ -289,17 +293,17 @@ void launch_counting_sort(const CountingPlan& plan, int n, uint32_t* counts, uin
                           const uint32_t* keys, const uint32_t* place, uint32_t* order, int* err, cudaStream_t s) {
     uint4* c4 = reinterpret_cast<uint4*>(counts);
     if (plan.blocks > 1)
-        counting_sums_kernel<<<plan.blocks, kThreads, 0, s>>>(c4, plan.chunks, plan.chunksPerBlock,
+        launch_chained(counting_sums_kernel, plan.blocks, kThreads, s, c4, plan.chunks, plan.chunksPerBlock,
                                                                       sums);
-    counting_scan_kernel<<<plan.blocks, kThreads, 0, s>>>(c4, plan.chunks, plan.chunksPerBlock, sums,
+    launch_chained(counting_scan_kernel, plan.blocks, kThreads, s, c4, plan.chunks, plan.chunksPerBlock, sums,
                                                           reinterpret_cast<uint4*>(starts));
-    cell_scatter_kernel<<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(n, keys, place, starts, order, err);
+    launch_chained(cell_scatter_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keys, place, starts, order, err);
 }
 
 void launch_cell_gather(int n, const uint32_t* keys, const uint32_t* starts, const uint32_t* order, uint32_t* keysOut,
                         uint32_t* permOut, const float4* pos, const float4* pred, const uint32_t* ids, float4* posOut,
                         float4* predOut, uint32_t* idsOut, int* err, cudaStream_t s) {
-    cell_gather_kernel<<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(n, keys, starts, order, keysOut, permOut, pos,
+    launch_chained(cell_gather_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keys, starts, order, keysOut, permOut, pos,
                                                                           pred, ids, posOut, predOut, idsOut, err);
 }
 
