@@ -12,8 +12,8 @@
 //   omega_i = -G sum (v2_j - v2_i) x k,  eta_i = -G sum |omega_j| k,
 //   v4 = v3 + dt eps_v (eta/|eta|) x omega_i.
 // Each kernel below walks the same friends as its forward kernel (the rows
-// the substep recorded, walk_friends) and scatters neighbour terms with atomics, so the sums are not ordered: these
-// are FP32 gradients, not bit-reproducible ones.  The derivation is the same
+// the substep recorded) and scatters neighbour terms with atomics, so the sums
+// are not ordered: these are FP32 gradients, not bit-reproducible ones.  The derivation is the same
 // as the FP64 adjoint the tests compare against.
 
 #include <cuda_runtime.h>
@@ -38,10 +38,10 @@ __device__ __forceinline__ float dot(F3 a, F3 b) { return a.x * b.x + a.y * b.y 
 __device__ __forceinline__ F3 cross(F3 a, F3 b) { return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x}; }
 __device__ __forceinline__ float len(F3 a) { return sqrtf(dot(a, a)); }
 
-__device__ __forceinline__ void add3(float4* a, F3 v) { atomicAdd(a, make_float4(v.x, v.y, v.z, 0.0f)); }
+__device__ __forceinline__ void add3(float4* a, F3 v, float w = 0.0f) { atomicAdd(a, make_float4(v.x, v.y, v.z, w)); }
 
-// A friend's records as the walks below load them, four friends in flight
-// (walk_friends): its index and one or two float4 records.
+// A friend's records as the walks below load them: its index and one or two
+// float4 records.
 struct Friend1 {
     uint32_t j;
     float4 a;
@@ -50,6 +50,34 @@ struct Friend2 {
     uint32_t j;
     float4 a, b;
 };
+
+// Four lanes share a particle: lane `sub` takes the friends sub, sub + 4, ...,
+// one word of each row entry, two in flight.  The sums are not ordered here, and
+// at 65,536 particles one thread per particle leaves 13 warps on an SM, each
+// waiting for its own loads (reverse pass of 20 substeps: 6.3 ms with one lane,
+// 5.8 with four).
+constexpr int kSplit = 4;
+template <typename LoadF, typename BodyF>
+__device__ __forceinline__ void walk_split(const uint4* __restrict__ rows, int n, int i, int total, int sub, LoadF load,
+                                           BodyF body) {
+    const uint32_t* p = reinterpret_cast<const uint32_t*>(rows + i) + sub;
+    const size_t stride = 4 * (size_t)n;
+    int t = sub;
+    for (; t + kSplit < total; t += 2 * kSplit, p += 2 * stride) {
+        const uint32_t j0 = __ldg(p), j1 = __ldg(p + stride);
+        const auto f0 = load(j0), f1 = load(j1);
+        body(f0);
+        body(f1);
+    }
+    if (t < total) body(load(__ldg(p)));
+}
+// The sum over a particle's lanes, in all of them.
+__device__ __forceinline__ float lanes_sum(float v) {
+    v += __shfl_xor_sync(0xFFFFFFFFu, v, 1);
+    v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
+    return v;
+}
+__device__ __forceinline__ F3 lanes_sum(F3 v) { return {lanes_sum(v.x), lanes_sum(v.y), lanes_sum(v.z)}; }
 
 // k(r) and the adjoint of its argument: d/dr [k . kb] = f kb + f'(|r|)(kb.r) r/|r|
 // with f = (h-|r|)^2/|r|, f' = -(h-|r|)(h+|r|)/|r|^2.  y is 1/|r| within an
@@ -86,43 +114,39 @@ template <typename T> __device__ __forceinline__ T block_sum(T v) {
     return s;
 }
 
+// The kernels leave the accumulators they are done with at zero for the next
+// use (each particle's own element, where only that particle reads it), so that
+// a substep starts with omb, v2b, pb and pbt zero and clears nothing.
+
 // v4 = v3 + dt*vort*(N x omega_i): adjoints of omega (omb) and of p^I (pb).
 __global__ void __launch_bounds__(kAdjBlock)
 adj_vorticity_kernel(DevConsts c, const float4* __restrict__ pI, const float4* __restrict__ omega,
-                     const uint4* __restrict__ rows, const uint2* __restrict__ meta,
+                     const float4* __restrict__ etas, const uint4* __restrict__ rows, const uint2* __restrict__ meta,
                      const float4* __restrict__ vb, float4* __restrict__ omb, float4* __restrict__ pb) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    chain_wait();
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / kSplit, sub = threadIdx.x % kSplit;
     const int n = c.n;
-    if (i >= n) return;
-    const uint64_t mt = load_meta(meta, i);
-    const F3 pi = f3(pI[i]);
+    const bool valid = i < n;
+    const F3 pi = valid ? f3(pI[i]) : F3{0.0f, 0.0f, 0.0f}, eta = valid ? f3(etas[i]) : F3{0.0f, 0.0f, 0.0f};
     const float G = c.gradSpiky;
-    F3 eta = {0.0f, 0.0f, 0.0f};
-    FlatFriends f1(mt, kept_other(mt));
     auto loadPO = [&](uint32_t j) {
         j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex);
         return Friend2{j, pI[j], omega[j]};
     };
-    walk_friends(rows, n, i, f1.total, loadPO, [&](const Friend2& f) {
-        const F3 r = pi - f3(f.a);
-        const float r2 = dot(r, r);
-        if (!xsph_pair(c, r2, f.a.w)) return;
-        float y;
-        const float rl = pair_length(r2, y);
-        eta = eta + len(f3(f.b)) * kvec(r, rl, y, c.h);
-    });
-    eta = -G * eta;
     const float l = len(eta);
-    if (!(l > 0.0f)) return;
-    const F3 N = (1.0f / l) * eta;
-    const F3 ub = (c.vort * c.dt) * f3(vb[i]);
-    const F3 oi = f3(omega[i]);
-    const F3 Nb = cross(oi, ub);
-    add3(&omb[i], cross(ub, N));
-    const F3 etab = (1.0f / l) * (Nb - dot(N, Nb) * N);
-    FlatFriends f2(mt, kept_other(mt));
+    const bool turns = valid && l > 0.0f;
+    F3 etab = {0.0f, 0.0f, 0.0f};
+    if (turns) {
+        const F3 N = (1.0f / l) * eta;
+        const F3 ub = (c.vort * c.dt) * f3(vb[i]);
+        const F3 oi = f3(omega[i]);
+        const F3 Nb = cross(oi, ub);
+        if (sub == 0) add3(&omb[i], cross(ub, N));
+        etab = (1.0f / l) * (Nb - dot(N, Nb) * N);
+    }
     F3 pbi = {0.0f, 0.0f, 0.0f};  // particle i's own terms, added once
-    walk_friends(rows, n, i, f2.total, loadPO, [&](const Friend2& f) {
+    const uint64_t mt = turns ? load_meta(meta, i) : 0u;
+    walk_split(rows, n, i, FlatFriends(mt, kept_other(mt)).total, sub, loadPO, [&](const Friend2& f) {
         const F3 r = pi - f3(f.a);
         const float r2 = dot(r, r);
         if (!xsph_pair(c, r2, f.a.w)) return;
@@ -136,30 +160,33 @@ adj_vorticity_kernel(DevConsts c, const float4* __restrict__ pI, const float4* _
         pbi = pbi + rb;
         add3(&pb[f.j], -1.0f * rb);
     });
-    add3(&pb[i], pbi);
+    pbi = lanes_sum(pbi);
+    if (turns && sub == 0) add3(&pb[i], pbi);
 }
 
 // v3 = v2 + c POLY6 sum (v2_j - v2_i) W and omega = -G sum (v2_j - v2_i) x k:
 // adjoints of v2 (v2b), p^I (pb) and of the XSPH factor (cbar).
 __global__ void __launch_bounds__(kAdjBlock)
 adj_viscosity_kernel(DevConsts c, const float4* __restrict__ pI, const float4* __restrict__ v2,
-                     const float4* __restrict__ omb, const float4* __restrict__ vb, const uint4* __restrict__ rows,
+                     float4* __restrict__ omb, const float4* __restrict__ vb, const uint4* __restrict__ rows,
                      const uint2* __restrict__ meta, float4* __restrict__ v2b, float4* __restrict__ pb,
                      float* __restrict__ cbar) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    chain_wait();
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / kSplit, sub = threadIdx.x % kSplit;
     const int n = c.n;
+    const bool valid = i < n;
     float cacc = 0.0f;
-    if (i < n) {
+    F3 v2bi = {0.0f, 0.0f, 0.0f}, pbi = {0.0f, 0.0f, 0.0f};  // particle i's own terms, added once
+    if (valid) {
         const uint64_t mt = load_meta(meta, i);
         const F3 pi = f3(pI[i]), v3b = f3(vb[i]), ob = f3(omb[i]), vi = f3(v2[i]);
         const float G = c.gradSpiky;
-        F3 v2bi = v3b, pbi = {0.0f, 0.0f, 0.0f};  // particle i's own terms, added once
-        FlatFriends fr(mt, kept_other(mt));
+        if (sub == 0) v2bi = v3b;
         auto loadPV = [&](uint32_t j) {
             j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex);
             return Friend2{j, pI[j], v2[j]};
         };
-        walk_friends(rows, n, i, fr.total, loadPV, [&](const Friend2& f) {
+        walk_split(rows, n, i, FlatFriends(mt, kept_other(mt)).total, sub, loadPV, [&](const Friend2& f) {
             const uint32_t j = f.j;
             const F3 r = pi - f3(f.a);
             const float r2 = dot(r, r);
@@ -179,113 +206,114 @@ adj_viscosity_kernel(DevConsts c, const float4* __restrict__ pI, const float4* _
             pbi = pbi + rb;
             add3(&pb[j], -1.0f * rb);
         });
+    }
+    v2bi = lanes_sum(v2bi);
+    pbi = lanes_sum(pbi);  // every lane has read omb[i] before this
+    if (valid && sub == 0) {
         add3(&v2b[i], v2bi);
         add3(&pb[i], pbi);
+        omb[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
     const float s = block_sum(cacc);
     if (threadIdx.x == 0 && s != 0.0f) atomicAdd(cbar, s);
 }
 
 // v2 = (p^I - x)/dt and x' = p^I.
-__global__ void adj_velocity_kernel(DevConsts c, const float4* __restrict__ xb, const float4* __restrict__ v2b,
+__global__ void adj_velocity_kernel(DevConsts c, const float4* __restrict__ xb, float4* __restrict__ v2b,
                                     float4* __restrict__ pb, float4* __restrict__ xsb) {
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
     const F3 v = f3(v2b[i]);
+    v2b[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const F3 p = f3(pb[i]) + f3(xb[i]) + (1.0f / c.dt) * v;
     pb[i] = make_float4(p.x, p.y, p.z, 0.0f);
     xsb[i] = make_float4(-v.x / c.dt, -v.y / c.dt, -v.z / c.dt, 0.0f);
 }
 
 // p^{t+1} = clamp(p^t + delta(p^t, lambda^t)): adjoints of p^t (pbt) and
-// lambda^t (lb) from that of p^{t+1} (pbn).  q = (p^t, lambda^t).
+// lambda^t (in pbt's w: one atomic for both) from that of p^{t+1} (pbn).
+// q = (p^t, lambda^t).
 __global__ void __launch_bounds__(kAdjBlock)
 adj_delta_kernel(DevConsts c, const float4* __restrict__ q, const uint8_t* __restrict__ mask,
                  const float4* __restrict__ pbn, const uint4* __restrict__ rows, const uint2* __restrict__ meta,
-                 float4* __restrict__ pbt, float* __restrict__ lb) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+                 float4* __restrict__ pbt) {
+    chain_wait();
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / kSplit, sub = threadIdx.x % kSplit;
     const int n = c.n;
-    if (i >= n) return;
-    F3 fb = f3(pbn[i]);
-    if (mask) {
-        const uint8_t m = mask[i];
-        if (m & 3) fb.x = 0.0f;
-        if (m & 12) fb.y = 0.0f;
-        if (m & 48) fb.z = 0.0f;
-    }
-    F3 pbi = fb;  // particle i's own terms, added once
+    const bool valid = i < n;
+    F3 pbi = {0.0f, 0.0f, 0.0f};  // particle i's own terms, added once
     float lbi = 0.0f;
-    const float4 qi = q[i];
-    const F3 pi = f3(qi);
-    const float a0 = -c.gradSpiky / c.rho0;
-    const uint64_t mt = load_meta(meta, i);
-    FlatFriends fr(mt, kept_other(mt));
-    auto loadQ = [&](uint32_t j) {
-        j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex);
-        return Friend1{j, q[j]};
-    };
-    walk_friends(rows, n, i, fr.total, loadQ, [&](const Friend1& f) {
-        const uint32_t j = f.j;
-        const float4 qj = f.a;
-        const F3 r = pi - f3(qj);
-        const float r2 = dot(r, r);
-        if (!in_support(c, r2)) return;
-        float y;
-        const float rl = pair_length(r2, y);
-        const float d = c.h2 - r2;
-        const float rq = d * d * d / c.poly6q;
-        const float a = qi.w + qj.w + c.K * rq * rq * rq * rq;
-        const F3 k = kvec(r, rl, y, c.h);
-        const float ab = a0 * dot(fb, k);
-        lbi += ab;
-        atomicAdd(&lb[j], ab);
-        const float sW = ab * 4.0f * c.K * rq * rq * rq / c.poly6q;
-        const F3 rb = (sW * -6.0f * d * d) * r + kvec_adj(r, rl, y, c.h, (a0 * a) * fb);
-        pbi = pbi + rb;
-        add3(&pbt[j], -1.0f * rb);
-    });
-    atomicAdd(&lb[i], lbi);
-    add3(&pbt[i], pbi);
+    if (valid) {
+        F3 fb = f3(pbn[i]);
+        if (mask) {
+            const uint8_t m = mask[i];
+            if (m & 3) fb.x = 0.0f;
+            if (m & 12) fb.y = 0.0f;
+            if (m & 48) fb.z = 0.0f;
+        }
+        if (sub == 0) pbi = fb;
+        const float4 qi = q[i];
+        const F3 pi = f3(qi);
+        const float a0 = -c.gradSpiky / c.rho0;
+        const uint64_t mt = load_meta(meta, i);
+        auto loadQ = [&](uint32_t j) {
+            j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex);
+            return Friend1{j, q[j]};
+        };
+        walk_split(rows, n, i, FlatFriends(mt, kept_other(mt)).total, sub, loadQ, [&](const Friend1& f) {
+            const uint32_t j = f.j;
+            const float4 qj = f.a;
+            const F3 r = pi - f3(qj);
+            const float r2 = dot(r, r);
+            if (!in_support(c, r2)) return;
+            float y;
+            const float rl = pair_length(r2, y);
+            const float d = c.h2 - r2;
+            const float rq = d * d * d / c.poly6q;
+            const float a = qi.w + qj.w + c.K * rq * rq * rq * rq;
+            const F3 k = kvec(r, rl, y, c.h);
+            const float ab = a0 * dot(fb, k);
+            lbi += ab;
+            const float sW = ab * 4.0f * c.K * rq * rq * rq / c.poly6q;
+            const F3 rb = (sW * -6.0f * d * d) * r + kvec_adj(r, rl, y, c.h, (a0 * a) * fb);
+            pbi = pbi + rb;
+            add3(&pbt[j], -1.0f * rb, ab);
+        });
+    }
+    lbi = lanes_sum(lbi);
+    pbi = lanes_sum(pbi);
+    if (valid && sub == 0) add3(&pbt[i], pbi, lbi);
 }
 
-// lambda^t from p^t: adjoint of p^t (pbt) from that of lambda^t (lb).
+// lambda^t from p^t: adjoint of p^t (pbt) from that of lambda^t (pbt's w, which
+// nothing changes here).  Clears pbn, which becomes the next iteration's pbt.
+// The sums over the friends are the forward pass' (sums, density).
 __global__ void __launch_bounds__(kAdjBlock)
-adj_scaling_kernel(DevConsts c, const float4* __restrict__ q, const float* __restrict__ lb,
-                   const uint4* __restrict__ rows, const uint2* __restrict__ meta, float4* __restrict__ pbt) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+adj_scaling_kernel(DevConsts c, const float4* __restrict__ q, const float4* __restrict__ sums,
+                   const float* __restrict__ density, const uint4* __restrict__ rows,
+                   const uint2* __restrict__ meta, float4* pbt, float4* __restrict__ pbn) {
+    chain_wait();
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / kSplit, sub = threadIdx.x % kSplit;
     const int n = c.n;
-    if (i >= n) return;
-    const float lbar = lb[i];
-    if (lbar == 0.0f) return;
-    const F3 pi = f3(q[i]);
-    const float G = c.gradSpiky;
-    const uint64_t mt = load_meta(meta, i);
-    float ds = 0.0f, gsk = 0.0f;
-    F3 S = {0.0f, 0.0f, 0.0f};
-    FlatFriends f1(mt, kept_density(mt));
+    const bool valid = i < n;
+    const float lbar = valid ? __ldcg(&pbt[i].w) : 0.0f;
+    const uint64_t mt = lbar != 0.0f ? load_meta(meta, i) : 0u;
+    const int total = FlatFriends(mt, kept_density(mt)).total;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const F3 pi = valid ? f3(q[i]) : f3(zero);
+    const float4 sum = valid ? sums[i] : zero;
+    const float rho = valid ? density[i] : 0.0f, G = c.gradSpiky, D = sum.w;
+    const F3 S = f3(sum);
     auto loadQ = [&](uint32_t j) {
         j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex);
         return Friend1{j, q[j]};
     };
-    walk_friends(rows, n, i, f1.total, loadQ, [&](const Friend1& f) {
-        const F3 r = pi - f3(f.a);
-        const float r2 = dot(r, r);
-        if (!in_support(c, r2)) return;
-        float y;
-        const float rl = pair_length(r2, y);
-        const F3 g = G * kvec(r, rl, y, c.h);
-        const float d = c.h2 - r2;
-        ds += d * d * d;
-        gsk += dot(g, g);
-        S = S + g;
-    });
-    const float rho = ds * c.poly6, D = gsk + dot(S, S);
     const float den = D / c.rho0sq + c.eps, Cc = rho / c.rho0 - 1.0f;
     const float rhob = (-lbar / den) / c.rho0;
     const float Db = lbar * Cc / (den * den) / c.rho0sq;
-    FlatFriends f2(mt, kept_density(mt));
     F3 pbi = {0.0f, 0.0f, 0.0f};  // particle i's own terms, added once
-    walk_friends(rows, n, i, f2.total, loadQ, [&](const Friend1& f) {
+    walk_split(rows, n, i, total, sub, loadQ, [&](const Friend1& f) {
         const uint32_t j = f.j;
         const F3 r = pi - f3(f.a);
         const float r2 = dot(r, r);
@@ -298,20 +326,26 @@ adj_scaling_kernel(DevConsts c, const float4* __restrict__ q, const float* __res
         pbi = pbi + rb;
         add3(&pbt[j], -1.0f * rb);
     });
-    add3(&pbt[i], pbi);
+    pbi = lanes_sum(pbi);
+    if (valid && sub == 0) {
+        if (total > 0) add3(&pbt[i], pbi);
+        pbn[i] = zero;
+    }
 }
 
 // Undo the sort and the prediction p0 = x + dt (v + dt g): adjoints of the
 // substep's inputs x, v (previous order) and of g.
 __global__ void __launch_bounds__(kAdjBlock)
 adj_unsort_predict_kernel(DevConsts c, const uint32_t* __restrict__ perm, const float4* __restrict__ xsb,
-                          const float4* __restrict__ pb0, float4* __restrict__ xo, float4* __restrict__ vo,
+                          float4* __restrict__ pb0, float4* __restrict__ xo, float4* __restrict__ vo,
                           float* __restrict__ gbar) {
+    chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     F3 g = {0.0f, 0.0f, 0.0f};
     if (k < c.n) {
         const uint32_t i = perm[k];
         const F3 p = f3(pb0[k]);
+        pb0[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         const F3 x = f3(xsb[k]) + p;
         xo[i] = make_float4(x.x, x.y, x.z, 0.0f);
         vo[i] = make_float4(c.dt * p.x, c.dt * p.y, c.dt * p.z, 0.0f);
@@ -347,26 +381,22 @@ inline unsigned grid_for(int n) { return (unsigned)((n + kAdjBlock - 1) / kAdjBl
 
 void adjoint_substep(const DevConsts& c, const AdjointTape& tp, AdjointBuffers& ab, cudaStream_t s) {
     const int n = c.n;
-    const size_t v4 = 16 * (size_t)n;
-    cudaMemsetAsync(ab.omb, 0, v4, s);
-    cudaMemsetAsync(ab.pb, 0, v4, s);
-    cudaMemsetAsync(ab.v2b, 0, v4, s);
-    adj_vorticity_kernel<<<grid_for(n), kAdjBlock, 0, s>>>(c, tp.pI, tp.omega, tp.rows, tp.meta, ab.vb, ab.omb, ab.pb);
-    adj_viscosity_kernel<<<grid_for(n), kAdjBlock, 0, s>>>(c, tp.pI, tp.v2, ab.omb, ab.vb, tp.rows, tp.meta, ab.v2b,
-                                                           ab.pb, ab.scalars);
-    adj_velocity_kernel<<<grid_for(n), kAdjBlock, 0, s>>>(c, ab.xb, ab.v2b, ab.pb, ab.xsb);
+    const unsigned wide = (unsigned)(((int64_t)n * kSplit + kAdjBlock - 1) / kAdjBlock);
+    launch_chained(adj_vorticity_kernel, wide, kAdjBlock, s, c, tp.pI, tp.omega, tp.eta, tp.rows, tp.meta, ab.vb,
+                   ab.omb, ab.pb);
+    launch_chained(adj_viscosity_kernel, wide, kAdjBlock, s, c, tp.pI, tp.v2, ab.omb, ab.vb, tp.rows, tp.meta, ab.v2b,
+                   ab.pb, ab.scalars);
+    launch_chained(adj_velocity_kernel, grid_for(n), kAdjBlock, s, c, ab.xb, ab.v2b, ab.pb, ab.xsb);
     for (int t = tp.iterations - 1; t >= 0; --t) {
-        cudaMemsetAsync(ab.pbt, 0, v4, s);
-        cudaMemsetAsync(ab.lb, 0, 4 * (size_t)n, s);
-        adj_delta_kernel<<<grid_for(n), kAdjBlock, 0, s>>>(c, tp.q[t], tp.mask ? tp.mask + (size_t)t * n : nullptr,
-                                                           ab.pb, tp.rows, tp.meta, ab.pbt, ab.lb);
-        adj_scaling_kernel<<<grid_for(n), kAdjBlock, 0, s>>>(c, tp.q[t], ab.lb, tp.rows, tp.meta, ab.pbt);
+        launch_chained(adj_delta_kernel, wide, kAdjBlock, s, c, tp.q[t], tp.mask ? tp.mask + (size_t)t * n : nullptr,
+                       ab.pb, tp.rows, tp.meta, ab.pbt);
+        launch_chained(adj_scaling_kernel, wide, kAdjBlock, s, c, tp.q[t], tp.sums[t], tp.rho[t], tp.rows, tp.meta, ab.pbt, ab.pb);
         float4* tmp = ab.pb;
         ab.pb = ab.pbt;
         ab.pbt = tmp;
     }
-    adj_unsort_predict_kernel<<<grid_for(n), kAdjBlock, 0, s>>>(c, tp.perm, ab.xsb, ab.pb, ab.xo, ab.vo,
-                                                                ab.scalars + 1);
+    launch_chained(adj_unsort_predict_kernel, grid_for(n), kAdjBlock, s, c, tp.perm, ab.xsb, ab.pb, ab.xo, ab.vo,
+                   ab.scalars + 1);
     float4* t1 = ab.xb;
     ab.xb = ab.xo;
     ab.xo = t1;

@@ -536,7 +536,8 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
         mark("sortParticles");
         if (counting) {
             ctx->keysIdx = 1;
-            pbf::launch_cell_gather(c.n, ctx->keys[0], ctx->cellStart, order, ctx->keys[1], ctx->perm[1], ctx->pos[P],
+            pbf::launch_cell_gather(c.n, ctx->keys[0], ctx->cellStart, order, ctx->keys[1], ctx->perm[1],
+                                    tape ? tape->perm : nullptr, ctx->pos[P],
                                     ctx->pred[0], ctx->ids, ctx->pos[P ^ 1], ctx->pred[1], ctx->idsTmp, ctx->errWord, s);
         } else {
             pbf::launch_gather_sorted(c.n, ctx->perm[ctx->keysIdx], ctx->pos[P], ctx->pred[0], ctx->ids, ctx->pos[P ^ 1],
@@ -553,7 +554,7 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
     uint4* rows = tape ? tape->rows : ctx->rows;
     uint2* meta = tape ? tape->meta : ctx->meta;
     float4* omega = tape ? tape->omega : ctx->omega;
-    if (tape) PBF_CUDA(ctx, cudaMemcpyAsync(tape->perm, ctx->perm[ctx->keysIdx], 4 * (size_t)c.n, cudaMemcpyDeviceToDevice, s));
+    if (tape && !counting) PBF_CUDA(ctx, cudaMemcpyAsync(tape->perm, ctx->perm[ctx->keysIdx], 4 * (size_t)c.n, cudaMemcpyDeviceToDevice, s));
     mark("updateCells");
     const uint32_t tableKeys = ctx->cellsWords * (uint32_t)(is_batch(ctx) ? ctx->sceneParams.size() : 1);
     c.keys = keys;  // the taint of irregular positions finds a cell's particles in them
@@ -572,11 +573,13 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
     }
     int a = sortedPred;
     const unsigned iters = ctx->params.simIterations;
-    const pbf::StepEnd end{ctx->pos[sortedPos ^ 1], ctx->vel[V], paused ? nullptr : ctx->idsTmp, ctx->ids};
+    const pbf::StepEnd end{ctx->pos[sortedPos ^ 1], ctx->vel[V], paused ? nullptr : ctx->idsTmp, ctx->ids,
+                           tape ? tape->pI : nullptr, tape ? tape->v2 : nullptr};
     for (unsigned it = 0; it < iters; ++it) {
         float4* packed = tape ? tape->q[it] : ctx->pred[a ^ 1];
         mark("computeScaling", (int)it);
-        pbf::launch_compute_scaling(c, ctx->pred[a], packed, ctx->density, meta, rows, ls.scaling, ls.balance, tiles(1), s);
+        pbf::launch_compute_scaling(c, ctx->pred[a], packed, ctx->density, tape ? tape->sums[it] : nullptr,
+                                    tape ? tape->rho[it] : nullptr, meta, rows, ls.scaling, ls.balance, tiles(1), s);
         mark("computeDelta", (int)it);
         pbf::launch_compute_delta(c, b, packed, ctx->pos[sortedPos], it + 1 == iters ? end : pbf::StepEnd{}, ctx->pred[a], ctx->density, meta,
                                   it + 1 == iters, tape && tape->mask ? tape->mask + (size_t)it * c.n : nullptr,
@@ -588,7 +591,6 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
         pack_density_kernel<<<(c.n + 255) / 256, 256, 0, s>>>(c.n, ctx->pred[a], ctx->density);
         ++launched;
     }
-    if (tape) PBF_CUDA(ctx, cudaMemcpyAsync(tape->pI, ctx->pred[a], v4, cudaMemcpyDeviceToDevice, s));
     mark("updateVelocities");
     if (iters == 0) {  // else by the last position pass
         pbf::launch_update_velocities(c, end, ctx->pred[a], ctx->pos[sortedPos], s);
@@ -600,24 +602,24 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
         PBF_CUDA(ctx, cudaMemcpyAsync(ctx->readPos, ctx->pos[sortedPos ^ 1], v4, cudaMemcpyDeviceToHost, ctx->copyStream));
         PBF_CUDA(ctx, cudaEventRecord(ctx->evCopyDone, ctx->copyStream));
     }
-    if (tape) PBF_CUDA(ctx, cudaMemcpyAsync(tape->v2, ctx->vel[V], v4, cudaMemcpyDeviceToDevice, s));
     mark("applyViscosity");
     float4* near = ctx->pred[a ^ 1];  // free: the iterations are done, and the next substep writes its predictions there
     pbf::launch_apply_viscosity(c, b, ctx->pred[a], ctx->vel[V], ctx->vel[V ^ 1], omega, near, meta, rows, ls.viscosity,
                                 ls.balance, tiles(3), s);
     mark("applyVorticity");
+    float4* eta = tape ? tape->eta : nullptr;
     const int vortTiles = (c.n + ls.vorticity - 1) / ls.vorticity;
     if (ctx->readVel && ctx->readPos && vortTiles >= 2) {
         // the first half of the particles' velocities copy out while the second half runs
         const int half = vortTiles / 2;
         const size_t headBytes = 16 * (size_t)half * (size_t)ls.vorticity;
-        pbf::launch_apply_vorticity(c, ctx->pred[a], near, omega, ctx->vel[V ^ 1], ctx->vel[V], meta, rows,
+        pbf::launch_apply_vorticity(c, ctx->pred[a], near, omega, ctx->vel[V ^ 1], ctx->vel[V], eta, meta, rows,
                                     ls.vorticity, ls.balance, nullptr, s, 0, half);
         PBF_CUDA(ctx, cudaEventRecord(ctx->evVelHead, s));
         PBF_CUDA(ctx, cudaStreamWaitEvent(ctx->copyStream, ctx->evVelHead, 0));
         PBF_CUDA(ctx, cudaMemcpyAsync(ctx->readVel, ctx->vel[V], headBytes, cudaMemcpyDeviceToHost, ctx->copyStream));
         PBF_CUDA(ctx, cudaEventRecord(ctx->evCopyDone, ctx->copyStream));
-        pbf::launch_apply_vorticity(c, ctx->pred[a], near, omega, ctx->vel[V ^ 1], ctx->vel[V], meta, rows,
+        pbf::launch_apply_vorticity(c, ctx->pred[a], near, omega, ctx->vel[V ^ 1], ctx->vel[V], eta, meta, rows,
                                     ls.vorticity, ls.balance, nullptr, s, half, vortTiles - half);
         PBF_CUDA(ctx, cudaMemcpyAsync(reinterpret_cast<char*>(ctx->readVel) + headBytes,
                                       reinterpret_cast<const char*>(ctx->vel[V]) + headBytes, v4 - headBytes,
@@ -625,7 +627,7 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
         velCopied = true;
         ++launched;
     } else {
-        pbf::launch_apply_vorticity(c, ctx->pred[a], near, omega, ctx->vel[V ^ 1], ctx->vel[V], meta, rows,
+        pbf::launch_apply_vorticity(c, ctx->pred[a], near, omega, ctx->vel[V ^ 1], ctx->vel[V], eta, meta, rows,
                                     ls.vorticity, ls.balance, tiles(4), s);
     }
     launched += 2;
@@ -762,7 +764,12 @@ int ensure_tape(pbf_ctx* ctx) {
         t.perm = (uint32_t*)take(4 * (size_t)n);
         t.rows = (uint4*)take(16 * pbf::row_entries(ctx->listSlots) * n);
         t.meta = (uint2*)take(8 * (size_t)n);
-        for (int it = 0; it < iters; ++it) t.q[it] = (float4*)take(v4);
+        for (int it = 0; it < iters; ++it) {
+            t.q[it] = (float4*)take(v4);
+            t.sums[it] = (float4*)take(v4);
+            t.rho[it] = (float*)take(4 * (size_t)n);
+        }
+        t.eta = (float4*)take(v4);
         t.mask = clamp ? (uint8_t*)take((size_t)iters * n) : nullptr;
         t.pI = (float4*)take(v4);
         t.v2 = (float4*)take(v4);
@@ -771,7 +778,6 @@ int ensure_tape(pbf_ctx* ctx) {
     pbf::AdjointBuffers& ab = ctx->adj;
     float4** vecs[] = {&ab.xb, &ab.vb, &ab.xo, &ab.vo, &ab.pb, &ab.pbt, &ab.omb, &ab.v2b, &ab.xsb, &ctx->adjById};
     for (float4** v : vecs) *v = (float4*)take(v4);
-    ab.lb = (float*)take(4 * (size_t)n);
     ab.scalars = (float*)take(16);
     cudaGetLastError();
     if (!ok) {
@@ -788,7 +794,7 @@ int ensure_tape(pbf_ctx* ctx) {
 
 bool same_buffers(const pbf::AdjointBuffers& a, const pbf::AdjointBuffers& b) {
     return a.xb == b.xb && a.vb == b.vb && a.xo == b.xo && a.vo == b.vo && a.pb == b.pb && a.pbt == b.pbt &&
-           a.omb == b.omb && a.v2b == b.v2b && a.xsb == b.xsb && a.lb == b.lb && a.scalars == b.scalars;
+           a.omb == b.omb && a.v2b == b.v2b && a.xsb == b.xsb && a.scalars == b.scalars;
 }
 
 // One segment of the reverse pass (its `len` substeps recomputed into the
@@ -1875,6 +1881,8 @@ int pbf_rollout_backward(pbf_ctx* ctx, const float* dL_dx, float* dL_dv0, float*
     pbf::scatter_by_id(n, ctx->ckptEnd.ids, ctx->adjById, ab.xb, s);
     PBF_CUDA(ctx, cudaMemsetAsync(ab.vb, 0, v4, s));
     PBF_CUDA(ctx, cudaMemsetAsync(ab.scalars, 0, 16, s));
+    // the accumulators start at zero, and the adjoint kernels leave them so
+    for (float4* v : {ab.pb, ab.pbt, ab.omb, ab.v2b}) PBF_CUDA(ctx, cudaMemsetAsync(v, 0, v4, s));
     ctx->launches += 1;
     const int segments = (int)ctx->ckpt.size();
     for (int sgm = segments - 1; sgm >= 0 && rc == PBF_OK; --sgm) {

@@ -148,17 +148,21 @@ void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const
                           cudaStream_t s);
 // uint4 entries per particle of the rows for `slots` friends.
 inline size_t row_entries(int slots) { return ((size_t)slots + 3) / 4; }
+// tapeSums, tapeRho, tapeEta below: a rollout's tape (AdjointTape; NULL without).
 void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* predPacked, float* density,
-                            const uint2* meta, const uint4* rows, int block, int balance, int* tileCounter,
+                            float4* tapeSums, float* tapeRho, const uint2* meta, const uint4* rows, int block, int balance, int* tileCounter,
                             cudaStream_t s);
 // What the last position pass of a substep also writes: the new positions and
-// velocities, and the particle ids (idsIn NULL: they stay).  posOut NULL: not
-// the last pass.
+// velocities, and the particle ids (idsIn NULL: they stay); for a rollout's tape
+// (NULL without one) the final predictions and the velocities again.  posOut
+// NULL: not the last pass.
 struct StepEnd {
     float4* posOut = nullptr;
     float4* vel = nullptr;
     const uint32_t* idsIn = nullptr;
     uint32_t* idsOut = nullptr;
+    float4* tapeP = nullptr;
+    float4* tapeV = nullptr;
 };
 // posPrev: the sorted positions, read by the force planes and the step's end.
 void launch_compute_delta(const DevConsts& c, Batch b, const float4* predPacked, const float4* posPrev,
@@ -176,7 +180,7 @@ void launch_apply_viscosity(const DevConsts& c, Batch b, const float4* pred, con
 // last vorticity pass so that the first part's velocities copy out while the
 // rest runs).
 void launch_apply_vorticity(const DevConsts& c, const float4* pred, const float4* near, const float4* omega,
-                            const float4* velIn, float4* velOut, const uint2* meta, const uint4* rows, int block, int balance,
+                            const float4* velIn, float4* velOut, float4* tapeEta, const uint2* meta, const uint4* rows, int block, int balance,
                             int* tileCounter, cudaStream_t s, int firstTile = 0, int tileCount = 0);
 
 // ---- radix sort (pbf_sort.cu) ----
@@ -216,10 +220,12 @@ CountingPlan make_counting_plan(int n, uint64_t keys);
 // in any order within a key, into `order`.  Zeroes the counts.
 void launch_counting_sort(const CountingPlan& plan, int n, uint32_t* counts, uint32_t* sums, uint32_t* starts,
                           const uint32_t* keys, const uint32_t* place, uint32_t* order, int* err, cudaStream_t s);
-// The stable order from it, with the records gathered (launch_gather_sorted).
+// The stable order from it, with the records gathered (launch_gather_sorted);
+// permCopy (may be NULL) receives the permutation too.
 void launch_cell_gather(int n, const uint32_t* keys, const uint32_t* starts, const uint32_t* order, uint32_t* keysOut,
-                        uint32_t* permOut, const float4* pos, const float4* pred, const uint32_t* ids, float4* posOut,
-                        float4* predOut, uint32_t* idsOut, int* err, cudaStream_t s);
+                        uint32_t* permOut, uint32_t* permCopy, const float4* pos, const float4* pred,
+                        const uint32_t* ids, float4* posOut, float4* predOut, uint32_t* idsOut, int* err,
+                        cudaStream_t s);
 
 // ---- adjoint (pbf_adjoint.cu) ----
 // What one substep of a rollout leaves for its reverse pass.
@@ -229,6 +235,9 @@ struct AdjointTape {
     uint4* rows = nullptr;         // the substep's kept friends in order, four per entry (walk_pairs)
     uint2* meta = nullptr;
     float4* q[64] = {};            // (p^t, lambda^t), t < iterations
+    float4* sums[64] = {};         // per iteration sum g and sum |g|^2 + |sum g|^2, g the density pass' gradients
+    float* rho[64] = {};           // per iteration the density
+    float4* eta = nullptr;         // the vorticity pass' eta, not normalised
     uint8_t* mask = nullptr;       // iterations x N box-clamp decisions (NULL: no clamp)
     float4* pI = nullptr;          // final predictions, w = density
     float4* v2 = nullptr;          // velocities before XSPH
@@ -238,9 +247,9 @@ struct AdjointTape {
 // and of its input on return (the pointers are swapped with xo / vo).
 struct AdjointBuffers {
     float4 *xb, *vb, *xo, *vo, *pb, *pbt, *omb, *v2b, *xsb;
-    float* lb;
     float* scalars;  // [0] dL/d viscosityFactor, [1..3] dL/d gravity
 };
+// Between substeps pb, pbt, omb and v2b are zero.
 void adjoint_substep(const DevConsts& c, const AdjointTape& tp, AdjointBuffers& ab, cudaStream_t s);
 int adjoint_launches(int iterations);
 void scatter_by_id(int n, const uint32_t* ids, const float4* byId, float4* out, cudaStream_t s);

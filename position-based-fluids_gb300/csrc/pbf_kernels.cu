@@ -704,6 +704,7 @@ __device__ __forceinline__ F2 spiky_over_r2(const DevConsts& c, F2 r2, F2& w) {
 template <bool R, bool Q>
 __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const float4* __restrict__ pred,
                                                      float4* __restrict__ predPacked, float* __restrict__ density,
+                                                     float4* __restrict__ tapeSums, float* __restrict__ tapeRho,
                                                      const uint4* __restrict__ rows, int i, const float4 pi, uint64_t mt) {
     const int n = c.n;
     // complete neighbour sets count the particle itself first: d = h^2 - 0
@@ -781,6 +782,10 @@ __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const f
     ds = ds * c.poly6;
     density[i] = ds;
     gsk = gsk + dot3(gx, gy, gz, gx, gy, gz);
+    if (tapeSums) {
+        tapeSums[i] = make_float4(gx, gy, gz, gsk);
+        tapeRho[i] = ds;
+    }
     const float constraint = (ds / c.rho0) - 1.0f;
     const float lambda = -1.0f * constraint / (gsk / c.rho0sq + c.eps);
     predPacked[i] = make_float4(pi.x, pi.y, pi.z, lambda);
@@ -789,8 +794,8 @@ __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const f
 template <bool R, bool B>
 __global__ void __launch_bounds__(kMaxBlock)
 compute_scaling_kernel(DevConsts c, const float4* __restrict__ pred, float4* __restrict__ predPacked,
-                       float* __restrict__ density, const uint2* __restrict__ meta, const uint4* __restrict__ rows,
-                       int tiles, int* tileCounter) {
+                       float* __restrict__ density, float4* __restrict__ tapeSums, float* __restrict__ tapeRho,
+                       const uint2* __restrict__ meta, const uint4* __restrict__ rows, int tiles, int* tileCounter) {
     chain_wait();
     for_tiles(tiles, tileCounter, [&](int tile) {
         const int i = B ? balanced_particle(meta, c.n, true, tile) : tile * (int)blockDim.x + (int)threadIdx.x;
@@ -798,8 +803,8 @@ compute_scaling_kernel(DevConsts c, const float4* __restrict__ pred, float4* __r
         const float4 pi = pred[i];
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) compute_scaling_body<R, true>(c, pred, predPacked, density, rows, i, pi, mt);
-        else compute_scaling_body<R, false>(c, pred, predPacked, density, rows, i, pi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) compute_scaling_body<R, true>(c, pred, predPacked, density, tapeSums, tapeRho, rows, i, pi, mt);
+        else compute_scaling_body<R, false>(c, pred, predPacked, density, tapeSums, tapeRho, rows, i, pi, mt);
     });
 }
 
@@ -813,6 +818,10 @@ __device__ __forceinline__ void end_of_step(const DevConsts& c, const StepEnd& e
     v.y = (p.y - q.y) / c.dt;
     v.z = (p.z - q.z) / c.dt;
     end.vel[i] = v;
+    if (end.tapeP) {
+        end.tapeP[i] = p;
+        end.tapeV[i] = v;
+    }
     end.posOut[i] = make_float4(p.x, p.y, p.z, sqrtf(dot3(v.x, v.y, v.z, v.x, v.y, v.z)));
 }
 
@@ -1072,7 +1081,8 @@ template <bool R, bool Q>
 __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const float4* __restrict__ near,
                                                      const float4* __restrict__ omega,
                                                      const float4* __restrict__ velIn, float4* __restrict__ velOut,
-                                                     const uint4* __restrict__ rows, int i, const float4 pi, uint64_t mt) {
+                                                     float4* __restrict__ tapeEta, const uint4* __restrict__ rows, int i,
+                                                     const float4 pi, uint64_t mt) {
     const int n = c.n;
     float ex = 0.0f, ey = 0.0f, ez = 0.0f;
     auto load = [&](uint32_t j) { return __ldg(near + checked_index(j, (uint32_t)n, c.err, kErrFriendIndex)); };
@@ -1120,6 +1130,7 @@ __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const f
     ex = ex * c.negGradSpiky;
     ey = ey * c.negGradSpiky;
     ez = ez * c.negGradSpiky;
+    if (tapeEta) tapeEta[i] = make_float4(ex, ey, ez, 0.0f);
     if (R) {
         const float l2 = fmaf(ez, ez, fmaf(ey, ey, ex * ex));
         if (l2 > 0.0f) {
@@ -1147,7 +1158,8 @@ __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const f
 template <bool R, bool B>
 __global__ void __launch_bounds__(kMaxBlock)
 apply_vorticity_kernel(DevConsts c, const float4* __restrict__ pred, const float4* __restrict__ near,
-                       const float4* __restrict__ omega, const float4* __restrict__ velIn, float4* __restrict__ velOut, const uint2* __restrict__ meta,
+                       const float4* __restrict__ omega, const float4* __restrict__ velIn, float4* __restrict__ velOut,
+                       float4* __restrict__ tapeEta, const uint2* __restrict__ meta,
                        const uint4* __restrict__ rows, int tiles, int* tileCounter, int tileOffset) {
     chain_wait();
     for_tiles(tiles, tileCounter, [&](int tile) {
@@ -1157,8 +1169,8 @@ apply_vorticity_kernel(DevConsts c, const float4* __restrict__ pred, const float
         const float4 pi = pred[i];
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) apply_vorticity_body<R, true>(c, near, omega, velIn, velOut, rows, i, pi, mt);
-        else apply_vorticity_body<R, false>(c, near, omega, velIn, velOut, rows, i, pi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) apply_vorticity_body<R, true>(c, near, omega, velIn, velOut, tapeEta, rows, i, pi, mt);
+        else apply_vorticity_body<R, false>(c, near, omega, velIn, velOut, tapeEta, rows, i, pi, mt);
     });
 }
 
@@ -1232,13 +1244,13 @@ void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const
 }
 
 void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* predPacked, float* density,
-                            const uint2* meta, const uint4* rows, int block, int balance, int* tileCounter,
+                            float4* tapeSums, float* tapeRho, const uint2* meta, const uint4* rows, int block, int balance, int* tileCounter,
                             cudaStream_t s) {
     auto k = c.relaxed ? (balance ? compute_scaling_kernel<true, true> : compute_scaling_kernel<true, false>)
                        : (balance ? compute_scaling_kernel<false, true> : compute_scaling_kernel<false, false>);
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
-    launch_chained(k, grid, block, s, c, pred, predPacked, density, meta, rows, tiles, tileCounter);
+    launch_chained(k, grid, block, s, c, pred, predPacked, density, tapeSums, tapeRho, meta, rows, tiles, tileCounter);
 }
 
 void launch_compute_delta(const DevConsts& c, Batch b, const float4* predPacked, const float4* posPrev,
@@ -1269,17 +1281,17 @@ void launch_apply_viscosity(const DevConsts& c, Batch b, const float4* pred, con
 }
 
 void launch_apply_vorticity(const DevConsts& c, const float4* pred, const float4* near, const float4* omega,
-                            const float4* velIn, float4* velOut, const uint2* meta, const uint4* rows, int block, int balance,
+                            const float4* velIn, float4* velOut, float4* tapeEta, const uint2* meta, const uint4* rows, int block, int balance,
                             int* tileCounter, cudaStream_t s, int firstTile, int tileCount) {
     auto k = c.relaxed ? (balance ? apply_vorticity_kernel<true, true> : apply_vorticity_kernel<true, false>)
                        : (balance ? apply_vorticity_kernel<false, true> : apply_vorticity_kernel<false, false>);
     if (tileCount > 0) {  // tiles [firstTile, firstTile + tileCount), one block each
-        launch_chained(k, (unsigned)tileCount, block, s, c, pred, near, omega, velIn, velOut, meta, rows, 0, nullptr, firstTile);
+        launch_chained(k, (unsigned)tileCount, block, s, c, pred, near, omega, velIn, velOut, tapeEta, meta, rows, 0, nullptr, firstTile);
         return;
     }
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
-    launch_chained(k, grid, block, s, c, pred, near, omega, velIn, velOut, meta, rows, tiles, tileCounter, 0);
+    launch_chained(k, grid, block, s, c, pred, near, omega, velIn, velOut, tapeEta, meta, rows, tiles, tileCounter, 0);
 }
 
 }  // namespace pbf

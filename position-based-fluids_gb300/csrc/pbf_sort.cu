@@ -256,6 +256,7 @@ cell_scatter_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __
 __global__ void __launch_bounds__(kThreads)
 cell_gather_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ starts,
                    const uint32_t* __restrict__ order, uint32_t* __restrict__ keysOut, uint32_t* __restrict__ permOut,
+                   uint32_t* __restrict__ permCopy,
                    const float4* __restrict__ pos, const float4* __restrict__ pred, const uint32_t* __restrict__ ids,
                    float4* __restrict__ posOut, float4* __restrict__ predOut, uint32_t* __restrict__ idsOut,
                    int* __restrict__ err) {
@@ -271,6 +272,7 @@ cell_gather_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __r
     to = checked_index(to, (uint32_t)n, err, kErrSortIndex);
     keysOut[to] = key;
     permOut[to] = i;
+    if (permCopy) permCopy[to] = i;
     posOut[to] = x;
     predOut[to] = p;
     idsOut[to] = id;
@@ -301,9 +303,10 @@ void launch_counting_sort(const CountingPlan& plan, int n, uint32_t* counts, uin
 }
 
 void launch_cell_gather(int n, const uint32_t* keys, const uint32_t* starts, const uint32_t* order, uint32_t* keysOut,
-                        uint32_t* permOut, const float4* pos, const float4* pred, const uint32_t* ids, float4* posOut,
-                        float4* predOut, uint32_t* idsOut, int* err, cudaStream_t s) {
-    launch_chained(cell_gather_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keys, starts, order, keysOut, permOut, pos,
+                        uint32_t* permOut, uint32_t* permCopy, const float4* pos, const float4* pred,
+                        const uint32_t* ids, float4* posOut, float4* predOut, uint32_t* idsOut, int* err,
+                        cudaStream_t s) {
+    launch_chained(cell_gather_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keys, starts, order, keysOut, permOut, permCopy, pos,
                                                                           pred, ids, posOut, predOut, idsOut, err);
 }
 
