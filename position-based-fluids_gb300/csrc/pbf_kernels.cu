@@ -655,6 +655,14 @@ __device__ __forceinline__ int balanced_particle(const uint2* __restrict__ meta,
     return t < valid ? order[t] : -1;
 }
 
+// Registers of the solver passes.  __launch_bounds__(512) makes the compiler
+// aim at the occupancy of 512-thread blocks and schedule the loads of a step
+// late; a register limit without it does not.  1M particles, two substeps:
+// density pass 0.835 ms with the bounds, 0.787 / 0.771 / 0.772 with limits of
+// 56 / 64 / 96; XSPH 0.259, 0.252 with 72; vorticity 0.190, 0.175 with 56; the
+// position pass 0.792, 0.797 / 0.794 with 56 / 64, so it keeps the bounds.
+// Limits below 52 spill and are slower.  512 threads of 72 registers fit an SM.
+
 // ---------------------------------------------------- tiles of a launch --
 // A launch covers `tiles` tiles of blockDim particles.  With tiles == 0, one
 // block per tile (tile = blockIdx.x).  Otherwise a persistent grid of at
@@ -792,7 +800,7 @@ __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const f
 }
 
 template <bool R, bool B>
-__global__ void __launch_bounds__(kMaxBlock)
+__global__ void __maxnreg__(64)
 compute_scaling_kernel(DevConsts c, const float4* __restrict__ pred, float4* __restrict__ predPacked,
                        float* __restrict__ density, float4* __restrict__ tapeSums, float* __restrict__ tapeRho,
                        const uint2* __restrict__ meta, const uint4* __restrict__ rows, int tiles, int* tileCounter) {
@@ -1060,7 +1068,7 @@ __device__ __forceinline__ void apply_viscosity_body(const DevConsts& c, const B
 }
 
 template <bool R, bool B>
-__global__ void __launch_bounds__(kMaxBlock)
+__global__ void __maxnreg__(72)
 apply_viscosity_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, const float4* __restrict__ velIn,
                        float4* __restrict__ velOut, float4* __restrict__ omega, float4* __restrict__ near,
                        const uint2* __restrict__ meta, const uint4* __restrict__ rows, int tiles, int* tileCounter) {
@@ -1156,7 +1164,7 @@ __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const f
 }
 
 template <bool R, bool B>
-__global__ void __launch_bounds__(kMaxBlock)
+__global__ void __maxnreg__(56)
 apply_vorticity_kernel(DevConsts c, const float4* __restrict__ pred, const float4* __restrict__ near,
                        const float4* __restrict__ omega, const float4* __restrict__ velIn, float4* __restrict__ velOut,
                        float4* __restrict__ tapeEta, const uint2* __restrict__ meta,
