@@ -709,7 +709,7 @@ __device__ __forceinline__ F2 spiky_over_r2(const DevConsts& c, F2 r2, F2& w) {
 
 // compute_scaling.cl:27-112 followed by pack_data.cl (w = lambda).  Q: the
 // exact quotients by |r| through one reciprocal (quotient_rn).
-template <bool R, bool Q>
+template <bool R, bool Q, int L>
 __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const float4* __restrict__ pred,
                                                      float4* __restrict__ predPacked, float* __restrict__ density,
                                                      float4* __restrict__ tapeSums, float* __restrict__ tapeRho,
@@ -730,7 +730,8 @@ __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const f
         gy = gy + g1;
         gz = gz + g2;
     };
-    walk_pairs(rows, n, i, FlatFriends(mt, kept_density(mt)).total, load, [&](const float4& pa, const float4& pb, bool va, bool vb) {
+    auto pass = [&](auto from) { ds = from(ds); gsk = from(gsk); gx = from(gx); gy = from(gy); gz = from(gz); };
+    walk_pairs<L>(rows, n, i, FlatFriends(mt, kept_density(mt)).total, load, [&](const float4& pa, const float4& pb, bool va, bool vb) {
         const F2 rx = pack2(pi.x - pa.x, pi.x - pb.x), ry = pack2(pi.y - pa.y, pi.y - pb.y),
                  rz = pack2(pi.z - pa.z, pi.z - pb.z);
         const F2 r2 = R ? fma2(rz, rz, fma2(ry, ry, mul2(rx, rx))) : dot2(c, rx, ry, rz, rx, ry, rz);
@@ -739,8 +740,10 @@ __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const f
         vb = vb && in_support(c, s2.y);
         if (!R && !Q) {
             const float2 x = unpack2(rx), y = unpack2(ry), z = unpack2(rz);
-            if (va) one(x.x, y.x, z.x, s2.x);
-            if (vb) one(x.y, y.y, z.y, s2.y);
+            in_turn<L>([&] {
+                if (va) one(x.x, y.x, z.x, s2.x);
+                if (vb) one(x.y, y.y, z.y, s2.y);
+            }, pass);
             return;
         }
         F2 g0, g1, g2;
@@ -763,30 +766,35 @@ __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const f
         const float2 x = unpack2(g0), y = unpack2(g1), z = unpack2(g2);
         if (R) {
             const float2 dd = unpack2(mul2(d, d)), d1 = unpack2(d);
-            if (va) {
-                ds = fmaf(dd.x, d1.x, ds);
-                gsk = fmaf(z.x, z.x, fmaf(y.x, y.x, fmaf(x.x, x.x, gsk)));
-                gx += x.x; gy += y.x; gz += z.x;
-            }
-            if (vb) {
-                ds = fmaf(dd.y, d1.y, ds);
-                gsk = fmaf(z.y, z.y, fmaf(y.y, y.y, fmaf(x.y, x.y, gsk)));
-                gx += x.y; gy += y.y; gz += z.y;
-            }
+            in_turn<L>([&] {
+                if (va) {
+                    ds = fmaf(dd.x, d1.x, ds);
+                    gsk = fmaf(z.x, z.x, fmaf(y.x, y.x, fmaf(x.x, x.x, gsk)));
+                    gx += x.x; gy += y.x; gz += z.x;
+                }
+                if (vb) {
+                    ds = fmaf(dd.y, d1.y, ds);
+                    gsk = fmaf(z.y, z.y, fmaf(y.y, y.y, fmaf(x.y, x.y, gsk)));
+                    gx += x.y; gy += y.y; gz += z.y;
+                }
+            }, pass);
         } else {
             const float2 d3 = unpack2(mul2(mul2(d, d), d)), gg = unpack2(dot2(c, g0, g1, g2, g0, g1, g2));
-            if (va) {
-                ds = ds + d3.x;
-                gsk = gsk + gg.x;
-                gx = gx + x.x; gy = gy + y.x; gz = gz + z.x;
-            }
-            if (vb) {
-                ds = ds + d3.y;
-                gsk = gsk + gg.y;
-                gx = gx + x.y; gy = gy + y.y; gz = gz + z.y;
-            }
+            in_turn<L>([&] {
+                if (va) {
+                    ds = ds + d3.x;
+                    gsk = gsk + gg.x;
+                    gx = gx + x.x; gy = gy + y.x; gz = gz + z.x;
+                }
+                if (vb) {
+                    ds = ds + d3.y;
+                    gsk = gsk + gg.y;
+                    gx = gx + x.y; gy = gy + y.y; gz = gz + z.y;
+                }
+            }, pass);
         }
     });
+    if (threadIdx.x % L) return;  // the sums are the first lane's
     ds = ds * c.poly6;
     density[i] = ds;
     gsk = gsk + dot3(gx, gy, gz, gx, gy, gz);
@@ -799,20 +807,20 @@ __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const f
     predPacked[i] = make_float4(pi.x, pi.y, pi.z, lambda);
 }
 
-template <bool R, bool B>
+template <bool R, bool B, int L>
 __global__ void __maxnreg__(64)
 compute_scaling_kernel(DevConsts c, const float4* __restrict__ pred, float4* __restrict__ predPacked,
                        float* __restrict__ density, float4* __restrict__ tapeSums, float* __restrict__ tapeRho,
                        const uint2* __restrict__ meta, const uint4* __restrict__ rows, int tiles, int* tileCounter) {
     chain_wait();
     for_tiles(tiles, tileCounter, [&](int tile) {
-        const int i = B ? balanced_particle(meta, c.n, true, tile) : tile * (int)blockDim.x + (int)threadIdx.x;
+        const int i = B ? balanced_particle(meta, c.n, true, tile) : (tile * (int)blockDim.x + (int)threadIdx.x) / L;
         if (i < 0 || i >= c.n) return;
         const float4 pi = pred[i];
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) compute_scaling_body<R, true>(c, pred, predPacked, density, tapeSums, tapeRho, rows, i, pi, mt);
-        else compute_scaling_body<R, false>(c, pred, predPacked, density, tapeSums, tapeRho, rows, i, pi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) compute_scaling_body<R, true, L>(c, pred, predPacked, density, tapeSums, tapeRho, rows, i, pi, mt);
+        else compute_scaling_body<R, false, L>(c, pred, predPacked, density, tapeSums, tapeRho, rows, i, pi, mt);
     });
 }
 
@@ -839,7 +847,7 @@ __device__ __forceinline__ void end_of_step(const DevConsts& c, const StepEnd& e
 // last iteration w carries the density (pack_data.cl with the density source,
 // src/Simulation.cpp:591), and the velocities are updated there as well
 // (end.posOut), which saves a launch and the prediction's way through memory.
-template <bool R, bool Q>
+template <bool R, bool Q, int L>
 __device__ __forceinline__ void compute_delta_body(const DevConsts& c, const Batch& b, const float4* __restrict__ pp,
                                                    const float4* __restrict__ posPrev, const StepEnd& end,
                                                    float4* __restrict__ predOut,
@@ -862,7 +870,8 @@ __device__ __forceinline__ void compute_delta_body(const DevConsts& c, const Bat
         sy = sy + a * g1;
         sz = sz + a * g2;
     };
-    walk_pairs(rows, n, i, FlatFriends(mt, kept_other(mt)).total, load, [&](const float4& pa, const float4& pb, bool va, bool vb) {
+    auto pass = [&](auto from) { sx = from(sx); sy = from(sy); sz = from(sz); };
+    walk_pairs<L>(rows, n, i, FlatFriends(mt, kept_other(mt)).total, load, [&](const float4& pa, const float4& pb, bool va, bool vb) {
         const F2 rx = pack2(pi.x - pa.x, pi.x - pb.x), ry = pack2(pi.y - pa.y, pi.y - pb.y),
                  rz = pack2(pi.z - pa.z, pi.z - pb.z);
         const F2 r2 = R ? fma2(rz, rz, fma2(ry, ry, mul2(rx, rx))) : dot2(c, rx, ry, rz, rx, ry, rz);
@@ -871,8 +880,10 @@ __device__ __forceinline__ void compute_delta_body(const DevConsts& c, const Bat
         vb = vb && in_support(c, s2.y);
         if (!R && !Q) {
             const float2 x = unpack2(rx), y = unpack2(ry), z = unpack2(rz);
-            if (va) one(x.x, y.x, z.x, s2.x, pa.w);
-            if (vb) one(x.y, y.y, z.y, s2.y, pb.w);
+            in_turn<L>([&] {
+                if (va) one(x.x, y.x, z.x, s2.x, pa.w);
+                if (vb) one(x.y, y.y, z.y, s2.y, pb.w);
+            }, pass);
             return;
         }
         const F2 d = sub2(both(c.h2), r2);
@@ -885,8 +896,10 @@ __device__ __forceinline__ void compute_delta_body(const DevConsts& c, const Bat
             const F2 rq2 = mul2(rq, rq);
             const float2 a = unpack2(mul2(fma2(mul2(both(c.K), rq2), rq2, wij), k));
             const float2 x = unpack2(rx), y = unpack2(ry), z = unpack2(rz);
-            if (va) { sx = fmaf(a.x, x.x, sx); sy = fmaf(a.x, y.x, sy); sz = fmaf(a.x, z.x, sz); }
-            if (vb) { sx = fmaf(a.y, x.y, sx); sy = fmaf(a.y, y.y, sy); sz = fmaf(a.y, z.y, sz); }
+            in_turn<L>([&] {
+                if (va) { sx = fmaf(a.x, x.x, sx); sy = fmaf(a.x, y.x, sy); sz = fmaf(a.x, z.x, sz); }
+                if (vb) { sx = fmaf(a.y, x.y, sx); sy = fmaf(a.y, y.y, sy); sz = fmaf(a.y, z.y, sz); }
+            }, pass);
         } else {
             F2 nrl, y;
             sqrt_recip_rn2(r2, nrl, y);
@@ -902,10 +915,13 @@ __device__ __forceinline__ void compute_delta_body(const DevConsts& c, const Bat
             }
             const F2 a = add2(wij, product2(c, mul2(mul2(mul2(both(c.K), rq), rq), rq), rq));
             const float2 x = unpack2(mul2(a, g0)), v = unpack2(mul2(a, g1)), z = unpack2(mul2(a, g2));
-            if (va) { sx = sx + x.x; sy = sy + v.x; sz = sz + z.x; }
-            if (vb) { sx = sx + x.y; sy = sy + v.y; sz = sz + z.y; }
+            in_turn<L>([&] {
+                if (va) { sx = sx + x.x; sy = sy + v.x; sz = sz + z.x; }
+                if (vb) { sx = sx + x.y; sy = sy + v.y; sz = sz + z.y; }
+            }, pass);
         }
     });
+    if (threadIdx.x % L) return;  // the sums are the first lane's
     float fx, fy, fz;
     if (R) {
         fx = fmaf(c.dpScale, sx, pi.x);
@@ -947,7 +963,7 @@ __device__ __forceinline__ void compute_delta_body(const DevConsts& c, const Bat
     if (end.posOut) end_of_step(c, end, i, out, posPrev[i]);
 }
 
-template <bool R, bool B>
+template <bool R, bool B, int L>
 __global__ void __launch_bounds__(kMaxBlock)
 compute_delta_kernel(DevConsts c, Batch b, const float4* __restrict__ pp, const float4* __restrict__ posPrev,
                      StepEnd end, float4* __restrict__ predOut, const float* __restrict__ density,
@@ -955,13 +971,13 @@ compute_delta_kernel(DevConsts c, Batch b, const float4* __restrict__ pp, const 
                      const uint4* __restrict__ rows, int tiles, int* tileCounter) {
     chain_wait();
     for_tiles(tiles, tileCounter, [&](int tile) {
-        const int i = B ? balanced_particle(meta, c.n, false, tile) : tile * (int)blockDim.x + (int)threadIdx.x;
+        const int i = B ? balanced_particle(meta, c.n, false, tile) : (tile * (int)blockDim.x + (int)threadIdx.x) / L;
         if (i < 0 || i >= c.n) return;
         const float4 pi = pp[i];
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) compute_delta_body<R, true>(c, b, pp, posPrev, end, predOut, density, lastIteration, clampMask, rows, i, pi, mt);
-        else compute_delta_body<R, false>(c, b, pp, posPrev, end, predOut, density, lastIteration, clampMask, rows, i, pi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) compute_delta_body<R, true, L>(c, b, pp, posPrev, end, predOut, density, lastIteration, clampMask, rows, i, pi, mt);
+        else compute_delta_body<R, false, L>(c, b, pp, posPrev, end, predOut, density, lastIteration, clampMask, rows, i, pi, mt);
     });
 }
 
@@ -981,7 +997,7 @@ __global__ void update_velocities_kernel(DevConsts c, StepEnd end, const float4*
 // (apply_vorticity.cl:44).  The vorticity pass was bound by the L1 wavefronts
 // of its two gathers per friend (79 %); with one it takes 0.191 ms instead of
 // 0.214 (1M particles, mid-collapse, two substeps).
-template <bool R, bool Q>
+template <bool R, bool Q, int L>
 __device__ __forceinline__ void apply_viscosity_body(const DevConsts& c, const Batch& b, const float4* __restrict__ pred,
                                                      const float4* __restrict__ velIn, float4* __restrict__ velOut,
                                                      float4* __restrict__ omega, float4* __restrict__ near,
@@ -990,7 +1006,8 @@ __device__ __forceinline__ void apply_viscosity_body(const DevConsts& c, const B
     const int n = c.n;
     float vsx = 0.0f, vsy = 0.0f, vsz = 0.0f, ox = 0.0f, oy = 0.0f, oz = 0.0f;
     auto load = [&](uint32_t j) { j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex); return PairRec{__ldg(pred + j), __ldg(velIn + j)}; };
-    walk_pairs<true>(rows, n, i, FlatFriends(mt, kept_other(mt)).total, load, [&](const PairRec& qa, const PairRec& qb, bool va, bool vb) {
+    auto pass = [&](auto from) { ox = from(ox); oy = from(oy); oz = from(oz); vsx = from(vsx); vsy = from(vsy); vsz = from(vsz); };
+    walk_pairs<L, true>(rows, n, i, FlatFriends(mt, kept_other(mt)).total, load, [&](const PairRec& qa, const PairRec& qb, bool va, bool vb) {
         const float4 pa = qa.a, pb = qb.a;
         const F2 rx = pack2(pi.x - pa.x, pi.x - pb.x), ry = pack2(pi.y - pa.y, pi.y - pb.y),
                  rz = pack2(pi.z - pa.z, pi.z - pb.z);
@@ -1028,28 +1045,33 @@ __device__ __forceinline__ void apply_viscosity_body(const DevConsts& c, const B
             const float2 x = unpack2(fma2(uy, g2, neg2(mul2(uz, g1)))), y = unpack2(fma2(uz, g0, neg2(mul2(ux, g2)))),
                          z = unpack2(fma2(ux, g1, neg2(mul2(uy, g0)))), t = unpack2(d3), a0 = unpack2(ux),
                          a1 = unpack2(uy), a2 = unpack2(uz);
-            if (va) {
-                ox += x.x; oy += y.x; oz += z.x;
-                vsx = fmaf(a0.x, t.x, vsx); vsy = fmaf(a1.x, t.x, vsy); vsz = fmaf(a2.x, t.x, vsz);
-            }
-            if (vb) {
-                ox += x.y; oy += y.y; oz += z.y;
-                vsx = fmaf(a0.y, t.y, vsx); vsy = fmaf(a1.y, t.y, vsy); vsz = fmaf(a2.y, t.y, vsz);
-            }
+            in_turn<L>([&] {
+                if (va) {
+                    ox += x.x; oy += y.x; oz += z.x;
+                    vsx = fmaf(a0.x, t.x, vsx); vsy = fmaf(a1.x, t.x, vsy); vsz = fmaf(a2.x, t.x, vsz);
+                }
+                if (vb) {
+                    ox += x.y; oy += y.y; oz += z.y;
+                    vsx = fmaf(a0.y, t.y, vsx); vsy = fmaf(a1.y, t.y, vsy); vsz = fmaf(a2.y, t.y, vsz);
+                }
+            }, pass);
         } else {
             const float2 p0 = unpack2(mul2(uy, g2)), p1 = unpack2(mul2(uz, g0)), p2 = unpack2(mul2(ux, g1)),
                          q0 = unpack2(mul2(uz, g1)), q1 = unpack2(mul2(ux, g2)), q2 = unpack2(mul2(uy, g0)),
                          a0 = unpack2(mul2(ux, d3)), a1 = unpack2(mul2(uy, d3)), a2 = unpack2(mul2(uz, d3));
-            if (va) {
-                ox = ox + (p0.x - q0.x); oy = oy + (p1.x - q1.x); oz = oz + (p2.x - q2.x);
-                vsx = vsx + a0.x; vsy = vsy + a1.x; vsz = vsz + a2.x;
-            }
-            if (vb) {
-                ox = ox + (p0.y - q0.y); oy = oy + (p1.y - q1.y); oz = oz + (p2.y - q2.y);
-                vsx = vsx + a0.y; vsy = vsy + a1.y; vsz = vsz + a2.y;
-            }
+            in_turn<L>([&] {
+                if (va) {
+                    ox = ox + (p0.x - q0.x); oy = oy + (p1.x - q1.x); oz = oz + (p2.x - q2.x);
+                    vsx = vsx + a0.x; vsy = vsy + a1.x; vsz = vsz + a2.x;
+                }
+                if (vb) {
+                    ox = ox + (p0.y - q0.y); oy = oy + (p1.y - q1.y); oz = oz + (p2.y - q2.y);
+                    vsx = vsx + a0.y; vsy = vsy + a1.y; vsz = vsz + a2.y;
+                }
+            }, pass);
         }
     });
+    if (threadIdx.x % L) return;  // the sums are the first lane's
     vsx = vsx * c.poly6;
     vsy = vsy * c.poly6;
     vsz = vsz * c.poly6;
@@ -1067,25 +1089,25 @@ __device__ __forceinline__ void apply_viscosity_body(const DevConsts& c, const B
     near[i] = make_float4(fabsf(pi.w) > 1e-8f ? pi.x : __int_as_float(0x7F800000), pi.y, pi.z, size);
 }
 
-template <bool R, bool B>
+template <bool R, bool B, int L>
 __global__ void __maxnreg__(72)
 apply_viscosity_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, const float4* __restrict__ velIn,
                        float4* __restrict__ velOut, float4* __restrict__ omega, float4* __restrict__ near,
                        const uint2* __restrict__ meta, const uint4* __restrict__ rows, int tiles, int* tileCounter) {
     chain_wait();
     for_tiles(tiles, tileCounter, [&](int tile) {
-        const int i = B ? balanced_particle(meta, c.n, false, tile) : tile * (int)blockDim.x + (int)threadIdx.x;
+        const int i = B ? balanced_particle(meta, c.n, false, tile) : (tile * (int)blockDim.x + (int)threadIdx.x) / L;
         if (i < 0 || i >= c.n) return;
         const float4 pi = pred[i], vi = velIn[i];
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) apply_viscosity_body<R, true>(c, b, pred, velIn, velOut, omega, near, rows, i, pi, vi, mt);
-        else apply_viscosity_body<R, false>(c, b, pred, velIn, velOut, omega, near, rows, i, pi, vi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) apply_viscosity_body<R, true, L>(c, b, pred, velIn, velOut, omega, near, rows, i, pi, vi, mt);
+        else apply_viscosity_body<R, false, L>(c, b, pred, velIn, velOut, omega, near, rows, i, pi, vi, mt);
     });
 }
 
 // apply_vorticity.cl:12-86; neighbours are read from near (apply_viscosity).
-template <bool R, bool Q>
+template <bool R, bool Q, int L>
 __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const float4* __restrict__ near,
                                                      const float4* __restrict__ omega,
                                                      const float4* __restrict__ velIn, float4* __restrict__ velOut,
@@ -1094,7 +1116,8 @@ __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const f
     const int n = c.n;
     float ex = 0.0f, ey = 0.0f, ez = 0.0f;
     auto load = [&](uint32_t j) { return __ldg(near + checked_index(j, (uint32_t)n, c.err, kErrFriendIndex)); };
-    walk_pairs(rows, n, i, FlatFriends(mt, kept_other(mt)).total, load, [&](const float4& pa, const float4& pb, bool va, bool vb) {
+    auto pass = [&](auto from) { ex = from(ex); ey = from(ey); ez = from(ez); };
+    walk_pairs<L>(rows, n, i, FlatFriends(mt, kept_other(mt)).total, load, [&](const float4& pa, const float4& pb, bool va, bool vb) {
         const F2 rx = pack2(pi.x - pa.x, pi.x - pb.x), ry = pack2(pi.y - pa.y, pi.y - pb.y),
                  rz = pack2(pi.z - pa.z, pi.z - pb.z);
         const F2 r2 = dot2(c, rx, ry, rz, rx, ry, rz);
@@ -1110,8 +1133,10 @@ __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const f
                 ey = fmaf(s, y1, ey);
                 ez = fmaf(s, z1, ez);
             };
-            if (va) add(pa.w, k.x, x.x, y.x, z.x);
-            if (vb) add(pb.w, k.y, x.y, y.y, z.y);
+            in_turn<L>([&] {
+                if (va) add(pa.w, k.x, x.x, y.x, z.x);
+                if (vb) add(pb.w, k.y, x.y, y.y, z.y);
+            }, pass);
         } else {
             F2 g0, g1, g2;
             if (Q) {
@@ -1131,10 +1156,13 @@ __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const f
             }
             const F2 ol = pack2(pa.w, pb.w);
             const float2 x = unpack2(mul2(ol, g0)), y = unpack2(mul2(ol, g1)), z = unpack2(mul2(ol, g2));
-            if (va) { ex = ex + x.x; ey = ey + y.x; ez = ez + z.x; }
-            if (vb) { ex = ex + x.y; ey = ey + y.y; ez = ez + z.y; }
+            in_turn<L>([&] {
+                if (va) { ex = ex + x.x; ey = ey + y.x; ez = ez + z.x; }
+                if (vb) { ex = ex + x.y; ey = ey + y.y; ez = ez + z.y; }
+            }, pass);
         }
     });
+    if (threadIdx.x % L) return;  // the sums are the first lane's
     ex = ex * c.negGradSpiky;
     ey = ey * c.negGradSpiky;
     ez = ez * c.negGradSpiky;
@@ -1163,7 +1191,7 @@ __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const f
     velOut[i] = make_float4(v.x + fx * c.dt, v.y + fy * c.dt, v.z + fz * c.dt, v.w + 0.0f);
 }
 
-template <bool R, bool B>
+template <bool R, bool B, int L>
 __global__ void __maxnreg__(56)
 apply_vorticity_kernel(DevConsts c, const float4* __restrict__ pred, const float4* __restrict__ near,
                        const float4* __restrict__ omega, const float4* __restrict__ velIn, float4* __restrict__ velOut,
@@ -1171,14 +1199,14 @@ apply_vorticity_kernel(DevConsts c, const float4* __restrict__ pred, const float
                        const uint4* __restrict__ rows, int tiles, int* tileCounter, int tileOffset) {
     chain_wait();
     for_tiles(tiles, tileCounter, [&](int tile) {
-        tile += tileOffset;  // a launch over part of the tiles (one block per tile)
-        const int i = B ? balanced_particle(meta, c.n, false, tile) : tile * (int)blockDim.x + (int)threadIdx.x;
+        tile += tileOffset * L;  // a launch over part of the tiles (L blocks per tile)
+        const int i = B ? balanced_particle(meta, c.n, false, tile) : (tile * (int)blockDim.x + (int)threadIdx.x) / L;
         if (i < 0 || i >= c.n) return;
         const float4 pi = pred[i];
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) apply_vorticity_body<R, true>(c, near, omega, velIn, velOut, tapeEta, rows, i, pi, mt);
-        else apply_vorticity_body<R, false>(c, near, omega, velIn, velOut, tapeEta, rows, i, pi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) apply_vorticity_body<R, true, L>(c, near, omega, velIn, velOut, tapeEta, rows, i, pi, mt);
+        else apply_vorticity_body<R, false, L>(c, near, omega, velIn, velOut, tapeEta, rows, i, pi, mt);
     });
 }
 
@@ -1207,6 +1235,14 @@ void launch_update_cells(int n, const uint32_t* keys, uint32_t* cells, uint32_t 
 
 void launch_reset_cells(int n, const uint32_t* keys, uint32_t* cells, uint32_t keyLimit, int* err, cudaStream_t s) {
     reset_cells_kernel<<<blocks_for(n), kBlock, 0, s>>>(n, keys, reinterpret_cast<uint2*>(cells), keyLimit, err);
+}
+
+// Lanes that share a particle in a solver pass (walk_pairs).  A substep of 2,048
+// / 8,192 / 16,384 / 32,768 / 65,536 particles takes 72 / 92 / 103 / 106 / 155 us
+// with one and 65 / 82 / 95 / 124 / 199 us with four: there the extra turns cost
+// more than the shorter chains save.
+int lanes_per_particle(int n, int balance, const int* tileCounter) {
+    return n <= 16384 && !balance && !tileCounter ? 4 : 1;
 }
 
 // Grid of a neighbour pass: one block per tile of `block` particles, or
@@ -1254,10 +1290,11 @@ void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const
 void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* predPacked, float* density,
                             float4* tapeSums, float* tapeRho, const uint2* meta, const uint4* rows, int block, int balance, int* tileCounter,
                             cudaStream_t s) {
-    auto k = c.relaxed ? (balance ? compute_scaling_kernel<true, true> : compute_scaling_kernel<true, false>)
-                       : (balance ? compute_scaling_kernel<false, true> : compute_scaling_kernel<false, false>);
+    const int lanes = lanes_per_particle(c.n, balance, tileCounter);
+    auto k = c.relaxed ? (lanes > 1 ? compute_scaling_kernel<true, false, 4> : balance ? compute_scaling_kernel<true, true, 1> : compute_scaling_kernel<true, false, 1>)
+                       : (lanes > 1 ? compute_scaling_kernel<false, false, 4> : balance ? compute_scaling_kernel<false, true, 1> : compute_scaling_kernel<false, false, 1>);
     int tiles = 0;
-    const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
+    const unsigned grid = grid_for_tiles(k, c.n * lanes, block, tileCounter != nullptr, &tiles);
     launch_chained(k, grid, block, s, c, pred, predPacked, density, tapeSums, tapeRho, meta, rows, tiles, tileCounter);
 }
 
@@ -1265,10 +1302,11 @@ void launch_compute_delta(const DevConsts& c, Batch b, const float4* predPacked,
                           const StepEnd& end, float4* predOut, const float* density, const uint2* meta, int lastIteration,
                           uint8_t* clampMask, const uint4* rows, int block, int balance, int* tileCounter,
                           cudaStream_t s) {
-    auto k = c.relaxed ? (balance ? compute_delta_kernel<true, true> : compute_delta_kernel<true, false>)
-                       : (balance ? compute_delta_kernel<false, true> : compute_delta_kernel<false, false>);
+    const int lanes = lanes_per_particle(c.n, balance, tileCounter);
+    auto k = c.relaxed ? (lanes > 1 ? compute_delta_kernel<true, false, 4> : balance ? compute_delta_kernel<true, true, 1> : compute_delta_kernel<true, false, 1>)
+                       : (lanes > 1 ? compute_delta_kernel<false, false, 4> : balance ? compute_delta_kernel<false, true, 1> : compute_delta_kernel<false, false, 1>);
     int tiles = 0;
-    const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
+    const unsigned grid = grid_for_tiles(k, c.n * lanes, block, tileCounter != nullptr, &tiles);
     launch_chained(k, grid, block, s, c, b, predPacked, posPrev, end, predOut, density, meta, lastIteration, clampMask, rows, tiles,
                              tileCounter);
 }
@@ -1281,24 +1319,26 @@ void launch_update_velocities(const DevConsts& c, const StepEnd& end, const floa
 void launch_apply_viscosity(const DevConsts& c, Batch b, const float4* pred, const float4* velIn, float4* velOut,
                             float4* omega, float4* near, const uint2* meta, const uint4* rows, int block, int balance,
                             int* tileCounter, cudaStream_t s) {
-    auto k = c.relaxed ? (balance ? apply_viscosity_kernel<true, true> : apply_viscosity_kernel<true, false>)
-                       : (balance ? apply_viscosity_kernel<false, true> : apply_viscosity_kernel<false, false>);
+    const int lanes = lanes_per_particle(c.n, balance, tileCounter);
+    auto k = c.relaxed ? (lanes > 1 ? apply_viscosity_kernel<true, false, 4> : balance ? apply_viscosity_kernel<true, true, 1> : apply_viscosity_kernel<true, false, 1>)
+                       : (lanes > 1 ? apply_viscosity_kernel<false, false, 4> : balance ? apply_viscosity_kernel<false, true, 1> : apply_viscosity_kernel<false, false, 1>);
     int tiles = 0;
-    const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
+    const unsigned grid = grid_for_tiles(k, c.n * lanes, block, tileCounter != nullptr, &tiles);
     launch_chained(k, grid, block, s, c, b, pred, velIn, velOut, omega, near, meta, rows, tiles, tileCounter);
 }
 
 void launch_apply_vorticity(const DevConsts& c, const float4* pred, const float4* near, const float4* omega,
                             const float4* velIn, float4* velOut, float4* tapeEta, const uint2* meta, const uint4* rows, int block, int balance,
                             int* tileCounter, cudaStream_t s, int firstTile, int tileCount) {
-    auto k = c.relaxed ? (balance ? apply_vorticity_kernel<true, true> : apply_vorticity_kernel<true, false>)
-                       : (balance ? apply_vorticity_kernel<false, true> : apply_vorticity_kernel<false, false>);
+    const int lanes = lanes_per_particle(c.n, balance, tileCounter);
+    auto k = c.relaxed ? (lanes > 1 ? apply_vorticity_kernel<true, false, 4> : balance ? apply_vorticity_kernel<true, true, 1> : apply_vorticity_kernel<true, false, 1>)
+                       : (lanes > 1 ? apply_vorticity_kernel<false, false, 4> : balance ? apply_vorticity_kernel<false, true, 1> : apply_vorticity_kernel<false, false, 1>);
     if (tileCount > 0) {  // tiles [firstTile, firstTile + tileCount), one block each
-        launch_chained(k, (unsigned)tileCount, block, s, c, pred, near, omega, velIn, velOut, tapeEta, meta, rows, 0, nullptr, firstTile);
+        launch_chained(k, (unsigned)(tileCount * lanes), block, s, c, pred, near, omega, velIn, velOut, tapeEta, meta, rows, 0, nullptr, firstTile);
         return;
     }
     int tiles = 0;
-    const unsigned grid = grid_for_tiles(k, c.n, block, tileCounter != nullptr, &tiles);
+    const unsigned grid = grid_for_tiles(k, c.n * lanes, block, tileCounter != nullptr, &tiles);
     launch_chained(k, grid, block, s, c, pred, near, omega, velIn, velOut, tapeEta, meta, rows, tiles, tileCounter, 0);
 }
 
