@@ -123,10 +123,10 @@ inline void launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, 
 // ---- kernels (pbf_kernels.cu) ----
 // counts (may be NULL): the number of particles of each key is added up there,
 // and perm receives each particle's place of arrival among them instead of its
-// own index.
+// own index (launch_compute_keys too).
 void launch_predict_keys(const DevConsts& c, Batch b, const float4* pos, float4* vel, float4* pred,
                          uint32_t* keys, uint32_t* perm, uint32_t* counts, int paused, cudaStream_t s);
-void launch_compute_keys(const DevConsts& c, Batch b, const float4* pred, uint32_t* keys, uint32_t* perm,
+void launch_compute_keys(const DevConsts& c, Batch b, const float4* pred, uint32_t* keys, uint32_t* perm, uint32_t* counts,
                          cudaStream_t s);
 // err (may be NULL): the error word that bounds-checked builds report bad
 // permutation entries or keys to; keyLimit: the number of cell-table entries.
@@ -206,9 +206,10 @@ int radix_sort_launches(const SortPlan& plan);
 // Taken by a substep whose keys are at most kCountingRatio times its particles
 // (or at most kCountingSmall), so that the scan over the key range (12 bytes a
 // key: 35 us for 2^24 keys at the measured copy rate) stays below the radix
-// passes that it replaces (65 us at 1M particles and three passes); the radix
-// sort above takes the others.
-constexpr uint64_t kCountingSmall = 1u << 20, kCountingRatio = 16;
+// passes that it replaces (65 us at 1M particles and three passes), and at least
+// a kCountingLoad-th of them: a particle reads its key's other particles.  The
+// radix sort above takes the others.
+constexpr uint64_t kCountingSmall = 1u << 20, kCountingRatio = 16, kCountingLoad = 64;
 struct CountingPlan {
     uint32_t blocks = 0;          // of the scan; 0: the radix sort
     uint32_t chunks = 0, chunksPerBlock = 0;
@@ -226,6 +227,12 @@ void launch_cell_gather(int n, const uint32_t* keys, const uint32_t* starts, con
                         uint32_t* permOut, uint32_t* permCopy, const float4* pos, const float4* pred,
                         const uint32_t* ids, float4* posOut, float4* predOut, uint32_t* idsOut, int* err,
                         cudaStream_t s);
+// For the entry points that sort without records: the stable permutation from
+// `order`, and the sorted keys (keysOut may still hold the particles' own keys
+// when the permutation is taken) and the cell table from `starts`.
+void launch_cell_rank(int n, const uint32_t* keys, const uint32_t* starts, const uint32_t* order, uint32_t* permOut,
+                      cudaStream_t s);
+void launch_cell_table(int n, uint32_t keys, const uint32_t* starts, uint32_t* keysOut, uint32_t* cells, cudaStream_t s);
 
 // ---- adjoint (pbf_adjoint.cu) ----
 // What one substep of a rollout leaves for its reverse pass.

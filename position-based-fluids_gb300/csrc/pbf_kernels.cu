@@ -42,6 +42,17 @@ __device__ __forceinline__ uint32_t key_base(const Batch& b, int i) {
     return b.scenes ? b.scenes[b.sceneOf[i]].keyBase : 0u;
 }
 
+// Adds the lanes of `valid` to their keys' counts; returns the lane's place
+// among its key's particles.  The particles come nearly sorted, a few keys to a
+// warp: one atomic per key and warp.
+__device__ __forceinline__ uint32_t place_of_arrival(unsigned valid, uint32_t key, uint32_t* __restrict__ counts) {
+    const unsigned peers = __match_any_sync(valid, key);
+    const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
+    uint32_t place = 0;
+    if (lane == leader) place = atomicAdd(&counts[key], (uint32_t)__popc(peers));
+    return __shfl_sync(valid, place, leader) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+}
+
 // ------------------------------------------------------------- predict --
 // predict_positions.cl:8-17 fused with computeKeys (radixsort.cl:7-19).
 __global__ void predict_keys_kernel(DevConsts c, Batch b, const float4* __restrict__ pos, float4* __restrict__ vel,
@@ -76,23 +87,21 @@ __global__ void predict_keys_kernel(DevConsts c, Batch b, const float4* __restri
             perm[i] = (uint32_t)i;
             return;
         }
-        // the particles come nearly sorted, a few keys to a warp: one atomic per key and warp
-        const unsigned peers = __match_any_sync(valid, key);
-        const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
-        uint32_t place = 0;
-        if (lane == leader) place = atomicAdd(&counts[key], (uint32_t)__popc(peers));
-        perm[i] = __shfl_sync(valid, place, leader) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+        perm[i] = place_of_arrival(valid, key, counts);
     }
 }
 
 // radixsort.cl:1-20 alone (keys of given predicted positions, no padding).
 __global__ void compute_keys_kernel(DevConsts c, Batch b, const float4* __restrict__ pred,
-                                    uint32_t* __restrict__ keys, uint32_t* __restrict__ perm) {
+                                    uint32_t* __restrict__ keys, uint32_t* __restrict__ perm,
+                                    uint32_t* __restrict__ counts) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned valid = __ballot_sync(0xFFFFFFFFu, i < c.n);
     if (i >= c.n) return;
     const float4 q = pred[i];
-    keys[i] = key_base(b, i) + grid_hash(__float2int_rz(q.x / c.h), __float2int_rz(q.y / c.h), __float2int_rz(q.z / c.h), c.grid);
-    perm[i] = (uint32_t)i;
+    const uint32_t key = key_base(b, i) + grid_hash(__float2int_rz(q.x / c.h), __float2int_rz(q.y / c.h), __float2int_rz(q.z / c.h), c.grid);
+    keys[i] = key;
+    perm[i] = counts ? place_of_arrival(valid, key, counts) : (uint32_t)i;
 }
 
 // radixsort.cl:22-37 (velocities are not permuted; they are recomputed
@@ -1218,9 +1227,9 @@ void launch_predict_keys(const DevConsts& c, Batch b, const float4* pos, float4*
     launch_chained(predict_keys_kernel, blocks_for(c.n), kBlock, s, c, b, pos, vel, pred, keys, perm, counts, paused);
 }
 
-void launch_compute_keys(const DevConsts& c, Batch b, const float4* pred, uint32_t* keys, uint32_t* perm,
+void launch_compute_keys(const DevConsts& c, Batch b, const float4* pred, uint32_t* keys, uint32_t* perm, uint32_t* counts,
                          cudaStream_t s) {
-    compute_keys_kernel<<<blocks_for(c.n), kBlock, 0, s>>>(c, b, pred, keys, perm);
+    compute_keys_kernel<<<blocks_for(c.n), kBlock, 0, s>>>(c, b, pred, keys, perm, counts);
 }
 
 void launch_gather_sorted(int n, const uint32_t* perm, const float4* pos, const float4* pred, const uint32_t* ids,

@@ -278,11 +278,50 @@ cell_gather_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __r
     idsOut[to] = id;
 }
 
+// The stable order without the records: permOut from the scattered order.
+__global__ void __launch_bounds__(kThreads)
+cell_rank_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ starts,
+                 const uint32_t* __restrict__ order, uint32_t* __restrict__ permOut) {
+    chain_wait();
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    const uint32_t i = order[s], key = keys[i], first = starts[key], end = starts[key + 1];
+    uint32_t to = first;
+    for (uint32_t q = first; q < end; ++q) to += order[q] < i;
+    permOut[to] = i;
+}
+
+// The sorted keys and the cell table (first and last particle of a key, both
+// all ones for none) from the first indices; the table may be NULL.  The last
+// particle of the only one of n = 1 is not written (update_cells.cl:11-25).
+__global__ void __launch_bounds__(kThreads)
+cell_table_kernel(int n, uint32_t keys, const uint32_t* __restrict__ starts, uint32_t* __restrict__ keysOut,
+                  uint32_t* __restrict__ cells) {
+    chain_wait();
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= keys) return;
+    const uint32_t first = starts[k], end = starts[k + 1];
+    if (cells) {
+        cells[2 * (size_t)k] = first < end ? first : kEmpty;
+        cells[2 * (size_t)k + 1] = first < end && n > 1 ? end - 1u : kEmpty;
+    }
+    for (uint32_t q = first; q < end; ++q) keysOut[q] = k;
+}
+
 }  // namespace
+
+void launch_cell_rank(int n, const uint32_t* keys, const uint32_t* starts, const uint32_t* order, uint32_t* permOut,
+                      cudaStream_t s) {
+    launch_chained(cell_rank_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keys, starts, order, permOut);
+}
+
+void launch_cell_table(int n, uint32_t keys, const uint32_t* starts, uint32_t* keysOut, uint32_t* cells, cudaStream_t s) {
+    launch_chained(cell_table_kernel, (keys + kThreads - 1) / kThreads, kThreads, s, n, keys, starts, keysOut, cells);
+}
 
 CountingPlan make_counting_plan(int n, uint64_t keys) {
     CountingPlan p;
-    if (keys > kCountingSmall && keys > kCountingRatio * (uint64_t)n) return p;
+    if ((keys > kCountingSmall && keys > kCountingRatio * (uint64_t)n) || (uint64_t)n > kCountingLoad * keys) return p;
     p.chunks = (uint32_t)((keys + 1 + kScanChunk - 1) / kScanChunk);  // one start beyond the last key
     // a key range of a few chunks is scanned by one block, which needs no sums of others before it
     p.chunksPerBlock = p.chunks <= kOneBlockChunks ? p.chunks : (p.chunks + kMaxScanBlocks - 1) / kMaxScanBlocks;
