@@ -321,8 +321,8 @@ void drop_graph(pbf_ctx* ctx);
 void free_render(pbf_ctx* ctx) {
     pbf::RenderBuffers& r = ctx->render;
     dev_free(r.dkey); dev_free(r.splat); dev_free(r.smooth); dev_free(r.out); dev_free(r.vis);
-    for (int k = 0; k < 2; ++k) { dev_free(r.keys[k]); dev_free(r.perm[k]); }
-    dev_free(r.hist); dev_free(r.cells);
+    dev_free(r.keys); dev_free(r.place); dev_free(r.order); dev_free(r.sorted);
+    dev_free(r.counts); dev_free(r.starts); dev_free(r.sums); dev_free(r.shownCount);
     r.width = r.height = r.n = 0;
 }
 
@@ -1231,22 +1231,23 @@ int pbf_render_frame(pbf_ctx* ctx, const PbfCamera* cam, int mode) {
     if (r.width != cam->width || r.height != cam->height || r.n != ctx->n) {
         free_render(ctx);
         const size_t n = (size_t)ctx->n;
-        r.plan = pbf::make_sort_plan(ctx->n, 1u << 23);
+        r.plan = pbf::make_scan_plan(pbf::render_grid_buckets());
         if ((rc = dev_alloc(ctx, &r.dkey, pixels)) || (rc = dev_alloc(ctx, &r.splat, pixels)) ||
             (rc = dev_alloc(ctx, &r.smooth, pixels)) || (rc = dev_alloc(ctx, &r.out, pixels)) ||
-            (rc = dev_alloc(ctx, &r.vis, n)) || (rc = dev_alloc(ctx, &r.keys[0], n)) ||
-            (rc = dev_alloc(ctx, &r.keys[1], n)) || (rc = dev_alloc(ctx, &r.perm[0], n)) ||
-            (rc = dev_alloc(ctx, &r.perm[1], n)) || (rc = dev_alloc(ctx, &r.hist, r.plan.histWords)) ||
-            (rc = dev_alloc(ctx, &r.cells, pbf::render_grid_words()))) {
+            (rc = dev_alloc(ctx, &r.vis, n)) || (rc = dev_alloc(ctx, &r.keys, n)) || (rc = dev_alloc(ctx, &r.place, n)) ||
+            (rc = dev_alloc(ctx, &r.order, n)) || (rc = dev_alloc(ctx, &r.sorted, n)) ||
+            (rc = dev_alloc(ctx, &r.counts, r.plan.words)) || (rc = dev_alloc(ctx, &r.starts, r.plan.words)) ||
+            (rc = dev_alloc(ctx, &r.sums, r.plan.blocks)) || (rc = dev_alloc(ctx, &r.shownCount, 1))) {
             free_render(ctx);
             return rc;
         }
+        PBF_CUDA(ctx, cudaMemsetAsync(r.counts, 0, 4 * r.plan.words, ctx->stream));
         r.width = cam->width;
         r.height = cam->height;
         r.n = ctx->n;
     }
     pbf::render_frame(*cam, mode, ctx->n, ctx->params.h, ctx->pos[ctx->curPos], r, ctx->stream);
-    ctx->launches += pbf::render_launches(mode, r.plan);
+    ctx->launches += pbf::render_launches(mode);
     ctx->renderMode = mode;
     PBF_CUDA(ctx, cudaGetLastError());
     PBF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -216,6 +216,10 @@ struct CountingPlan {
     size_t words = 0;             // counters, and first indices, as allocated
 };
 CountingPlan make_counting_plan(int n, uint64_t keys);
+CountingPlan make_scan_plan(uint64_t keys);  // whatever the number of particles
+// The first index of every key, and one beyond the last, from the counts, which
+// it leaves at zero.
+void launch_counting_scan(const CountingPlan& plan, uint32_t* counts, uint32_t* sums, uint32_t* starts, cudaStream_t s);
 // From the counts and the particles' places of arrival (launch_predict_keys):
 // the first index of every key into `starts`, and the particles grouped by key,
 // in any order within a key, into `order`.  Zeroes the counts.
@@ -270,14 +274,18 @@ struct RenderBuffers {
     float4* smooth = nullptr;            // fluid_depth_smoothing.fs output
     float4* out = nullptr;               // the frame
     uint8_t* vis = nullptr;              // per particle: seen in the splat
-    uint32_t* keys[2] = {nullptr, nullptr};
-    uint32_t* perm[2] = {nullptr, nullptr};
-    uint32_t* hist = nullptr;
-    uint32_t* cells = nullptr;           // 2 x 2048^2: first / last sorted index per bucket
-    SortPlan plan{};
+    uint32_t* keys = nullptr;            // per particle: its bucket
+    uint32_t* place = nullptr;           // per particle: its place of arrival in the bucket
+    uint32_t* order = nullptr;           // the visible particles grouped by bucket
+    float4* sorted = nullptr;            // their positions, by index within a bucket
+    uint32_t* counts = nullptr;          // per bucket (2048^2): its particles; zero between frames
+    uint32_t* starts = nullptr;          // per bucket: its first particle, and one beyond the last bucket
+    uint32_t* sums = nullptr;
+    uint32_t* shownCount = nullptr;      // sprites that draw_kernel draws
+    CountingPlan plan{};
 };
 void render_frame(const PbfCamera& cam, int mode, int n, float h, const float4* pos, RenderBuffers& rb, cudaStream_t s);
-int render_launches(int mode, const SortPlan& plan);
-size_t render_grid_words();
+int render_launches(int mode);
+uint64_t render_grid_buckets();
 
 }  // namespace pbf

@@ -14,7 +14,7 @@
 //             into 2048 x 2048 buckets.  The shader chains them with atomic
 //             exchanges (order left to the hardware); here the chain of a
 //             bucket is its particles in decreasing index order, from a
-//             stable radix sort by bucket.
+//             counting sort of the visible ones by bucket.
 //   smooth    fluid_depth_smoothing.fs: two Newton steps of the pixel's point
 //             along the camera ray towards the density shell sum (h^2 - r^2)^3
 //             = 1; colour = (window depth, normalized gradient).
@@ -119,20 +119,129 @@ __device__ __forceinline__ bool sprite(const PbfCamera& cam, float4 p, float& ex
     return true;
 }
 
-__global__ void splat_kernel(PbfCamera cam, int n, const float4* __restrict__ pos, unsigned long long* __restrict__ dkey) {
+// The pixels of a sprite's square.
+struct Rect {
+    int i0, i1, j0, j1;
+};
+__device__ __forceinline__ Rect sprite_rect(const PbfCamera& cam, float xw, float yw, float s) {
+    return {max(0, (int)ceilf(xw - s * 0.5f - 0.5f)), min(cam.width - 1, (int)ceilf(xw + s * 0.5f - 0.5f) - 1),
+            max(0, (int)ceilf(yw - s * 0.5f - 0.5f)), min(cam.height - 1, (int)ceilf(yw + s * 0.5f - 0.5f) - 1)};
+}
+
+// ---- occlusion ----
+//
+// A volume of particles is tens of sprites deep, and all but the nearest
+// fragments lose the depth test.  Under a perspective projection (checked on the
+// host: depth depends on the eye-space z alone, and grows with the distance) a
+// sprite that covers a tile of 8 x 8 pixels bounds the tile's final depth: its
+// farthest fragment there.  occlude_kernel takes the least such bound of every
+// tile; splat_kernel drops the tiles of a sprite whose nearest possible fragment
+// lies behind the bound, and most sprites altogether (262,144 particles at 1280 x
+// 720: 572 us for all fragments, one thread and one atomic after another for each
+// sprite; 45 us for the bounds, the list and the listed sprites).  The bounds leave kSlack,
+// above the few 2^-24 that the rounded depths can be off, so no fragment that
+// could win is dropped and the image is the same.
+constexpr int kTilePixels = 8;
+constexpr float kSlack = 1.0e-6f;
+__device__ __forceinline__ float depth_at(const PbfCamera& cam, float z) {
+    return ((cam.projection[10] * z + cam.projection[14]) / -z + 1.0f) / 2.0f;
+}
+
+__global__ void __launch_bounds__(128)
+occlude_kernel(PbfCamera cam, int n, const float4* __restrict__ pos, uint32_t* __restrict__ tileDepth) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     float ex, ey, ez, xw, yw, s;
     if (!sprite(cam, pos[p], ex, ey, ez, xw, yw, s)) return;
-    const int i0 = max(0, (int)ceilf(xw - s * 0.5f - 0.5f)), i1 = min(cam.width - 1, (int)ceilf(xw + s * 0.5f - 0.5f) - 1);
-    const int j0 = max(0, (int)ceilf(yw - s * 0.5f - 0.5f)), j1 = min(cam.height - 1, (int)ceilf(yw + s * 0.5f - 0.5f) - 1);
-    for (int j = j0; j <= j1; ++j)
-        for (int i = i0; i <= i1; ++i) {
-            Frag f;
-            if (!fragment(cam, ex, ey, ez, xw, yw, s, i, j, f)) continue;
-            const unsigned long long key = ((unsigned long long)__float_as_uint(f.depth) << 32) | (0xFFFFFFFFu - (uint32_t)p);
-            atomicMin(dkey + (size_t)j * cam.width + i, key);
+    // only sprites that lie inside the depth range as a whole, and wide enough to cover a tile
+    if (s < 1.5f * kTilePixels || !(ez + cam.pointSize < 0.0f)) return;
+    if (!(depth_at(cam, ez + cam.pointSize) > kSlack) || !(depth_at(cam, ez) < 1.0f - kSlack)) return;
+    const Rect r = sprite_rect(cam, xw, yw, s);
+    const int tilesX = (cam.width + kTilePixels - 1) / kTilePixels;
+    const float scale = 2.0f / s;
+    for (int tj = r.j0 / kTilePixels; tj <= r.j1 / kTilePixels; ++tj) {
+        const float y0 = ((float)(tj * kTilePixels) + 0.5f - yw) * scale, y1 = y0 + (float)(kTilePixels - 1) * scale;
+        const float y = fmaxf(fabsf(y0), fabsf(y1));
+        for (int ti = r.i0 / kTilePixels; ti <= r.i1 / kTilePixels; ++ti) {
+            const float x0 = ((float)(ti * kTilePixels) + 0.5f - xw) * scale, x1 = x0 + (float)(kTilePixels - 1) * scale;
+            const float x = fmaxf(fabsf(x0), fabsf(x1));
+            const float mag = x * x + y * y;  // of the tile's farthest pixel centre
+            if (!(mag < 0.99f)) continue;
+            const float far = depth_at(cam, ez + 0.999f * sqrtf(1.0f - mag) * cam.pointSize) + kSlack;
+            uint32_t* bound = tileDepth + (size_t)tj * tilesX + ti;
+            if (__float_as_uint(far) < *bound) atomicMin(bound, __float_as_uint(far));
         }
+    }
+}
+
+// A fragment's depth test.
+__device__ __forceinline__ void draw(const PbfCamera& cam, float ex, float ey, float ez, float xw, float yw, float s,
+                                     int p, int i, int j, unsigned long long* __restrict__ dkey) {
+    Frag f;
+    if (!fragment(cam, ex, ey, ez, xw, yw, s, i, j, f)) return;
+    const unsigned long long key = ((unsigned long long)__float_as_uint(f.depth) << 32) | (0xFFFFFFFFu - (uint32_t)p);
+    unsigned long long* at = dkey + (size_t)j * cam.width + i;
+    if (key < *at) atomicMin(at, key);  // an old value is larger, so a stale read only costs the atomic
+}
+
+__device__ __forceinline__ uint32_t nearest_depth(const PbfCamera& cam, float ez) {
+    const float nearest = ez + cam.pointSize < 0.0f ? depth_at(cam, ez + cam.pointSize) - kSlack : 0.0f;
+    return nearest > 0.0f ? __float_as_uint(nearest) : 0u;
+}
+
+// Draws the small sprites, a thread each, and lists the others that are not
+// hidden in every tile.  tileDepth NULL: no occlusion bounds.
+constexpr int kSmallSprite = 36;  // pixels that one thread draws
+__global__ void __launch_bounds__(128)
+splat_kernel(PbfCamera cam, int n, const float4* __restrict__ pos, const uint32_t* __restrict__ tileDepth,
+             unsigned long long* __restrict__ dkey, uint32_t* __restrict__ shown, uint32_t* __restrict__ shownCount) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    float ex, ey, ez, xw, yw, s;
+    if (!sprite(cam, pos[p], ex, ey, ez, xw, yw, s)) return;
+    const Rect r = sprite_rect(cam, xw, yw, s);
+    const int tilesX = (cam.width + kTilePixels - 1) / kTilePixels;
+    const uint32_t nearest = nearest_depth(cam, ez);
+    bool visible = tileDepth == nullptr;
+    for (int tj = r.j0 / kTilePixels; !visible && tj <= r.j1 / kTilePixels; ++tj)
+        for (int ti = r.i0 / kTilePixels; !visible && ti <= r.i1 / kTilePixels; ++ti)
+            visible = nearest <= tileDepth[(size_t)tj * tilesX + ti];
+    if (!visible) return;
+    if ((r.i1 - r.i0 + 1) * (r.j1 - r.j0 + 1) <= kSmallSprite) {
+        for (int j = r.j0; j <= r.j1; ++j)
+            for (int i = r.i0; i <= r.i1; ++i) draw(cam, ex, ey, ez, xw, yw, s, p, i, j, dkey);
+    } else {
+        shown[atomicAdd(shownCount, 1u)] = (uint32_t)p;
+    }
+}
+
+// The listed sprites, a warp each, tile by tile: the sprites that remain lie
+// together in memory, so they are dealt out over the whole chip.
+constexpr int kDrawBlocks = 152 * 16;
+__global__ void __launch_bounds__(128)
+draw_kernel(PbfCamera cam, const float4* __restrict__ pos, const uint32_t* __restrict__ tileDepth,
+            unsigned long long* __restrict__ dkey, const uint32_t* __restrict__ shown,
+            const uint32_t* __restrict__ shownCount) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t count = *shownCount;
+    const int tilesX = (cam.width + kTilePixels - 1) / kTilePixels;
+    for (uint32_t k = blockIdx.x * 4 + (threadIdx.x >> 5); k < count; k += kDrawBlocks * 4) {
+        const int p = (int)shown[k];
+        float ex, ey, ez, xw, yw, s;
+        sprite(cam, pos[p], ex, ey, ez, xw, yw, s);
+        const Rect r = sprite_rect(cam, xw, yw, s);
+        const uint32_t nearest = nearest_depth(cam, ez);
+        for (int tj = r.j0 / kTilePixels; tj <= r.j1 / kTilePixels; ++tj)
+            for (int ti = r.i0 / kTilePixels; ti <= r.i1 / kTilePixels; ++ti) {
+                if (tileDepth && nearest > tileDepth[(size_t)tj * tilesX + ti]) continue;
+                const int i = ti * kTilePixels + lane % kTilePixels;
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int j = tj * kTilePixels + 4 * half + lane / kTilePixels;
+                    if (i >= r.i0 && i <= r.i1 && j >= r.j0 && j <= r.j1) draw(cam, ex, ey, ez, xw, yw, s, p, i, j, dkey);
+                }
+            }
+    }
 }
 
 // hsv2rgb of particles_color.fs, mix(a, b, t) = a (1 - t) + b t
@@ -145,18 +254,26 @@ __device__ __forceinline__ float hsv_channel(float h, float k, float s, float v)
 }
 
 __global__ void resolve_kernel(PbfCamera cam, int n, int mode, const float4* __restrict__ pos,
-                               const unsigned long long* __restrict__ dkey, float4* __restrict__ splat) {
+                               const unsigned long long* __restrict__ dkey, float4* __restrict__ splat,
+                               uint8_t* __restrict__ vis) {
     const int pix = blockIdx.x * blockDim.x + threadIdx.x;
     if (pix >= cam.width * cam.height) return;
     const unsigned long long key = dkey[pix];
+    // vis_scan.cms, in mode 0: the particle that the pixel's colour names, also an empty pixel's
+    auto mark = [&](float colour) {
+        const uint32_t x = (uint32_t)(colour + 0.5f);
+        if (x < (uint32_t)n && vis[x] == 0) vis[x] = 1;
+    };
     if (key == kEmptyKey) {
         splat[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (mode == 0) mark(0.0f);
         return;
     }
     const uint32_t p = 0xFFFFFFFFu - (uint32_t)(key & 0xFFFFFFFFu);
     const float depth = __uint_as_float((uint32_t)(key >> 32));
     if (mode == 0) {
         splat[pix] = make_float4(depth, (float)(int)p, 0.0f, 1.0f);
+        mark((float)(int)p);
         return;
     }
     const int i = pix % cam.width, j = pix / cam.width;
@@ -181,48 +298,60 @@ __global__ void resolve_kernel(PbfCamera cam, int n, int mode, const float4* __r
     splat[pix] = make_float4(r * cosA, g * cosA, b * cosA, 1.0f * cosA);
 }
 
-__global__ void visible_kernel(int pixels, int n, const float4* __restrict__ splat, uint8_t* __restrict__ vis) {
-    const int pix = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pix >= pixels) return;
-    const uint32_t x = (uint32_t)(splat[pix].y + 0.5f);
-    if (x < (uint32_t)n) vis[x] = 1;
-}
-
-__global__ void grid_keys_kernel(int n, float h, const float4* __restrict__ pos, const uint8_t* __restrict__ vis,
-                                 uint32_t* __restrict__ keys, uint32_t* __restrict__ perm) {
+// Bucket and place of arrival of the visible particles (kGridBuckets: not visible).
+__global__ void grid_count_kernel(int n, float h, const float4* __restrict__ pos, const uint8_t* __restrict__ vis,
+                                  uint32_t* __restrict__ keys, uint32_t* __restrict__ place, uint32_t* __restrict__ counts) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float4 p = pos[i];
-    keys[i] = vis[i] ? render_hash(to_int(p.x / h), to_int(p.y / h), to_int(p.z / h)) : kGridBuckets;
-    perm[i] = (uint32_t)i;
+    uint32_t key = kGridBuckets;
+    if (vis[i]) {
+        const float4 p = pos[i];
+        key = render_hash(to_int(p.x / h), to_int(p.y / h), to_int(p.z / h));
+        place[i] = atomicAdd(&counts[key], 1u);
+    }
+    keys[i] = key;
 }
 
-// first / last sorted index of every bucket (0xFFFFFFFF where empty)
-__global__ void grid_cells_kernel(int n, const uint32_t* __restrict__ keys, uint32_t* __restrict__ cells) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const uint32_t key = keys[k];
-    if (key >= kGridBuckets) return;
-    if (k == 0 || keys[k - 1] != key) cells[2 * (size_t)key] = (uint32_t)k;
-    if (k == n - 1 || keys[k + 1] != key) cells[2 * (size_t)key + 1] = (uint32_t)k;
+__global__ void grid_scatter_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ place,
+                                    const uint32_t* __restrict__ starts, uint32_t* __restrict__ order) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n || keys[i] >= kGridBuckets) return;
+    order[starts[keys[i]] + place[i]] = (uint32_t)i;
+}
+
+// The positions of each bucket's particles by increasing index.
+__global__ void grid_rank_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ starts,
+                                 const uint32_t* __restrict__ order, const float4* __restrict__ pos,
+                                 float4* __restrict__ sorted) {
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= starts[kGridBuckets]) return;
+    const uint32_t i = order[s], key = keys[i], first = starts[key], end = starts[key + 1];
+    uint32_t to = first;
+    for (uint32_t q = first; q < end; ++q) to += order[q] < i;
+    sorted[to] = pos[i];
 }
 
 // fluid_depth_smoothing.fs SampleDensityAndGradient
-__device__ void sample_density(float h, const float4* __restrict__ pos, const uint32_t* __restrict__ perm,
-                               const uint32_t* __restrict__ cells, float wx, float wy, float wz, float& density,
+__device__ void sample_density(float h, const float4* __restrict__ sorted, const uint32_t* __restrict__ starts, float wx, float wy, float wz, float& density,
                                float& gx, float& gy, float& gz) {
     const float h2 = h * h;
     density = 0.0f;
     gx = gy = gz = 0.0f;
     const int cx = to_int(wx / h), cy = to_int(wy / h), cz = to_int(wz / h);
+    // render_hash of the 27 buckets from the spread coordinates of each axis; the Morton number is below 2^30
+    const uint32_t sx0 = expand_bits_i(cx - 1), sx1 = expand_bits_i(cx), sx2 = expand_bits_i(cx + 1);
+#pragma unroll 1
     for (int iz = -1; iz <= 1; ++iz)
-        for (int iy = -1; iy <= 1; ++iy)
-            for (int ix = -1; ix <= 1; ++ix) {
-                const uint32_t b = render_hash(cx + ix, cy + iy, cz + iz);
-                const uint32_t first = cells[2 * (size_t)b];
-                if (first == 0xFFFFFFFFu) continue;
-                for (int k = (int)cells[2 * (size_t)b + 1]; k >= (int)first; --k) {
-                    const float4 pp = pos[perm[k]];
+#pragma unroll 1
+        for (int iy = -1; iy <= 1; ++iy) {
+            const uint32_t yz = (expand_bits_i(cy + iy) << 1) | (expand_bits_i(cz + iz) << 2);
+#pragma unroll 1
+            for (int ix = 0; ix < 3; ++ix) {
+                const uint32_t b = ((ix == 0 ? sx0 : ix == 1 ? sx1 : sx2) | yz) & (kGridBuckets - 1u);
+                const int first = (int)starts[b];
+#pragma unroll 4
+                for (int k = (int)starts[b + 1] - 1; k >= first; --k) {
+                    const float4 pp = __ldg(sorted + k);
                     const float dx = pp.x - wx, dy = pp.y - wy, dz = pp.z - wz;
                     const float r2 = dot3f(dx, dy, dz, dx, dy, dz);
                     if (r2 < h2) {
@@ -234,6 +363,7 @@ __device__ void sample_density(float h, const float4* __restrict__ pos, const ui
                     }
                 }
             }
+        }
     density = density * 1.0f;
     gx = gx * -6.0f;
     gy = gy * -6.0f;
@@ -256,12 +386,16 @@ __device__ __forceinline__ void normalize3(float& x, float& y, float& z) {
     z = z / l;
 }
 
-__global__ void smooth_kernel(PbfCamera cam, float h, const float4* __restrict__ pos, const uint32_t* __restrict__ perm,
-                              const uint32_t* __restrict__ cells, const float4* __restrict__ splat,
-                              float4* __restrict__ out) {
-    const int pix = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pix >= cam.width * cam.height) return;
-    const int i = pix % cam.width, j = pix / cam.width;
+// A warp takes 8 x 4 pixels, whose points lie in the same few buckets; bound by
+// instruction issue (85 %): 141 us with a row of pixels and the positions behind
+// the permutation, 118 like this (the scene above).
+__global__ void __launch_bounds__(128)
+smooth_kernel(PbfCamera cam, float h, const float4* __restrict__ sorted, const uint32_t* __restrict__ starts,
+              const float4* __restrict__ splat, float4* __restrict__ out) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = blockIdx.x * 16 + 8 * (warp & 1) + (lane & 7), j = blockIdx.y * 8 + 4 * (warp >> 1) + (lane >> 3);
+    if (i >= cam.width || j >= cam.height) return;
+    const int pix = j * cam.width + i;
     const float z = splat[pix].x;
     out[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (z == 1.0f) return;  // the far plane: discard
@@ -272,7 +406,7 @@ __global__ void smooth_kernel(PbfCamera cam, float h, const float4* __restrict__
     float tp = 0.0f, sx = m.x, sy = m.y, sz = m.z;
     float density, gx = 0.0f, gy = 0.0f, gz = 0.0f;
     for (int it = 0; it < 2; ++it) {
-        sample_density(h, pos, perm, cells, sx, sy, sz, density, gx, gy, gz);
+        sample_density(h, sorted, starts, sx, sy, sz, density, gx, gy, gz);
         const float dd = density - 1.0f;
         const float ga = dot3f(nx, ny, nz, gx, gy, gz);
         tp += dd / ga;
@@ -323,32 +457,49 @@ __global__ void final_kernel(PbfCamera cam, const float4* __restrict__ smooth, f
 
 inline unsigned blocks(size_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
+// A perspective projection as depth_at takes it: the clip z and w depend on the
+// eye-space z alone, w is the distance, and depth grows with it.
+bool plain_perspective(const PbfCamera& cam) {
+    const float* m = cam.projection;
+    return m[2] == 0.0f && m[6] == 0.0f && m[3] == 0.0f && m[7] == 0.0f && m[11] == -1.0f && m[15] == 0.0f &&
+           m[10] < 0.0f && m[10] >= -2.0f && m[14] < 0.0f && m[14] > -1.0e6f && cam.pointSize > 0.0f &&
+           cam.pointSize < 1.0e6f;
+}
+
 }  // namespace
 
-int render_launches(int mode, const SortPlan& plan) {
-    return mode == 0 ? 6 + radix_sort_launches(plan) : 2;
-}
+int render_launches(int mode) { return mode == 0 ? 11 : 4; }
 
 void render_frame(const PbfCamera& cam, int mode, int n, float h, const float4* pos, RenderBuffers& rb,
                   cudaStream_t s) {
     const size_t pixels = (size_t)cam.width * cam.height;
     cudaMemsetAsync(rb.dkey, 0xFF, 8 * pixels, s);
-    splat_kernel<<<blocks(n, 128), 128, 0, s>>>(cam, n, pos, rb.dkey);
-    resolve_kernel<<<blocks(pixels, 256), 256, 0, s>>>(cam, n, mode, pos, rb.dkey, rb.splat);
+    // the bounds of the tiles live in the smoothed image, and the list of sprites in the grid's order: both are
+    // written later
+    uint32_t* tileDepth = plain_perspective(cam) ? reinterpret_cast<uint32_t*>(rb.smooth) : nullptr;
+    cudaMemsetAsync(rb.shownCount, 0, 4, s);
+    if (tileDepth) {
+        const size_t tiles = (size_t)((cam.width + kTilePixels - 1) / kTilePixels) * ((cam.height + kTilePixels - 1) / kTilePixels);
+        cudaMemsetAsync(tileDepth, 0x7F, 4 * tiles, s);  // a depth above every other
+        occlude_kernel<<<blocks(n, 128), 128, 0, s>>>(cam, n, pos, tileDepth);
+    }
+    splat_kernel<<<blocks(n, 128), 128, 0, s>>>(cam, n, pos, tileDepth, rb.dkey, rb.order, rb.shownCount);
+    draw_kernel<<<kDrawBlocks, 128, 0, s>>>(cam, pos, tileDepth, rb.dkey, rb.order, rb.shownCount);
+    if (mode == 0) cudaMemsetAsync(rb.vis, 0, (size_t)n, s);
+    resolve_kernel<<<blocks(pixels, 256), 256, 0, s>>>(cam, n, mode, pos, rb.dkey, rb.splat, rb.vis);
     if (mode != 0) {
         cudaMemcpyAsync(rb.out, rb.splat, 16 * pixels, cudaMemcpyDeviceToDevice, s);
         return;
     }
-    cudaMemsetAsync(rb.vis, 0, (size_t)n, s);
-    visible_kernel<<<blocks(pixels, 256), 256, 0, s>>>((int)pixels, n, rb.splat, rb.vis);
-    grid_keys_kernel<<<blocks(n, 256), 256, 0, s>>>(n, h, pos, rb.vis, rb.keys[0], rb.perm[0]);
-    const int cur = launch_radix_sort(rb.plan, rb.keys, rb.perm, rb.hist, nullptr, nullptr, nullptr, nullptr, s);
-    cudaMemsetAsync(rb.cells, 0xFF, 8 * (size_t)kGridBuckets, s);
-    grid_cells_kernel<<<blocks(n, 256), 256, 0, s>>>(n, rb.keys[cur], rb.cells);
-    smooth_kernel<<<blocks(pixels, 128), 128, 0, s>>>(cam, h, pos, rb.perm[cur], rb.cells, rb.splat, rb.smooth);
+    grid_count_kernel<<<blocks(n, 256), 256, 0, s>>>(n, h, pos, rb.vis, rb.keys, rb.place, rb.counts);
+    launch_counting_scan(rb.plan, rb.counts, rb.sums, rb.starts, s);
+    grid_scatter_kernel<<<blocks(n, 256), 256, 0, s>>>(n, rb.keys, rb.place, rb.starts, rb.order);
+    grid_rank_kernel<<<blocks(n, 256), 256, 0, s>>>(rb.keys, rb.starts, rb.order, pos, rb.sorted);
+    smooth_kernel<<<dim3(blocks(cam.width, 16), blocks(cam.height, 8)), 128, 0, s>>>(cam, h, rb.sorted, rb.starts, rb.splat,
+                                                                                    rb.smooth);
     final_kernel<<<blocks(pixels, 256), 256, 0, s>>>(cam, rb.smooth, rb.out);
 }
 
-size_t render_grid_words() { return 2 * (size_t)kGridBuckets; }
+uint64_t render_grid_buckets() { return kGridBuckets; }
 
 }  // namespace pbf

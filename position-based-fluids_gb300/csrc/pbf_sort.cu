@@ -216,8 +216,8 @@ counting_scan_kernel(uint4* __restrict__ counts, uint32_t chunks, uint32_t chunk
     for (uint32_t k = first; k < last; ++k) {
         const size_t at = (size_t)k * kThreads + t;
         const uint4 v = counts[at];
-        counts[at] = make_uint4(0u, 0u, 0u, 0u);
         const uint32_t sum = (v.x + v.y) + (v.z + v.w);
+        if (sum) counts[at] = make_uint4(0u, 0u, 0u, 0u);
         uint32_t incl = sum;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -320,8 +320,13 @@ void launch_cell_table(int n, uint32_t keys, const uint32_t* starts, uint32_t* k
 }
 
 CountingPlan make_counting_plan(int n, uint64_t keys) {
+    if ((keys > kCountingSmall && keys > kCountingRatio * (uint64_t)n) || (uint64_t)n > kCountingLoad * keys)
+        return CountingPlan{};
+    return make_scan_plan(keys);
+}
+
+CountingPlan make_scan_plan(uint64_t keys) {
     CountingPlan p;
-    if ((keys > kCountingSmall && keys > kCountingRatio * (uint64_t)n) || (uint64_t)n > kCountingLoad * keys) return p;
     p.chunks = (uint32_t)((keys + 1 + kScanChunk - 1) / kScanChunk);  // one start beyond the last key
     // a key range of a few chunks is scanned by one block, which needs no sums of others before it
     p.chunksPerBlock = p.chunks <= kOneBlockChunks ? p.chunks : (p.chunks + kMaxScanBlocks - 1) / kMaxScanBlocks;
@@ -330,14 +335,18 @@ CountingPlan make_counting_plan(int n, uint64_t keys) {
     return p;
 }
 
-void launch_counting_sort(const CountingPlan& plan, int n, uint32_t* counts, uint32_t* sums, uint32_t* starts,
-                          const uint32_t* keys, const uint32_t* place, uint32_t* order, int* err, cudaStream_t s) {
+void launch_counting_scan(const CountingPlan& plan, uint32_t* counts, uint32_t* sums, uint32_t* starts, cudaStream_t s) {
     uint4* c4 = reinterpret_cast<uint4*>(counts);
     if (plan.blocks > 1)
         launch_chained(counting_sums_kernel, plan.blocks, kThreads, s, c4, plan.chunks, plan.chunksPerBlock,
                                                                       sums);
     launch_chained(counting_scan_kernel, plan.blocks, kThreads, s, c4, plan.chunks, plan.chunksPerBlock, sums,
                                                           reinterpret_cast<uint4*>(starts));
+}
+
+void launch_counting_sort(const CountingPlan& plan, int n, uint32_t* counts, uint32_t* sums, uint32_t* starts,
+                          const uint32_t* keys, const uint32_t* place, uint32_t* order, int* err, cudaStream_t s) {
+    launch_counting_scan(plan, counts, sums, starts, s);
     launch_chained(cell_scatter_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keys, place, starts, order, err);
 }
 
