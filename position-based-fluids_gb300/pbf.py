@@ -476,7 +476,8 @@ class Simulation:
         return ids
 
     def positions_by_id(self) -> np.ndarray:
-        pos, _, _ = self.read_state()
+        pos = np.empty((self.n, 4), np.float32)
+        self.read_state_into(pos.ctypes.data)
         out = np.empty_like(pos)
         out[self.read_ids()] = pos
         return out
