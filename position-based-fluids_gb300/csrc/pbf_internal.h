@@ -146,8 +146,9 @@ void launch_reset_cells(int n, const uint32_t* keys, uint32_t* cells, uint32_t k
 void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const uint32_t* cells,
                           const uint32_t* starts, uint4* rows, uint2* meta, int* errorWord, int block, int algorithm,
                           cudaStream_t s);
-// uint4 entries per particle of the rows for `slots` friends.
-inline size_t row_entries(int slots) { return ((size_t)slots + 3) / 4; }
+// uint4 entries per particle of the rows for `slots` friends, at least the four
+// that eight lanes read ahead (first_entry in pbf_device.cuh).
+inline size_t row_entries(int slots) { return slots > 16 ? ((size_t)slots + 3) / 4 : 4; }
 // tapeSums, tapeRho, tapeEta below: a rollout's tape (AdjointTape; NULL without).
 void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* predPacked, float* density,
                             float4* tapeSums, float* tapeRho, const uint2* meta, const uint4* rows, int block, int balance, int* tileCounter,

@@ -722,7 +722,7 @@ template <bool R, bool Q, int L>
 __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const float4* __restrict__ pred,
                                                      float4* __restrict__ predPacked, float* __restrict__ density,
                                                      float4* __restrict__ tapeSums, float* __restrict__ tapeRho,
-                                                     const uint4* __restrict__ rows, int i, const float4 pi, uint64_t mt) {
+                                                     const uint4* __restrict__ rows, int i, uint4 head, const float4 pi, uint64_t mt) {
     const int n = c.n;
     // complete neighbour sets count the particle itself first: d = h^2 - 0
     float ds = c.complete ? c.h2 * c.h2 * c.h2 : 0.0f, gsk = 0.0f, gx = 0.0f, gy = 0.0f, gz = 0.0f;
@@ -739,8 +739,11 @@ __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const f
         gy = gy + g1;
         gz = gz + g2;
     };
+    constexpr bool kLaneSums = L > 1 && Q && !R;  // the other forms go in_turn
+    __shared__ __align__(16) float terms[kLaneSums ? kMaxBlock / L * LaneSums<L, 5>::kStride : 1];
+    LaneSums<L, 5> sums(terms, {ds, gsk, gx, gy, gz});
     auto pass = [&](auto from) { ds = from(ds); gsk = from(gsk); gx = from(gx); gy = from(gy); gz = from(gz); };
-    walk_pairs<L>(rows, n, i, FlatFriends(mt, kept_density(mt)).total, load, [&](const float4& pa, const float4& pb, bool va, bool vb) {
+    walk_pairs<L>(rows, n, i, head, FlatFriends(mt, kept_density(mt)).total, load, [&](const float4& pa, const float4& pb, bool va, bool vb) {
         const F2 rx = pack2(pi.x - pa.x, pi.x - pb.x), ry = pack2(pi.y - pa.y, pi.y - pb.y),
                  rz = pack2(pi.z - pa.z, pi.z - pb.z);
         const F2 r2 = R ? fma2(rz, rz, fma2(ry, ry, mul2(rx, rx))) : dot2(c, rx, ry, rz, rx, ry, rz);
@@ -789,6 +792,10 @@ __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const f
             }, pass);
         } else {
             const float2 d3 = unpack2(mul2(mul2(d, d), d)), gg = unpack2(dot2(c, g0, g1, g2, g0, g1, g2));
+            if constexpr (kLaneSums) {
+                sums.add(va, vb, {d3, gg, x, y, z});
+                return;
+            }
             in_turn<L>([&] {
                 if (va) {
                     ds = ds + d3.x;
@@ -803,6 +810,13 @@ __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const f
             }, pass);
         }
     });
+    if constexpr (kLaneSums) {
+        ds = sums.template get<0>();
+        gsk = sums.template get<1>();
+        gx = sums.template get<2>();
+        gy = sums.template get<3>();
+        gz = sums.template get<4>();
+    }
     if (threadIdx.x % L) return;  // the sums are the first lane's
     ds = ds * c.poly6;
     density[i] = ds;
@@ -826,10 +840,11 @@ compute_scaling_kernel(DevConsts c, const float4* __restrict__ pred, float4* __r
         const int i = B ? balanced_particle(meta, c.n, true, tile) : (tile * (int)blockDim.x + (int)threadIdx.x) / L;
         if (i < 0 || i >= c.n) return;
         const float4 pi = pred[i];
+        const uint4 head = first_entry<L>(rows, c.n, i);
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) compute_scaling_body<R, true, L>(c, pred, predPacked, density, tapeSums, tapeRho, rows, i, pi, mt);
-        else compute_scaling_body<R, false, L>(c, pred, predPacked, density, tapeSums, tapeRho, rows, i, pi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) compute_scaling_body<R, true, L>(c, pred, predPacked, density, tapeSums, tapeRho, rows, i, head, pi, mt);
+        else compute_scaling_body<R, false, L>(c, pred, predPacked, density, tapeSums, tapeRho, rows, i, head, pi, mt);
     });
 }
 
@@ -862,7 +877,7 @@ __device__ __forceinline__ void compute_delta_body(const DevConsts& c, const Bat
                                                    float4* __restrict__ predOut,
                                                    const float* __restrict__ density, int lastIteration,
                                                    uint8_t* __restrict__ clampMask, const uint4* __restrict__ rows,
-                                                   int i, const float4 pi, uint64_t mt) {
+                                                   int i, uint4 head, const float4 pi, uint64_t mt) {
     const int n = c.n;
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
     auto load = [&](uint32_t j) { return __ldg(pp + checked_index(j, (uint32_t)n, c.err, kErrFriendIndex)); };
@@ -879,8 +894,11 @@ __device__ __forceinline__ void compute_delta_body(const DevConsts& c, const Bat
         sy = sy + a * g1;
         sz = sz + a * g2;
     };
+    constexpr bool kLaneSums = L > 1 && Q && !R;  // the other forms go in_turn
+    __shared__ __align__(16) float terms[kLaneSums ? kMaxBlock / L * LaneSums<L, 3>::kStride : 1];
+    LaneSums<L, 3> sums(terms, {0.0f, 0.0f, 0.0f});
     auto pass = [&](auto from) { sx = from(sx); sy = from(sy); sz = from(sz); };
-    walk_pairs<L>(rows, n, i, FlatFriends(mt, kept_other(mt)).total, load, [&](const float4& pa, const float4& pb, bool va, bool vb) {
+    walk_pairs<L>(rows, n, i, head, FlatFriends(mt, kept_other(mt)).total, load, [&](const float4& pa, const float4& pb, bool va, bool vb) {
         const F2 rx = pack2(pi.x - pa.x, pi.x - pb.x), ry = pack2(pi.y - pa.y, pi.y - pb.y),
                  rz = pack2(pi.z - pa.z, pi.z - pb.z);
         const F2 r2 = R ? fma2(rz, rz, fma2(ry, ry, mul2(rx, rx))) : dot2(c, rx, ry, rz, rx, ry, rz);
@@ -924,12 +942,21 @@ __device__ __forceinline__ void compute_delta_body(const DevConsts& c, const Bat
             }
             const F2 a = add2(wij, product2(c, mul2(mul2(mul2(both(c.K), rq), rq), rq), rq));
             const float2 x = unpack2(mul2(a, g0)), v = unpack2(mul2(a, g1)), z = unpack2(mul2(a, g2));
+            if constexpr (kLaneSums) {
+                sums.add(va, vb, {x, v, z});
+                return;
+            }
             in_turn<L>([&] {
                 if (va) { sx = sx + x.x; sy = sy + v.x; sz = sz + z.x; }
                 if (vb) { sx = sx + x.y; sy = sy + v.y; sz = sz + z.y; }
             }, pass);
         }
     });
+    if constexpr (kLaneSums) {
+        sx = sums.template get<0>();
+        sy = sums.template get<1>();
+        sz = sums.template get<2>();
+    }
     if (threadIdx.x % L) return;  // the sums are the first lane's
     float fx, fy, fz;
     if (R) {
@@ -983,10 +1010,11 @@ compute_delta_kernel(DevConsts c, Batch b, const float4* __restrict__ pp, const 
         const int i = B ? balanced_particle(meta, c.n, false, tile) : (tile * (int)blockDim.x + (int)threadIdx.x) / L;
         if (i < 0 || i >= c.n) return;
         const float4 pi = pp[i];
+        const uint4 head = first_entry<L>(rows, c.n, i);
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) compute_delta_body<R, true, L>(c, b, pp, posPrev, end, predOut, density, lastIteration, clampMask, rows, i, pi, mt);
-        else compute_delta_body<R, false, L>(c, b, pp, posPrev, end, predOut, density, lastIteration, clampMask, rows, i, pi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) compute_delta_body<R, true, L>(c, b, pp, posPrev, end, predOut, density, lastIteration, clampMask, rows, i, head, pi, mt);
+        else compute_delta_body<R, false, L>(c, b, pp, posPrev, end, predOut, density, lastIteration, clampMask, rows, i, head, pi, mt);
     });
 }
 
@@ -1010,13 +1038,16 @@ template <bool R, bool Q, int L>
 __device__ __forceinline__ void apply_viscosity_body(const DevConsts& c, const Batch& b, const float4* __restrict__ pred,
                                                      const float4* __restrict__ velIn, float4* __restrict__ velOut,
                                                      float4* __restrict__ omega, float4* __restrict__ near,
-                                                     const uint4* __restrict__ rows, int i, const float4 pi,
+                                                     const uint4* __restrict__ rows, int i, uint4 head, const float4 pi,
                                                      const float4 vi, uint64_t mt) {
     const int n = c.n;
     float vsx = 0.0f, vsy = 0.0f, vsz = 0.0f, ox = 0.0f, oy = 0.0f, oz = 0.0f;
     auto load = [&](uint32_t j) { j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex); return PairRec{__ldg(pred + j), __ldg(velIn + j)}; };
+    constexpr bool kLaneSums = L > 1 && Q && !R;  // the other forms go in_turn
+    __shared__ __align__(16) float terms[kLaneSums ? kMaxBlock / L * LaneSums<L, 6>::kStride : 1];
+    LaneSums<L, 6> sums(terms, {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f});
     auto pass = [&](auto from) { ox = from(ox); oy = from(oy); oz = from(oz); vsx = from(vsx); vsy = from(vsy); vsz = from(vsz); };
-    walk_pairs<L, true>(rows, n, i, FlatFriends(mt, kept_other(mt)).total, load, [&](const PairRec& qa, const PairRec& qb, bool va, bool vb) {
+    walk_pairs<L, true>(rows, n, i, head, FlatFriends(mt, kept_other(mt)).total, load, [&](const PairRec& qa, const PairRec& qb, bool va, bool vb) {
         const float4 pa = qa.a, pb = qb.a;
         const F2 rx = pack2(pi.x - pa.x, pi.x - pb.x), ry = pack2(pi.y - pa.y, pi.y - pb.y),
                  rz = pack2(pi.z - pa.z, pi.z - pb.z);
@@ -1068,6 +1099,11 @@ __device__ __forceinline__ void apply_viscosity_body(const DevConsts& c, const B
             const float2 p0 = unpack2(mul2(uy, g2)), p1 = unpack2(mul2(uz, g0)), p2 = unpack2(mul2(ux, g1)),
                          q0 = unpack2(mul2(uz, g1)), q1 = unpack2(mul2(ux, g2)), q2 = unpack2(mul2(uy, g0)),
                          a0 = unpack2(mul2(ux, d3)), a1 = unpack2(mul2(uy, d3)), a2 = unpack2(mul2(uz, d3));
+            if constexpr (kLaneSums) {
+                sums.add(va, vb, {make_float2(p0.x - q0.x, p0.y - q0.y), make_float2(p1.x - q1.x, p1.y - q1.y),
+                                  make_float2(p2.x - q2.x, p2.y - q2.y), a0, a1, a2});
+                return;
+            }
             in_turn<L>([&] {
                 if (va) {
                     ox = ox + (p0.x - q0.x); oy = oy + (p1.x - q1.x); oz = oz + (p2.x - q2.x);
@@ -1080,6 +1116,14 @@ __device__ __forceinline__ void apply_viscosity_body(const DevConsts& c, const B
             }, pass);
         }
     });
+    if constexpr (kLaneSums) {
+        ox = sums.template get<0>();
+        oy = sums.template get<1>();
+        oz = sums.template get<2>();
+        vsx = sums.template get<3>();
+        vsy = sums.template get<4>();
+        vsz = sums.template get<5>();
+    }
     if (threadIdx.x % L) return;  // the sums are the first lane's
     vsx = vsx * c.poly6;
     vsy = vsy * c.poly6;
@@ -1108,10 +1152,11 @@ apply_viscosity_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, co
         const int i = B ? balanced_particle(meta, c.n, false, tile) : (tile * (int)blockDim.x + (int)threadIdx.x) / L;
         if (i < 0 || i >= c.n) return;
         const float4 pi = pred[i], vi = velIn[i];
+        const uint4 head = first_entry<L>(rows, c.n, i);
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) apply_viscosity_body<R, true, L>(c, b, pred, velIn, velOut, omega, near, rows, i, pi, vi, mt);
-        else apply_viscosity_body<R, false, L>(c, b, pred, velIn, velOut, omega, near, rows, i, pi, vi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) apply_viscosity_body<R, true, L>(c, b, pred, velIn, velOut, omega, near, rows, i, head, pi, vi, mt);
+        else apply_viscosity_body<R, false, L>(c, b, pred, velIn, velOut, omega, near, rows, i, head, pi, vi, mt);
     });
 }
 
@@ -1121,12 +1166,15 @@ __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const f
                                                      const float4* __restrict__ omega,
                                                      const float4* __restrict__ velIn, float4* __restrict__ velOut,
                                                      float4* __restrict__ tapeEta, const uint4* __restrict__ rows, int i,
-                                                     const float4 pi, uint64_t mt) {
+                                                     uint4 head, const float4 pi, uint64_t mt) {
     const int n = c.n;
     float ex = 0.0f, ey = 0.0f, ez = 0.0f;
     auto load = [&](uint32_t j) { return __ldg(near + checked_index(j, (uint32_t)n, c.err, kErrFriendIndex)); };
+    constexpr bool kLaneSums = L > 1 && Q && !R;  // the other forms go in_turn
+    __shared__ __align__(16) float terms[kLaneSums ? kMaxBlock / L * LaneSums<L, 3>::kStride : 1];
+    LaneSums<L, 3> sums(terms, {0.0f, 0.0f, 0.0f});
     auto pass = [&](auto from) { ex = from(ex); ey = from(ey); ez = from(ez); };
-    walk_pairs<L>(rows, n, i, FlatFriends(mt, kept_other(mt)).total, load, [&](const float4& pa, const float4& pb, bool va, bool vb) {
+    walk_pairs<L>(rows, n, i, head, FlatFriends(mt, kept_other(mt)).total, load, [&](const float4& pa, const float4& pb, bool va, bool vb) {
         const F2 rx = pack2(pi.x - pa.x, pi.x - pb.x), ry = pack2(pi.y - pa.y, pi.y - pb.y),
                  rz = pack2(pi.z - pa.z, pi.z - pb.z);
         const F2 r2 = dot2(c, rx, ry, rz, rx, ry, rz);
@@ -1165,12 +1213,21 @@ __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const f
             }
             const F2 ol = pack2(pa.w, pb.w);
             const float2 x = unpack2(mul2(ol, g0)), y = unpack2(mul2(ol, g1)), z = unpack2(mul2(ol, g2));
+            if constexpr (kLaneSums) {
+                sums.add(va, vb, {x, y, z});
+                return;
+            }
             in_turn<L>([&] {
                 if (va) { ex = ex + x.x; ey = ey + y.x; ez = ez + z.x; }
                 if (vb) { ex = ex + x.y; ey = ey + y.y; ez = ez + z.y; }
             }, pass);
         }
     });
+    if constexpr (kLaneSums) {
+        ex = sums.template get<0>();
+        ey = sums.template get<1>();
+        ez = sums.template get<2>();
+    }
     if (threadIdx.x % L) return;  // the sums are the first lane's
     ex = ex * c.negGradSpiky;
     ey = ey * c.negGradSpiky;
@@ -1212,10 +1269,11 @@ apply_vorticity_kernel(DevConsts c, const float4* __restrict__ pred, const float
         const int i = B ? balanced_particle(meta, c.n, false, tile) : (tile * (int)blockDim.x + (int)threadIdx.x) / L;
         if (i < 0 || i >= c.n) return;
         const float4 pi = pred[i];
+        const uint4 head = first_entry<L>(rows, c.n, i);
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) apply_vorticity_body<R, true, L>(c, near, omega, velIn, velOut, tapeEta, rows, i, pi, mt);
-        else apply_vorticity_body<R, false, L>(c, near, omega, velIn, velOut, tapeEta, rows, i, pi, mt);
+        if (!R && c.quotients && !quotients_tainted(c, i)) apply_vorticity_body<R, true, L>(c, near, omega, velIn, velOut, tapeEta, rows, i, head, pi, mt);
+        else apply_vorticity_body<R, false, L>(c, near, omega, velIn, velOut, tapeEta, rows, i, head, pi, mt);
     });
 }
 
@@ -1247,11 +1305,16 @@ void launch_reset_cells(int n, const uint32_t* keys, uint32_t* cells, uint32_t k
 }
 
 // Lanes that share a particle in a solver pass (walk_pairs).  A substep of 2,048
-// / 8,192 / 16,384 / 32,768 / 65,536 particles takes 72 / 92 / 103 / 106 / 155 us
-// with one and 65 / 82 / 95 / 124 / 199 us with four: there the extra turns cost
-// more than the shorter chains save.
-int lanes_per_particle(int n, int balance, const int* tileCounter) {
-    return n <= 16384 && !balance && !tileCounter ? 4 : 1;
+// / 4,096 / 8,192 / 16,384 / 24,576 / 32,768 particles takes 70 / 80 / 89 / 96 /
+// 98 / 101 us with one lane, 56 / 61 / 65 / 80 / 94 / 109 with four and 51 / 57 /
+// 68 / 90 / 119 / 133 with eight: beyond, the chip is full, and what the lanes
+// exchange costs more than the shorter chains save.  Relaxed sums go in turns:
+// 65 / 82 / 95 / 124 us at 2,048 / 8,192 / 16,384 / 32,768 against 72 / 92 / 103 /
+// 106 with one lane (the exact passes' figures when theirs went in turns).
+int lanes_per_particle(const DevConsts& c, int balance, const int* tileCounter) {
+    if (balance || tileCounter) return 1;
+    if (c.relaxed) return c.n <= 16384 ? 4 : 1;
+    return c.n <= 4096 ? 8 : c.n <= 24576 ? 4 : 1;
 }
 
 // Grid of a neighbour pass: one block per tile of `block` particles, or
@@ -1299,9 +1362,9 @@ void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const
 void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* predPacked, float* density,
                             float4* tapeSums, float* tapeRho, const uint2* meta, const uint4* rows, int block, int balance, int* tileCounter,
                             cudaStream_t s) {
-    const int lanes = lanes_per_particle(c.n, balance, tileCounter);
+    const int lanes = lanes_per_particle(c, balance, tileCounter);
     auto k = c.relaxed ? (lanes > 1 ? compute_scaling_kernel<true, false, 4> : balance ? compute_scaling_kernel<true, true, 1> : compute_scaling_kernel<true, false, 1>)
-                       : (lanes > 1 ? compute_scaling_kernel<false, false, 4> : balance ? compute_scaling_kernel<false, true, 1> : compute_scaling_kernel<false, false, 1>);
+                       : (lanes == 8 ? compute_scaling_kernel<false, false, 8> : lanes == 4 ? compute_scaling_kernel<false, false, 4> : balance ? compute_scaling_kernel<false, true, 1> : compute_scaling_kernel<false, false, 1>);
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n * lanes, block, tileCounter != nullptr, &tiles);
     launch_chained(k, grid, block, s, c, pred, predPacked, density, tapeSums, tapeRho, meta, rows, tiles, tileCounter);
@@ -1311,9 +1374,9 @@ void launch_compute_delta(const DevConsts& c, Batch b, const float4* predPacked,
                           const StepEnd& end, float4* predOut, const float* density, const uint2* meta, int lastIteration,
                           uint8_t* clampMask, const uint4* rows, int block, int balance, int* tileCounter,
                           cudaStream_t s) {
-    const int lanes = lanes_per_particle(c.n, balance, tileCounter);
+    const int lanes = lanes_per_particle(c, balance, tileCounter);
     auto k = c.relaxed ? (lanes > 1 ? compute_delta_kernel<true, false, 4> : balance ? compute_delta_kernel<true, true, 1> : compute_delta_kernel<true, false, 1>)
-                       : (lanes > 1 ? compute_delta_kernel<false, false, 4> : balance ? compute_delta_kernel<false, true, 1> : compute_delta_kernel<false, false, 1>);
+                       : (lanes == 8 ? compute_delta_kernel<false, false, 8> : lanes == 4 ? compute_delta_kernel<false, false, 4> : balance ? compute_delta_kernel<false, true, 1> : compute_delta_kernel<false, false, 1>);
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n * lanes, block, tileCounter != nullptr, &tiles);
     launch_chained(k, grid, block, s, c, b, predPacked, posPrev, end, predOut, density, meta, lastIteration, clampMask, rows, tiles,
@@ -1328,9 +1391,9 @@ void launch_update_velocities(const DevConsts& c, const StepEnd& end, const floa
 void launch_apply_viscosity(const DevConsts& c, Batch b, const float4* pred, const float4* velIn, float4* velOut,
                             float4* omega, float4* near, const uint2* meta, const uint4* rows, int block, int balance,
                             int* tileCounter, cudaStream_t s) {
-    const int lanes = lanes_per_particle(c.n, balance, tileCounter);
+    const int lanes = lanes_per_particle(c, balance, tileCounter);
     auto k = c.relaxed ? (lanes > 1 ? apply_viscosity_kernel<true, false, 4> : balance ? apply_viscosity_kernel<true, true, 1> : apply_viscosity_kernel<true, false, 1>)
-                       : (lanes > 1 ? apply_viscosity_kernel<false, false, 4> : balance ? apply_viscosity_kernel<false, true, 1> : apply_viscosity_kernel<false, false, 1>);
+                       : (lanes == 8 ? apply_viscosity_kernel<false, false, 8> : lanes == 4 ? apply_viscosity_kernel<false, false, 4> : balance ? apply_viscosity_kernel<false, true, 1> : apply_viscosity_kernel<false, false, 1>);
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n * lanes, block, tileCounter != nullptr, &tiles);
     launch_chained(k, grid, block, s, c, b, pred, velIn, velOut, omega, near, meta, rows, tiles, tileCounter);
@@ -1339,9 +1402,9 @@ void launch_apply_viscosity(const DevConsts& c, Batch b, const float4* pred, con
 void launch_apply_vorticity(const DevConsts& c, const float4* pred, const float4* near, const float4* omega,
                             const float4* velIn, float4* velOut, float4* tapeEta, const uint2* meta, const uint4* rows, int block, int balance,
                             int* tileCounter, cudaStream_t s, int firstTile, int tileCount) {
-    const int lanes = lanes_per_particle(c.n, balance, tileCounter);
+    const int lanes = lanes_per_particle(c, balance, tileCounter);
     auto k = c.relaxed ? (lanes > 1 ? apply_vorticity_kernel<true, false, 4> : balance ? apply_vorticity_kernel<true, true, 1> : apply_vorticity_kernel<true, false, 1>)
-                       : (lanes > 1 ? apply_vorticity_kernel<false, false, 4> : balance ? apply_vorticity_kernel<false, true, 1> : apply_vorticity_kernel<false, false, 1>);
+                       : (lanes == 8 ? apply_vorticity_kernel<false, false, 8> : lanes == 4 ? apply_vorticity_kernel<false, false, 4> : balance ? apply_vorticity_kernel<false, true, 1> : apply_vorticity_kernel<false, false, 1>);
     if (tileCount > 0) {  // tiles [firstTile, firstTile + tileCount), one block each
         launch_chained(k, (unsigned)(tileCount * lanes), block, s, c, pred, near, omega, velIn, velOut, tapeEta, meta, rows, 0, nullptr, firstTile);
         return;
