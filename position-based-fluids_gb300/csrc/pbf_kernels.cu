@@ -1352,10 +1352,12 @@ void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const
         launch_chained(build_friends_scan_kernel, blocks_for(c.n, block), block, s, c, b, pred, table, rows, meta, errorWord);
         return;
     }
+    // a substep of 1,024 / 2,048 / 4,096 / 8,192 particles takes 43 / 48 / 54 / 68 us with one particle to a warp,
+    // 46 / 52 / 56 / 66 with 4 (nothing else fills the chip, and a warp takes its members one after another);
     // friends of 2,048 / 16,384 / 65,536 / 131,072 / 262,144 particles, us: 13 / 20 / 45 / 81 / 152 with 4 to a
     // warp, 17 / 23 / 38 / 65 / 120 with 8, 22 / 32 / 38 / 58 / 105 with 16, 34 / 41 / 47 / 63 / 104 with 32
-    const int w = c.n <= 16384 ? 4 : c.n <= 49152 ? 8 : c.n <= 196608 ? 16 : 32;
-    auto k = w == 4 ? build_friends_kernel<4> : w == 8 ? build_friends_kernel<8> : w == 16 ? build_friends_kernel<16> : build_friends_kernel<32>;
+    const int w = c.n <= 4096 ? 1 : c.n <= 16384 ? 4 : c.n <= 49152 ? 8 : c.n <= 196608 ? 16 : 32;
+    auto k = w == 1 ? build_friends_kernel<1> : w == 4 ? build_friends_kernel<4> : w == 8 ? build_friends_kernel<8> : w == 16 ? build_friends_kernel<16> : build_friends_kernel<32>;
     launch_chained(k, blocks_for(c.n, w * kFriendWarps), 32 * kFriendWarps, s, c, b, pred, table, rows, meta, errorWord);
 }
 
