@@ -232,12 +232,13 @@ void launch_cell_gather(int n, const uint32_t* keys, const uint32_t* starts, con
                         uint32_t* permOut, uint32_t* permCopy, const float4* pos, const float4* pred,
                         const uint32_t* ids, float4* posOut, float4* predOut, uint32_t* idsOut, int* err,
                         cudaStream_t s);
-// For the entry points that sort without records: the stable permutation from
-// `order`, and the sorted keys (keysOut may still hold the particles' own keys
-// when the permutation is taken) and the cell table from `starts`.
-void launch_cell_rank(int n, const uint32_t* keys, const uint32_t* starts, const uint32_t* order, uint32_t* permOut,
-                      cudaStream_t s);
-void launch_cell_table(int n, uint32_t keys, const uint32_t* starts, uint32_t* keysOut, uint32_t* cells, cudaStream_t s);
+// For the entry point that sorts without records (at most PBF_NOALLOC_MAX_KEYS
+// particles): the stable permutation, the sorted keys (in place of the
+// particles' own) and the cell table (may be NULL) from `order` and `starts`.
+// crowded: a word more than there are keys, the first one zero, such as the
+// counts after the scan.
+cudaError_t launch_cell_finish(int n, uint32_t keyCount, const uint32_t* starts, const uint32_t* order, uint32_t* keys,
+                               uint32_t* permOut, uint32_t* cells, uint32_t* crowded, cudaStream_t s);
 
 // ---- adjoint (pbf_adjoint.cu) ----
 // What one substep of a rollout leaves for its reverse pass.

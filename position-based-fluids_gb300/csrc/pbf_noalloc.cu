@@ -145,9 +145,9 @@ extern "C" int pbf_sort_state_noalloc(const PbfParameters* params, const float* 
         if (e == cudaSuccess) {
             pbf::launch_compute_keys(c, pbf::Batch{nullptr, nullptr}, reinterpret_cast<const float4*>(d_pred), d_keys, d_perm, counts, s);
             pbf::launch_counting_sort(counting, (int)n, counts, sums, starts, d_keys, d_perm, order, nullptr, s);
-            pbf::launch_cell_rank((int)n, d_keys, starts, order, d_perm, s);
-            pbf::launch_cell_table((int)n, params->gridBufSize, starts, d_keys, d_cells, s);
-            e = cudaGetLastError();
+            e = pbf::launch_cell_finish((int)n, params->gridBufSize, starts, order, d_keys, d_perm, d_cells, counts, s);
+            const cudaError_t launched = cudaGetLastError();
+            if (e == cudaSuccess) e = launched;
         }
         if (e != cudaSuccess) return pbf::fail(nullptr, PBF_ERR_CUDA, std::string("pbf_sort_state_noalloc: ") + cudaGetErrorString(e));
         return PBF_OK;

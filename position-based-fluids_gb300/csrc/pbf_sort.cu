@@ -278,14 +278,22 @@ cell_gather_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __r
     idsOut[to] = id;
 }
 
-// The stable order without the records: permOut from the scattered order.
+// The stable order without the records: permOut from the scattered order.  The
+// comparisons are as many as the cell holds, for each particle; cells of more
+// than kCrowdedCell go to the list `crowded` (its length first, zero before the
+// launch).
+constexpr uint32_t kCrowdedCell = 1024;
 __global__ void __launch_bounds__(kThreads)
 cell_rank_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ starts,
-                 const uint32_t* __restrict__ order, uint32_t* __restrict__ permOut) {
+                 const uint32_t* __restrict__ order, uint32_t* __restrict__ permOut, uint32_t* __restrict__ crowded) {
     chain_wait();
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= (uint32_t)n) return;
     const uint32_t i = order[s], key = keys[i], first = starts[key], end = starts[key + 1];
+    if (end - first > kCrowdedCell) {
+        if (s == first) crowded[1u + atomicAdd(crowded, 1u)] = key;
+        return;
+    }
     uint32_t to = first;
     for (uint32_t q = first; q < end; ++q) to += order[q] < i;
     permOut[to] = i;
@@ -294,29 +302,143 @@ cell_rank_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __res
 // The sorted keys and the cell table (first and last particle of a key, both
 // all ones for none) from the first indices; the table may be NULL.  The last
 // particle of the only one of n = 1 is not written (update_cells.cl:11-25).
+// A warp writes the keys of the cells of more than 16 particles, one thread 512
+// of them one after another took 100 us; those of crowded cells are left to
+// crowded_cells_kernel.
 __global__ void __launch_bounds__(kThreads)
 cell_table_kernel(int n, uint32_t keys, const uint32_t* __restrict__ starts, uint32_t* __restrict__ keysOut,
                   uint32_t* __restrict__ cells) {
     chain_wait();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= keys) return;
-    const uint32_t first = starts[k], end = starts[k + 1];
-    if (cells) {
-        cells[2 * (size_t)k] = first < end ? first : kEmpty;
-        cells[2 * (size_t)k + 1] = first < end && n > 1 ? end - 1u : kEmpty;
+    const int lane = threadIdx.x & 31;
+    uint32_t first = 0, end = 0;
+    if (k < keys) {
+        first = starts[k];
+        end = starts[k + 1];
+        if (cells) {
+            cells[2 * (size_t)k] = first < end ? first : kEmpty;
+            cells[2 * (size_t)k + 1] = first < end && n > 1 ? end - 1u : kEmpty;
+        }
     }
-    for (uint32_t q = first; q < end; ++q) keysOut[q] = k;
+    const bool many = end - first > 16u;
+    if (!many)
+        for (uint32_t q = first; q < end; ++q) keysOut[q] = k;
+    for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, many && end - first <= kCrowdedCell); todo; todo &= todo - 1u) {
+        const int src = __ffs(todo) - 1;
+        const uint32_t f = __shfl_sync(0xFFFFFFFFu, first, src), e = __shfl_sync(0xFFFFFFFFu, end, src);
+        for (uint32_t q = f + lane; q < e; q += 32) keysOut[q] = k - lane + src;
+    }
+}
+
+// The crowded cells, each by one block, or by up to kMostParts that take an
+// equal part of the span of the cell's indices: the indices in the part are
+// marked in a bitmap and read out in order, behind those below the part.  So a
+// cell costs its particles and its span, however many it holds (2^20 particles,
+// 16,384 to a cell: 0.12 ms, all in one: 0.24; a comparison with each would take
+// 0.13 us for every particle that a cell holds).  Word w of the map is at
+// [w % each][w / each], a thread's words in a column.
+constexpr int kCrowdedThreads = 1024, kCrowdedBlocks = 152;
+constexpr uint32_t kMostParts = 16, kPartCell = 16384;
+constexpr int kMostShift = 5;  // 2^5 words to a thread
+static_assert(PBF_NOALLOC_MAX_KEYS == (kCrowdedThreads * 32) << kMostShift, "the bitmap holds every index");
+__global__ void __launch_bounds__(kCrowdedThreads)
+crowded_cells_kernel(const uint32_t* __restrict__ crowded, const uint32_t* __restrict__ starts,
+                     const uint32_t* __restrict__ order, uint32_t* __restrict__ keysOut, uint32_t* __restrict__ permOut) {
+    chain_wait();
+    extern __shared__ uint32_t marks[];  // kCrowdedThreads words for every word to a thread
+    __shared__ uint32_t warpSums[kCrowdedThreads / 32], below, least, largest;
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const uint32_t count = crowded[0];
+    for (uint32_t c = 0; c < count; ++c) {
+        const uint32_t part = (blockIdx.x + kCrowdedBlocks - c * 17u % kCrowdedBlocks) % kCrowdedBlocks;
+        if (part >= kMostParts) continue;
+        const uint32_t key = crowded[1u + c], first = starts[key], end = starts[key + 1];
+        int parts = 0;  // 2^parts of them
+        while ((1u << parts) < kMostParts && (end - first) >> parts > kPartCell) ++parts;
+        if (part >= 1u << parts) continue;
+        if (t == 0) {
+            below = largest = 0u;
+            least = 0xFFFFFFFFu;
+        }
+        __syncthreads();
+        uint32_t low = 0xFFFFFFFFu, high = 0u;
+#pragma unroll 4
+        for (uint32_t s = first + t; s < end; s += kCrowdedThreads) {
+            low = min(low, order[s]);
+            high = max(high, order[s]);
+            if (part == 0) keysOut[s] = key;
+        }
+        low = __reduce_min_sync(0xFFFFFFFFu, low);
+        high = __reduce_max_sync(0xFFFFFFFFu, high);
+        if (lane == 0) {
+            atomicMin(&least, low);
+            atomicMax(&largest, high);
+        }
+        __syncthreads();
+        const uint32_t begin = least & ~31u, span = largest - begin;  // the bitmap's first index, its last one's place
+        int shift = 0;  // 2^shift words to a thread of all parts
+        while (shift < kMostShift && span >> shift >= kCrowdedThreads * 32u) ++shift;
+        const int down = max(shift - parts, 0);  // 2^down words to a thread of this part
+        const uint32_t each = 1u << down, lo = begin + part * ((uint32_t)kCrowdedThreads << down) * 32u;
+        if (lo <= largest) {
+            for (uint32_t r = 0; r < each; ++r) marks[r * kCrowdedThreads + t] = 0u;
+            __syncthreads();
+            uint32_t less = 0;
+#pragma unroll 4
+            for (uint32_t s = first + t; s < end; s += kCrowdedThreads) {
+                const uint32_t i = order[s], w = (i - lo) >> 5;
+                less += i < lo;
+                if (i >= lo && w >> down < kCrowdedThreads)
+                    atomicOr(&marks[(w & (each - 1u)) * kCrowdedThreads + (w >> down)], 1u << (i & 31u));
+            }
+            less = __reduce_add_sync(0xFFFFFFFFu, less);
+            if (lane == 0 && less) atomicAdd(&below, less);
+            __syncthreads();
+            uint32_t mine = 0;
+            for (uint32_t r = 0; r < each; ++r) mine += __popc(marks[r * kCrowdedThreads + t]);
+            uint32_t incl = mine;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+                if (lane >= (uint32_t)d) incl += u;
+            }
+            if (lane == 31) warpSums[warp] = incl;
+            __syncthreads();
+            uint32_t to = first + below + incl - mine;
+            for (uint32_t w = 0; w < warp; ++w) to += warpSums[w];
+            for (uint32_t r = 0; r < each; ++r)
+                for (uint32_t m = marks[r * kCrowdedThreads + t]; m; m &= m - 1u)
+                    permOut[to++] = lo + 32u * ((t << down) + r) + (uint32_t)__ffs(m) - 1u;
+        }
+        __syncthreads();  // all is read before the next cell writes it
+    }
 }
 
 }  // namespace
 
-void launch_cell_rank(int n, const uint32_t* keys, const uint32_t* starts, const uint32_t* order, uint32_t* permOut,
-                      cudaStream_t s) {
-    launch_chained(cell_rank_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keys, starts, order, permOut);
-}
-
-void launch_cell_table(int n, uint32_t keys, const uint32_t* starts, uint32_t* keysOut, uint32_t* cells, cudaStream_t s) {
-    launch_chained(cell_table_kernel, (keys + kThreads - 1) / kThreads, kThreads, s, n, keys, starts, keysOut, cells);
+cudaError_t launch_cell_finish(int n, uint32_t keyCount, const uint32_t* starts, const uint32_t* order, uint32_t* keys,
+                               uint32_t* permOut, uint32_t* cells, uint32_t* crowded, cudaStream_t s) {
+    launch_chained(cell_rank_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keys, starts, order, permOut, crowded);
+    launch_chained(cell_table_kernel, (keyCount + kThreads - 1) / kThreads, kThreads, s, n, keyCount, starts, keys, cells);
+    if ((uint32_t)n <= kCrowdedCell) return cudaGetLastError();
+    int shift = 0;
+    while (shift < kMostShift && ((uint64_t)kCrowdedThreads * 32 << shift) < (uint64_t)n) ++shift;
+    constexpr size_t kRow = kCrowdedThreads * sizeof(uint32_t);
+    // always the same limit: callers on other threads launch the kernel too
+    const cudaError_t e = cudaFuncSetAttribute(crowded_cells_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)(kRow << kMostShift));
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kCrowdedBlocks);
+    cfg.blockDim = dim3(kCrowdedThreads);
+    cfg.dynamicSmemBytes = kRow << shift;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, crowded_cells_kernel, static_cast<const uint32_t*>(crowded), starts, order, keys, permOut);
 }
 
 CountingPlan make_counting_plan(int n, uint64_t keys) {
