@@ -219,6 +219,11 @@ __device__ __forceinline__ void put_friend(uint4* __restrict__ rows, int n, int 
     *reinterpret_cast<uint32_t*>(entry + 4u * ((uint32_t)pos & 3u)) = j;
 }
 
+__device__ __forceinline__ uint32_t friend_at(const uint4* rows, int n, int i, int pos) {
+    const char* entry = reinterpret_cast<const char*>(rows + i) + (uint64_t)((uint32_t)pos >> 2) * (16u * (uint32_t)n);
+    return *reinterpret_cast<const uint32_t*>(entry + 4u * ((uint32_t)pos & 3u));
+}
+
 // The friend circle of r^2 < h^2: min(int(adj^3 * C), C-1) with
 // adj = max(0, (r - 0.3h) / 0.7h) (build_friends_list.cl:58-95), read off
 // precomputed r^2 thresholds (DevConsts::circT): the same integer the sqrt /
@@ -292,31 +297,31 @@ __device__ __forceinline__ void scan_neighbours(const DevConsts& c, uint32_t bas
     }
 }
 
-// Particle i's friends by one thread: the circles are counted in one scan, and
-// each friend is put in its place in a second.  Circle counts saturate at
-// perCircle (later candidates are dropped, build_friends_list.cl:79-83).
+// Particle i's friends by one thread, in one scan: friend q of circle k goes to
+// place perCircle * k + q of the rows, and when the circles' counts are known the
+// kept ones move up to their places, none past one that has yet to move.  Circle
+// counts saturate at perCircle (later candidates are dropped,
+// build_friends_list.cl:79-83).
 __device__ __noinline__ void friends_of_one(const DevConsts& c, uint32_t base, const float4* __restrict__ pred,
                                             const CellTable& cells, uint4* __restrict__ rows,
                                             uint2* __restrict__ meta, int* __restrict__ err, int i, const float4 pi,
                                             int cx, int cy, int cz) {
     uint64_t cnt = 0;  // 8 circles x 8-bit counters
-    scan_neighbours(c, base, pred, cells, err, i, pi, cx, cy, cz, [&](uint32_t, float r2) {
-        const int k = circle_of(c, r2);
-        if ((int)byte_of(cnt, k) < c.perCircle) cnt += 1ull << (8 * k);
+    scan_neighbours(c, base, pred, cells, err, i, pi, cx, cy, cz, [&](uint32_t j, float r2) {
+        const int k = circle_of(c, r2), have = (int)byte_of(cnt, k);
+        if (have >= c.perCircle) return;
+        cnt += 1ull << (8 * k);
+        put_friend(rows, c.n, i, c.perCircle * k + have, j);
     });
     int dense;
-    const uint2 m = make_meta(c, cnt, &dense);
-    meta[i] = m;
-    uint64_t left = cnt;  // places not taken yet
-    scan_neighbours(c, base, pred, cells, err, i, pi, cx, cy, cz, [&](uint32_t j, float r2) {
-        const int k = circle_of(c, r2);
-        const int free = (int)byte_of(left, k);
-        if (free == 0) return;
-        left -= 1ull << (8 * k);
-        int pos = -free;
-        for (int q = 0; q <= k; ++q) pos += (int)byte_of(cnt, q);
-        if (pos < dense) put_friend(rows, c.n, i, pos, j);
-    });
+    meta[i] = make_meta(c, cnt, &dense);
+    int to = (int)byte_of(cnt, 0);
+    for (int k = 1; to < dense; ++k) {
+        const int nk = (int)byte_of(cnt, k);
+        if (to < c.perCircle * k)
+            for (int q = 0; q < nk; ++q) put_friend(rows, c.n, i, to + q, friend_at(rows, c.n, i, c.perCircle * k + q));
+        to += nk;
+    }
     for (int t = dense; t & 3; ++t) put_friend(rows, c.n, i, t, (uint32_t)i);
 }
 
@@ -572,7 +577,8 @@ build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, Cell
             const bool low = ex >= ey && ex >= ez ? pi.x < lx + 0.5f * ex : ey >= ez ? pi.y < ly + 0.5f * ey : pi.z < lz + 0.5f * ez;
             uint32_t part = __ballot_sync(kFull, member && low);
             if (part == 0u || part == runMask) part = runMask & (0u - runMask);
-            if (part == runMask) scan |= runMask;  // a single member
+            if (kept > 4u * (uint32_t)kCandidates) part = runMask;  // most of them would be too many for a member alone
+            if (part == runMask) scan |= runMask;  // a single member, or far too many
             else { now = part; later |= runMask & ~part; }
             continue;
         }
