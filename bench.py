@@ -70,22 +70,25 @@ def survey_bytes(stage: str, passes: int = 3):
             "applyViscosity": 64.0, "applyVorticity": 64.0}.get(stage)
 
 
+# Stages whose work other stages do (the counting sort's scan is the cell
+# table, the last position pass updates the velocities); their own times are
+# the gap between two events, and they get no bandwidth.  Parameters that the
+# radix sort serves still run the first two.
+FUSED_STAGES = ("updateCells", "resetPartList", "updateVelocities")
+
 # Bytes per particle of one launch of each stage as this build moves them:
 # the model's bytes plus the friend list it keeps (4 B per entry written or
 # read).  `nl` / `nd` are the mean list lengths of the density pass / the
 # other passes.
 STAGE_BYTES = {
     "predictPositions": lambda nl, nd, it=4: 72.0,
-    "sortParticles": lambda nl, nd, it=4: 68.0,
-    "updateCells": lambda nl, nd, it=4: 12.0,
+    "sortParticles": lambda nl, nd, it=4: 88.0,
     "buildFriendsList": lambda nl, nd, it=4: 20.0 + 4.0 * nl,
-    "resetPartList": lambda nl, nd, it=4: 12.0,
-    # per density pass: the friend entries read; the first pass of a substep
-    # also writes them as flat rows for the passes after it (it = iterations)
-    "computeScaling": lambda nl, nd, it=4: 40.0 + 4.0 * nl + 4.0 * nl / max(it, 1),
-    "computeDelta": lambda nl, nd, it=4: 40.0 + 4.0 * nd,
-    "updateVelocities": lambda nl, nd, it=4: 80.0,
-    "applyViscosity": lambda nl, nd, it=4: 68.0 + 4.0 * nd,
+    "computeScaling": lambda nl, nd, it=4: 40.0 + 4.0 * nl,
+    # per position pass; the last of a substep also writes the step's end
+    # (positions, velocities and ids: 88 B)
+    "computeDelta": lambda nl, nd, it=4: 40.0 + 4.0 * nd + 88.0 / max(it, 1),
+    "applyViscosity": lambda nl, nd, it=4: 84.0 + 4.0 * nd,
     "applyVorticity": lambda nl, nd, it=4: 68.0 + 4.0 * nd,
 }
 
@@ -93,23 +96,19 @@ STAGE_BYTES = {
 # instructions (smsp__inst_executed.sum) per launch from an ncu capture of the
 # dam_break_1m scene in the first substep of frame 51, with the mean list
 # lengths of that frame (density pass nl, other passes nd): the friends build,
-# and the mean over the four launches of each solver pass in the substep (for
-# the density pass: the one that records the flat friend rows and three that
-# read them).  Launch shape of the capture: the autotuner's for that state
-# under ncu (friends 128-thread blocks, density passes 128, position passes
-# 64, plain thread map).
+# and the mean over the four launches of each solver pass in the substep.
 # Scaled to the measured list lengths: the traffic by the stage's
 # list-inclusive bytes, the instructions in proportion to the list length of
 # the pass (for the friends build, whose candidates grow with the density,
 # to nl).
-CAPTURE_SOURCE = ("ncu capture of the first substep of frame 51 (friends 128-thread blocks, density passes 128, "
-                  "position passes 64, list lengths 38.52 / 32.79), scaled by list length")
-TRAFFIC_CAPTURE = {"buildFriendsList": {"bytes": 813.3e6, "nl": 38.52, "nd": 32.79},
-                   "computeScaling": {"bytes": 308.8e6, "nl": 38.52, "nd": 32.79},
-                   "computeDelta": {"bytes": 216.4e6, "nl": 38.52, "nd": 32.79}}
-ISSUE_CAPTURE = {"buildFriendsList": {"inst": 650.0e6, "nl": 38.52, "nd": 32.79},
-                 "computeScaling": {"inst": 114.5e6, "nl": 38.52, "nd": 32.79},
-                 "computeDelta": {"inst": 116.6e6, "nl": 38.52, "nd": 32.79}}
+CAPTURE_SOURCE = ("ncu capture of the first substep of frame 51 (friends by warps, 128-thread blocks, "
+                  "list lengths 38.52 / 32.79; position passes: the mean of the four), scaled by list length")
+TRAFFIC_CAPTURE = {"buildFriendsList": {"bytes": 207.1e6, "nl": 38.52, "nd": 32.79},
+                   "computeScaling": {"bytes": 228.6e6, "nl": 38.52, "nd": 32.79},
+                   "computeDelta": {"bytes": 219.8e6, "nl": 38.52, "nd": 32.79}}
+ISSUE_CAPTURE = {"buildFriendsList": {"inst": 454.9e6, "nl": 38.52, "nd": 32.79},
+                 "computeScaling": {"inst": 71.4e6, "nl": 38.52, "nd": 32.79},
+                 "computeDelta": {"inst": 74.8e6, "nl": 38.52, "nd": 32.79}}
 SM_COUNT = 152
 SCHEDULERS_PER_SM = 4
 
@@ -234,7 +233,7 @@ def stage_rooflines(stage_ms: dict, n: int, iters: int, sub: int, nl: float, nd:
     for k, ms in stage_ms.items():
         per = launches_per_frame(k, iters, sub)
         launch_ms = ms / per
-        model = survey_bytes(k)
+        model = survey_bytes(k) if k not in FUSED_STAGES else None
         own = STAGE_BYTES[k](nl, nd, iters) if k in STAGE_BYTES else None
         if k == "radixsort":
             model_bytes = model * n  # all passes of one substep's sort
@@ -898,19 +897,19 @@ def render(args) -> None:
 def friends_compare(args) -> None:
     """The friends build of the 1M dam break after the warm-up frames, once
     with each algorithm from the same state (a short run to profile: one
-    substep with the shared-memory brick gather, one with the L1 scan)."""
+    substep with the build by warps, one with the scan by threads)."""
     import pbf
     params, pos, vel = pbf.make_scene(SCENE)
     sim = pbf.Simulation.create(params, pos, vel, device=0)
     for _ in range(args.warmup):
         sim.step_async(int(params.subSteps))
     sim.synchronize()
-    for algorithm in (2, 0):
+    for algorithm in (0, 1):
         sim.set_launch_shape([256, 128, 128, 128, 128, algorithm, 0, 0])
         sim.Step(1)
     sim.synchronize()
     sim.close()
-    print(json.dumps({"friends_compare": "one substep each with friends algorithms 2 and 0", "warmup": args.warmup}))
+    print(json.dumps({"friends_compare": "one substep each with friends algorithms 0 and 1", "warmup": args.warmup}))
 
 
 def main() -> None:

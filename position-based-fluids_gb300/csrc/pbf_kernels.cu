@@ -374,10 +374,12 @@ __device__ __forceinline__ float max_nan(float a, float b) {
 // instructions, 649 -> 462 us at 81 % issue active, DRAM writes 489 -> 160 MB,
 // and the density pass that used to copy the friends into rows (149 us) is one
 // of the others (100 us).  Per particle the candidate sequence takes about 100
-// instructions, the tests 160 and the sorting 170.  Against the scan below, which
-// has to run twice to write the rows: faster from one particle to a cell on
-// (500,000 particles: 0.21 against 0.25 ms there, 0.17 against 0.46 at four), 13 %
-// slower at one particle to two cells.  A run whose candidates do not fit is split
+// instructions, the tests 160 and the sorting 170.  Against the scan by threads:
+// 0.105 / 0.095 / 0.174 / 0.156 / 0.180 ms at 0.5 / 1 / 2 / 4 / 8 particles to a
+// cell and 0.062 / 0.063 / 0.162 / 0.217 / 0.310 there (200,000 particles for the
+// first two, then 500,000); a rule within the kernel that scans the warps of many
+// short runs gains a fifth of that at 0.5 to a cell and loses at 1 and above.
+// A run whose candidates do not fit is split
 // across the longest side of its box; a member that alone has too many, and runs
 // with coordinates that are not finite, take the scan.
 // 384 candidates leave room for 7 blocks per SM: 320 is 2 % faster on the scene
