@@ -221,7 +221,7 @@ __device__ __forceinline__ void put_friend(uint4* __restrict__ rows, int n, int 
 
 __device__ __forceinline__ uint32_t friend_at(const uint4* rows, int n, int i, int pos) {
     const char* entry = reinterpret_cast<const char*>(rows + i) + (uint64_t)((uint32_t)pos >> 2) * (16u * (uint32_t)n);
-    return *reinterpret_cast<const uint32_t*>(entry + 4u * ((uint32_t)pos & 3u));
+    return *reinterpret_cast<const volatile uint32_t*>(entry + 4u * ((uint32_t)pos & 3u));  // another lane may have written it
 }
 
 // The friend circle of r^2 < h^2: min(int(adj^3 * C), C-1) with
@@ -297,10 +297,21 @@ __device__ __forceinline__ void scan_neighbours(const DevConsts& c, uint32_t bas
     }
 }
 
-// Particle i's friends by one thread, in one scan: friend q of circle k goes to
-// place perCircle * k + q of the rows, and when the circles' counts are known the
-// kept ones move up to their places, none past one that has yet to move.  Circle
-// counts saturate at perCircle (later candidates are dropped,
+// Moves the kept friends of particle i up from the places of their circles
+// (friend q of circle k at perCircle * k + q), none past one that has yet to move.
+__device__ __forceinline__ void close_up(const DevConsts& c, uint4* __restrict__ rows, int i, uint64_t cnt, int dense) {
+    int to = (int)byte_of(cnt, 0);
+    for (int k = 1; to < dense; ++k) {
+        const int nk = (int)byte_of(cnt, k);
+        if (to < c.perCircle * k)
+            for (int q = 0; q < nk; ++q) put_friend(rows, c.n, i, to + q, friend_at(rows, c.n, i, c.perCircle * k + q));
+        to += nk;
+    }
+}
+
+// Particle i's friends by one thread, in one scan: they go to the places of their
+// circles and are closed up when the circles' counts are known.  Circle counts
+// saturate at perCircle (later candidates are dropped,
 // build_friends_list.cl:79-83).
 __device__ __noinline__ void friends_of_one(const DevConsts& c, uint32_t base, const float4* __restrict__ pred,
                                             const CellTable& cells, uint4* __restrict__ rows,
@@ -315,13 +326,7 @@ __device__ __noinline__ void friends_of_one(const DevConsts& c, uint32_t base, c
     });
     int dense;
     meta[i] = make_meta(c, cnt, &dense);
-    int to = (int)byte_of(cnt, 0);
-    for (int k = 1; to < dense; ++k) {
-        const int nk = (int)byte_of(cnt, k);
-        if (to < c.perCircle * k)
-            for (int q = 0; q < nk; ++q) put_friend(rows, c.n, i, to + q, friend_at(rows, c.n, i, c.perCircle * k + q));
-        to += nk;
-    }
+    close_up(c, rows, i, cnt, dense);
     for (int t = dense; t & 3; ++t) put_friend(rows, c.n, i, t, (uint32_t)i);
 }
 
@@ -379,12 +384,17 @@ __device__ __forceinline__ float max_nan(float a, float b) {
 // cell and 0.062 / 0.063 / 0.162 / 0.217 / 0.310 there (200,000 particles for the
 // first two, then 500,000); a rule within the kernel that scans the warps of many
 // short runs gains a fifth of that at 0.5 to a cell and loses at 1 and above.
-// A run whose candidates do not fit is split
-// across the longest side of its box; a member that alone has too many, and runs
-// with coordinates that are not finite, take the scan.
+// Runs with
+// coordinates that are not finite take the scan.  A run with up to half as many
+// candidates again as fit is split across the longest side of its box, and the
+// candidates of others pass through in chunks (friends_in_chunks).  262,144
+// particles in two colliding columns, where 560 candidates are common: a frame
+// takes 0.76 ms with that line, 0.84 with chunks alone; 400,000 particles with 30 /
+// 50 / 80 to a cell take 1.8 / 2.1 / 2.7 ms and 1.4 / 2.0 / 2.7 (without chunks 1.9 /
+// 3.6 / 7.1, by one thread each 1.7 / 2.5 / 3.3), 65,536 in 16 clusters of 4,096
+// take 1.7 (4.6 and 2.7).
 // 384 candidates leave room for 7 blocks per SM: 320 is 2 % faster on the scene
-// above and 10 % slower where 560 candidates are common (262,144 particles in two
-// colliding columns: 0.300 against 0.273 ms), 448 is 5 % slower on the former.
+// above and 10 % slower where 560 are common, 448 is 5 % slower on the former.
 constexpr int kFriendWarps = 4, kCandidates = 384, kMostFriends = 128;
 struct FriendShared {
     float x[kCandidates], y[kCandidates], z[kCandidates];
@@ -475,6 +485,85 @@ __device__ __noinline__ uint64_t sort_many_friends(const DevConsts& c, const Fri
     return (uint64_t)lo | ((uint64_t)hi << 32);
 }
 
+// The members of a run with far more candidates than fit, which pass through shared
+// memory in chunks; friends go to the places of their circles and
+// are closed up at the end.  end, shift: the cells (see below).  Returns the lane's
+// circle counts.
+__device__ __noinline__ uint64_t friends_in_chunks(const DevConsts& c, FriendShared& sh, const float4* __restrict__ pred,
+                                                   uint4* __restrict__ rows, uint32_t total, uint32_t end, uint32_t shift,
+                                                   float lx, float ly, float lz, float hx, float hy, float hz,
+                                                   uint32_t runMask, const float4 pi, int warpBase, uint64_t counts) {
+    constexpr unsigned kFull = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    const uint32_t ltMask = (1u << lane) - 1u, limit = (uint32_t)c.perCircle * 0x01010101u;
+    uint32_t kept = 0;
+    int firstCell = 0;
+    for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+        const uint32_t t = t0 + (uint32_t)lane;
+        const uint32_t ending = __reduce_or_sync(kFull, end - t0 < 32u ? 1u << (end - t0) : 0u);
+        const int q = firstCell + __popc(ending & (ltMask | (1u << lane)));
+        firstCell += __popc(ending);
+        const uint32_t j = t + __shfl_sync(kFull, shift, q);
+        const float4 pj = t < total ? __ldg(pred + j) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float dx = max_nan(max_nan(lx - pj.x, pj.x - hx), 0.0f), dy = max_nan(max_nan(ly - pj.y, pj.y - hy), 0.0f),
+                    dz = max_nan(max_nan(lz - pj.z, pj.z - hz), 0.0f);
+        const bool keep = t < total && !(dot3(dx, dy, dz, dx, dy, dz) >= c.h2);
+        const uint32_t km = __ballot_sync(kFull, keep);
+        if (keep) {
+            const uint32_t pos = kept + (uint32_t)__popc(km & ltMask);
+            sh.x[pos] = pj.x;
+            sh.y[pos] = pj.y;
+            sh.z[pos] = pj.z;
+            sh.j[pos] = j;
+        }
+        kept += (uint32_t)__popc(km);
+        if (t0 + 32u < total && kept + 32u <= (uint32_t)kCandidates) continue;
+        for (uint32_t e = kept + (uint32_t)lane; e < ((kept + 63u) & ~63u); e += 32) {
+            sh.x[e] = __int_as_float(0x7F800000);
+            sh.y[e] = sh.z[e] = 0.0f;
+        }
+        __syncwarp();
+        for (uint32_t rm = runMask; rm; rm &= rm - 1u) {
+            const int pl = __ffs(rm) - 1, ip = warpBase + pl;
+            const F2 px = both(__shfl_sync(kFull, pi.x, pl)), py = both(__shfl_sync(kFull, pi.y, pl)),
+                     pz = both(__shfl_sync(kFull, pi.z, pl));
+            uint32_t lo = __shfl_sync(kFull, (uint32_t)counts, pl), hi = __shfl_sync(kFull, (uint32_t)(counts >> 32), pl);
+            int cnt = 0;
+            for (uint32_t k = 0; k < kept; k += 64) {
+                const uint32_t e = k + 2u * (uint32_t)lane;
+                const F2 rx = sub2(px, load2(sh.x + e)), ry = sub2(py, load2(sh.y + e)), rz = sub2(pz, load2(sh.z + e));
+                const float2 r2 = unpack2(dot2(c, rx, ry, rz, rx, ry, rz));
+                const bool a0 = !(r2.x >= c.h2), a1 = !(r2.y >= c.h2);
+                const uint32_t m0 = __ballot_sync(kFull, a0), m1 = __ballot_sync(kFull, a1);
+                const int pos = cnt + __popc(m0 & ltMask) + __popc(m1 & ltMask);
+                if (a0) sh.list[pos] = make_uint2(e, __float_as_uint(r2.x));
+                if (a1) sh.list[pos + (a0 ? 1 : 0)] = make_uint2(e + 1u, __float_as_uint(r2.y));
+                cnt += __popc(m0) + __popc(m1);
+                if (cnt <= kMostFriends && k + 64u < kept) continue;
+                __syncwarp();
+                for (int r = 0; r < cnt; r += 32) {
+                    const uint2 entry = sh.list[r + lane];
+                    const uint32_t friendOf = sh.j[r + lane < cnt ? entry.x : 0u];
+                    const bool valid = r + lane < cnt && (int)friendOf != ip;
+                    const uint32_t circ = valid ? (uint32_t)circle_of(c, __uint_as_float(entry.y)) : 8u;
+                    const uint32_t peers = __match_any_sync(kFull, circ);
+                    const int rank = __popc(peers & ltMask) + (int)(__byte_perm(lo, hi, circ & 7u) & 0xFFu);
+                    if (valid && rank < c.perCircle) put_friend(rows, c.n, ip, c.perCircle * (int)circ + rank, friendOf);
+                    const uint32_t one = valid ? 1u << (8u * (circ & 3u)) : 0u, one0 = circ < 4u ? one : 0u;
+                    lo = __vminu4(lo + __reduce_add_sync(kFull, one0), limit);
+                    hi = __vminu4(hi + __reduce_add_sync(kFull, one - one0), limit);
+                }
+                cnt = 0;
+                __syncwarp();  // the list is read before it is written again
+            }
+            if (lane == pl) counts = (uint64_t)lo | ((uint64_t)hi << 32);
+        }
+        __syncwarp();
+        kept = 0;
+    }
+    return counts;
+}
+
 // W particles to a warp: 32, or fewer where that leaves the chip without warps
 // (a warp takes its members one after another).
 template <int W>
@@ -506,6 +595,7 @@ build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, Cell
     const float inf = __int_as_float(0x7F800000);
     uint32_t scan = 0;   // lanes whose particles take the scan
     uint64_t counts = 0; // this lane's particle: its circles' counts
+    uint32_t spread = 0; // lanes whose particles' friends are at the places of their circles
     uint32_t now = 0, later = 0;  // the parts of a split run: the one to do next, and the rest
     while (heads | now | later) {
         uint32_t runMask = now;
@@ -574,14 +664,19 @@ build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, Cell
             }
             kept += (uint32_t)__popc(km);
         }
-        if (kept > (uint32_t)kCandidates) {  // the members on one side of the box's middle first, across its longest side
+        if (kept > (uint32_t)kCandidates) {
+            // the members on one side of the box's middle first, across its longest side
             const float ex = hx - lx, ey = hy - ly, ez = hz - lz;
             const bool low = ex >= ey && ex >= ez ? pi.x < lx + 0.5f * ex : ey >= ez ? pi.y < ly + 0.5f * ey : pi.z < lz + 0.5f * ez;
             uint32_t part = __ballot_sync(kFull, member && low);
             if (part == 0u || part == runMask) part = runMask & (0u - runMask);
-            if (kept > 4u * (uint32_t)kCandidates) part = runMask;  // most of them would be too many for a member alone
-            if (part == runMask) scan |= runMask;  // a single member, or far too many
-            else { now = part; later |= runMask & ~part; }
+            if (2u * kept > 3u * (uint32_t)kCandidates || part == runMask) {  // too many for that, or a single member
+                counts = friends_in_chunks(c, sh, pred, rows, total, end, shift, lx, ly, lz, hx, hy, hz, runMask, pi, warpBase, counts);
+                spread |= runMask;
+            } else {
+                now = part;
+                later |= runMask & ~part;
+            }
             continue;
         }
         for (uint32_t e = kept + (uint32_t)lane; e < ((kept + 63u) & ~63u); e += 32) {  // up to a step of 64: out of reach
@@ -617,6 +712,7 @@ build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, Cell
             __syncwarp();  // the list is read before the next member's is written
         }
     }
+    __syncwarp();  // spread friends are read by the lane that closes them up
     if (!valid) return;
     if ((scan >> lane) & 1u) {
         friends_of_one(c, base, pred, cells, rows, meta, err, i, pi, cx, cy, cz);
@@ -624,6 +720,7 @@ build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, Cell
     }
     int dense;
     meta[i] = make_meta(c, counts, &dense);
+    if ((spread >> lane) & 1u) close_up(c, rows, i, counts, dense);
     for (int t = dense; t & 3; ++t) put_friend(rows, n, i, t, (uint32_t)i);
 }
 
