@@ -294,7 +294,8 @@ int pbf_perf_export_json(pbf_ctx* ctx, char* buf, size_t capacity, size_t* lengt
    one by one). */
 int pbf_launch_count(pbf_ctx* ctx, uint64_t* count);
 
-/* Use (1) or stop using (0) a captured CUDA graph for each substep. */
+/* Use (1) or stop using (0) a captured CUDA graph for each substep.  Rollouts
+   launch their kernels one by one either way. */
 int pbf_use_graph(pbf_ctx* ctx, int enable);
 
 /* ------------------------------------------------ allocation-free variant -- */

@@ -3,8 +3,8 @@ a GPU): the builds by warps (friends algorithms 0 and 2) and by one thread per
 particle (1) must give the oracle's substep bit for bit, and the same lists.
 
 The configurations cover ragged particle counts, candidate sequences longer than
-the shared buffer (runs taken member by member), more accepted candidates than
-the list holds (the scan), circles over their limit, one to eight circles, hash
+the shared buffer (split runs and chunks), more accepted candidates than the
+list holds (a second walk), circles over their limit, one to eight circles, hash
 collisions under a modulo that is no power of two, and cells with few particles.
 Integer decisions and the exact contract: no tolerance."""
 from __future__ import annotations
@@ -67,12 +67,3 @@ def test_coordinates_that_are_not_finite(pbf_mod, cuda_device, value):
             sim.Step(1)
             lists.append(sim.read_friends())
     assert np.array_equal(lists[0][0], lists[1][0]) and np.array_equal(lists[0][1], lists[1][1])
-
-
-def test_integer_form_of_the_circle_cuts():
-    """5 p > 3 t and 2 p > t decide as the float quotients do, for every count."""
-    p, t = np.meshgrid(np.arange(513), np.arange(513), indexing="ij")
-    with np.errstate(invalid="ignore", divide="ignore"):
-        q = p.astype(np.float32) / t.astype(np.float32)
-    assert np.array_equal((q > np.float32(0.6))[p <= t], (5 * p > 3 * t)[p <= t])
-    assert np.array_equal((q > np.float32(0.5))[p <= t], (2 * p > t)[p <= t])
