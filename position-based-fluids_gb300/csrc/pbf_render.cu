@@ -337,7 +337,7 @@ __global__ void grid_scatter_kernel(int n, const uint32_t* __restrict__ keys, co
     order[starts[keys[i]] + place[i]] = (uint32_t)i;
 }
 
-// The positions of each bucket's particles by increasing index.
+// The positions of each bucket's particles by decreasing index, the order of its chain.
 __global__ void grid_rank_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ starts,
                                  const uint32_t* __restrict__ order, const float4* __restrict__ pos,
                                  float4* __restrict__ sorted) {
@@ -345,7 +345,7 @@ __global__ void grid_rank_kernel(const uint32_t* __restrict__ keys, const uint32
     if (s >= starts[kGridBuckets]) return;
     const uint32_t i = order[s], key = keys[i], first = starts[key], end = starts[key + 1];
     uint32_t to = first;
-    for (uint32_t q = first; q < end; ++q) to += order[q] < i;
+    for (uint32_t q = first; q < end; ++q) to += order[q] > i;
     sorted[to] = pos[i];
 }
 
@@ -356,19 +356,22 @@ __device__ void sample_density(float h, const float4* __restrict__ sorted, const
     density = 0.0f;
     gx = gy = gz = 0.0f;
     const int cx = to_int(wx / h), cy = to_int(wy / h), cz = to_int(wz / h);
-    // render_hash of the 27 buckets from the spread coordinates of each axis; the Morton number is below 2^30
+    // render_hash of the 27 buckets from the spread coordinates of each axis; the Morton number is below 2^30.  x is
+    // its lowest bit: of three buckets in a row the first two (cx odd) or the last two lie together, and are one range
     const uint32_t sx0 = expand_bits_i(cx - 1), sx1 = expand_bits_i(cx), sx2 = expand_bits_i(cx + 1);
+    const bool odd = cx & 1;
+    const uint32_t from[2] = {sx0, odd ? sx2 : sx1}, length[2] = {odd ? 2u : 1u, odd ? 1u : 2u};
 #pragma unroll 1
     for (int iz = -1; iz <= 1; ++iz)
 #pragma unroll 1
         for (int iy = -1; iy <= 1; ++iy) {
             const uint32_t yz = (expand_bits_i(cy + iy) << 1) | (expand_bits_i(cz + iz) << 2);
-#pragma unroll 1
-            for (int ix = 0; ix < 3; ++ix) {
-                const uint32_t b = ((ix == 0 ? sx0 : ix == 1 ? sx1 : sx2) | yz) & (kGridBuckets - 1u);
-                const int first = (int)starts[b];
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+                const uint32_t b = (from[part] | yz) & (kGridBuckets - 1u);
+                const int end = (int)starts[b + length[part]];
 #pragma unroll 4
-                for (int k = (int)starts[b + 1] - 1; k >= first; --k) {
+                for (int k = (int)starts[b]; k < end; ++k) {
                     const float4 pp = __ldg(sorted + k);
                     const float dx = pp.x - wx, dy = pp.y - wy, dz = pp.z - wz;
                     const float r2 = dot3f(dx, dy, dz, dx, dy, dz);
