@@ -409,7 +409,8 @@ __device__ __forceinline__ void normalize3(float& x, float& y, float& z) {
 
 // A warp takes 8 x 4 pixels, whose points lie in the same few buckets; bound by
 // instruction issue (85 %): 141 us with a row of pixels and the positions behind
-// the permutation, 118 like this (the scene above).
+// the permutation, 118 like this, and 110 with two buckets to a range (the scene
+// above; pairs of candidates in packed arithmetic: 105, and slower at 1M sprites).
 __global__ void __launch_bounds__(128)
 smooth_kernel(PbfCamera cam, float h, const float4* __restrict__ sorted, const uint32_t* __restrict__ starts,
               const float4* __restrict__ splat, float4* __restrict__ out) {
