@@ -58,18 +58,18 @@ struct Friend2 {
 // 5.8 with four).
 constexpr int kSplit = 4;
 template <typename LoadF, typename BodyF>
-__device__ __forceinline__ void walk_split(const uint4* __restrict__ rows, int n, int i, int total, int sub, LoadF load,
+__device__ __forceinline__ void walk_split(const uint4* rows, int n, int i, int total, int sub, LoadF load,
                                            BodyF body) {
     const uint32_t* p = reinterpret_cast<const uint32_t*>(rows + i) + sub;
     const size_t stride = 4 * (size_t)n;
     int t = sub;
     for (; t + kSplit < total; t += 2 * kSplit, p += 2 * stride) {
-        const uint32_t j0 = __ldg(p), j1 = __ldg(p + stride);
+        const uint32_t j0 = *p, j1 = p[stride];
         const auto f0 = load(j0), f1 = load(j1);
         body(f0);
         body(f1);
     }
-    if (t < total) body(load(__ldg(p)));
+    if (t < total) body(load(*p));
 }
 // The sum over a particle's lanes, in all of them.
 __device__ __forceinline__ float lanes_sum(float v) {
@@ -120,9 +120,9 @@ template <typename T> __device__ __forceinline__ T block_sum(T v) {
 
 // v4 = v3 + dt*vort*(N x omega_i): adjoints of omega (omb) and of p^I (pb).
 __global__ void __launch_bounds__(kAdjBlock)
-adj_vorticity_kernel(DevConsts c, const float4* __restrict__ pI, const float4* __restrict__ omega,
-                     const float4* __restrict__ etas, const uint4* __restrict__ rows, const uint2* __restrict__ meta,
-                     const float4* __restrict__ vb, float4* __restrict__ omb, float4* __restrict__ pb) {
+adj_vorticity_kernel(DevConsts c, const float4* pI, const float4* omega,
+                     const float4* etas, const uint4* rows, const uint2* meta,
+                     const float4* vb, float4* omb, float4* pb) {
     chain_wait();
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) / kSplit, sub = threadIdx.x % kSplit;
     const int n = c.n;
@@ -167,10 +167,10 @@ adj_vorticity_kernel(DevConsts c, const float4* __restrict__ pI, const float4* _
 // v3 = v2 + c POLY6 sum (v2_j - v2_i) W and omega = -G sum (v2_j - v2_i) x k:
 // adjoints of v2 (v2b), p^I (pb) and of the XSPH factor (cbar).
 __global__ void __launch_bounds__(kAdjBlock)
-adj_viscosity_kernel(DevConsts c, const float4* __restrict__ pI, const float4* __restrict__ v2,
-                     float4* __restrict__ omb, const float4* __restrict__ vb, const uint4* __restrict__ rows,
-                     const uint2* __restrict__ meta, float4* __restrict__ v2b, float4* __restrict__ pb,
-                     float* __restrict__ cbar) {
+adj_viscosity_kernel(DevConsts c, const float4* pI, const float4* v2,
+                     float4* omb, const float4* vb, const uint4* rows,
+                     const uint2* meta, float4* v2b, float4* pb,
+                     float* cbar) {
     chain_wait();
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) / kSplit, sub = threadIdx.x % kSplit;
     const int n = c.n;
@@ -219,8 +219,8 @@ adj_viscosity_kernel(DevConsts c, const float4* __restrict__ pI, const float4* _
 }
 
 // v2 = (p^I - x)/dt and x' = p^I.
-__global__ void adj_velocity_kernel(DevConsts c, const float4* __restrict__ xb, float4* __restrict__ v2b,
-                                    float4* __restrict__ pb, float4* __restrict__ xsb) {
+__global__ void adj_velocity_kernel(DevConsts c, const float4* xb, float4* v2b,
+                                    float4* pb, float4* xsb) {
     chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
@@ -235,9 +235,9 @@ __global__ void adj_velocity_kernel(DevConsts c, const float4* __restrict__ xb, 
 // lambda^t (in pbt's w: one atomic for both) from that of p^{t+1} (pbn).
 // q = (p^t, lambda^t).
 __global__ void __launch_bounds__(kAdjBlock)
-adj_delta_kernel(DevConsts c, const float4* __restrict__ q, const uint8_t* __restrict__ mask,
-                 const float4* __restrict__ pbn, const uint4* __restrict__ rows, const uint2* __restrict__ meta,
-                 float4* __restrict__ pbt) {
+adj_delta_kernel(DevConsts c, const float4* q, const uint8_t* mask,
+                 const float4* pbn, const uint4* rows, const uint2* meta,
+                 float4* pbt) {
     chain_wait();
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) / kSplit, sub = threadIdx.x % kSplit;
     const int n = c.n;
@@ -290,9 +290,9 @@ adj_delta_kernel(DevConsts c, const float4* __restrict__ q, const uint8_t* __res
 // nothing changes here).  Clears pbn, which becomes the next iteration's pbt.
 // The sums over the friends are the forward pass' (sums, density).
 __global__ void __launch_bounds__(kAdjBlock)
-adj_scaling_kernel(DevConsts c, const float4* __restrict__ q, const float4* __restrict__ sums,
-                   const float* __restrict__ density, const uint4* __restrict__ rows,
-                   const uint2* __restrict__ meta, float4* pbt, float4* __restrict__ pbn) {
+adj_scaling_kernel(DevConsts c, const float4* q, const float4* sums,
+                   const float* density, const uint4* rows,
+                   const uint2* meta, float4* pbt, float4* pbn) {
     chain_wait();
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) / kSplit, sub = threadIdx.x % kSplit;
     const int n = c.n;
@@ -336,9 +336,9 @@ adj_scaling_kernel(DevConsts c, const float4* __restrict__ q, const float4* __re
 // Undo the sort and the prediction p0 = x + dt (v + dt g): adjoints of the
 // substep's inputs x, v (previous order) and of g.
 __global__ void __launch_bounds__(kAdjBlock)
-adj_unsort_predict_kernel(DevConsts c, const uint32_t* __restrict__ perm, const float4* __restrict__ xsb,
-                          float4* __restrict__ pb0, float4* __restrict__ xo, float4* __restrict__ vo,
-                          float* __restrict__ gbar) {
+adj_unsort_predict_kernel(DevConsts c, const uint32_t* perm, const float4* xsb,
+                          float4* pb0, float4* xo, float4* vo,
+                          float* gbar) {
     chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     F3 g = {0.0f, 0.0f, 0.0f};
@@ -364,13 +364,13 @@ adj_unsort_predict_kernel(DevConsts c, const uint32_t* __restrict__ perm, const 
 }
 
 // xb[k] = src[ids[k]] (to the current order) or dst[ids[k]] = xb[k] (back).
-__global__ void scatter_by_id_kernel(int n, const uint32_t* __restrict__ ids, const float4* __restrict__ byId,
-                                     float4* __restrict__ out) {
+__global__ void scatter_by_id_kernel(int n, const uint32_t* ids, const float4* byId,
+                                     float4* out) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < n) out[k] = byId[ids[k]];
 }
-__global__ void gather_to_id_kernel(int n, const uint32_t* __restrict__ ids, const float4* __restrict__ in,
-                                    float4* __restrict__ byId) {
+__global__ void gather_to_id_kernel(int n, const uint32_t* ids, const float4* in,
+                                    float4* byId) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < n) byId[ids[k]] = in[k];
 }

@@ -45,7 +45,7 @@ __device__ __forceinline__ uint32_t key_base(const Batch& b, int i) {
 // Adds the lanes of `valid` to their keys' counts; returns the lane's place
 // among its key's particles.  The particles come nearly sorted, a few keys to a
 // warp: one atomic per key and warp.
-__device__ __forceinline__ uint32_t place_of_arrival(unsigned valid, uint32_t key, uint32_t* __restrict__ counts) {
+__device__ __forceinline__ uint32_t place_of_arrival(unsigned valid, uint32_t key, uint32_t* counts) {
     const unsigned peers = __match_any_sync(valid, key);
     const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
     uint32_t place = 0;
@@ -55,9 +55,9 @@ __device__ __forceinline__ uint32_t place_of_arrival(unsigned valid, uint32_t ke
 
 // ------------------------------------------------------------- predict --
 // predict_positions.cl:8-17 fused with computeKeys (radixsort.cl:7-19).
-__global__ void predict_keys_kernel(DevConsts c, Batch b, const float4* __restrict__ pos, float4* __restrict__ vel,
-                                    float4* __restrict__ pred, uint32_t* __restrict__ keys,
-                                    uint32_t* __restrict__ perm, uint32_t* __restrict__ counts, int paused) {
+__global__ void predict_keys_kernel(DevConsts c, Batch b, const float4* pos, float4* vel,
+                                    float4* pred, uint32_t* keys,
+                                    uint32_t* perm, uint32_t* counts, int paused) {
     chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned valid = __ballot_sync(0xFFFFFFFFu, i < c.n);
@@ -92,9 +92,9 @@ __global__ void predict_keys_kernel(DevConsts c, Batch b, const float4* __restri
 }
 
 // radixsort.cl:1-20 alone (keys of given predicted positions, no padding).
-__global__ void compute_keys_kernel(DevConsts c, Batch b, const float4* __restrict__ pred,
-                                    uint32_t* __restrict__ keys, uint32_t* __restrict__ perm,
-                                    uint32_t* __restrict__ counts) {
+__global__ void compute_keys_kernel(DevConsts c, Batch b, const float4* pred,
+                                    uint32_t* keys, uint32_t* perm,
+                                    uint32_t* counts) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned valid = __ballot_sync(0xFFFFFFFFu, i < c.n);
     if (i >= c.n) return;
@@ -108,10 +108,10 @@ __global__ void compute_keys_kernel(DevConsts c, Batch b, const float4* __restri
 // before any read, update_velocities.cl:13).
 // Particle ids (the original index of each record) follow the same
 // permutation into idsOut.
-__global__ void gather_sorted_kernel(int n, const uint32_t* __restrict__ perm, const float4* __restrict__ pos,
-                                     const float4* __restrict__ pred, const uint32_t* __restrict__ ids,
-                                     float4* __restrict__ posOut, float4* __restrict__ predOut,
-                                     uint32_t* __restrict__ idsOut, int* err) {
+__global__ void gather_sorted_kernel(int n, const uint32_t* perm, const float4* pos,
+                                     const float4* pred, const uint32_t* ids,
+                                     float4* posOut, float4* predOut,
+                                     uint32_t* idsOut, int* err) {
     chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -125,8 +125,8 @@ __global__ void gather_sorted_kernel(int n, const uint32_t* __restrict__ perm, c
 // update_cells.cl:6-25 on a table that holds END_OF_CELL_LIST everywhere.
 // cellStart (may be NULL) also receives each occupied cell's first particle;
 // it is never reset (taint_around checks an entry against the keys).
-__global__ void update_cells_kernel(int n, const uint32_t* __restrict__ keys, uint32_t* __restrict__ cells,
-                                    uint32_t keyLimit, int* err, uint32_t* __restrict__ cellStart) {
+__global__ void update_cells_kernel(int n, const uint32_t* keys, uint32_t* cells,
+                                    uint32_t keyLimit, int* err, uint32_t* cellStart) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t k = checked_index(keys[i], keyLimit, err, kErrCellKey);
@@ -145,7 +145,7 @@ __global__ void update_cells_kernel(int n, const uint32_t* __restrict__ keys, ui
 }
 
 // reset_grid.cl:6-14
-__global__ void reset_cells_kernel(int n, const uint32_t* __restrict__ keys, uint2* __restrict__ cells,
+__global__ void reset_cells_kernel(int n, const uint32_t* keys, uint2* cells,
                                    uint32_t keyLimit, int* err) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -193,7 +193,7 @@ struct CellTable {
     const uint2* ranges;     // first and last particle, kEmpty for none (update_cells.cl)
     const uint32_t* starts;  // or the first particle of every key, and one beyond the last
 };
-__device__ __forceinline__ void cell_range(const CellTable& cells, uint32_t key, int n, int* __restrict__ err,
+__device__ __forceinline__ void cell_range(const CellTable& cells, uint32_t key, int n, int* err,
                                            uint32_t& first, uint32_t& count) {
     uint32_t last;
     count = 0;
@@ -214,7 +214,7 @@ __device__ __forceinline__ void cell_range(const CellTable& cells, uint32_t key,
 }
 
 // Friend `pos` of particle i in the rows.
-__device__ __forceinline__ void put_friend(uint4* __restrict__ rows, int n, int i, int pos, uint32_t j) {
+__device__ __forceinline__ void put_friend(uint4* rows, int n, int i, int pos, uint32_t j) {
     char* entry = reinterpret_cast<char*>(rows + i) + (uint64_t)((uint32_t)pos >> 2) * (16u * (uint32_t)n);
     *reinterpret_cast<uint32_t*>(entry + 4u * ((uint32_t)pos & 3u)) = j;
 }
@@ -250,8 +250,8 @@ __device__ __forceinline__ int circle_of(const DevConsts& c, float r2) {
 // reach (a NaN distance is taken, as in the reference's test).  The 27 hashes
 // are formed from the three spread coordinates of each axis.
 template <typename F>
-__device__ __forceinline__ void scan_neighbours(const DevConsts& c, uint32_t base, const float4* __restrict__ pred,
-                                                const CellTable& cells, int* __restrict__ err, int i,
+__device__ __forceinline__ void scan_neighbours(const DevConsts& c, uint32_t base, const float4* pred,
+                                                const CellTable& cells, int* err, int i,
                                                 const float4 pi, int cx, int cy, int cz, F consider) {
     const int n = c.n;
     const bool pow2 = (c.grid & (c.grid - 1)) == 0;
@@ -268,11 +268,11 @@ __device__ __forceinline__ void scan_neighbours(const DevConsts& c, uint32_t bas
     auto scan = [&](uint32_t lo, uint32_t hi) {
         uint32_t j = lo;
         for (; j + 1 <= hi; j += 2) {
-            const float4 p0 = __ldg(pred + j), p1 = __ldg(pred + j + 1);
+            const float4 p0 = pred[j], p1 = pred[j + 1];
             test(j, p0);
             test(j + 1, p1);
         }
-        if (j <= hi) test(j, __ldg(pred + j));
+        if (j <= hi) test(j, pred[j]);
     };
     for (int x = -1; x <= 1; ++x) {
         const uint32_t ex = x < 0 ? exm : (x > 0 ? exp_ : ex0);
@@ -299,7 +299,7 @@ __device__ __forceinline__ void scan_neighbours(const DevConsts& c, uint32_t bas
 
 // Moves the kept friends of particle i up from the places of their circles
 // (friend q of circle k at perCircle * k + q), none past one that has yet to move.
-__device__ __forceinline__ void close_up(const DevConsts& c, uint4* __restrict__ rows, int i, uint64_t cnt, int dense) {
+__device__ __forceinline__ void close_up(const DevConsts& c, uint4* rows, int i, uint64_t cnt, int dense) {
     int to = (int)byte_of(cnt, 0);
     for (int k = 1; to < dense; ++k) {
         const int nk = (int)byte_of(cnt, k);
@@ -313,9 +313,9 @@ __device__ __forceinline__ void close_up(const DevConsts& c, uint4* __restrict__
 // circles and are closed up when the circles' counts are known.  Circle counts
 // saturate at perCircle (later candidates are dropped,
 // build_friends_list.cl:79-83).
-__device__ __noinline__ void friends_of_one(const DevConsts& c, uint32_t base, const float4* __restrict__ pred,
-                                            const CellTable& cells, uint4* __restrict__ rows,
-                                            uint2* __restrict__ meta, int* __restrict__ err, int i, const float4 pi,
+__device__ __noinline__ void friends_of_one(const DevConsts& c, uint32_t base, const float4* pred,
+                                            const CellTable& cells, uint4* rows,
+                                            uint2* meta, int* err, int i, const float4 pi,
                                             int cx, int cy, int cz) {
     uint64_t cnt = 0;  // 8 circles x 8-bit counters
     scan_neighbours(c, base, pred, cells, err, i, pi, cx, cy, cz, [&](uint32_t j, float r2) {
@@ -331,8 +331,8 @@ __device__ __noinline__ void friends_of_one(const DevConsts& c, uint32_t base, c
 }
 
 __global__ void __launch_bounds__(kMaxBlock)
-build_friends_scan_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, CellTable cells,
-                          uint4* __restrict__ rows, uint2* __restrict__ meta, int* __restrict__ err) {
+build_friends_scan_kernel(const __grid_constant__ DevConsts c, Batch b, const float4* pred, CellTable cells,
+                          uint4* rows, uint2* meta, int* err) {
     chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
@@ -409,7 +409,7 @@ struct FriendShared {
 // summed up to each circle by one multiplication, at once.
 template <int NR>
 __device__ __forceinline__ uint64_t sort_friends(const DevConsts& c, const FriendShared& sh, int lane, uint32_t ltMask,
-                                                 int cnt, int ip, uint4* __restrict__ rows) {
+                                                 int cnt, int ip, uint4* rows) {
     constexpr unsigned kFull = 0xFFFFFFFFu;
     constexpr uint32_t kOnes = 0x01010101u;
     uint32_t j[NR], circ[NR], rank[NR];
@@ -454,7 +454,7 @@ __device__ __forceinline__ uint64_t sort_friends(const DevConsts& c, const Frien
 // friend in its place.
 __device__ __noinline__ uint64_t sort_many_friends(const DevConsts& c, const FriendShared& sh, int lane, uint32_t ltMask,
                                                    uint32_t kept, float px, float py, float pz, int ip,
-                                                   uint4* __restrict__ rows) {
+                                                   uint4* rows) {
     constexpr unsigned kFull = 0xFFFFFFFFu;
     const uint32_t limit = (uint32_t)c.perCircle * 0x01010101u;
     uint32_t lo = 0, hi = 0;  // counts of circles 0-3 and 4-7, a byte each, at most perCircle
@@ -489,8 +489,8 @@ __device__ __noinline__ uint64_t sort_many_friends(const DevConsts& c, const Fri
 // memory in chunks; friends go to the places of their circles and
 // are closed up at the end.  end, shift: the cells (see below).  Returns the lane's
 // circle counts.
-__device__ __noinline__ uint64_t friends_in_chunks(const DevConsts& c, FriendShared& sh, const float4* __restrict__ pred,
-                                                   uint4* __restrict__ rows, uint32_t total, uint32_t end, uint32_t shift,
+__device__ __noinline__ uint64_t friends_in_chunks(const DevConsts& c, FriendShared& sh, const float4* pred,
+                                                   uint4* rows, uint32_t total, uint32_t end, uint32_t shift,
                                                    float lx, float ly, float lz, float hx, float hy, float hz,
                                                    uint32_t runMask, const float4 pi, int warpBase, uint64_t counts) {
     constexpr unsigned kFull = 0xFFFFFFFFu;
@@ -504,7 +504,7 @@ __device__ __noinline__ uint64_t friends_in_chunks(const DevConsts& c, FriendSha
         const int q = firstCell + __popc(ending & (ltMask | (1u << lane)));
         firstCell += __popc(ending);
         const uint32_t j = t + __shfl_sync(kFull, shift, q);
-        const float4 pj = t < total ? __ldg(pred + j) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float4 pj = t < total ? pred[j] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         const float dx = max_nan(max_nan(lx - pj.x, pj.x - hx), 0.0f), dy = max_nan(max_nan(ly - pj.y, pj.y - hy), 0.0f),
                     dz = max_nan(max_nan(lz - pj.z, pj.z - hz), 0.0f);
         const bool keep = t < total && !(dot3(dx, dy, dz, dx, dy, dz) >= c.h2);
@@ -568,8 +568,8 @@ __device__ __noinline__ uint64_t friends_in_chunks(const DevConsts& c, FriendSha
 // (a warp takes its members one after another).
 template <int W>
 __global__ void __launch_bounds__(32 * kFriendWarps)
-build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, CellTable cells,
-                     uint4* __restrict__ rows, uint2* __restrict__ meta, int* __restrict__ err) {
+build_friends_kernel(const __grid_constant__ DevConsts c, Batch b, const float4* pred, CellTable cells,
+                     uint4* rows, uint2* meta, int* err) {
     chain_wait();
     constexpr unsigned kFull = 0xFFFFFFFFu;
     __shared__ FriendShared shared[kFriendWarps];
@@ -650,7 +650,7 @@ build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, Cell
             const int q = firstCell + __popc(ending & (ltMask | (1u << lane)));
             firstCell += __popc(ending);
             const uint32_t j = t + __shfl_sync(kFull, shift, q);
-            const float4 pj = t < total ? __ldg(pred + j) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 pj = t < total ? pred[j] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             const float dx = max_nan(max_nan(lx - pj.x, pj.x - hx), 0.0f), dy = max_nan(max_nan(ly - pj.y, pj.y - hy), 0.0f),
                         dz = max_nan(max_nan(lz - pj.z, pj.z - hz), 0.0f);
             const bool keep = t < total && !(dot3(dx, dy, dz, dx, dy, dz) >= c.h2);
@@ -731,7 +731,7 @@ build_friends_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, Cell
 // sort in shared memory over the kept-circle count (saturated at 255), ties
 // in any order.  Every thread of the block must call it (it synchronises);
 // returns the particle index, or -1 for threads beyond the block's particles.
-__device__ __forceinline__ int balanced_particle(const uint2* __restrict__ meta, int n, bool densityPass, int tile) {
+__device__ __forceinline__ int balanced_particle(const uint2* meta, int n, bool densityPass, int tile) {
     __shared__ uint32_t bins[256];
     __shared__ int order[kMaxBlock];
     const int t = threadIdx.x;
@@ -824,14 +824,14 @@ __device__ __forceinline__ F2 spiky_over_r2(const DevConsts& c, F2 r2, F2& w) {
 // compute_scaling.cl:27-112 followed by pack_data.cl (w = lambda).  Q: the
 // exact quotients by |r| through one reciprocal (quotient_rn).
 template <bool R, bool Q, int L>
-__device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const float4* __restrict__ pred,
-                                                     float4* __restrict__ predPacked, float* __restrict__ density,
-                                                     float4* __restrict__ tapeSums, float* __restrict__ tapeRho,
-                                                     const uint4* __restrict__ rows, int i, uint4 head, const float4 pi, uint64_t mt) {
+__device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const float4* pred,
+                                                     float4* predPacked, float* density,
+                                                     float4* tapeSums, float* tapeRho,
+                                                     const uint4* rows, int i, uint4 head, const float4 pi, uint64_t mt) {
     const int n = c.n;
     // complete neighbour sets count the particle itself first: d = h^2 - 0
     float ds = c.complete ? c.h2 * c.h2 * c.h2 : 0.0f, gsk = 0.0f, gx = 0.0f, gy = 0.0f, gz = 0.0f;
-    auto load = [&](uint32_t j) { return __ldg(pred + checked_index(j, (uint32_t)n, c.err, kErrFriendIndex)); };
+    auto load = [&](uint32_t j) { return pred[checked_index(j, (uint32_t)n, c.err, kErrFriendIndex)]; };
     auto one = [&](float rx, float ry, float rz, float r2) {  // a friend in support, divided the IEEE way
         const float rl = sqrtf(r2);
         const float hr = c.h - rl;
@@ -937,9 +937,9 @@ __device__ __forceinline__ void compute_scaling_body(const DevConsts& c, const f
 
 template <bool R, bool B, int L>
 __global__ void __maxnreg__(64)
-compute_scaling_kernel(DevConsts c, const float4* __restrict__ pred, float4* __restrict__ predPacked,
-                       float* __restrict__ density, float4* __restrict__ tapeSums, float* __restrict__ tapeRho,
-                       const uint2* __restrict__ meta, const uint4* __restrict__ rows, int tiles, int* tileCounter) {
+compute_scaling_kernel(const __grid_constant__ DevConsts c, const float4* pred, float4* predPacked,
+                       float* density, float4* tapeSums, float* tapeRho,
+                       const uint2* meta, const uint4* rows, int tiles, int* tileCounter) {
     chain_wait();
     for_tiles(tiles, tileCounter, [&](int tile) {
         const int i = B ? balanced_particle(meta, c.n, true, tile) : (tile * (int)blockDim.x + (int)threadIdx.x) / L;
@@ -977,15 +977,15 @@ __device__ __forceinline__ void end_of_step(const DevConsts& c, const StepEnd& e
 // src/Simulation.cpp:591), and the velocities are updated there as well
 // (end.posOut), which saves a launch and the prediction's way through memory.
 template <bool R, bool Q, int L>
-__device__ __forceinline__ void compute_delta_body(const DevConsts& c, const Batch& b, const float4* __restrict__ pp,
-                                                   const float4* __restrict__ posPrev, const StepEnd& end,
-                                                   float4* __restrict__ predOut,
-                                                   const float* __restrict__ density, int lastIteration,
-                                                   uint8_t* __restrict__ clampMask, const uint4* __restrict__ rows,
+__device__ __forceinline__ void compute_delta_body(const DevConsts& c, const Batch& b, const float4* pp,
+                                                   const float4* posPrev, const StepEnd& end,
+                                                   float4* predOut,
+                                                   const float* density, int lastIteration,
+                                                   uint8_t* clampMask, const uint4* rows,
                                                    int i, uint4 head, const float4 pi, uint64_t mt) {
     const int n = c.n;
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-    auto load = [&](uint32_t j) { return __ldg(pp + checked_index(j, (uint32_t)n, c.err, kErrFriendIndex)); };
+    auto load = [&](uint32_t j) { return pp[checked_index(j, (uint32_t)n, c.err, kErrFriendIndex)]; };
     auto one = [&](float rx, float ry, float rz, float r2, float wj) {  // a friend in support, divided the IEEE way
         const float rl = sqrtf(r2);
         const float hr = c.h - rl;
@@ -1106,10 +1106,10 @@ __device__ __forceinline__ void compute_delta_body(const DevConsts& c, const Bat
 
 template <bool R, bool B, int L>
 __global__ void __launch_bounds__(kMaxBlock)
-compute_delta_kernel(DevConsts c, Batch b, const float4* __restrict__ pp, const float4* __restrict__ posPrev,
-                     StepEnd end, float4* __restrict__ predOut, const float* __restrict__ density,
-                     const uint2* __restrict__ meta, int lastIteration, uint8_t* __restrict__ clampMask,
-                     const uint4* __restrict__ rows, int tiles, int* tileCounter) {
+compute_delta_kernel(const __grid_constant__ DevConsts c, Batch b, const float4* pp, const float4* posPrev,
+                     StepEnd end, float4* predOut, const float* density,
+                     const uint2* meta, int lastIteration, uint8_t* clampMask,
+                     const uint4* rows, int tiles, int* tileCounter) {
     chain_wait();
     for_tiles(tiles, tileCounter, [&](int tile) {
         const int i = B ? balanced_particle(meta, c.n, false, tile) : (tile * (int)blockDim.x + (int)threadIdx.x) / L;
@@ -1125,8 +1125,8 @@ compute_delta_kernel(DevConsts c, Batch b, const float4* __restrict__ pp, const 
 
 // ----------------------------------------------------------- velocities --
 // The end of a step without solver iterations.
-__global__ void update_velocities_kernel(DevConsts c, StepEnd end, const float4* __restrict__ pred,
-                                         const float4* __restrict__ posIn) {
+__global__ void update_velocities_kernel(DevConsts c, StepEnd end, const float4* pred,
+                                         const float4* posIn) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < c.n) end_of_step(c, end, i, pred[i], posIn[i]);
 }
@@ -1140,14 +1140,14 @@ __global__ void update_velocities_kernel(DevConsts c, StepEnd end, const float4*
 // of its two gathers per friend (79 %); with one it takes 0.191 ms instead of
 // 0.214 (1M particles, mid-collapse, two substeps).
 template <bool R, bool Q, int L>
-__device__ __forceinline__ void apply_viscosity_body(const DevConsts& c, const Batch& b, const float4* __restrict__ pred,
-                                                     const float4* __restrict__ velIn, float4* __restrict__ velOut,
-                                                     float4* __restrict__ omega, float4* __restrict__ near,
-                                                     const uint4* __restrict__ rows, int i, uint4 head, const float4 pi,
+__device__ __forceinline__ void apply_viscosity_body(const DevConsts& c, const Batch& b, const float4* pred,
+                                                     const float4* velIn, float4* velOut,
+                                                     float4* omega, float4* near,
+                                                     const uint4* rows, int i, uint4 head, const float4 pi,
                                                      const float4 vi, uint64_t mt) {
     const int n = c.n;
     float vsx = 0.0f, vsy = 0.0f, vsz = 0.0f, ox = 0.0f, oy = 0.0f, oz = 0.0f;
-    auto load = [&](uint32_t j) { j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex); return PairRec{__ldg(pred + j), __ldg(velIn + j)}; };
+    auto load = [&](uint32_t j) { j = checked_index(j, (uint32_t)n, c.err, kErrFriendIndex); return PairRec{pred[j], velIn[j]}; };
     constexpr bool kLaneSums = L > 1 && Q && !R;  // the other forms go in_turn
     __shared__ __align__(16) float terms[kLaneSums ? kMaxBlock / L * LaneSums<L, 6>::kStride : 1];
     LaneSums<L, 6> sums(terms, {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f});
@@ -1249,9 +1249,9 @@ __device__ __forceinline__ void apply_viscosity_body(const DevConsts& c, const B
 
 template <bool R, bool B, int L>
 __global__ void __maxnreg__(72)
-apply_viscosity_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, const float4* __restrict__ velIn,
-                       float4* __restrict__ velOut, float4* __restrict__ omega, float4* __restrict__ near,
-                       const uint2* __restrict__ meta, const uint4* __restrict__ rows, int tiles, int* tileCounter) {
+apply_viscosity_kernel(const __grid_constant__ DevConsts c, Batch b, const float4* pred, const float4* velIn,
+                       float4* velOut, float4* omega, float4* near,
+                       const uint2* meta, const uint4* rows, int tiles, int* tileCounter) {
     chain_wait();
     for_tiles(tiles, tileCounter, [&](int tile) {
         const int i = B ? balanced_particle(meta, c.n, false, tile) : (tile * (int)blockDim.x + (int)threadIdx.x) / L;
@@ -1267,14 +1267,14 @@ apply_viscosity_kernel(DevConsts c, Batch b, const float4* __restrict__ pred, co
 
 // apply_vorticity.cl:12-86; neighbours are read from near (apply_viscosity).
 template <bool R, bool Q, int L>
-__device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const float4* __restrict__ near,
-                                                     const float4* __restrict__ omega,
-                                                     const float4* __restrict__ velIn, float4* __restrict__ velOut,
-                                                     float4* __restrict__ tapeEta, const uint4* __restrict__ rows, int i,
+__device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const float4* near,
+                                                     const float4* omega,
+                                                     const float4* velIn, float4* velOut,
+                                                     float4* tapeEta, const uint4* rows, int i,
                                                      uint4 head, const float4 pi, uint64_t mt) {
     const int n = c.n;
     float ex = 0.0f, ey = 0.0f, ez = 0.0f;
-    auto load = [&](uint32_t j) { return __ldg(near + checked_index(j, (uint32_t)n, c.err, kErrFriendIndex)); };
+    auto load = [&](uint32_t j) { return near[checked_index(j, (uint32_t)n, c.err, kErrFriendIndex)]; };
     constexpr bool kLaneSums = L > 1 && Q && !R;  // the other forms go in_turn
     __shared__ __align__(16) float terms[kLaneSums ? kMaxBlock / L * LaneSums<L, 3>::kStride : 1];
     LaneSums<L, 3> sums(terms, {0.0f, 0.0f, 0.0f});
@@ -1364,10 +1364,10 @@ __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const f
 
 template <bool R, bool B, int L>
 __global__ void __maxnreg__(56)
-apply_vorticity_kernel(DevConsts c, const float4* __restrict__ pred, const float4* __restrict__ near,
-                       const float4* __restrict__ omega, const float4* __restrict__ velIn, float4* __restrict__ velOut,
-                       float4* __restrict__ tapeEta, const uint2* __restrict__ meta,
-                       const uint4* __restrict__ rows, int tiles, int* tileCounter, int tileOffset) {
+apply_vorticity_kernel(const __grid_constant__ DevConsts c, const float4* pred, const float4* near,
+                       const float4* omega, const float4* velIn, float4* velOut,
+                       float4* tapeEta, const uint2* meta,
+                       const uint4* rows, int tiles, int* tileCounter, int tileOffset) {
     chain_wait();
     for_tiles(tiles, tileCounter, [&](int tile) {
         tile += tileOffset * L;  // a launch over part of the tiles (L blocks per tile)

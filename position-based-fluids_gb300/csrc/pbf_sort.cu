@@ -172,8 +172,8 @@ constexpr int kScanChunk = 4 * kThreads;  // counters a block takes at a time
 
 // Sum of each block's tile of counters.
 __global__ void __launch_bounds__(kThreads)
-counting_sums_kernel(const uint4* __restrict__ counts, uint32_t chunks, uint32_t chunksPerBlock,
-                     uint32_t* __restrict__ sums) {
+counting_sums_kernel(const uint4* counts, uint32_t chunks, uint32_t chunksPerBlock,
+                     uint32_t* sums) {
     chain_wait();
     __shared__ uint32_t warpSums[kWarps];
     const uint32_t first = blockIdx.x * chunksPerBlock, last = min(first + chunksPerBlock, chunks);
@@ -199,8 +199,8 @@ counting_sums_kernel(const uint4* __restrict__ counts, uint32_t chunks, uint32_t
 // of them), so no block waits for another.
 constexpr uint32_t kMaxScanBlocks = 1024, kOneBlockChunks = 16;
 __global__ void __launch_bounds__(kThreads)
-counting_scan_kernel(uint4* __restrict__ counts, uint32_t chunks, uint32_t chunksPerBlock,
-                     const uint32_t* __restrict__ sums, uint4* __restrict__ starts) {
+counting_scan_kernel(uint4* counts, uint32_t chunks, uint32_t chunksPerBlock,
+                     const uint32_t* sums, uint4* starts) {
     chain_wait();
     __shared__ uint32_t warpSums[kWarps];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -242,8 +242,8 @@ counting_scan_kernel(uint4* __restrict__ counts, uint32_t chunks, uint32_t chunk
 
 // order[first index of the key + place of arrival] = particle
 __global__ void __launch_bounds__(kThreads)
-cell_scatter_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ place,
-                    const uint32_t* __restrict__ starts, uint32_t* __restrict__ order, int* __restrict__ err) {
+cell_scatter_kernel(int n, const uint32_t* keys, const uint32_t* place,
+                    const uint32_t* starts, uint32_t* order, int* err) {
     chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) order[checked_index(starts[keys[i]] + place[i], (uint32_t)n, err, kErrSortIndex)] = (uint32_t)i;
@@ -254,12 +254,12 @@ cell_scatter_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __
 // its key, index, position, prediction and id (radixsort.cl:22-37; velocities
 // are not permuted, they are recomputed before any read, update_velocities.cl:13).
 __global__ void __launch_bounds__(kThreads)
-cell_gather_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ starts,
-                   const uint32_t* __restrict__ order, uint32_t* __restrict__ keysOut, uint32_t* __restrict__ permOut,
-                   uint32_t* __restrict__ permCopy,
-                   const float4* __restrict__ pos, const float4* __restrict__ pred, const uint32_t* __restrict__ ids,
-                   float4* __restrict__ posOut, float4* __restrict__ predOut, uint32_t* __restrict__ idsOut,
-                   int* __restrict__ err) {
+cell_gather_kernel(int n, const uint32_t* keys, const uint32_t* starts,
+                   const uint32_t* order, uint32_t* keysOut, uint32_t* permOut,
+                   uint32_t* permCopy,
+                   const float4* pos, const float4* pred, const uint32_t* ids,
+                   float4* posOut, float4* predOut, uint32_t* idsOut,
+                   int* err) {
     chain_wait();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
@@ -284,8 +284,8 @@ cell_gather_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __r
 // launch).
 constexpr uint32_t kCrowdedCell = 1024;
 __global__ void __launch_bounds__(kThreads)
-cell_rank_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ starts,
-                 const uint32_t* __restrict__ order, uint32_t* __restrict__ permOut, uint32_t* __restrict__ crowded) {
+cell_rank_kernel(int n, const uint32_t* keys, const uint32_t* starts,
+                 const uint32_t* order, uint32_t* permOut, uint32_t* crowded) {
     chain_wait();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= (uint32_t)n) return;
@@ -306,8 +306,8 @@ cell_rank_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __res
 // of them one after another took 100 us; those of crowded cells are left to
 // crowded_cells_kernel.
 __global__ void __launch_bounds__(kThreads)
-cell_table_kernel(int n, uint32_t keys, const uint32_t* __restrict__ starts, uint32_t* __restrict__ keysOut,
-                  uint32_t* __restrict__ cells) {
+cell_table_kernel(int n, uint32_t keys, const uint32_t* starts, uint32_t* keysOut,
+                  uint32_t* cells) {
     chain_wait();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
@@ -342,8 +342,8 @@ constexpr uint32_t kMostParts = 16, kPartCell = 16384;
 constexpr int kMostShift = 5;  // 2^5 words to a thread
 static_assert(PBF_NOALLOC_MAX_KEYS == (kCrowdedThreads * 32) << kMostShift, "the bitmap holds every index");
 __global__ void __launch_bounds__(kCrowdedThreads)
-crowded_cells_kernel(const uint32_t* __restrict__ crowded, const uint32_t* __restrict__ starts,
-                     const uint32_t* __restrict__ order, uint32_t* __restrict__ keysOut, uint32_t* __restrict__ permOut) {
+crowded_cells_kernel(const uint32_t* crowded, const uint32_t* starts,
+                     const uint32_t* order, uint32_t* keysOut, uint32_t* permOut) {
     chain_wait();
     extern __shared__ uint32_t marks[];  // kCrowdedThreads words for every word to a thread
     __shared__ uint32_t warpSums[kCrowdedThreads / 32], below, least, largest;
