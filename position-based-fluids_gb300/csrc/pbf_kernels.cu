@@ -948,7 +948,7 @@ compute_scaling_kernel(const __grid_constant__ DevConsts c, const float4* pred, 
         const uint4 head = first_entry<L>(rows, c.n, i);
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) compute_scaling_body<R, true, L>(c, pred, predPacked, density, tapeSums, tapeRho, rows, i, head, pi, mt);
+        if (!R && c.quotients && !quotients_tainted<L>(c, i)) compute_scaling_body<R, true, L>(c, pred, predPacked, density, tapeSums, tapeRho, rows, i, head, pi, mt);
         else compute_scaling_body<R, false, L>(c, pred, predPacked, density, tapeSums, tapeRho, rows, i, head, pi, mt);
     });
 }
@@ -1118,7 +1118,7 @@ compute_delta_kernel(const __grid_constant__ DevConsts c, Batch b, const float4*
         const uint4 head = first_entry<L>(rows, c.n, i);
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) compute_delta_body<R, true, L>(c, b, pp, posPrev, end, predOut, density, lastIteration, clampMask, rows, i, head, pi, mt);
+        if (!R && c.quotients && !quotients_tainted<L>(c, i)) compute_delta_body<R, true, L>(c, b, pp, posPrev, end, predOut, density, lastIteration, clampMask, rows, i, head, pi, mt);
         else compute_delta_body<R, false, L>(c, b, pp, posPrev, end, predOut, density, lastIteration, clampMask, rows, i, head, pi, mt);
     });
 }
@@ -1260,7 +1260,7 @@ apply_viscosity_kernel(const __grid_constant__ DevConsts c, Batch b, const float
         const uint4 head = first_entry<L>(rows, c.n, i);
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) apply_viscosity_body<R, true, L>(c, b, pred, velIn, velOut, omega, near, rows, i, head, pi, vi, mt);
+        if (!R && c.quotients && !quotients_tainted<L>(c, i)) apply_viscosity_body<R, true, L>(c, b, pred, velIn, velOut, omega, near, rows, i, head, pi, vi, mt);
         else apply_viscosity_body<R, false, L>(c, b, pred, velIn, velOut, omega, near, rows, i, head, pi, vi, mt);
     });
 }
@@ -1377,7 +1377,7 @@ apply_vorticity_kernel(const __grid_constant__ DevConsts c, const float4* pred, 
         const uint4 head = first_entry<L>(rows, c.n, i);
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted(c, i)) apply_vorticity_body<R, true, L>(c, near, omega, velIn, velOut, tapeEta, rows, i, head, pi, mt);
+        if (!R && c.quotients && !quotients_tainted<L>(c, i)) apply_vorticity_body<R, true, L>(c, near, omega, velIn, velOut, tapeEta, rows, i, head, pi, mt);
         else apply_vorticity_body<R, false, L>(c, near, omega, velIn, velOut, tapeEta, rows, i, head, pi, mt);
     });
 }
