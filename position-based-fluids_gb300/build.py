@@ -11,9 +11,10 @@ arithmetic contract:
   host are the same on x86-64 and aarch64.
 
 ``build(checked=True)`` builds libpbf_gb300_checked.so from the same sources
-with ``-DPBF_CHECK_BOUNDS``: every index the kernels read from device memory
-(friend-list entries, the sort permutation, keys) is checked before use and
-an out-of-range one is reported through the context's error word.  The
+with ``-DPBF_CHECK_BOUNDS``: the indices that the kernels read from device
+memory (friend-list entries, sort permutations, keys and the ranges they stand
+for) are checked before use and an out-of-range one is reported through the
+context's error word.  The
 arithmetic is the same, so its results are identical.  ``pbf.py`` loads it
 when ``PBF_CHECK_BOUNDS=1`` is set.
 """

@@ -343,7 +343,7 @@ adj_unsort_predict_kernel(DevConsts c, const uint32_t* perm, const float4* xsb,
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     F3 g = {0.0f, 0.0f, 0.0f};
     if (k < c.n) {
-        const uint32_t i = perm[k];
+        const uint32_t i = checked_index(perm[k], (uint32_t)c.n, c.err, kErrSortIndex);
         const F3 p = f3(pb0[k]);
         pb0[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         const F3 x = f3(xsb[k]) + p;

@@ -495,6 +495,7 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
     auto tiles = [&](int kernel) { return ls.persistent ? ctx->tileCounters + 2 * kernel : nullptr; };
     // a paused substep keeps the last sort's keys, and takes its cells from them
     const bool counting = ctx->counting.blocks > 0 && !paused;
+    const uint32_t tableKeys = ctx->cellsWords * (uint32_t)(is_batch(ctx) ? ctx->sceneParams.size() : 1);
     uint32_t* order = reinterpret_cast<uint32_t*>(ctx->vel[V ^ 1]);  // free until XSPH
     pbf::launch_predict_keys(c, b, ctx->pos[P], ctx->vel[V], ctx->pred[0], ctx->keys[0], ctx->perm[0],
                              counting ? ctx->cellCounts : nullptr, paused, s);
@@ -504,7 +505,7 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
         mark("radixsort");
         if (counting) {
             pbf::launch_counting_sort(ctx->counting, c.n, ctx->cellCounts, ctx->scanSums, ctx->cellStart, ctx->keys[0],
-                                      ctx->perm[0], order, ctx->errWord, s);
+                                      ctx->perm[0], order, tableKeys, ctx->errWord, s);
             launched += ctx->counting.blocks > 1 ? 3 : 2;
         } else {
             ctx->keysIdx = pbf::launch_radix_sort(ctx->plan, ctx->keys, ctx->perm, ctx->hist, nullptr, nullptr, nullptr,
@@ -516,7 +517,8 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
             ctx->keysIdx = 1;
             pbf::launch_cell_gather(c.n, ctx->keys[0], ctx->cellStart, order, ctx->keys[1], ctx->perm[1],
                                     tape ? tape->perm : nullptr, ctx->pos[P],
-                                    ctx->pred[0], ctx->ids, ctx->pos[P ^ 1], ctx->pred[1], ctx->idsTmp, ctx->errWord, s);
+                                    ctx->pred[0], ctx->ids, ctx->pos[P ^ 1], ctx->pred[1], ctx->idsTmp, tableKeys,
+                                    ctx->errWord, s);
         } else {
             pbf::launch_gather_sorted(c.n, ctx->perm[ctx->keysIdx], ctx->pos[P], ctx->pred[0], ctx->ids, ctx->pos[P ^ 1],
                                       ctx->pred[1], ctx->idsTmp, ctx->errWord, s);
@@ -534,7 +536,6 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
     float4* omega = tape ? tape->omega : ctx->omega;
     if (tape && !counting) PBF_CUDA(ctx, cudaMemcpyAsync(tape->perm, ctx->perm[ctx->keysIdx], 4 * (size_t)c.n, cudaMemcpyDeviceToDevice, s));
     mark("updateCells");
-    const uint32_t tableKeys = ctx->cellsWords * (uint32_t)(is_batch(ctx) ? ctx->sceneParams.size() : 1);
     c.keys = keys;  // the taint of irregular positions finds a cell's particles in them
     if (!counting) {
         pbf::launch_update_cells(c.n, keys, ctx->cells, tableKeys, ctx->errWord, s, ctx->cellStart);
@@ -1191,6 +1192,7 @@ int pbf_render_frame(pbf_ctx* ctx, const PbfCamera* cam, int mode) {
         r.height = cam->height;
         r.n = ctx->n;
     }
+    r.err = ctx->errWord;
     pbf::render_frame(*cam, mode, ctx->n, ctx->params.h, ctx->pos[ctx->curPos], r, ctx->stream);
     ctx->launches += pbf::render_launches(mode);
     ctx->renderMode = mode;

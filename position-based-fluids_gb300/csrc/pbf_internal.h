@@ -223,14 +223,16 @@ CountingPlan make_scan_plan(uint64_t keys);  // whatever the number of particles
 void launch_counting_scan(const CountingPlan& plan, uint32_t* counts, uint32_t* sums, uint32_t* starts, cudaStream_t s);
 // From the counts and the particles' places of arrival (launch_predict_keys):
 // the first index of every key into `starts`, and the particles grouped by key,
-// in any order within a key, into `order`.  Zeroes the counts.
+// in any order within a key, into `order`.  Zeroes the counts.  keyLimit, err: as
+// for launch_update_cells.
 void launch_counting_sort(const CountingPlan& plan, int n, uint32_t* counts, uint32_t* sums, uint32_t* starts,
-                          const uint32_t* keys, const uint32_t* place, uint32_t* order, int* err, cudaStream_t s);
+                          const uint32_t* keys, const uint32_t* place, uint32_t* order, uint32_t keyLimit, int* err,
+                          cudaStream_t s);
 // The stable order from it, with the records gathered (launch_gather_sorted);
 // permCopy (may be NULL) receives the permutation too.
 void launch_cell_gather(int n, const uint32_t* keys, const uint32_t* starts, const uint32_t* order, uint32_t* keysOut,
                         uint32_t* permOut, uint32_t* permCopy, const float4* pos, const float4* pred,
-                        const uint32_t* ids, float4* posOut, float4* predOut, uint32_t* idsOut, int* err,
+                        const uint32_t* ids, float4* posOut, float4* predOut, uint32_t* idsOut, uint32_t keyLimit, int* err,
                         cudaStream_t s);
 // For the entry point that sorts without records (at most PBF_NOALLOC_MAX_KEYS
 // particles): the stable permutation, the sorted keys (in place of the
@@ -285,6 +287,7 @@ struct RenderBuffers {
     uint32_t* sums = nullptr;
     uint32_t* shownCount = nullptr;      // sprites that draw_kernel draws
     CountingPlan plan{};
+    int* err = nullptr;                  // the context's error word (bounds-checked builds)
 };
 void render_frame(const PbfCamera& cam, int mode, int n, float h, const float4* pos, RenderBuffers& rb, cudaStream_t s);
 int render_launches(int mode);

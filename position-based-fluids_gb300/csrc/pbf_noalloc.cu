@@ -144,7 +144,7 @@ extern "C" int pbf_sort_state_noalloc(const PbfParameters* params, const float* 
         e = cudaMemsetAsync(counts, 0, 4 * counting.words, s);
         if (e == cudaSuccess) {
             pbf::launch_compute_keys(c, pbf::Batch{nullptr, nullptr}, reinterpret_cast<const float4*>(d_pred), d_keys, d_perm, counts, s);
-            pbf::launch_counting_sort(counting, (int)n, counts, sums, starts, d_keys, d_perm, order, nullptr, s);
+            pbf::launch_counting_sort(counting, (int)n, counts, sums, starts, d_keys, d_perm, order, params->gridBufSize, nullptr, s);
             e = pbf::launch_cell_finish((int)n, params->gridBufSize, starts, order, d_keys, d_perm, d_cells, counts, s);
             const cudaError_t launched = cudaGetLastError();
             if (e == cudaSuccess) e = launched;

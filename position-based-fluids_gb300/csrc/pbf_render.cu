@@ -27,6 +27,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "pbf_device.cuh"
 #include "pbf_internal.h"
 
 namespace pbf {
@@ -236,14 +237,14 @@ splat_kernel(PbfCamera cam, int n, const float4* __restrict__ pos, const uint32_
 // together in memory, so they are dealt out over the whole chip.
 constexpr int kDrawBlocks = 152 * 16;
 __global__ void __launch_bounds__(128)
-draw_kernel(PbfCamera cam, const float4* __restrict__ pos, const uint32_t* __restrict__ tileDepth,
+draw_kernel(PbfCamera cam, int n, const float4* __restrict__ pos, const uint32_t* __restrict__ tileDepth,
             unsigned long long* __restrict__ dkey, const uint32_t* __restrict__ shown,
-            const uint32_t* __restrict__ shownCount) {
+            const uint32_t* __restrict__ shownCount, int* err) {
     const int lane = threadIdx.x & 31;
-    const uint32_t count = *shownCount;
+    const uint32_t count = checked_index(*shownCount, (uint32_t)n + 1u, err, kErrSortIndex);
     const int tilesX = (cam.width + kTilePixels - 1) / kTilePixels;
     for (uint32_t k = blockIdx.x * 4 + (threadIdx.x >> 5); k < count; k += kDrawBlocks * 4) {
-        const int p = (int)shown[k];
+        const int p = (int)checked_index(shown[k], (uint32_t)n, err, kErrSortIndex);
         float ex, ey, ez, xw, yw, s;
         sprite(cam, pos[p], ex, ey, ez, xw, yw, s);
         const Rect r = sprite_rect(cam, xw, yw, s);
@@ -334,27 +335,28 @@ __global__ void grid_count_kernel(int n, float h, const float4* __restrict__ pos
 }
 
 __global__ void grid_scatter_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ place,
-                                    const uint32_t* __restrict__ starts, uint32_t* __restrict__ order) {
+                                    const uint32_t* __restrict__ starts, uint32_t* __restrict__ order, int* err) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || keys[i] >= kGridBuckets) return;
-    order[starts[keys[i]] + place[i]] = (uint32_t)i;
+    order[checked_index(starts[keys[i]] + place[i], (uint32_t)n, err, kErrSortIndex)] = (uint32_t)i;
 }
 
 // The positions of each bucket's particles by decreasing index, the order of its chain.
-__global__ void grid_rank_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ starts,
+__global__ void grid_rank_kernel(int n, const uint32_t* __restrict__ keys, const uint32_t* __restrict__ starts,
                                  const uint32_t* __restrict__ order, const float4* __restrict__ pos,
-                                 float4* __restrict__ sorted) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= starts[kGridBuckets]) return;
-    const uint32_t i = order[s], key = keys[i], first = starts[key], end = starts[key + 1];
+                                 float4* __restrict__ sorted, int* err) {
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x, limit = (uint32_t)n;
+    if (s >= checked_index(starts[kGridBuckets], limit + 1u, err, kErrSortIndex)) return;
+    const uint32_t i = checked_index(order[s], limit, err, kErrSortIndex), key = checked_index(keys[i], kGridBuckets, err, kErrCellKey);
+    const uint32_t first = starts[key], end = checked_index(starts[key + 1], limit + 1u, err, kErrSortIndex);
     uint32_t to = first;
     for (uint32_t q = first; q < end; ++q) to += order[q] > i;
-    sorted[to] = pos[i];
+    sorted[checked_index(to, limit, err, kErrSortIndex)] = pos[i];
 }
 
 // fluid_depth_smoothing.fs SampleDensityAndGradient
-__device__ void sample_density(float h, const float4* __restrict__ sorted, const uint32_t* __restrict__ starts, float wx, float wy, float wz, float& density,
-                               float& gx, float& gy, float& gz) {
+__device__ void sample_density(float h, int n, const float4* __restrict__ sorted, const uint32_t* __restrict__ starts,
+                               int* err, float wx, float wy, float wz, float& density, float& gx, float& gy, float& gz) {
     const float h2 = h * h;
     density = 0.0f;
     gx = gy = gz = 0.0f;
@@ -372,7 +374,7 @@ __device__ void sample_density(float h, const float4* __restrict__ sorted, const
 #pragma unroll
             for (int part = 0; part < 2; ++part) {
                 const uint32_t b = (from[part] | yz) & (kGridBuckets - 1u);
-                const int end = (int)starts[b + length[part]];
+                const int end = (int)checked_index(starts[b + length[part]], (uint32_t)n + 1u, err, kErrSortIndex);
 #pragma unroll 4
                 for (int k = (int)starts[b]; k < end; ++k) {
                     const float4 pp = __ldg(sorted + k);
@@ -415,8 +417,8 @@ __device__ __forceinline__ void normalize3(float& x, float& y, float& z) {
 // the permutation, 118 like this, and 110 with two buckets to a range (the scene
 // above; pairs of candidates in packed arithmetic: 105, and slower at 1M sprites).
 __global__ void __launch_bounds__(128)
-smooth_kernel(PbfCamera cam, float h, const float4* __restrict__ sorted, const uint32_t* __restrict__ starts,
-              const float4* __restrict__ splat, float4* __restrict__ out) {
+smooth_kernel(PbfCamera cam, float h, int n, const float4* __restrict__ sorted, const uint32_t* __restrict__ starts,
+              const float4* __restrict__ splat, float4* __restrict__ out, int* err) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int i = blockIdx.x * 16 + 8 * (warp & 1) + (lane & 7), j = blockIdx.y * 8 + 4 * (warp >> 1) + (lane >> 3);
     if (i >= cam.width || j >= cam.height) return;
@@ -431,7 +433,7 @@ smooth_kernel(PbfCamera cam, float h, const float4* __restrict__ sorted, const u
     float tp = 0.0f, sx = m.x, sy = m.y, sz = m.z;
     float density, gx = 0.0f, gy = 0.0f, gz = 0.0f;
     for (int it = 0; it < 2; ++it) {
-        sample_density(h, sorted, starts, sx, sy, sz, density, gx, gy, gz);
+        sample_density(h, n, sorted, starts, err, sx, sy, sz, density, gx, gy, gz);
         const float dd = density - 1.0f;
         const float ga = dot3f(nx, ny, nz, gx, gy, gz);
         tp += dd / ga;
@@ -509,7 +511,7 @@ void render_frame(const PbfCamera& cam, int mode, int n, float h, const float4* 
         occlude_kernel<<<blocks(n, 128), 128, 0, s>>>(cam, n, pos, tileDepth);
     }
     splat_kernel<<<blocks(n, 128), 128, 0, s>>>(cam, n, pos, tileDepth, rb.dkey, rb.order, rb.shownCount);
-    draw_kernel<<<kDrawBlocks, 128, 0, s>>>(cam, pos, tileDepth, rb.dkey, rb.order, rb.shownCount);
+    draw_kernel<<<kDrawBlocks, 128, 0, s>>>(cam, n, pos, tileDepth, rb.dkey, rb.order, rb.shownCount, rb.err);
     if (mode == 0) cudaMemsetAsync(rb.vis, 0, (size_t)n, s);
     resolve_kernel<<<blocks(pixels, 256), 256, 0, s>>>(cam, n, mode, pos, rb.dkey, rb.splat, rb.vis);
     if (mode != 0) {
@@ -518,10 +520,10 @@ void render_frame(const PbfCamera& cam, int mode, int n, float h, const float4* 
     }
     grid_count_kernel<<<blocks(n, 256), 256, 0, s>>>(n, h, pos, rb.vis, rb.keys, rb.place, rb.counts);
     launch_counting_scan(rb.plan, rb.counts, rb.sums, rb.starts, s);
-    grid_scatter_kernel<<<blocks(n, 256), 256, 0, s>>>(n, rb.keys, rb.place, rb.starts, rb.order);
-    grid_rank_kernel<<<blocks(n, 256), 256, 0, s>>>(rb.keys, rb.starts, rb.order, pos, rb.sorted);
-    smooth_kernel<<<dim3(blocks(cam.width, 16), blocks(cam.height, 8)), 128, 0, s>>>(cam, h, rb.sorted, rb.starts, rb.splat,
-                                                                                    rb.smooth);
+    grid_scatter_kernel<<<blocks(n, 256), 256, 0, s>>>(n, rb.keys, rb.place, rb.starts, rb.order, rb.err);
+    grid_rank_kernel<<<blocks(n, 256), 256, 0, s>>>(n, rb.keys, rb.starts, rb.order, pos, rb.sorted, rb.err);
+    smooth_kernel<<<dim3(blocks(cam.width, 16), blocks(cam.height, 8)), 128, 0, s>>>(cam, h, n, rb.sorted, rb.starts, rb.splat,
+                                                                                    rb.smooth, rb.err);
     final_kernel<<<blocks(pixels, 256), 256, 0, s>>>(cam, rb.smooth, rb.out);
 }
 

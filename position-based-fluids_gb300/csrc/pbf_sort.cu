@@ -243,10 +243,12 @@ counting_scan_kernel(uint4* counts, uint32_t chunks, uint32_t chunksPerBlock,
 // order[first index of the key + place of arrival] = particle
 __global__ void __launch_bounds__(kThreads)
 cell_scatter_kernel(int n, const uint32_t* keys, const uint32_t* place,
-                    const uint32_t* starts, uint32_t* order, int* err) {
+                    const uint32_t* starts, uint32_t* order, uint32_t keyLimit, int* err) {
     chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) order[checked_index(starts[keys[i]] + place[i], (uint32_t)n, err, kErrSortIndex)] = (uint32_t)i;
+    if (i >= n) return;
+    const uint32_t first = starts[checked_index(keys[i], keyLimit, err, kErrCellKey)];
+    order[checked_index(first + place[i], (uint32_t)n, err, kErrSortIndex)] = (uint32_t)i;
 }
 
 // The particle in slot s of the scattered order goes to its cell's first index
@@ -259,14 +261,14 @@ cell_gather_kernel(int n, const uint32_t* keys, const uint32_t* starts,
                    uint32_t* permCopy,
                    const float4* pos, const float4* pred, const uint32_t* ids,
                    float4* posOut, float4* predOut, uint32_t* idsOut,
-                   int* err) {
+                   uint32_t keyLimit, int* err) {
     chain_wait();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const uint32_t i = checked_index(order[s], (uint32_t)n, err, kErrSortIndex);
     const float4 x = pos[i], p = pred[i];
-    const uint32_t id = ids[i], key = keys[i];
-    const uint32_t first = starts[key], end = starts[key + 1];
+    const uint32_t id = ids[i], key = checked_index(keys[i], keyLimit, err, kErrCellKey);
+    const uint32_t first = starts[key], end = checked_index(starts[key + 1], (uint32_t)n + 1u, err, kErrSortIndex);
     uint32_t to = first;
     for (uint32_t q = first; q < end; ++q) to += order[q] < i;
     to = checked_index(to, (uint32_t)n, err, kErrSortIndex);
@@ -284,12 +286,14 @@ cell_gather_kernel(int n, const uint32_t* keys, const uint32_t* starts,
 // launch).
 constexpr uint32_t kCrowdedCell = 1024;
 __global__ void __launch_bounds__(kThreads)
-cell_rank_kernel(int n, const uint32_t* keys, const uint32_t* starts,
+cell_rank_kernel(int n, uint32_t keyLimit, const uint32_t* keys, const uint32_t* starts,
                  const uint32_t* order, uint32_t* permOut, uint32_t* crowded) {
     chain_wait();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= (uint32_t)n) return;
-    const uint32_t i = order[s], key = keys[i], first = starts[key], end = starts[key + 1];
+    const uint32_t i = checked_index(order[s], (uint32_t)n, nullptr, kErrSortIndex);
+    const uint32_t key = checked_index(keys[i], keyLimit, nullptr, kErrCellKey);
+    const uint32_t first = starts[key], end = checked_index(starts[key + 1], (uint32_t)n + 1u, nullptr, kErrSortIndex);
     if (end - first > kCrowdedCell) {
         if (s == first) crowded[1u + atomicAdd(crowded, 1u)] = key;
         return;
@@ -418,7 +422,7 @@ crowded_cells_kernel(const uint32_t* crowded, const uint32_t* starts,
 
 cudaError_t launch_cell_finish(int n, uint32_t keyCount, const uint32_t* starts, const uint32_t* order, uint32_t* keys,
                                uint32_t* permOut, uint32_t* cells, uint32_t* crowded, cudaStream_t s) {
-    launch_chained(cell_rank_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keys, starts, order, permOut, crowded);
+    launch_chained(cell_rank_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keyCount, keys, starts, order, permOut, crowded);
     launch_chained(cell_table_kernel, (keyCount + kThreads - 1) / kThreads, kThreads, s, n, keyCount, starts, keys, cells);
     if ((uint32_t)n <= kCrowdedCell) return cudaGetLastError();
     int shift = 0;
@@ -467,17 +471,18 @@ void launch_counting_scan(const CountingPlan& plan, uint32_t* counts, uint32_t* 
 }
 
 void launch_counting_sort(const CountingPlan& plan, int n, uint32_t* counts, uint32_t* sums, uint32_t* starts,
-                          const uint32_t* keys, const uint32_t* place, uint32_t* order, int* err, cudaStream_t s) {
+                          const uint32_t* keys, const uint32_t* place, uint32_t* order, uint32_t keyLimit, int* err,
+                          cudaStream_t s) {
     launch_counting_scan(plan, counts, sums, starts, s);
-    launch_chained(cell_scatter_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keys, place, starts, order, err);
+    launch_chained(cell_scatter_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keys, place, starts, order, keyLimit, err);
 }
 
 void launch_cell_gather(int n, const uint32_t* keys, const uint32_t* starts, const uint32_t* order, uint32_t* keysOut,
                         uint32_t* permOut, uint32_t* permCopy, const float4* pos, const float4* pred,
-                        const uint32_t* ids, float4* posOut, float4* predOut, uint32_t* idsOut, int* err,
+                        const uint32_t* ids, float4* posOut, float4* predOut, uint32_t* idsOut, uint32_t keyLimit, int* err,
                         cudaStream_t s) {
     launch_chained(cell_gather_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keys, starts, order, keysOut, permOut, permCopy, pos,
-                                                                          pred, ids, posOut, predOut, idsOut, err);
+                                                                          pred, ids, posOut, predOut, idsOut, keyLimit, err);
 }
 
 SortPlan make_sort_plan(int n, uint32_t gridBufSize) {
