@@ -505,7 +505,7 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
         mark("radixsort");
         if (counting) {
             pbf::launch_counting_sort(ctx->counting, c.n, ctx->cellCounts, ctx->scanSums, ctx->cellStart, ctx->keys[0],
-                                      ctx->perm[0], order, tableKeys, ctx->errWord, s);
+                                      ctx->perm[0], order, nullptr, tableKeys, ctx->errWord, s);
             launched += ctx->counting.blocks > 1 ? 3 : 2;
         } else {
             ctx->keysIdx = pbf::launch_radix_sort(ctx->plan, ctx->keys, ctx->perm, ctx->hist, nullptr, nullptr, nullptr,
@@ -1447,7 +1447,7 @@ int pbf_sort_state(pbf_ctx* ctx, const float* pred, uint32_t* keys, uint32_t* pe
     auto keep = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };  // the first error of the sequence
     keep(cudaMemcpyAsync(dPred, pred, 16 * (size_t)n, cudaMemcpyHostToDevice, s));
     keep(cudaMemsetAsync(dCells, 0xFF, 8 * (size_t)grid, s));
-    pbf::launch_compute_keys(ctx->consts, batch_of(ctx), dPred, k[0], pm[0], nullptr, s);
+    pbf::launch_compute_keys(ctx->consts, batch_of(ctx), dPred, k[0], pm[0], nullptr, nullptr, s);
     const int r = pbf::launch_radix_sort(ctx->plan, k, pm, dHist, nullptr, nullptr, nullptr, nullptr, s);
     pbf::launch_update_cells(n, k[r], dCells, grid, nullptr, s);
     const uint32_t nKeys = ((uint32_t)n + 2047u) / 2048u * 2048u;

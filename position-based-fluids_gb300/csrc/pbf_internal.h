@@ -126,8 +126,12 @@ inline void launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, 
 // own index (launch_compute_keys too).
 void launch_predict_keys(const DevConsts& c, Batch b, const float4* pos, float4* vel, float4* pred,
                          uint32_t* keys, uint32_t* perm, uint32_t* counts, int paused, cudaStream_t s);
+// hot: NULL, or the word that launch_clear_counts set.
 void launch_compute_keys(const DevConsts& c, Batch b, const float4* pred, uint32_t* keys, uint32_t* perm, uint32_t* counts,
-                         cudaStream_t s);
+                         const uint32_t* hot, cudaStream_t s);
+// Clears the counts (words: a multiple of 4) before launch_compute_keys, and tells
+// in *hot whether few cells hold most of the particles of this single scene.
+void launch_clear_counts(const DevConsts& c, const float4* pred, uint32_t* counts, size_t words, uint32_t* hot, cudaStream_t s);
 // err (may be NULL): the error word that bounds-checked builds report bad
 // permutation entries or keys to; keyLimit: the number of cell-table entries.
 void launch_gather_sorted(int n, const uint32_t* perm, const float4* pos, const float4* pred, const uint32_t* ids,
@@ -223,11 +227,12 @@ CountingPlan make_scan_plan(uint64_t keys);  // whatever the number of particles
 void launch_counting_scan(const CountingPlan& plan, uint32_t* counts, uint32_t* sums, uint32_t* starts, cudaStream_t s);
 // From the counts and the particles' places of arrival (launch_predict_keys):
 // the first index of every key into `starts`, and the particles grouped by key,
-// in any order within a key, into `order`.  Zeroes the counts.  keyLimit, err: as
-// for launch_update_cells.
+// in any order within a key, into `order`.  Zeroes the counts.  crowded: `counts`
+// where launch_cell_finish follows, else NULL.  keyLimit, err: as for
+// launch_update_cells.
 void launch_counting_sort(const CountingPlan& plan, int n, uint32_t* counts, uint32_t* sums, uint32_t* starts,
-                          const uint32_t* keys, const uint32_t* place, uint32_t* order, uint32_t keyLimit, int* err,
-                          cudaStream_t s);
+                          const uint32_t* keys, const uint32_t* place, uint32_t* order, uint32_t* crowded,
+                          uint32_t keyLimit, int* err, cudaStream_t s);
 // The stable order from it, with the records gathered (launch_gather_sorted);
 // permCopy (may be NULL) receives the permutation too.
 void launch_cell_gather(int n, const uint32_t* keys, const uint32_t* starts, const uint32_t* order, uint32_t* keysOut,
@@ -236,11 +241,10 @@ void launch_cell_gather(int n, const uint32_t* keys, const uint32_t* starts, con
                         cudaStream_t s);
 // For the entry point that sorts without records (at most PBF_NOALLOC_MAX_KEYS
 // particles): the stable permutation, the sorted keys (in place of the
-// particles' own) and the cell table (may be NULL) from `order` and `starts`.
-// crowded: a word more than there are keys, the first one zero, such as the
-// counts after the scan.
-cudaError_t launch_cell_finish(int n, uint32_t keyCount, const uint32_t* starts, const uint32_t* order, uint32_t* keys,
-                               uint32_t* permOut, uint32_t* cells, uint32_t* crowded, cudaStream_t s);
+// particles' own) and the cell table (may be NULL) from `order`, which it uses up,
+// `starts` and the list of crowded cells.
+void launch_cell_finish(const CountingPlan& plan, int n, uint32_t keyCount, const uint32_t* starts, uint32_t* order,
+                        uint32_t* keys, uint32_t* permOut, uint32_t* cells, const uint32_t* crowded, cudaStream_t s);
 
 // ---- adjoint (pbf_adjoint.cu) ----
 // What one substep of a rollout leaves for its reverse pass.

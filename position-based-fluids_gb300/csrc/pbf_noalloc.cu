@@ -136,19 +136,21 @@ extern "C" int pbf_sort_state_noalloc(const PbfParameters* params, const float* 
 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const pbf::DevConsts c = pbf::make_consts(*params, (int)n);
-    // 1M particles and 2^19 keys: 105 us by radix passes (11 launches, a copy and a clear), 41 by counting
+    // 1M particles and 2^19 keys: 105 us by radix passes (11 launches, a copy and a clear), 40 by counting
     const pbf::CountingPlan counting = pbf::make_counting_plan((int)n, params->gridBufSize);
     const size_t grouped = ((size_t)n + 3) / 4 * 4;  // the counts are read 16 bytes at a time
-    if (counting.blocks > 0 && grouped + 2 * counting.words + counting.blocks <= kScratchWords) {
+    // many particles to every key of a range that two radix passes sort: 2^20 particles and 2^14 keys, sorted before /
+    // in random order, 57 / 77 us by radix passes and 71 / 119 by counting; 2^15 keys 58 / 80 and 49 / 72
+    const bool crowded = n > 65536u && n > 32u * params->gridBufSize;
+    if (counting.blocks > 0 && !crowded && grouped + 2 * counting.words + counting.blocks <= kScratchWords) {
         uint32_t *order = scratch, *counts = order + grouped, *starts = counts + counting.words, *sums = starts + counting.words;
-        e = cudaMemsetAsync(counts, 0, 4 * counting.words, s);
-        if (e == cudaSuccess) {
-            pbf::launch_compute_keys(c, pbf::Batch{nullptr, nullptr}, reinterpret_cast<const float4*>(d_pred), d_keys, d_perm, counts, s);
-            pbf::launch_counting_sort(counting, (int)n, counts, sums, starts, d_keys, d_perm, order, params->gridBufSize, nullptr, s);
-            e = pbf::launch_cell_finish((int)n, params->gridBufSize, starts, order, d_keys, d_perm, d_cells, counts, s);
-            const cudaError_t launched = cudaGetLastError();
-            if (e == cudaSuccess) e = launched;
-        }
+        const float4* pred = reinterpret_cast<const float4*>(d_pred);
+        uint32_t* hot = starts;  // until the scan writes them
+        pbf::launch_clear_counts(c, pred, counts, counting.words, hot, s);
+        pbf::launch_compute_keys(c, pbf::Batch{nullptr, nullptr}, pred, d_keys, d_perm, counts, hot, s);
+        pbf::launch_counting_sort(counting, (int)n, counts, sums, starts, d_keys, d_perm, order, counts, params->gridBufSize, nullptr, s);
+        pbf::launch_cell_finish(counting, (int)n, params->gridBufSize, starts, order, d_keys, d_perm, d_cells, counts, s);
+        e = cudaGetLastError();
         if (e != cudaSuccess) return pbf::fail(nullptr, PBF_ERR_CUDA, std::string("pbf_sort_state_noalloc: ") + cudaGetErrorString(e));
         return PBF_OK;
     }
@@ -159,7 +161,7 @@ extern "C" int pbf_sort_state_noalloc(const PbfParameters* params, const float* 
     uint32_t* perm[2] = {d_perm, scratch + kMaxKeys};
     uint32_t* hist = scratch + 2 * kMaxKeys;
 
-    pbf::launch_compute_keys(c, pbf::Batch{nullptr, nullptr}, reinterpret_cast<const float4*>(d_pred), keys[0], perm[0], nullptr, s);
+    pbf::launch_compute_keys(c, pbf::Batch{nullptr, nullptr}, reinterpret_cast<const float4*>(d_pred), keys[0], perm[0], nullptr, nullptr, s);
     const int r = pbf::launch_radix_sort(plan, keys, perm, hist, nullptr, nullptr, nullptr, nullptr, s);
     if (r == 1) {  // an odd number of passes left the result in the scratch half
         if ((e = cudaMemcpyAsync(d_keys, keys[1], 4 * (size_t)n, cudaMemcpyDeviceToDevice, s)) == cudaSuccess)

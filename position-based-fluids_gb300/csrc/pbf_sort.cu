@@ -240,15 +240,24 @@ counting_scan_kernel(uint4* counts, uint32_t chunks, uint32_t chunksPerBlock,
     }
 }
 
-// order[first index of the key + place of arrival] = particle
+// order[first index of the key + place of arrival] = particle.  crowded (may be
+// NULL; words of it, the first two zero): the keys of the cells that
+// launch_cell_finish does not order by comparing, by the first particle to arrive
+// in each: [0] and [1] count those of up to kBlockCell particles, listed from [2]
+// on, and the larger ones, listed from the end on downwards.
+constexpr uint32_t kComparedCell = 128, kWarpCell = 512, kBlockCell = 4096;
 __global__ void __launch_bounds__(kThreads)
 cell_scatter_kernel(int n, const uint32_t* keys, const uint32_t* place,
-                    const uint32_t* starts, uint32_t* order, uint32_t keyLimit, int* err) {
+                    const uint32_t* starts, uint32_t* order, uint32_t* crowded, uint32_t words, uint32_t keyLimit, int* err) {
     chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const uint32_t first = starts[checked_index(keys[i], keyLimit, err, kErrCellKey)];
-    order[checked_index(first + place[i], (uint32_t)n, err, kErrSortIndex)] = (uint32_t)i;
+    const uint32_t key = checked_index(keys[i], keyLimit, err, kErrCellKey), first = starts[key], at = place[i];
+    order[checked_index(first + at, (uint32_t)n, err, kErrSortIndex)] = (uint32_t)i;
+    if (!crowded || at != 0u) return;
+    const uint32_t holds = starts[key + 1] - first;
+    if (holds > kBlockCell) crowded[words - 1u - atomicAdd(crowded + 1, 1u)] = key;
+    else if (holds > kComparedCell) crowded[2u + atomicAdd(crowded, 1u)] = key;
 }
 
 // The particle in slot s of the scattered order goes to its cell's first index
@@ -280,38 +289,253 @@ cell_gather_kernel(int n, const uint32_t* keys, const uint32_t* starts,
     idsOut[to] = id;
 }
 
-// The stable order without the records: permOut from the scattered order.  The
-// comparisons are as many as the cell holds, for each particle; cells of more
-// than kCrowdedCell go to the list `crowded` (its length first, zero before the
-// launch).
-constexpr uint32_t kCrowdedCell = 1024;
+// ---- the stable order without the records ----
+//
+// cell_scatter leaves a cell's particles in any order.  Up to kComparedCell of them
+// are ranked by comparing, up to kWarpCell are sorted by a warp, up to kBlockCell by
+// a block, and the particles of larger cells, at most kMostBig of them, are counted
+// and placed tile by tile of the particles' own order, as a radix pass does with
+// its digits.  A call with 2^20 particles in 2^17 keys, sorted before / in random
+// order, us: 128 to a cell 53 / 80, 512 45 / 73, 2,100 42 / 67, 4,096 45 / 90,
+// 16,384 37 / 71, all in one 34; by radix passes 81-85 / 85-106 whatever they hold;
+// comparing with every other one takes 104 / 145 at 512 and 181 / 284 at 1,024.
+
+constexpr uint32_t kMostBig = PBF_NOALLOC_MAX_KEYS / (kBlockCell + 1);
+constexpr int kTileRounds = 16, kTileKeys = kThreads * kTileRounds;
+constexpr uint32_t kMostTiles = PBF_NOALLOC_MAX_KEYS / kTileKeys;
+constexpr uint32_t kBigSlots = 512;  // of the table, a power of two above kMostBig
+static_assert(kMostBig < kBigSlots / 2 + 1 && kMostTiles <= kBlockCell, "bins and tiles of the large cells");
+
+// The large cells' numbers by key, and their first indices by number, for a block.
+struct BigCells {
+    uint32_t key[kBigSlots], bin[kBigSlots], first[kMostBig];
+    __device__ __forceinline__ static uint32_t slot(uint32_t k) { return (k * 2654435761u) >> 23; }
+    // All threads; they are in step afterwards.
+    __device__ __forceinline__ void fill(const uint32_t* crowded, uint32_t words, uint32_t big, const uint32_t* starts) {
+        for (uint32_t q = threadIdx.x; q < kBigSlots; q += kThreads) key[q] = kEmpty;
+        __syncthreads();
+        for (uint32_t b = threadIdx.x; b < big; b += kThreads) {
+            const uint32_t k = crowded[words - 1u - b];
+            uint32_t q = slot(k);
+            while (atomicCAS(&key[q], kEmpty, k) != kEmpty) q = (q + 1u) % kBigSlots;
+            bin[q] = b;
+            first[b] = starts[k];
+        }
+        __syncthreads();
+    }
+    // kEmpty: not a large cell's key.
+    __device__ __forceinline__ uint32_t find(uint32_t k) const {
+        for (uint32_t q = slot(k);; q = (q + 1u) % kBigSlots) {
+            const uint32_t at = key[q];
+            if (at == k) return bin[q];
+            if (at == kEmpty) return kEmpty;
+        }
+    }
+};
+
+// permOut of the cells that are ranked by comparing.  The first `tiles` blocks also
+// count the particles that each tile has of each large cell, into the cell's slots
+// of permOut, one per tile.
 __global__ void __launch_bounds__(kThreads)
-cell_rank_kernel(int n, uint32_t keyLimit, const uint32_t* keys, const uint32_t* starts,
-                 const uint32_t* order, uint32_t* permOut, uint32_t* crowded) {
+cell_rank_kernel(int n, uint32_t keyLimit, const uint32_t* keys, const uint32_t* starts, const uint32_t* order,
+                 uint32_t* permOut, const uint32_t* crowded, uint32_t words, uint32_t tiles) {
     chain_wait();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= (uint32_t)n) return;
-    const uint32_t i = checked_index(order[s], (uint32_t)n, nullptr, kErrSortIndex);
-    const uint32_t key = checked_index(keys[i], keyLimit, nullptr, kErrCellKey);
-    const uint32_t first = starts[key], end = checked_index(starts[key + 1], (uint32_t)n + 1u, nullptr, kErrSortIndex);
-    if (end - first > kCrowdedCell) {
-        if (s == first) crowded[1u + atomicAdd(crowded, 1u)] = key;
-        return;
+    if (s < (uint32_t)n) {
+        const uint32_t i = checked_index(order[s], (uint32_t)n, nullptr, kErrSortIndex);
+        const uint32_t key = checked_index(keys[i], keyLimit, nullptr, kErrCellKey);
+        const uint32_t first = starts[key], end = checked_index(starts[key + 1], (uint32_t)n + 1u, nullptr, kErrSortIndex);
+        if (end - first <= kComparedCell) {
+            uint32_t to = first;
+            for (uint32_t q = first; q < end; ++q) to += order[q] < i;
+            permOut[to] = i;
+        }
     }
-    uint32_t to = first;
-    for (uint32_t q = first; q < end; ++q) to += order[q] < i;
-    permOut[to] = i;
+    if (blockIdx.x >= tiles) return;
+    const uint32_t big = crowded[1];
+    if (big == 0u) return;
+    __shared__ BigCells cells;
+    __shared__ uint32_t counts[kMostBig];
+    for (uint32_t b = threadIdx.x; b < big; b += kThreads) counts[b] = 0u;
+    cells.fill(crowded, words, big, starts);
+    uint32_t key[kTileRounds];
+#pragma unroll
+    for (int r = 0; r < kTileRounds; ++r) {
+        const uint32_t i = blockIdx.x * kTileKeys + r * kThreads + threadIdx.x;
+        key[r] = i < (uint32_t)n ? keys[i] : kEmpty;
+    }
+#pragma unroll
+    for (int r = 0; r < kTileRounds; ++r) {
+        const uint32_t bin = key[r] != kEmpty ? cells.find(key[r]) : kEmpty;
+        const unsigned peers = __match_any_sync(0xFFFFFFFFu, bin);
+        if (bin != kEmpty && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&counts[bin], (uint32_t)__popc(peers));
+    }
+    __syncthreads();
+    for (uint32_t b = threadIdx.x; b < big; b += kThreads) permOut[cells.first[b] + blockIdx.x] = counts[b];
+}
+
+// Sorts the particles of one cell of more than kComparedCell and at most 16 G, G
+// threads (a warp or the block): a counting sort by the upper bits of their indices,
+// about as many buckets as particles, and the few of a bucket are put in order by
+// comparing them.
+template <uint32_t G>
+struct SharedCell {
+    static constexpr uint32_t kMost = 16 * G;
+    uint32_t index[kMost], buckets[kMost];
+    uint32_t warpSums[G / 32], least, largest;
+};
+static_assert(kWarpCell == SharedCell<32>::kMost && kBlockCell == SharedCell<kThreads>::kMost, "what a warp and a block sort");
+template <uint32_t G>
+__device__ __forceinline__ void sort_cell(SharedCell<G>& sh, uint32_t first, uint32_t count, const uint32_t* order, uint32_t* permOut) {
+    const uint32_t t = threadIdx.x % G, lane = t & 31, warp = t >> 5;
+    auto sync = [] {
+        if constexpr (G == 32) __syncwarp();
+        else __syncthreads();
+    };
+    int log = 0;  // 2^log buckets to a thread, bucket b at [b % 2^log][b / 2^log]
+    while (G << log < count) ++log;
+    const uint32_t each = 1u << log;
+    if (t == 0) {
+        sh.least = 0xFFFFFFFFu;
+        sh.largest = 0u;
+    }
+    for (uint32_t r = 0; r < each; ++r) sh.buckets[r * G + t] = 0u;
+    sync();
+    uint32_t low = 0xFFFFFFFFu, high = 0u;
+#pragma unroll 4
+    for (uint32_t q = t; q < count; q += G) {
+        const uint32_t i = order[first + q];
+        low = min(low, i);
+        high = max(high, i);
+    }
+    low = __reduce_min_sync(0xFFFFFFFFu, low);
+    high = __reduce_max_sync(0xFFFFFFFFu, high);
+    if (lane == 0) {
+        atomicMin(&sh.least, low);
+        atomicMax(&sh.largest, high);
+    }
+    sync();
+    const uint32_t begin = sh.least, span = sh.largest - begin;
+    int shift = 0;  // 2^shift indices to a bucket
+    while (span >> shift >> log >= G) ++shift;
+    auto place = [&](uint32_t b) -> uint32_t& { return sh.buckets[(b & (each - 1u)) * G + (b >> log)]; };
+#pragma unroll 4
+    for (uint32_t q = t; q < count; q += G) atomicAdd(&place((order[first + q] - begin) >> shift), 1u);
+    sync();
+    uint32_t mine = 0;
+    for (uint32_t r = 0; r < each; ++r) mine += sh.buckets[r * G + t];
+    uint32_t incl = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+        if (lane >= (uint32_t)d) incl += u;
+    }
+    uint32_t run = incl - mine;
+    if constexpr (G > 32) {
+        if (lane == 31) sh.warpSums[warp] = incl;
+        sync();
+        for (uint32_t w = 0; w < warp; ++w) run += sh.warpSums[w];
+    }
+    for (uint32_t r = 0; r < each; ++r) {
+        const uint32_t c = sh.buckets[r * G + t];
+        sh.buckets[r * G + t] = run;
+        run += c;
+    }
+    sync();
+#pragma unroll 4
+    for (uint32_t q = t; q < count; q += G) {
+        const uint32_t i = order[first + q];
+        sh.index[atomicAdd(&place((i - begin) >> shift), 1u)] = i;
+    }
+    sync();
+    for (uint32_t q = t; q < count; q += G) {  // a bucket's place is its end now
+        const uint32_t i = sh.index[q], b = (i - begin) >> shift, from = b ? place(b - 1u) : 0u, end = place(b);
+        uint32_t to = from;
+        for (uint32_t k = from; k < end; ++k) to += sh.index[k] < i;
+        permOut[first + to] = i;
+    }
+    sync();  // all is read before the next cell writes it
+}
+
+// The cells that a block sorts go to permOut, a block taking one after another; of
+// the larger ones, block b places the particles of tile b into the cells' slots of
+// `order`, behind those of the tiles before it.
+struct BigTile {
+    BigCells cells;
+    uint32_t warpCount[kWarps][kMostBig], base[kMostBig];
+};
+__global__ void __launch_bounds__(kThreads)
+crowded_cells_kernel(int n, const uint32_t* keys, const uint32_t* starts, uint32_t* order, uint32_t* permOut,
+                     const uint32_t* crowded, uint32_t words, uint32_t tiles) {
+    chain_wait();
+    __shared__ union {
+        SharedCell<32> warpCell[kWarps];
+        SharedCell<kThreads> cell;
+        BigTile tile;
+    } sh;
+    const uint32_t count = crowded[0], big = crowded[1], t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    for (uint32_t c = blockIdx.x * kWarps + warp; c < count; c += gridDim.x * kWarps) {
+        const uint32_t key = crowded[2u + c], first = starts[key], holds = starts[key + 1] - first;
+        if (holds <= kWarpCell) sort_cell<32>(sh.warpCell[warp], first, holds, order, permOut);
+    }
+    __syncthreads();
+    for (uint32_t c = blockIdx.x; c < count; c += gridDim.x) {
+        const uint32_t key = crowded[2u + c], first = starts[key], holds = starts[key + 1] - first;
+        if (holds > kWarpCell && holds <= kBlockCell) sort_cell<kThreads>(sh.cell, first, holds, order, permOut);
+    }
+    if (big == 0u || blockIdx.x >= tiles) return;
+    BigTile& tile = sh.tile;
+    tile.cells.fill(crowded, words, big, starts);
+    for (uint32_t b = warp; b < big; b += kWarps) {
+        const uint32_t first = tile.cells.first[b];
+        uint32_t before = 0;
+#pragma unroll
+        for (uint32_t q = lane; q < kMostTiles; q += 32) before += q < blockIdx.x ? permOut[first + q] : 0u;
+        before = __reduce_add_sync(0xFFFFFFFFu, before);
+        if (lane == 0) tile.base[b] = first + before;
+        for (uint32_t w = lane; w < kWarps; w += 32) tile.warpCount[w][b] = 0u;
+    }
+    __syncthreads();
+    const uint32_t from = blockIdx.x * kTileKeys + warp * (32 * kTileRounds) + lane;  // a warp's particles are consecutive
+    uint32_t bins[kTileRounds], rank[kTileRounds];
+#pragma unroll
+    for (int r = 0; r < kTileRounds; ++r) bins[r] = from + 32 * r < (uint32_t)n ? keys[from + 32 * r] : kEmpty;
+#pragma unroll
+    for (int r = 0; r < kTileRounds; ++r) {
+        const uint32_t bin = bins[r] != kEmpty ? tile.cells.find(bins[r]) : kEmpty;
+        const unsigned peers = __match_any_sync(0xFFFFFFFFu, bin);
+        const uint32_t prior = bin != kEmpty ? tile.warpCount[warp][bin] : 0u;
+        __syncwarp();
+        if (bin != kEmpty && lane == (uint32_t)__ffs(peers) - 1u) tile.warpCount[warp][bin] = prior + (uint32_t)__popc(peers);
+        __syncwarp();
+        bins[r] = bin;
+        rank[r] = prior + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+    }
+    __syncthreads();
+    for (uint32_t b = t; b < big; b += kThreads) {
+        uint32_t run = tile.base[b];
+        for (int w = 0; w < kWarps; ++w) {
+            const uint32_t c = tile.warpCount[w][b];
+            tile.warpCount[w][b] = run;
+            run += c;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kTileRounds; ++r)
+        if (bins[r] != kEmpty)
+            order[checked_index(tile.warpCount[warp][bins[r]] + rank[r], (uint32_t)n, nullptr, kErrSortIndex)] = from + 32 * r;
 }
 
 // The sorted keys and the cell table (first and last particle of a key, both
 // all ones for none) from the first indices; the table may be NULL.  The last
 // particle of the only one of n = 1 is not written (update_cells.cl:11-25).
-// A warp writes the keys of the cells of more than 16 particles, one thread 512
-// of them one after another took 100 us; those of crowded cells are left to
-// crowded_cells_kernel.
+// A warp writes the keys of the cells of more than 16 particles (one thread 512 of
+// them one after another took 100 us), a block those of the cells of more than
+// kComparedCell, and all blocks those of the large ones, with their order.
 __global__ void __launch_bounds__(kThreads)
-cell_table_kernel(int n, uint32_t keys, const uint32_t* starts, uint32_t* keysOut,
-                  uint32_t* cells) {
+cell_table_kernel(int n, uint32_t keys, const uint32_t* starts, const uint32_t* order, uint32_t* keysOut, uint32_t* permOut,
+                  uint32_t* cells, const uint32_t* crowded, uint32_t words) {
     chain_wait();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
@@ -327,122 +551,41 @@ cell_table_kernel(int n, uint32_t keys, const uint32_t* starts, uint32_t* keysOu
     const bool many = end - first > 16u;
     if (!many)
         for (uint32_t q = first; q < end; ++q) keysOut[q] = k;
-    for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, many && end - first <= kCrowdedCell); todo; todo &= todo - 1u) {
+    for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, many && end - first <= kComparedCell); todo; todo &= todo - 1u) {
         const int src = __ffs(todo) - 1;
         const uint32_t f = __shfl_sync(0xFFFFFFFFu, first, src), e = __shfl_sync(0xFFFFFFFFu, end, src);
         for (uint32_t q = f + lane; q < e; q += 32) keysOut[q] = k - lane + src;
     }
-}
-
-// The crowded cells, each by one block, or by up to kMostParts that take an
-// equal part of the span of the cell's indices: the indices in the part are
-// marked in a bitmap and read out in order, behind those below the part.  So a
-// cell costs its particles and its span, however many it holds (2^20 particles,
-// 16,384 to a cell: 0.12 ms, all in one: 0.24; a comparison with each would take
-// 0.13 us for every particle that a cell holds).  Word w of the map is at
-// [w % each][w / each], a thread's words in a column.
-constexpr int kCrowdedThreads = 1024, kCrowdedBlocks = 152;
-constexpr uint32_t kMostParts = 16, kPartCell = 16384;
-constexpr int kMostShift = 5;  // 2^5 words to a thread
-static_assert(PBF_NOALLOC_MAX_KEYS == (kCrowdedThreads * 32) << kMostShift, "the bitmap holds every index");
-__global__ void __launch_bounds__(kCrowdedThreads)
-crowded_cells_kernel(const uint32_t* crowded, const uint32_t* starts,
-                     const uint32_t* order, uint32_t* keysOut, uint32_t* permOut) {
-    chain_wait();
-    extern __shared__ uint32_t marks[];  // kCrowdedThreads words for every word to a thread
-    __shared__ uint32_t warpSums[kCrowdedThreads / 32], below, least, largest;
-    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const uint32_t count = crowded[0];
-    for (uint32_t c = 0; c < count; ++c) {
-        const uint32_t part = (blockIdx.x + kCrowdedBlocks - c * 17u % kCrowdedBlocks) % kCrowdedBlocks;
-        if (part >= kMostParts) continue;
-        const uint32_t key = crowded[1u + c], first = starts[key], end = starts[key + 1];
-        int parts = 0;  // 2^parts of them
-        while ((1u << parts) < kMostParts && (end - first) >> parts > kPartCell) ++parts;
-        if (part >= 1u << parts) continue;
-        if (t == 0) {
-            below = largest = 0u;
-            least = 0xFFFFFFFFu;
+    if ((uint32_t)n <= kComparedCell) return;
+    const uint32_t count = crowded[0], big = crowded[1];
+    for (uint32_t b = blockIdx.x; b < count; b += gridDim.x) {
+        const uint32_t key = crowded[2u + b], e = min(starts[key + 1], (uint32_t)n);
+        for (uint32_t q = starts[key] + threadIdx.x; q < e; q += kThreads) keysOut[q] = key;
+    }
+    if (big == 0u) return;
+    const uint32_t parts = max(gridDim.x / big, 1u), part = blockIdx.x % parts;  // blocks to a cell
+    for (uint32_t b = blockIdx.x / parts; b < big; b += gridDim.x) {
+        const uint32_t key = crowded[words - 1u - b], e = min(starts[key + 1], (uint32_t)n);
+        for (uint32_t q = starts[key] + part * kThreads + threadIdx.x; q < e; q += parts * kThreads) {
+            keysOut[q] = key;
+            permOut[q] = order[q];
         }
-        __syncthreads();
-        uint32_t low = 0xFFFFFFFFu, high = 0u;
-#pragma unroll 4
-        for (uint32_t s = first + t; s < end; s += kCrowdedThreads) {
-            low = min(low, order[s]);
-            high = max(high, order[s]);
-            if (part == 0) keysOut[s] = key;
-        }
-        low = __reduce_min_sync(0xFFFFFFFFu, low);
-        high = __reduce_max_sync(0xFFFFFFFFu, high);
-        if (lane == 0) {
-            atomicMin(&least, low);
-            atomicMax(&largest, high);
-        }
-        __syncthreads();
-        const uint32_t begin = least & ~31u, span = largest - begin;  // the bitmap's first index, its last one's place
-        int shift = 0;  // 2^shift words to a thread of all parts
-        while (shift < kMostShift && span >> shift >= kCrowdedThreads * 32u) ++shift;
-        const int down = max(shift - parts, 0);  // 2^down words to a thread of this part
-        const uint32_t each = 1u << down, lo = begin + part * ((uint32_t)kCrowdedThreads << down) * 32u;
-        if (lo <= largest) {
-            for (uint32_t r = 0; r < each; ++r) marks[r * kCrowdedThreads + t] = 0u;
-            __syncthreads();
-            uint32_t less = 0;
-#pragma unroll 4
-            for (uint32_t s = first + t; s < end; s += kCrowdedThreads) {
-                const uint32_t i = order[s], w = (i - lo) >> 5;
-                less += i < lo;
-                if (i >= lo && w >> down < kCrowdedThreads)
-                    atomicOr(&marks[(w & (each - 1u)) * kCrowdedThreads + (w >> down)], 1u << (i & 31u));
-            }
-            less = __reduce_add_sync(0xFFFFFFFFu, less);
-            if (lane == 0 && less) atomicAdd(&below, less);
-            __syncthreads();
-            uint32_t mine = 0;
-            for (uint32_t r = 0; r < each; ++r) mine += __popc(marks[r * kCrowdedThreads + t]);
-            uint32_t incl = mine;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-                if (lane >= (uint32_t)d) incl += u;
-            }
-            if (lane == 31) warpSums[warp] = incl;
-            __syncthreads();
-            uint32_t to = first + below + incl - mine;
-            for (uint32_t w = 0; w < warp; ++w) to += warpSums[w];
-            for (uint32_t r = 0; r < each; ++r)
-                for (uint32_t m = marks[r * kCrowdedThreads + t]; m; m &= m - 1u)
-                    permOut[to++] = lo + 32u * ((t << down) + r) + (uint32_t)__ffs(m) - 1u;
-        }
-        __syncthreads();  // all is read before the next cell writes it
     }
 }
 
 }  // namespace
 
-cudaError_t launch_cell_finish(int n, uint32_t keyCount, const uint32_t* starts, const uint32_t* order, uint32_t* keys,
-                               uint32_t* permOut, uint32_t* cells, uint32_t* crowded, cudaStream_t s) {
-    launch_chained(cell_rank_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keyCount, keys, starts, order, permOut, crowded);
-    launch_chained(cell_table_kernel, (keyCount + kThreads - 1) / kThreads, kThreads, s, n, keyCount, starts, keys, cells);
-    if ((uint32_t)n <= kCrowdedCell) return cudaGetLastError();
-    int shift = 0;
-    while (shift < kMostShift && ((uint64_t)kCrowdedThreads * 32 << shift) < (uint64_t)n) ++shift;
-    constexpr size_t kRow = kCrowdedThreads * sizeof(uint32_t);
-    // always the same limit: callers on other threads launch the kernel too
-    const cudaError_t e = cudaFuncSetAttribute(crowded_cells_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)(kRow << kMostShift));
-    if (e != cudaSuccess) return e;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(kCrowdedBlocks);
-    cfg.blockDim = dim3(kCrowdedThreads);
-    cfg.dynamicSmemBytes = kRow << shift;
-    cfg.stream = s;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, crowded_cells_kernel, static_cast<const uint32_t*>(crowded), starts, order, keys, permOut);
+void launch_cell_finish(const CountingPlan& plan, int n, uint32_t keyCount, const uint32_t* starts, uint32_t* order,
+                        uint32_t* keys, uint32_t* permOut, uint32_t* cells, const uint32_t* crowded, cudaStream_t s) {
+    const uint32_t words = (uint32_t)plan.words, tiles = (uint32_t)n > kBlockCell ? ((uint32_t)n + kTileKeys - 1) / kTileKeys : 0u;
+    launch_chained(cell_rank_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keyCount, keys, starts, order, permOut,
+                   crowded, words, tiles);
+    if ((uint32_t)n > kComparedCell) {
+        const uint32_t most = min((uint32_t)n / kComparedCell, 912u);  // 6 blocks to an SM
+        launch_chained(crowded_cells_kernel, max(most, tiles), kThreads, s, n, keys, starts, order, permOut, crowded, words, tiles);
+    }
+    launch_chained(cell_table_kernel, (keyCount + kThreads - 1) / kThreads, kThreads, s, n, keyCount, starts, order, keys,
+                   permOut, cells, crowded, words);
 }
 
 CountingPlan make_counting_plan(int n, uint64_t keys) {
@@ -453,7 +596,7 @@ CountingPlan make_counting_plan(int n, uint64_t keys) {
 
 CountingPlan make_scan_plan(uint64_t keys) {
     CountingPlan p;
-    p.chunks = (uint32_t)((keys + 1 + kScanChunk - 1) / kScanChunk);  // one start beyond the last key
+    p.chunks = (uint32_t)((keys + 2 + kScanChunk - 1) / kScanChunk);  // one start beyond the last key; two counts (cell_scatter)
     // a key range of a few chunks is scanned by one block, which needs no sums of others before it
     p.chunksPerBlock = p.chunks <= kOneBlockChunks ? p.chunks : (p.chunks + kMaxScanBlocks - 1) / kMaxScanBlocks;
     p.blocks = (p.chunks + p.chunksPerBlock - 1) / p.chunksPerBlock;
@@ -471,10 +614,11 @@ void launch_counting_scan(const CountingPlan& plan, uint32_t* counts, uint32_t* 
 }
 
 void launch_counting_sort(const CountingPlan& plan, int n, uint32_t* counts, uint32_t* sums, uint32_t* starts,
-                          const uint32_t* keys, const uint32_t* place, uint32_t* order, uint32_t keyLimit, int* err,
-                          cudaStream_t s) {
+                          const uint32_t* keys, const uint32_t* place, uint32_t* order, uint32_t* crowded,
+                          uint32_t keyLimit, int* err, cudaStream_t s) {
     launch_counting_scan(plan, counts, sums, starts, s);
-    launch_chained(cell_scatter_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keys, place, starts, order, keyLimit, err);
+    launch_chained(cell_scatter_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keys, place, starts, order, crowded,
+                   (uint32_t)plan.words, keyLimit, err);
 }
 
 void launch_cell_gather(int n, const uint32_t* keys, const uint32_t* starts, const uint32_t* order, uint32_t* keysOut,

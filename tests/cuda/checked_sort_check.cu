@@ -29,7 +29,7 @@ extern "C" int checked_sort(int n, uint32_t limit, const uint32_t* keys, const u
     cudaMemset(v, 0, 64 * (size_t)n);
     cudaMemset(ids, 0, 8 * (size_t)n);
     cudaMemset(err, 0, 4);
-    pbf::launch_counting_sort(plan, n, d[2], d[3], d[4], d[0], d[1], d[5], limit, err, nullptr);
+    pbf::launch_counting_sort(plan, n, d[2], d[3], d[4], d[0], d[1], d[5], nullptr, limit, err, nullptr);
     cudaMemcpy(errors, err, 4, cudaMemcpyDeviceToHost);
     cudaMemset(err, 0, 4);
     pbf::launch_cell_gather(n, d[0], d[4], d[5], d[6], d[7], nullptr, v, v + n, ids, v + 2 * n, v + 3 * n, ids + n, limit,
