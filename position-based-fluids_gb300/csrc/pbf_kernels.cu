@@ -474,12 +474,16 @@ __device__ __forceinline__ float max_nan(float a, float b) {
 // Runs with
 // coordinates that are not finite take the scan.  A run with up to half as many
 // candidates again as fit is split across the longest side of its box, and the
-// candidates of others pass through in chunks (friends_in_chunks).  262,144
+// candidates of others pass through in chunks (friends_in_chunks): at once where the
+// cells hold twice as many as fit, of which a run keeps about three of four.  262,144
 // particles in two colliding columns, where 560 candidates are common: a frame
-// takes 0.76 ms with that line, 0.84 with chunks alone; 400,000 particles with 30 /
-// 50 / 80 to a cell take 1.8 / 2.1 / 2.7 ms and 1.4 / 2.0 / 2.7 (without chunks 1.9 /
-// 3.6 / 7.1, by one thread each 1.7 / 2.5 / 3.3), 65,536 in 16 clusters of 4,096
-// take 1.7 (4.6 and 2.7).
+// takes 0.76 ms with that line, 0.84 with chunks alone.  A substep of 400,000
+// particles with 30 / 50 / 80 to a cell takes 1.56 / 2.11 / 2.73 ms (1.74 / 2.19 /
+// 2.76 when the chunks wait for the first walk's count; without chunks 1.9 / 3.6 /
+// 7.1; two scans by one thread each, with the passes of then, 1.69 / 2.51 / 3.33).
+// In chunks of more than 8 times as many candidates, circles at their limit take no
+// part: 65,536 particles in 16 clusters of 4,096 take 1.1 ms (1.8), 32,768 in one
+// cell 2.9 (5.2; the scans 4.7).
 // 384 candidates leave room for 7 blocks per SM: 320 is 2 % faster on the scene
 // above and 10 % slower where 560 are common, 448 is 5 % slower on the former.
 constexpr int kFriendWarps = 4, kCandidates = 384, kMostFriends = 128;
@@ -616,11 +620,18 @@ __device__ __noinline__ uint64_t friends_in_chunks(const DevConsts& c, FriendSha
                      pz = both(__shfl_sync(kFull, pi.z, pl));
             uint32_t lo = __shfl_sync(kFull, (uint32_t)counts, pl), hi = __shfl_sync(kFull, (uint32_t)(counts >> 32), pl);
             int cnt = 0;
+            uint32_t full = 0;  // of many chunks most candidates belong to circles that take no more
+            if (total > 8u * (uint32_t)kCandidates)
+                for (int k = 0; k < 8; ++k) full |= (__byte_perm(lo, hi, k) & 0xFFu) == (uint32_t)c.perCircle ? 1u << k : 0u;
             for (uint32_t k = 0; k < kept; k += 64) {
                 const uint32_t e = k + 2u * (uint32_t)lane;
                 const F2 rx = sub2(px, load2(sh.x + e)), ry = sub2(py, load2(sh.y + e)), rz = sub2(pz, load2(sh.z + e));
                 const float2 r2 = unpack2(dot2(c, rx, ry, rz, rx, ry, rz));
-                const bool a0 = !(r2.x >= c.h2), a1 = !(r2.y >= c.h2);
+                bool a0 = !(r2.x >= c.h2), a1 = !(r2.y >= c.h2);
+                if (full) {
+                    a0 = a0 && !((full >> circle_of(c, r2.x)) & 1u);
+                    a1 = a1 && !((full >> circle_of(c, r2.y)) & 1u);
+                }
                 const uint32_t m0 = __ballot_sync(kFull, a0), m1 = __ballot_sync(kFull, a1);
                 const int pos = cnt + __popc(m0 & ltMask) + __popc(m1 & ltMask);
                 if (a0) sh.list[pos] = make_uint2(e, __float_as_uint(r2.x));
@@ -728,6 +739,11 @@ build_friends_kernel(const __grid_constant__ DevConsts c, Batch b, const float4*
         end = lane < __popc(occupied) ? cell.x : 0xFFFFFFFFu;
         const uint32_t shift = cell.y;
         __syncwarp();
+        if (total > 2u * (uint32_t)kCandidates) {  // a run of this many keeps about three of four: too many to split
+            counts = friends_in_chunks(c, sh, pred, rows, total, end, shift, lx, ly, lz, hx, hy, hz, runMask, pi, warpBase, counts);
+            spread |= runMask;
+            continue;
+        }
         uint32_t kept = 0;
         int firstCell = 0;  // of candidate t0
         for (uint32_t t0 = 0; t0 < total; t0 += 32) {

@@ -15,7 +15,7 @@ def _bits(a):
     return a.view(np.uint32)
 
 
-@pytest.mark.parametrize("counts", [[256, 257], [1000], [31, 700, 288, 1, 33, 320], [5, 2500]])
+@pytest.mark.parametrize("counts", [[256, 257], [1000], [31, 700, 288, 1, 33, 320], [5, 2500], [3300]])
 @pytest.mark.parametrize("sort", [True, False])
 def test_crowded_cells_of_a_substep(pbf_mod, oracle_mod, cuda_device, counts, sort):
     params = pbf_mod.load_scenario("dam_break_32k")
