@@ -420,7 +420,8 @@ int pbf_render_read(pbf_ctx* ctx, int which, float* rgba);
    viscosity, vorticity (multiples of 32 in [32, 512]), then the friends
    algorithm (0, and 2 as well: warps test the candidates of each run of
    same-cell particles together, in blocks of 128 threads whatever the friends
-   block size; 1: one thread scans the 27 cells per particle), then the balance
+   block size, and sparse scenes of 600,000 particles or more are scanned as
+   with 1; 1: one thread scans the 27 cells per particle), then the balance
    flag (1: the four solver passes hand each block's particles to its threads
    in decreasing order of friend count, so warps walk lists of similar
    length), then the persistent flag (1: the four solver passes launch at

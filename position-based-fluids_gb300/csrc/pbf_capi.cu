@@ -515,7 +515,7 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
         mark("sortParticles");
         if (counting) {
             ctx->keysIdx = 1;
-            pbf::launch_cell_gather(c.n, ctx->keys[0], ctx->cellStart, order, ctx->keys[1], ctx->perm[1],
+            pbf::launch_cell_gather(c, ctx->keys[0], ctx->cellStart, order, ctx->keys[1], ctx->perm[1],
                                     tape ? tape->perm : nullptr, ctx->pos[P],
                                     ctx->pred[0], ctx->ids, ctx->pos[P ^ 1], ctx->pred[1], ctx->idsTmp, tableKeys,
                                     ctx->errWord, s);
@@ -542,9 +542,8 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
         ++launched;
     }
     mark("buildFriendsList");
-    pbf::launch_build_friends(c, b, ctx->pred[sortedPred], ctx->cells, counting ? ctx->cellStart : nullptr, rows, meta,
-                              ctx->errWord, ls.friends, ls.friendsAlgorithm, s);
-    ++launched;
+    launched += pbf::launch_build_friends(c, b, ctx->pred[sortedPred], ctx->cells, counting ? ctx->cellStart : nullptr, rows,
+                                          meta, ctx->errWord, ls.friends, ls.friendsAlgorithm, s);
     mark("resetPartList");
     if (!counting) {
         pbf::launch_reset_cells(c.n, keys, ctx->cells, tableKeys, ctx->errWord, s);
@@ -857,9 +856,9 @@ int pbf_create(const PbfParameters* params, int device, pbf_ctx** out) {
     ctx->device = device;
     PBF_CUDA(nullptr, cudaSetDevice(device));
     PBF_CUDA(nullptr, cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
-    // [0]: the error word; [1]: the substep counter of the taint marks (pbf::DevConsts::epoch)
-    PBF_CUDA(nullptr, cudaMalloc((void**)&ctx->errWord, 2 * sizeof(int)));
-    PBF_CUDA(nullptr, cudaMemset(ctx->errWord, 0, 2 * sizeof(int)));
+    // [0]: the error word; [1]: the substep counter of the taint marks; [2]: sampled cells (pbf::DevConsts::epoch)
+    PBF_CUDA(nullptr, cudaMalloc((void**)&ctx->errWord, 3 * sizeof(int)));
+    PBF_CUDA(nullptr, cudaMemset(ctx->errWord, 0, 3 * sizeof(int)));
     PBF_CUDA(nullptr, cudaMallocHost((void**)&ctx->errHost, sizeof(int)));
     PBF_CUDA(nullptr, cudaMalloc((void**)&ctx->tileCounters, 10 * sizeof(int)));
     PBF_CUDA(nullptr, cudaMemset(ctx->tileCounters, 0, 10 * sizeof(int)));
@@ -998,7 +997,7 @@ int pbf_init_cells(pbf_ctx* ctx) {
     PBF_CUDA(ctx, cudaMemset(ctx->meta, 0, 8 * (size_t)ctx->n));
     // taint marks are substep numbers from 1 on (the counter restarts with them); no cell start yet
     PBF_CUDA(ctx, cudaMemset(ctx->taint, 0, 4 * (size_t)ctx->n));
-    PBF_CUDA(ctx, cudaMemset(ctx->errWord + 1, 0, sizeof(int)));
+    PBF_CUDA(ctx, cudaMemset(ctx->errWord + 1, 0, 2 * sizeof(int)));
     PBF_CUDA(ctx, cudaMemset(ctx->cellStart, 0xFF, 4 * tableWords));
     apply_planes(ctx);
     ctx->cellsReady = true;

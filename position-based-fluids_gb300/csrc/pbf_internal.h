@@ -52,7 +52,8 @@ struct DevConsts {
     int quotients;               // divisions by |r| in the four neighbour passes
     int quotientPoly6q;          // the s_corr division by poly6q in the position pass
     float recipPoly6q;           // RN(1 / poly6q)
-    uint32_t* epoch;             // device word: the substep's number, counted by the predict kernel
+    uint32_t* epoch;             // device words: the substep's number, counted by the predict kernel, and the cells of the
+                                 // particles that the counting sort samples (kSparseLeast)
     uint32_t* taint;             // per particle: the last substep that tainted it (quotients_tainted)
     int4* cellXYZ;               // per particle: the cell its friends were taken around, and the scene's first key
                                  // (NULL in relaxed mode: nothing is tainted)
@@ -102,6 +103,13 @@ struct LaunchShape {
                                // the particle tiles from a counter (no waits between blocks)
 };
 constexpr int kMaxBlock = 512;
+// Particles from which on a substep that sorts by counting looks whether the scene is
+// sparse (sparse_scene): an idle launch more, and below the build by warps is no slower
+// than the two scans that it replaced (200,000 at 0.5 to a cell 207 us a substep and
+// 224; 500,000 404 and 393).  kSampleBlocks x 256 particles add kSampleOne over the
+// particles of their cell each.
+constexpr int kSparseLeast = 600000;
+constexpr uint32_t kSampleBlocks = 32, kSampleOne = 1024;
 
 // Launches a kernel of the substep's chain: it may start before the kernel
 // before it on the stream has ended, and waits for that one's end itself
@@ -146,8 +154,8 @@ void launch_reset_cells(int n, const uint32_t* keys, uint32_t* cells, uint32_t k
 // Writes the rows (walk_pairs in pbf_device.cuh) and meta.  algorithm:
 // LaunchShape::friendsAlgorithm; block is the scan's.
 // The cells come as ranges (launch_update_cells) or, where starts is given, as
-// the first index of every key and one beyond the last.
-void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const uint32_t* cells,
+// the first index of every key and one beyond the last.  Returns the launches.
+int launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const uint32_t* cells,
                           const uint32_t* starts, uint4* rows, uint2* meta, int* errorWord, int block, int algorithm,
                           cudaStream_t s);
 // uint4 entries per particle of the rows for `slots` friends, at least the four
@@ -234,8 +242,8 @@ void launch_counting_sort(const CountingPlan& plan, int n, uint32_t* counts, uin
                           const uint32_t* keys, const uint32_t* place, uint32_t* order, uint32_t* crowded,
                           uint32_t keyLimit, int* err, cudaStream_t s);
 // The stable order from it, with the records gathered (launch_gather_sorted);
-// permCopy (may be NULL) receives the permutation too.
-void launch_cell_gather(int n, const uint32_t* keys, const uint32_t* starts, const uint32_t* order, uint32_t* keysOut,
+// permCopy (may be NULL) receives the permutation too; c: its n, h and epoch.
+void launch_cell_gather(const DevConsts& c, const uint32_t* keys, const uint32_t* starts, const uint32_t* order, uint32_t* keysOut,
                         uint32_t* permOut, uint32_t* permCopy, const float4* pos, const float4* pred,
                         const uint32_t* ids, float4* posOut, float4* predOut, uint32_t* idsOut, uint32_t keyLimit, int* err,
                         cudaStream_t s);

@@ -79,7 +79,10 @@ __global__ void predict_keys_kernel(DevConsts c, Batch b, const float4* pos, flo
     const float4 p = pos[i];
     const float4 q = make_float4(p.x + c.dt * v.x, p.y + c.dt * v.y, p.z + c.dt * v.z, p.w + c.dt * v.w);
     pred[i] = q;
-    if (i == 0) *c.epoch += 1u;  // a new substep: earlier taint marks lapse
+    if (i == 0) {
+        c.epoch[0] += 1u;  // a new substep: earlier taint marks lapse
+        c.epoch[1] = 0u;
+    }
     if (!paused) {
         const uint32_t key = base + grid_hash(__float2int_rz(q.x / c.h), __float2int_rz(q.y / c.h), __float2int_rz(q.z / c.h), c.grid);
         keys[i] = key;
@@ -469,8 +472,7 @@ __device__ __forceinline__ float max_nan(float a, float b) {
 // instructions, the tests 160 and the sorting 170.  Against the scan by threads:
 // 0.105 / 0.095 / 0.174 / 0.156 / 0.180 ms at 0.5 / 1 / 2 / 4 / 8 particles to a
 // cell and 0.062 / 0.063 / 0.162 / 0.217 / 0.310 there (200,000 particles for the
-// first two, then 500,000); a rule within the kernel that scans the warps of many
-// short runs gains a fifth of that at 0.5 to a cell and loses at 1 and above.
+// first two, then 500,000; sparse_scene).
 // Runs with
 // coordinates that are not finite take the scan.  A run with up to half as many
 // candidates again as fit is split across the longest side of its box, and the
@@ -662,6 +664,35 @@ __device__ __noinline__ uint64_t friends_in_chunks(const DevConsts& c, FriendSha
     return counts;
 }
 
+// Whether the scene's cells hold fewer than two particles on average (sample_cells):
+// a warp then takes a run for every particle or two, and the scan by threads is the faster one.  A substep of 1M random
+// particles at 0.5 / 1 / 1.5 / 2 / 3 to a cell of space takes 739 / 785 / 797 / 801 /
+// 810 us by warps and 590 / 705 / 780 / 858 / 968 by threads (4M at 0.5 / 1 / 2:
+// 3,990 / 4,100 / 3,840 and 2,815 / 3,250 / 3,710); two scans by one thread each,
+// with the passes of then, took 704 / 776 / - / 894 / 985 (3,516 / 3,703 / 3,845).
+// Dense scenes pay 4 us a substep for the question.
+// Decided for single warps it is slower: the few of a dense scene take 30 to 70 us
+// after all others have ended.
+__device__ __forceinline__ bool sparse_scene(const DevConsts& c) {
+    return 2u * c.epoch[1] > kSampleBlocks * 256u * kSampleOne;
+}
+
+// The friends of a sparse scene by one thread each, where build_friends_kernel<32>
+// leaves them; an idle launch (about 1.5 us) in others.
+__global__ void __launch_bounds__(kBlock, 6)
+build_friends_sparse_kernel(const __grid_constant__ DevConsts c, Batch b, const float4* pred, CellTable cells, uint4* rows,
+                            uint2* meta, int* err) {
+    chain_wait();
+    if (!sparse_scene(c)) return;
+#pragma unroll 1
+    for (uint32_t k = blockIdx.x * kBlock + threadIdx.x; k < (uint32_t)c.n; k += gridDim.x * kBlock) {
+        const int i = (int)k;
+        const float4 pi = pred[i];
+        const int cx = __float2int_rz(pi.x / c.h), cy = __float2int_rz(pi.y / c.h), cz = __float2int_rz(pi.z / c.h);
+        friends_of_one(c, key_base(b, i), pred, cells, rows, meta, err, i, pi, cx, cy, cz);
+    }
+}
+
 // W particles to a warp: 32, or fewer where that leaves the chip without warps
 // (a warp takes its members one after another).
 template <int W>
@@ -678,10 +709,12 @@ build_friends_kernel(const __grid_constant__ DevConsts c, Batch b, const float4*
     const int n = c.n;
     if (warpBase >= n) return;  // whole warp idle
     const bool valid = lane < W && i < n;
+    const bool sparse = W == 32 && c.n >= kSparseLeast && sparse_scene(c);  // read beside the position
     const float4 pi = valid ? pred[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const int cx = __float2int_rz(pi.x / c.h), cy = __float2int_rz(pi.y / c.h), cz = __float2int_rz(pi.z / c.h);
     const uint32_t base = valid ? key_base(b, i) : 0u;
     if (valid) record_cell(c, i, pi, cx, cy, cz, base);
+    if (W == 32 && sparse) return;
     const bool pow2 = (c.grid & (c.grid - 1)) == 0;
     const uint32_t gmask = c.grid - 1;
     const int ux = __shfl_up_sync(kFull, cx, 1), uy = __shfl_up_sync(kFull, cy, 1), uz = __shfl_up_sync(kFull, cz, 1);
@@ -1558,13 +1591,13 @@ unsigned grid_for_tiles(K kernel, int n, int block, bool persistent, int* tiles)
     return cap;
 }
 
-void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const uint32_t* cells,
+int launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const uint32_t* cells,
                           const uint32_t* starts, uint4* rows, uint2* meta, int* errorWord, int block, int algorithm,
                           cudaStream_t s) {
     const CellTable table{reinterpret_cast<const uint2*>(cells), starts};
     if (algorithm == 1) {
         launch_chained(build_friends_scan_kernel, blocks_for(c.n, block), block, s, c, b, pred, table, rows, meta, errorWord);
-        return;
+        return 1;
     }
     // a substep of 1,024 / 2,048 / 4,096 / 8,192 particles takes 43 / 48 / 54 / 68 us with one particle to a warp,
     // 46 / 52 / 56 / 66 with 4 (nothing else fills the chip, and a warp takes its members one after another);
@@ -1573,6 +1606,9 @@ void launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const
     const int w = c.n <= 4096 ? 1 : c.n <= 16384 ? 4 : c.n <= 49152 ? 8 : c.n <= 196608 ? 16 : 32;
     auto k = w == 1 ? build_friends_kernel<1> : w == 4 ? build_friends_kernel<4> : w == 8 ? build_friends_kernel<8> : w == 16 ? build_friends_kernel<16> : build_friends_kernel<32>;
     launch_chained(k, blocks_for(c.n, w * kFriendWarps), 32 * kFriendWarps, s, c, b, pred, table, rows, meta, errorWord);
+    if (c.n < kSparseLeast) return 1;
+    launch_chained(build_friends_sparse_kernel, 912u, kBlock, s, c, b, pred, table, rows, meta, errorWord);
+    return 2;
 }
 
 void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* predPacked, float* density,

@@ -301,19 +301,45 @@ __device__ __noinline__ uint32_t smaller_in_long_cell(const uint32_t* order, uin
     return less;
 }
 
+// What a particle's cell holds, for sparse_scene: each thread draws one from its part
+// of the order and adds its share of kSampleOne.  Other cells of the same key do not
+// count.  The gather's first blocks do that and nothing else: they end long before
+// its last.
+__device__ __forceinline__ void sample_cells(int n, float perH, const uint32_t* keys, const uint32_t* starts,
+                                          const uint32_t* order, const float4* pred, uint32_t* sampled) {
+    const uint32_t k = blockIdx.x * kThreads + threadIdx.x, part = (uint32_t)n / (kSampleBlocks * kThreads);
+    const uint32_t i = order[k * part + ((k * 2654435761u) >> 8) % part];
+    const float4 p = pred[i];
+    const uint32_t key = keys[i], first = starts[key], end = min(starts[key + 1], first + 16u);
+    const int cx = __float2int_rz(p.x * perH), cy = __float2int_rz(p.y * perH), cz = __float2int_rz(p.z * perH);
+    uint32_t together = 0;
+#pragma unroll 8
+    for (uint32_t q = first; q < end; ++q) {
+        const float4 o = pred[order[q]];
+        together += __float2int_rz(o.x * perH) == cx && __float2int_rz(o.y * perH) == cy && __float2int_rz(o.z * perH) == cz;
+    }
+    const uint32_t share = __reduce_add_sync(0xFFFFFFFFu, kSampleOne / max(together, 1u));
+    if ((threadIdx.x & 31) == 0) atomicAdd(sampled, share);
+}
+
 // The particle in slot s of the scattered order goes to its cell's first index
 // plus the number of smaller indices in the cell: the stable order.  With it go
 // its key, index, position, prediction and id (radixsort.cl:22-37; velocities
 // are not permuted, they are recomputed before any read, update_velocities.cl:13).
-__global__ void __launch_bounds__(kThreads)
-cell_gather_kernel(int n, const uint32_t* keys, const uint32_t* starts,
+template <bool Sample>
+__global__ void __launch_bounds__(kThreads, 8)
+cell_gather_kernel(int n, float h, uint32_t* sampled, const uint32_t* keys, const uint32_t* starts,
                    const uint32_t* order, uint32_t* keysOut, uint32_t* permOut,
                    uint32_t* permCopy,
                    const float4* pos, const float4* pred, const uint32_t* ids,
                    float4* posOut, float4* predOut, uint32_t* idsOut,
                    uint32_t keyLimit, int* err) {
     chain_wait();
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (Sample && blockIdx.x < kSampleBlocks) {
+        sample_cells(n, 1.0f / h, keys, starts, order, pred, sampled);
+        return;
+    }
+    const int s = (blockIdx.x - (Sample ? kSampleBlocks : 0u)) * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const uint32_t i = checked_index(order[s], (uint32_t)n, err, kErrSortIndex);
     const float4 x = pos[i], p = pred[i];
@@ -664,11 +690,14 @@ void launch_counting_sort(const CountingPlan& plan, int n, uint32_t* counts, uin
                    (uint32_t)plan.words, keyLimit, err);
 }
 
-void launch_cell_gather(int n, const uint32_t* keys, const uint32_t* starts, const uint32_t* order, uint32_t* keysOut,
+void launch_cell_gather(const DevConsts& c, const uint32_t* keys, const uint32_t* starts, const uint32_t* order, uint32_t* keysOut,
                         uint32_t* permOut, uint32_t* permCopy, const float4* pos, const float4* pred,
                         const uint32_t* ids, float4* posOut, float4* predOut, uint32_t* idsOut, uint32_t keyLimit, int* err,
                         cudaStream_t s) {
-    launch_chained(cell_gather_kernel, (n + kThreads - 1) / kThreads, kThreads, s, n, keys, starts, order, keysOut, permOut, permCopy, pos,
+    const int n = c.n;
+    const bool sample = n >= kSparseLeast;
+    auto k = sample ? cell_gather_kernel<true> : cell_gather_kernel<false>;
+    launch_chained(k, (n + kThreads - 1) / kThreads + (sample ? kSampleBlocks : 0u), kThreads, s, n, c.h, c.epoch + 1, keys, starts, order, keysOut, permOut, permCopy, pos,
                                                                           pred, ids, posOut, predOut, idsOut, keyLimit, err);
 }
 

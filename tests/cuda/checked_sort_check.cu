@@ -32,7 +32,10 @@ extern "C" int checked_sort(int n, uint32_t limit, const uint32_t* keys, const u
     pbf::launch_counting_sort(plan, n, d[2], d[3], d[4], d[0], d[1], d[5], nullptr, limit, err, nullptr);
     cudaMemcpy(errors, err, 4, cudaMemcpyDeviceToHost);
     cudaMemset(err, 0, 4);
-    pbf::launch_cell_gather(n, d[0], d[4], d[5], d[6], d[7], nullptr, v, v + n, ids, v + 2 * n, v + 3 * n, ids + n, limit,
+    pbf::DevConsts c{};
+    c.n = n;
+    c.h = 0.1f;
+    pbf::launch_cell_gather(c, d[0], d[4], d[5], d[6], d[7], nullptr, v, v + n, ids, v + 2 * n, v + 3 * n, ids + n, limit,
                             err, nullptr);
     cudaError_t e = cudaDeviceSynchronize();
     if (e == cudaSuccess) e = cudaMemcpy(errors + 1, err, 4, cudaMemcpyDeviceToHost);
