@@ -1192,8 +1192,7 @@ int pbf_render_frame(pbf_ctx* ctx, const PbfCamera* cam, int mode) {
         r.n = ctx->n;
     }
     r.err = ctx->errWord;
-    pbf::render_frame(*cam, mode, ctx->n, ctx->params.h, ctx->pos[ctx->curPos], r, ctx->stream);
-    ctx->launches += pbf::render_launches(mode);
+    ctx->launches += (uint64_t)pbf::render_frame(*cam, mode, ctx->n, ctx->params.h, ctx->pos[ctx->curPos], r, ctx->stream);
     ctx->renderMode = mode;
     PBF_CUDA(ctx, cudaGetLastError());
     PBF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -301,8 +301,8 @@ struct RenderBuffers {
     CountingPlan plan{};
     int* err = nullptr;                  // the context's error word (bounds-checked builds)
 };
-void render_frame(const PbfCamera& cam, int mode, int n, float h, const float4* pos, RenderBuffers& rb, cudaStream_t s);
-int render_launches(int mode);
+// Returns the launches.
+int render_frame(const PbfCamera& cam, int mode, int n, float h, const float4* pos, RenderBuffers& rb, cudaStream_t s);
 uint64_t render_grid_buckets();
 
 }  // namespace pbf

@@ -495,9 +495,7 @@ bool plain_perspective(const PbfCamera& cam) {
 
 }  // namespace
 
-int render_launches(int mode) { return mode == 0 ? 11 : 4; }
-
-void render_frame(const PbfCamera& cam, int mode, int n, float h, const float4* pos, RenderBuffers& rb,
+int render_frame(const PbfCamera& cam, int mode, int n, float h, const float4* pos, RenderBuffers& rb,
                   cudaStream_t s) {
     const size_t pixels = (size_t)cam.width * cam.height;
     cudaMemsetAsync(rb.dkey, 0xFF, 8 * pixels, s);
@@ -516,7 +514,7 @@ void render_frame(const PbfCamera& cam, int mode, int n, float h, const float4* 
     resolve_kernel<<<blocks(pixels, 256), 256, 0, s>>>(cam, n, mode, pos, rb.dkey, rb.splat, rb.vis);
     if (mode != 0) {
         cudaMemcpyAsync(rb.out, rb.splat, 16 * pixels, cudaMemcpyDeviceToDevice, s);
-        return;
+        return tileDepth ? 4 : 3;
     }
     grid_count_kernel<<<blocks(n, 256), 256, 0, s>>>(n, h, pos, rb.vis, rb.keys, rb.place, rb.counts);
     launch_counting_scan(rb.plan, rb.counts, rb.sums, rb.starts, s);
@@ -525,6 +523,7 @@ void render_frame(const PbfCamera& cam, int mode, int n, float h, const float4* 
     smooth_kernel<<<dim3(blocks(cam.width, 16), blocks(cam.height, 8)), 128, 0, s>>>(cam, h, n, rb.sorted, rb.starts, rb.splat,
                                                                                     rb.smooth, rb.err);
     final_kernel<<<blocks(pixels, 256), 256, 0, s>>>(cam, rb.smooth, rb.out);
+    return (tileDepth ? 9 : 8) + (rb.plan.blocks > 1 ? 2 : 1);
 }
 
 uint64_t render_grid_buckets() { return kGridBuckets; }
