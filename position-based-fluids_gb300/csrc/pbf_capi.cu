@@ -508,8 +508,7 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
                                       ctx->perm[0], order, nullptr, tableKeys, ctx->errWord, s);
             launched += ctx->counting.blocks > 1 ? 3 : 2;
         } else {
-            ctx->keysIdx = pbf::launch_radix_sort(ctx->plan, ctx->keys, ctx->perm, ctx->hist, nullptr, nullptr, nullptr,
-                                                  nullptr, s);
+            ctx->keysIdx = pbf::launch_radix_sort(ctx->plan, ctx->keys, ctx->perm, ctx->hist, s);
             launched += pbf::radix_sort_launches(ctx->plan);
         }
         mark("sortParticles");
@@ -1446,7 +1445,7 @@ int pbf_sort_state(pbf_ctx* ctx, const float* pred, uint32_t* keys, uint32_t* pe
     keep(cudaMemcpyAsync(dPred, pred, 16 * (size_t)n, cudaMemcpyHostToDevice, s));
     keep(cudaMemsetAsync(dCells, 0xFF, 8 * (size_t)grid, s));
     pbf::launch_compute_keys(ctx->consts, batch_of(ctx), dPred, k[0], pm[0], nullptr, nullptr, s);
-    const int r = pbf::launch_radix_sort(ctx->plan, k, pm, dHist, nullptr, nullptr, nullptr, nullptr, s);
+    const int r = pbf::launch_radix_sort(ctx->plan, k, pm, dHist, s);
     pbf::launch_update_cells(n, k[r], dCells, grid, nullptr, s);
     const uint32_t nKeys = ((uint32_t)n + 2047u) / 2048u * 2048u;
     if (keys) keep(cudaMemcpyAsync(keys, k[r], 4 * (size_t)n, cudaMemcpyDeviceToHost, s));

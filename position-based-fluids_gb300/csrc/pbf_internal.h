@@ -207,11 +207,7 @@ struct SortPlan {
 SortPlan make_sort_plan(int n, uint32_t gridBufSize);
 // Sorts (keys[0], perm[0]) by key, stably, ping-ponging through keys[1] /
 // perm[1]; returns the index (0 or 1) of the buffers holding the result.
-// When posIn/predIn are given, the last pass also writes posOut/predOut
-// gathered through the permutation (the reference's sortParticles).
-int launch_radix_sort(const SortPlan& plan, uint32_t* keys[2], uint32_t* perm[2], uint32_t* hist,
-                      const float4* posIn, const float4* predIn, float4* posOut, float4* predOut,
-                      cudaStream_t s);
+int launch_radix_sort(const SortPlan& plan, uint32_t* keys[2], uint32_t* perm[2], uint32_t* hist, cudaStream_t s);
 // Kernels launched by one launch_radix_sort call.
 int radix_sort_launches(const SortPlan& plan);
 

@@ -162,7 +162,7 @@ extern "C" int pbf_sort_state_noalloc(const PbfParameters* params, const float* 
     uint32_t* hist = scratch + 2 * kMaxKeys;
 
     pbf::launch_compute_keys(c, pbf::Batch{nullptr, nullptr}, reinterpret_cast<const float4*>(d_pred), keys[0], perm[0], nullptr, nullptr, s);
-    const int r = pbf::launch_radix_sort(plan, keys, perm, hist, nullptr, nullptr, nullptr, nullptr, s);
+    const int r = pbf::launch_radix_sort(plan, keys, perm, hist, s);
     if (r == 1) {  // an odd number of passes left the result in the scratch half
         if ((e = cudaMemcpyAsync(d_keys, keys[1], 4 * (size_t)n, cudaMemcpyDeviceToDevice, s)) == cudaSuccess)
             e = cudaMemcpyAsync(d_perm, perm[1], 4 * (size_t)n, cudaMemcpyDeviceToDevice, s);

@@ -716,8 +716,7 @@ SortPlan make_sort_plan(int n, uint32_t gridBufSize) {
 
 int radix_sort_launches(const SortPlan& plan) { return 3 * plan.passes; }
 
-int launch_radix_sort(const SortPlan& plan, uint32_t* keys[2], uint32_t* perm[2], uint32_t* hist,
-                      const float4*, const float4*, float4*, float4*, cudaStream_t s) {
+int launch_radix_sort(const SortPlan& plan, uint32_t* keys[2], uint32_t* perm[2], uint32_t* hist, cudaStream_t s) {
     int cur = 0;
     uint32_t* totals = hist + (size_t)256 * plan.tiles;
     for (int pass = 0; pass < plan.passes; ++pass) {
