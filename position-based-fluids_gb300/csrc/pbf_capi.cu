@@ -1674,9 +1674,9 @@ int pbf_autotune(pbf_ctx* ctx, int trial_substeps, int* blocks_out) {
     };
     const char* names[5] = {"buildFriendsList", "computeScaling", "computeDelta", "applyViscosity", "applyVorticity"};
     const int candidates[4] = {64, 128, 256, 512};
-    // friends: best over block size x algorithm; the solver passes: best
-    // block size per balance setting, then the balance setting with the
-    // smaller sum
+    // friends: best over algorithm, and over block size for the scan by threads
+    // (the build by warps has its own); the solver passes: best block size per
+    // balance setting, then the balance setting with the smaller sum
     float friendsMs = 1e30f;
     int friendsBlock = shape0.friends, algorithm = shape0.friendsAlgorithm;
     float solverMs[2][4];
@@ -1699,7 +1699,7 @@ int pbf_autotune(pbf_ctx* ctx, int trial_substeps, int* blocks_out) {
             for (size_t k = 0; k < ctx->stageNames.size(); ++k) {
                 if (ctx->stageNames[k] != names[q]) continue;
                 const float ms = ctx->stageMs[k];
-                if (q == 0 && ms < friendsMs) { friendsMs = ms; friendsBlock = cand; algorithm = algo; }
+                if (q == 0 && ms < friendsMs) { friendsMs = ms; friendsBlock = algo == 1 ? cand : shape0.friends; algorithm = algo; }
                 if (q > 0 && ms < solverMs[bal][q - 1]) { solverMs[bal][q - 1] = ms; solverBlock[bal][q - 1] = cand; }
             }
     }
