@@ -480,9 +480,11 @@ __device__ __forceinline__ float max_nan(float a, float b) {
 // cells hold twice as many as fit, of which a run keeps about three of four.  262,144
 // particles in two colliding columns, where 560 candidates are common: a frame
 // takes 0.76 ms with that line, 0.84 with chunks alone.  A substep of 400,000
-// particles with 30 / 50 / 80 to a cell takes 1.56 / 2.11 / 2.73 ms (1.74 / 2.19 /
+// particles with 30 / 50 / 80 to a cell takes 1.61 / 2.15 / 2.74 ms (1.74 / 2.19 /
 // 2.76 when the chunks wait for the first walk's count; without chunks 1.9 / 3.6 /
 // 7.1; two scans by one thread each, with the passes of then, 1.69 / 2.51 / 3.33).
+// A run that is a small part of what its key holds takes the walk all the same:
+// 150,000 particles in 1,024 keys 1.28 ms (1.96 in chunks at once, 1.32 the scans).
 // In chunks of more than 8 times as many candidates, circles at their limit take no
 // part: 65,536 particles in 16 clusters of 4,096 take 1.1 ms (1.8), 32,768 in one
 // cell 2.9 (5.2; the scans 4.7).
@@ -772,7 +774,8 @@ build_friends_kernel(const __grid_constant__ DevConsts c, Batch b, const float4*
         end = lane < __popc(occupied) ? cell.x : 0xFFFFFFFFu;
         const uint32_t shift = cell.y;
         __syncwarp();
-        if (total > 2u * (uint32_t)kCandidates) {  // a run of this many keeps about three of four: too many to split
+        // cells this full keep about three of four, too many to split, unless it is other cells' particles that fill their keys
+        if (total > 2u * (uint32_t)kCandidates && 2 * __popc(runMask) >= (int)min(__shfl_sync(kFull, count, 13), (uint32_t)W)) {
             counts = friends_in_chunks(c, sh, pred, rows, total, end, shift, lx, ly, lz, hx, hy, hz, runMask, pi, warpBase, counts);
             spread |= runMask;
             continue;

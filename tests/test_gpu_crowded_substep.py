@@ -37,3 +37,21 @@ def test_crowded_cells_of_a_substep(pbf_mod, oracle_mod, cuda_device, counts, so
             assert np.array_equal(cells, debug["cells"])
             for g, o in zip(got, want):
                 assert np.array_equal(_bits(g), _bits(o))
+
+
+@pytest.mark.parametrize("grid", [16, 64, 150])
+@pytest.mark.parametrize("per_cell", [8, 40])
+def test_keys_that_many_cells_share(pbf_mod, oracle_mod, cuda_device, grid, per_cell):
+    """Runs whose candidates are many and mostly another cell's, beside runs of truly crowded cells."""
+    params = pbf_mod.load_scenario("dam_break_32k")
+    n = params.particleCount = 6000
+    params.gridBufSize, params.boxClamp = grid, 0
+    rng = np.random.default_rng(grid + per_cell)
+    pos = np.zeros((n, 4), np.float32)
+    pos[:, :3] = 0.3 + rng.random((n, 3)) * (n / per_cell) ** (1.0 / 3.0) * params.h
+    vel = np.zeros_like(pos)
+    with pbf_mod.Simulation.create(params, pos, vel, device=cuda_device) as sim:
+        sim.Step(2)
+        got = sim.read_state()
+    for g, o in zip(got, oracle_mod.step(params, pos, vel, 2)):
+        assert np.array_equal(_bits(g), _bits(o))
