@@ -313,7 +313,7 @@ void free_render(pbf_ctx* ctx) {
     pbf::RenderBuffers& r = ctx->render;
     dev_free(r.dkey); dev_free(r.splat); dev_free(r.smooth); dev_free(r.out); dev_free(r.vis);
     dev_free(r.keys); dev_free(r.place); dev_free(r.order); dev_free(r.sorted);
-    dev_free(r.counts); dev_free(r.starts); dev_free(r.sums); dev_free(r.shownCount);
+    dev_free(r.counts); dev_free(r.starts); dev_free(r.sums);
     r.width = r.height = r.n = 0;
 }
 
@@ -1178,10 +1178,10 @@ int pbf_render_frame(pbf_ctx* ctx, const PbfCamera* cam, int mode) {
         r.plan = pbf::make_scan_plan(pbf::render_grid_buckets());
         if ((rc = dev_alloc(ctx, &r.dkey, pixels)) || (rc = dev_alloc(ctx, &r.splat, pixels)) ||
             (rc = dev_alloc(ctx, &r.smooth, pixels)) || (rc = dev_alloc(ctx, &r.out, pixels)) ||
-            (rc = dev_alloc(ctx, &r.vis, n)) || (rc = dev_alloc(ctx, &r.keys, n)) || (rc = dev_alloc(ctx, &r.place, n)) ||
+            (rc = dev_alloc(ctx, &r.vis, (n + 3) / 4 * 4)) || (rc = dev_alloc(ctx, &r.keys, n)) || (rc = dev_alloc(ctx, &r.place, n)) ||
             (rc = dev_alloc(ctx, &r.order, n)) || (rc = dev_alloc(ctx, &r.sorted, n)) ||
             (rc = dev_alloc(ctx, &r.counts, r.plan.words)) || (rc = dev_alloc(ctx, &r.starts, r.plan.words)) ||
-            (rc = dev_alloc(ctx, &r.sums, r.plan.blocks)) || (rc = dev_alloc(ctx, &r.shownCount, 1))) {
+            (rc = dev_alloc(ctx, &r.sums, r.plan.blocks))) {
             free_render(ctx);
             return rc;
         }

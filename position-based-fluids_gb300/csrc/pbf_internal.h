@@ -293,7 +293,6 @@ struct RenderBuffers {
     uint32_t* counts = nullptr;          // per bucket (2048^2): its particles; zero between frames
     uint32_t* starts = nullptr;          // per bucket: its first particle, and one beyond the last bucket
     uint32_t* sums = nullptr;
-    uint32_t* shownCount = nullptr;      // sprites that draw_kernel draws
     CountingPlan plan{};
     int* err = nullptr;                  // the context's error word (bounds-checked builds)
 };

@@ -148,14 +148,48 @@ __device__ __forceinline__ float depth_at(const PbfCamera& cam, float z) {
     return ((cam.projection[10] * z + cam.projection[14]) / -z + 1.0f) / 2.0f;
 }
 
+// A fragment's depth test.  Most fragments lie behind what is drawn already: one
+// whose sprite's nearest depth does is dropped before its own is formed (1M
+// sprites of 5 pixels, 48M -> 33M warp instructions in splat_kernel, and 61 -> 43
+// us with four pixels' loads in flight; one by one they took the gain away).  An old
+// value of the pixel is larger, so a stale read only costs the work.
+__device__ __forceinline__ void draw(const PbfCamera& cam, float ex, float ey, float ez, float xw, float yw, float s,
+                                     uint32_t nearest, int p, int i, int j, unsigned long long* at,
+                                     unsigned long long drawn) {
+    if (nearest > (uint32_t)(drawn >> 32)) return;
+    Frag f;
+    if (!fragment(cam, ex, ey, ez, xw, yw, s, i, j, f)) return;
+    const unsigned long long key = ((unsigned long long)__float_as_uint(f.depth) << 32) | (0xFFFFFFFFu - (uint32_t)p);
+    if (key < drawn) atomicMin(at, key);
+}
+
+__device__ __forceinline__ uint32_t nearest_depth(const PbfCamera& cam, float ez) {
+    const float nearest = ez + cam.pointSize < 0.0f ? depth_at(cam, ez + cam.pointSize) - kSlack : 0.0f;
+    return nearest > 0.0f ? __float_as_uint(nearest) : 0u;
+}
+
+// Also clears what a frame starts from: no fragment, and no particle seen (visWords
+// words).  tileDepth NULL: that alone.  Each had a clear of its own; with those, and
+// the launches up to the resolve not chained, 262,144 sprites of 2 pixels at 640 x 480
+// took 48 us in a colour mode, 27 like this.
+constexpr uint32_t kNoSprites = 0x7F7F7F7Fu;  // what the sprites' counter and the bounds start from
 __global__ void __launch_bounds__(128)
-occlude_kernel(PbfCamera cam, int n, const float4* __restrict__ pos, uint32_t* __restrict__ tileDepth) {
+occlude_kernel(PbfCamera cam, int n, const float4* pos, uint32_t* tileDepth, unsigned long long* dkey, uint32_t* vis,
+               uint32_t visWords) {
+    chain_wait();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
+    const size_t pixels = (size_t)cam.width * cam.height, stride = gridDim.x * (size_t)blockDim.x;
+    for (size_t k = p; k < pixels; k += stride) dkey[k] = kEmptyKey;
+    for (size_t k = p; k < visWords; k += stride) vis[k] = 0u;
+    if (p >= n || !tileDepth) return;
+    const float4 at = pos[p];
+    // only sprites that lie inside the depth range as a whole, and wide enough to cover a tile: the size is known from
+    // the eye-space z alone (w = -z)
+    const float* m = cam.modelView;
+    const float z = ((m[2] * at.x + m[6] * at.y) + m[10] * at.z) + m[14] * 1.0f;
+    if (!(z + cam.pointSize < 0.0f) || cam.widthOfNearPlane * cam.pointSize / -z < 1.5f * kTilePixels) return;
     float ex, ey, ez, xw, yw, s;
-    if (!sprite(cam, pos[p], ex, ey, ez, xw, yw, s)) return;
-    // only sprites that lie inside the depth range as a whole, and wide enough to cover a tile
-    if (s < 1.5f * kTilePixels || !(ez + cam.pointSize < 0.0f)) return;
+    if (!sprite(cam, at, ex, ey, ez, xw, yw, s)) return;
     if (!(depth_at(cam, ez + cam.pointSize) > kSlack) || !(depth_at(cam, ez) < 1.0f - kSlack)) return;
     const Rect r = sprite_rect(cam, xw, yw, s);
     const int tilesX = (cam.width + kTilePixels - 1) / kTilePixels;
@@ -175,75 +209,64 @@ occlude_kernel(PbfCamera cam, int n, const float4* __restrict__ pos, uint32_t* _
     }
 }
 
-// A fragment's depth test.  Most fragments lie behind what is drawn already: one
-// whose sprite's nearest depth does is dropped before its own is formed (1M
-// sprites of 5 pixels, 48M -> 33M warp instructions in splat_kernel, and 61 -> 43
-// us with four pixels' loads in flight; one by one they took the gain away).  An old
-// value of the pixel is larger, so a stale read only costs the work.
-__device__ __forceinline__ void draw(const PbfCamera& cam, float ex, float ey, float ez, float xw, float yw, float s,
-                                     uint32_t nearest, int p, int i, int j, unsigned long long* __restrict__ at,
-                                     unsigned long long drawn) {
-    if (nearest > (uint32_t)(drawn >> 32)) return;
-    Frag f;
-    if (!fragment(cam, ex, ey, ez, xw, yw, s, i, j, f)) return;
-    const unsigned long long key = ((unsigned long long)__float_as_uint(f.depth) << 32) | (0xFFFFFFFFu - (uint32_t)p);
-    if (key < drawn) atomicMin(at, key);
-}
-
-__device__ __forceinline__ uint32_t nearest_depth(const PbfCamera& cam, float ez) {
-    const float nearest = ez + cam.pointSize < 0.0f ? depth_at(cam, ez + cam.pointSize) - kSlack : 0.0f;
-    return nearest > 0.0f ? __float_as_uint(nearest) : 0u;
-}
-
-// Draws the small sprites, a thread each, and lists the others that are not
-// hidden in every tile.  tileDepth NULL: no occlusion bounds.
-// Pixels that one thread draws: sprites too small to cover a tile, which nothing
-// hides beforehand (494,820 particles at 750 x 981, 10 pixels wide: 355 us a frame;
-// a warp to each of more than 36 pixels: 642; every fragment formed: 522).
-constexpr int kSmallSprite = 144;
+// Draws the small sprites, a thread each, and lists the others (*counter of them)
+// that are not hidden in every tile.  tileDepth NULL: no bounds.
+// Pixels that one thread draws: sprites too small to cover a tile (494,820
+// particles at 750 x 981, 10 pixels wide: 355 us a frame; a warp to each of more than
+// 36 pixels: 642; every fragment formed: 522).
+// Below kEarlyLeast particles the chip has too few threads to hide the loads of the
+// early depth test (30,000 of 6 pixels at 640 x 480 93 us a frame with it, 57 without
+// it and without the look at the tiles).  Tiny sprites skip both too: they cost as
+// much as the few fragments do (1M of 2 to 3 pixels: 46 us in this kernel with them,
+// 38 to 40 without; at 3 to 4 pixels a frame of 262,144, many over one another, takes
+// 39 and 51).
+constexpr int kSmallSprite = 144, kEarlyLeast = 100000;
+template <bool Early>
 __global__ void __launch_bounds__(128)
-splat_kernel(PbfCamera cam, int n, const float4* __restrict__ pos, const uint32_t* __restrict__ tileDepth,
-             unsigned long long* __restrict__ dkey, uint32_t* __restrict__ shown, uint32_t* __restrict__ shownCount) {
+splat_kernel(PbfCamera cam, int n, const float4* pos, const uint32_t* tileDepth, unsigned long long* dkey, uint32_t* shown,
+             uint32_t* counter) {
+    chain_wait();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     float ex, ey, ez, xw, yw, s;
     if (!sprite(cam, pos[p], ex, ey, ez, xw, yw, s)) return;
     const Rect r = sprite_rect(cam, xw, yw, s);
     const int tilesX = (cam.width + kTilePixels - 1) / kTilePixels;
+    const bool tiny = s <= (Early ? 3.0f : 8.0f);
     const uint32_t nearest = tileDepth ? nearest_depth(cam, ez) : 0u;
-    bool visible = tileDepth == nullptr;
+    bool visible = tiny || tileDepth == nullptr;
     for (int tj = r.j0 / kTilePixels; !visible && tj <= r.j1 / kTilePixels; ++tj)
         for (int ti = r.i0 / kTilePixels; !visible && ti <= r.i1 / kTilePixels; ++ti)
             visible = nearest <= tileDepth[(size_t)tj * tilesX + ti];
     if (!visible) return;
-    if ((r.i1 - r.i0 + 1) * (r.j1 - r.j0 + 1) <= kSmallSprite) {
-        for (int j = r.j0; j <= r.j1; ++j) {
-            unsigned long long* row = dkey + (size_t)j * cam.width;
-            for (int i = r.i0; i <= r.i1; i += 4) {  // four pixels' loads in flight
-                unsigned long long drawn[4];
+    if ((r.i1 - r.i0 + 1) * (r.j1 - r.j0 + 1) > kSmallSprite) {
+        shown[atomicAdd(counter, 1u) - kNoSprites] = (uint32_t)p;
+        return;
+    }
+    for (int j = r.j0; j <= r.j1; ++j) {
+        unsigned long long* row = dkey + (size_t)j * cam.width;
+        for (int i = r.i0; i <= r.i1; i += 4) {  // four pixels' loads in flight
+            unsigned long long drawn[4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) drawn[k] = i + k <= r.i1 ? row[i + k] : 0ull;  // 0: nothing is in front of it
+            for (int k = 0; k < 4; ++k) drawn[k] = !Early || tiny ? kEmptyKey : i + k <= r.i1 ? row[i + k] : 0ull;  // 0: nothing is in front of it
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (i + k <= r.i1) draw(cam, ex, ey, ez, xw, yw, s, nearest, p, i + k, j, row + i + k, drawn[k]);
-            }
+            for (int k = 0; k < 4; ++k)
+                if (i + k <= r.i1) draw(cam, ex, ey, ez, xw, yw, s, nearest, p, i + k, j, row + i + k, drawn[k]);
         }
-    } else {
-        shown[atomicAdd(shownCount, 1u)] = (uint32_t)p;
     }
 }
 
-// The listed sprites, a warp each, tile by tile: the sprites that remain lie
-// together in memory, so they are dealt out over the whole chip.
-constexpr int kDrawBlocks = 152 * 16;
-__global__ void __launch_bounds__(128)
-draw_kernel(PbfCamera cam, int n, const float4* __restrict__ pos, const uint32_t* __restrict__ tileDepth,
-            unsigned long long* __restrict__ dkey, const uint32_t* __restrict__ shown,
-            const uint32_t* __restrict__ shownCount, int* err) {
+// The sprites that remain, a warp each, tile by tile: they lie together in memory, so
+// they are dealt out over the whole chip.  tileDepth NULL: no occlusion bounds.
+constexpr int kDrawBlocks = 152 * 16, kDrawWarps = 4;
+__global__ void __launch_bounds__(32 * kDrawWarps)
+draw_kernel(PbfCamera cam, int n, const float4* pos, const uint32_t* tileDepth, unsigned long long* dkey,
+            const uint32_t* shown, const uint32_t* shownCount, int* err) {
+    chain_wait();
     const int lane = threadIdx.x & 31;
-    const uint32_t count = checked_index(*shownCount, (uint32_t)n + 1u, err, kErrSortIndex);
+    const uint32_t count = checked_index(*shownCount - kNoSprites, (uint32_t)n + 1u, err, kErrSortIndex);
     const int tilesX = (cam.width + kTilePixels - 1) / kTilePixels;
-    for (uint32_t k = blockIdx.x * 4 + (threadIdx.x >> 5); k < count; k += kDrawBlocks * 4) {
+    for (uint32_t k = blockIdx.x * kDrawWarps + (threadIdx.x >> 5); k < count; k += kDrawBlocks * kDrawWarps) {
         const int p = (int)checked_index(shown[k], (uint32_t)n, err, kErrSortIndex);
         float ex, ey, ez, xw, yw, s;
         sprite(cam, pos[p], ex, ey, ez, xw, yw, s);
@@ -273,9 +296,10 @@ __device__ __forceinline__ float hsv_channel(float h, float k, float s, float v)
     return v * (1.0f * (1.0f - s) + q * s);
 }
 
-__global__ void resolve_kernel(PbfCamera cam, int n, int mode, const float4* __restrict__ pos,
-                               const unsigned long long* __restrict__ dkey, float4* __restrict__ splat,
-                               uint8_t* __restrict__ vis) {
+__global__ void __launch_bounds__(256)
+resolve_kernel(PbfCamera cam, int n, int mode, const float4* pos, const unsigned long long* dkey, float4* splat,
+               uint8_t* vis, float4* out) {
+    chain_wait();
     const int pix = blockIdx.x * blockDim.x + threadIdx.x;
     const bool inside = pix < cam.width * cam.height;
     const unsigned long long key = inside ? dkey[pix] : 0ull;
@@ -289,6 +313,7 @@ __global__ void resolve_kernel(PbfCamera cam, int n, int mode, const float4* __r
     if (!inside) return;
     if (key == kEmptyKey) {
         splat[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (mode != 0) out[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // the colour modes' frame is the splat
         return;
     }
     const uint32_t p = 0xFFFFFFFFu - (uint32_t)(key & 0xFFFFFFFFu);
@@ -317,7 +342,7 @@ __global__ void resolve_kernel(PbfCamera cam, int n, int mode, const float4* __r
         g = hsv_channel(hue, 2.0f / 3.0f, 0.9f, 0.9f);
         b = hsv_channel(hue, 1.0f / 3.0f, 0.9f, 0.9f);
     }
-    splat[pix] = make_float4(r * cosA, g * cosA, b * cosA, 1.0f * cosA);
+    splat[pix] = out[pix] = make_float4(r * cosA, g * cosA, b * cosA, 1.0f * cosA);
 }
 
 // Bucket and place of arrival of the visible particles (kGridBuckets: not visible).
@@ -495,27 +520,21 @@ bool plain_perspective(const PbfCamera& cam) {
 
 }  // namespace
 
-int render_frame(const PbfCamera& cam, int mode, int n, float h, const float4* pos, RenderBuffers& rb,
-                  cudaStream_t s) {
+int render_frame(const PbfCamera& cam, int mode, int n, float h, const float4* pos, RenderBuffers& rb, cudaStream_t s) {
     const size_t pixels = (size_t)cam.width * cam.height;
-    cudaMemsetAsync(rb.dkey, 0xFF, 8 * pixels, s);
-    // the bounds of the tiles live in the smoothed image, and the list of sprites in the grid's order: both are
-    // written later
-    uint32_t* tileDepth = plain_perspective(cam) ? reinterpret_cast<uint32_t*>(rb.smooth) : nullptr;
-    cudaMemsetAsync(rb.shownCount, 0, 4, s);
-    if (tileDepth) {
-        const size_t tiles = (size_t)((cam.width + kTilePixels - 1) / kTilePixels) * ((cam.height + kTilePixels - 1) / kTilePixels);
-        cudaMemsetAsync(tileDepth, 0x7F, 4 * tiles, s);  // a depth above every other
-        occlude_kernel<<<blocks(n, 128), 128, 0, s>>>(cam, n, pos, tileDepth);
-    }
-    splat_kernel<<<blocks(n, 128), 128, 0, s>>>(cam, n, pos, tileDepth, rb.dkey, rb.order, rb.shownCount);
-    draw_kernel<<<kDrawBlocks, 128, 0, s>>>(cam, n, pos, tileDepth, rb.dkey, rb.order, rb.shownCount, rb.err);
-    if (mode == 0) cudaMemsetAsync(rb.vis, 0, (size_t)n, s);
-    resolve_kernel<<<blocks(pixels, 256), 256, 0, s>>>(cam, n, mode, pos, rb.dkey, rb.splat, rb.vis);
-    if (mode != 0) {
-        cudaMemcpyAsync(rb.out, rb.splat, 16 * pixels, cudaMemcpyDeviceToDevice, s);
-        return tileDepth ? 4 : 3;
-    }
+    // the counter of the listed sprites and the bounds of the tiles live in the smoothed image, and the list in the
+    // grid's order: both are written later
+    uint32_t* counter = reinterpret_cast<uint32_t*>(rb.smooth);
+    uint32_t* tileDepth = plain_perspective(cam) ? counter + 1 : nullptr;
+    const size_t tiles = (size_t)((cam.width + kTilePixels - 1) / kTilePixels) * ((cam.height + kTilePixels - 1) / kTilePixels);
+    cudaMemsetAsync(counter, 0x7F, 4 * (1 + tiles), s);  // no sprite, and a depth above every other
+    launch_chained(occlude_kernel, max(blocks(n, 128), min(blocks(pixels, 128), 1216u)), 128, s, cam, n, pos, tileDepth, rb.dkey,
+                   reinterpret_cast<uint32_t*>(rb.vis), mode == 0 ? (uint32_t)((n + 3) / 4) : 0u);
+    launch_chained(n >= kEarlyLeast ? splat_kernel<true> : splat_kernel<false>, blocks(n, 128), 128, s, cam, n, pos, tileDepth,
+                   rb.dkey, rb.order, counter);
+    launch_chained(draw_kernel, kDrawBlocks, 32 * kDrawWarps, s, cam, n, pos, tileDepth, rb.dkey, rb.order, counter, rb.err);
+    launch_chained(resolve_kernel, blocks(pixels, 256), 256, s, cam, n, mode, pos, rb.dkey, rb.splat, rb.vis, rb.out);
+    if (mode != 0) return 4;
     grid_count_kernel<<<blocks(n, 256), 256, 0, s>>>(n, h, pos, rb.vis, rb.keys, rb.place, rb.counts);
     launch_counting_scan(rb.plan, rb.counts, rb.sums, rb.starts, s);
     grid_scatter_kernel<<<blocks(n, 256), 256, 0, s>>>(n, rb.keys, rb.place, rb.starts, rb.order, rb.err);
@@ -523,7 +542,7 @@ int render_frame(const PbfCamera& cam, int mode, int n, float h, const float4* p
     smooth_kernel<<<dim3(blocks(cam.width, 16), blocks(cam.height, 8)), 128, 0, s>>>(cam, h, n, rb.sorted, rb.starts, rb.splat,
                                                                                     rb.smooth, rb.err);
     final_kernel<<<blocks(pixels, 256), 256, 0, s>>>(cam, rb.smooth, rb.out);
-    return (tileDepth ? 9 : 8) + (rb.plan.blocks > 1 ? 2 : 1);
+    return 9 + (rb.plan.blocks > 1 ? 2 : 1);
 }
 
 uint64_t render_grid_buckets() { return kGridBuckets; }
