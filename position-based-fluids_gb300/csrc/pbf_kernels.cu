@@ -102,7 +102,8 @@ __global__ void predict_keys_kernel(DevConsts c, Batch b, const float4* pos, flo
 // tile's count of a key with one atomic.
 constexpr int kKeyThreads = 1024, kHotLeast = 65536;  // fewer particles do not contend
 constexpr uint32_t kHotTile = 4096;                   // as many slots as particles: the table does not overflow
-__global__ void __launch_bounds__(kKeyThreads)
+template <int Threads>
+__global__ void __launch_bounds__(Threads)
 compute_keys_kernel(DevConsts c, Batch b, const float4* pred, uint32_t* keys, uint32_t* perm, uint32_t* counts,
                     const uint32_t* hot) {
     chain_wait();
@@ -110,8 +111,8 @@ compute_keys_kernel(DevConsts c, Batch b, const float4* pred, uint32_t* keys, ui
         const float4 q = pred[i];
         return key_base(b, i) + grid_hash(__float2int_rz(q.x / c.h), __float2int_rz(q.y / c.h), __float2int_rz(q.z / c.h), c.grid);
     };
-    if (!hot || *hot == 0u) {
-        const int i = blockIdx.x * kKeyThreads + threadIdx.x;
+    if (Threads < kKeyThreads || *hot == 0u) {
+        const int i = blockIdx.x * Threads + threadIdx.x;
         const unsigned valid = __ballot_sync(0xFFFFFFFFu, i < c.n);
         if (i >= c.n) return;
         const uint32_t key = key_of(i);
@@ -121,7 +122,8 @@ compute_keys_kernel(DevConsts c, Batch b, const float4* pred, uint32_t* keys, ui
     }
     if (blockIdx.x * kHotTile >= (uint32_t)c.n) return;
     constexpr int kRounds = kHotTile / kKeyThreads;
-    __shared__ uint32_t slotKey[kHotTile], slotCount[kHotTile];  // a slot's count, then its first place
+    constexpr uint32_t kSlots = Threads < kKeyThreads ? 1 : kHotTile;
+    __shared__ uint32_t slotKey[kSlots], slotCount[kSlots];  // a slot's count, then its first place
     for (uint32_t q = threadIdx.x; q < kHotTile; q += kKeyThreads) {
         slotKey[q] = kEmpty;
         slotCount[q] = 0u;
@@ -1531,7 +1533,8 @@ void launch_predict_keys(const DevConsts& c, Batch b, const float4* pos, float4*
 
 void launch_compute_keys(const DevConsts& c, Batch b, const float4* pred, uint32_t* keys, uint32_t* perm, uint32_t* counts,
                          const uint32_t* hot, cudaStream_t s) {
-    launch_chained(compute_keys_kernel, blocks_for(c.n, kKeyThreads), kKeyThreads, s, c, b, pred, keys, perm, counts, hot);
+    if (hot) launch_chained(compute_keys_kernel<kKeyThreads>, blocks_for(c.n, kKeyThreads), kKeyThreads, s, c, b, pred, keys, perm, counts, hot);
+    else launch_chained(compute_keys_kernel<kBlock>, blocks_for(c.n), kBlock, s, c, b, pred, keys, perm, counts, hot);
 }
 
 void launch_clear_counts(const DevConsts& c, const float4* pred, uint32_t* counts, size_t words, uint32_t* hot, cudaStream_t s) {
