@@ -103,11 +103,11 @@ STAGE_BYTES = {
 # to nl).
 CAPTURE_SOURCE = ("ncu capture of the first substep of frame 51 (friends by warps, 128-thread blocks, "
                   "list lengths 38.52 / 32.79; position passes: the mean of the four), scaled by list length")
-TRAFFIC_CAPTURE = {"buildFriendsList": {"bytes": 207.1e6, "nl": 38.52, "nd": 32.79},
-                   "computeScaling": {"bytes": 228.6e6, "nl": 38.52, "nd": 32.79},
+TRAFFIC_CAPTURE = {"buildFriendsList": {"bytes": 207.6e6, "nl": 38.52, "nd": 32.79},
+                   "computeScaling": {"bytes": 228.8e6, "nl": 38.52, "nd": 32.79},
                    "computeDelta": {"bytes": 219.8e6, "nl": 38.52, "nd": 32.79}}
-ISSUE_CAPTURE = {"buildFriendsList": {"inst": 454.9e6, "nl": 38.52, "nd": 32.79},
-                 "computeScaling": {"inst": 71.4e6, "nl": 38.52, "nd": 32.79},
+ISSUE_CAPTURE = {"buildFriendsList": {"inst": 455.5e6, "nl": 38.52, "nd": 32.79},
+                 "computeScaling": {"inst": 71.3e6, "nl": 38.52, "nd": 32.79},
                  "computeDelta": {"inst": 74.8e6, "nl": 38.52, "nd": 32.79}}
 SM_COUNT = 152
 SCHEDULERS_PER_SM = 4

@@ -1558,12 +1558,11 @@ void launch_reset_cells(int n, const uint32_t* keys, uint32_t* cells, uint32_t k
 }
 
 // Lanes that share a particle in a solver pass (walk_pairs).  A substep of 2,048
-// / 4,096 / 8,192 / 16,384 / 24,576 / 32,768 particles takes 70 / 80 / 89 / 96 /
-// 98 / 101 us with one lane, 56 / 61 / 65 / 80 / 94 / 109 with four and 51 / 57 /
-// 68 / 90 / 119 / 133 with eight: beyond, the chip is full, and what the lanes
-// exchange costs more than the shorter chains save.  Relaxed sums go in turns:
-// 65 / 82 / 95 / 124 us at 2,048 / 8,192 / 16,384 / 32,768 against 72 / 92 / 103 /
-// 106 with one lane (the exact passes' figures when theirs went in turns).
+// / 4,096 / 8,192 / 16,384 / 24,576 / 32,768 particles takes 68 / 77 / 86 / 99 /
+// 102 / 109 us with one lane, 54 / 60 / 66 / 84 / 96 / 112 with four and 52 / 57 /
+// 68 / 96 / 118 / 136 with eight: beyond, the chip is full, and what the lanes
+// exchange costs more than the shorter chains save.  Relaxed sums go in turns: 60 /
+// 68 / 75 / 85 / 86 / 89 us with one lane, 56 / 63 / 68 / 82 / 95 / 118 with four.
 int lanes_per_particle(const DevConsts& c, int balance, const int* tileCounter) {
     if (balance || tileCounter) return 1;
     if (c.relaxed) return c.n <= 16384 ? 4 : 1;
