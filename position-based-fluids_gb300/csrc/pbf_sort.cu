@@ -375,7 +375,9 @@ constexpr uint32_t kMostTiles = PBF_NOALLOC_MAX_KEYS / kTileKeys;
 constexpr uint32_t kBigSlots = 512;  // of the table, a power of two above kMostBig
 static_assert(kMostBig < kBigSlots / 2 + 1 && kMostTiles <= kBlockCell, "bins and tiles of the large cells");
 
-// The large cells' numbers by key, and their first indices by number, for a block.
+// The large cells' numbers by key, and their first indices by number, for a block.  The
+// counts and the probes are limited to what a call can need: calls must not overlap on
+// the array, and where they do all the same no loop here runs on what the other left.
 struct BigCells {
     uint32_t key[kBigSlots], bin[kBigSlots], first[kMostBig];
     __device__ __forceinline__ static uint32_t slot(uint32_t k) { return (k * 2654435761u) >> 23; }
@@ -386,7 +388,7 @@ struct BigCells {
         for (uint32_t b = threadIdx.x; b < big; b += kThreads) {
             const uint32_t k = crowded[words - 1u - b];
             uint32_t q = slot(k);
-            while (atomicCAS(&key[q], kEmpty, k) != kEmpty) q = (q + 1u) % kBigSlots;
+            for (uint32_t tries = 0; tries < kBigSlots && atomicCAS(&key[q], kEmpty, k) != kEmpty; ++tries) q = (q + 1u) % kBigSlots;
             bin[q] = b;
             first[b] = starts[k];
         }
@@ -394,11 +396,12 @@ struct BigCells {
     }
     // kEmpty: not a large cell's key.
     __device__ __forceinline__ uint32_t find(uint32_t k) const {
-        for (uint32_t q = slot(k);; q = (q + 1u) % kBigSlots) {
+        for (uint32_t q = slot(k), tries = 0; tries < kBigSlots; q = (q + 1u) % kBigSlots, ++tries) {
             const uint32_t at = key[q];
             if (at == k) return bin[q];
-            if (at == kEmpty) return kEmpty;
+            if (at == kEmpty) break;
         }
+        return kEmpty;
     }
 };
 
@@ -421,7 +424,7 @@ cell_rank_kernel(int n, uint32_t keyLimit, const uint32_t* keys, const uint32_t*
         }
     }
     if (blockIdx.x >= tiles) return;
-    const uint32_t big = crowded[1];
+    const uint32_t big = min(crowded[1], kMostBig);
     if (big == 0u) return;
     __shared__ BigCells cells;
     __shared__ uint32_t counts[kMostBig];
@@ -542,7 +545,7 @@ crowded_cells_kernel(int n, const uint32_t* keys, const uint32_t* starts, uint32
         SharedCell<kThreads> cell;
         BigTile tile;
     } sh;
-    const uint32_t count = crowded[0], big = crowded[1], t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const uint32_t count = min(crowded[0], words - 2u), big = min(crowded[1], kMostBig), t = threadIdx.x, lane = t & 31, warp = t >> 5;
     for (uint32_t c = blockIdx.x * kWarps + warp; c < count; c += gridDim.x * kWarps) {
         const uint32_t key = crowded[2u + c], first = starts[key], holds = starts[key + 1] - first;
         if (holds <= kWarpCell) sort_cell<32>(sh.warpCell[warp], first, holds, order, permOut);
@@ -626,7 +629,7 @@ cell_table_kernel(int n, uint32_t keys, const uint32_t* starts, const uint32_t* 
         for (uint32_t q = f + lane; q < e; q += 32) keysOut[q] = k - lane + src;
     }
     if ((uint32_t)n <= kComparedCell) return;
-    const uint32_t count = crowded[0], big = crowded[1];
+    const uint32_t count = min(crowded[0], words - 2u), big = min(crowded[1], kMostBig);
     for (uint32_t b = blockIdx.x; b < count; b += gridDim.x) {
         const uint32_t key = crowded[2u + b], e = min(starts[key + 1], (uint32_t)n);
         for (uint32_t q = starts[key] + threadIdx.x; q < e; q += kThreads) keysOut[q] = key;
