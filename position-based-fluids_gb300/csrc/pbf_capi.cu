@@ -1499,10 +1499,10 @@ int pbf_read_friends(pbf_ctx* ctx, uint32_t* counts, uint32_t* list, int list_sl
     std::vector<uint2> meta(n);
     PBF_CUDA(ctx, cudaMemcpyAsync(meta.data(), ctx->meta, 8 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
     // the kept friends of every particle in order: the rows the passes walk
-    const int slots = list ? std::min(list_slots, ctx->listSlots) : 0;
-    std::vector<uint4> rows(pbf::row_entries(std::max(slots, 0)) * n);
+    const int slots = list ? std::max(0, std::min(list_slots, ctx->listSlots)) : 0;
+    std::unique_ptr<uint4[]> rows(new uint4[(size_t)((slots + 3) / 4) * n]);  // not initialised: the copy fills it
     if (slots > 0)
-        PBF_CUDA(ctx, cudaMemcpyAsync(rows.data(), ctx->rows, 16 * rows.size(), cudaMemcpyDeviceToHost, ctx->stream));
+        PBF_CUDA(ctx, cudaMemcpyAsync(rows.get(), ctx->rows, 16 * (size_t)((slots + 3) / 4) * n, cudaMemcpyDeviceToHost, ctx->stream));
     PBF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     for (int i = 0; i < n; ++i) {
         const uint64_t m = (uint64_t)meta[i].x | ((uint64_t)meta[i].y << 32);
