@@ -855,9 +855,9 @@ int pbf_create(const PbfParameters* params, int device, pbf_ctx** out) {
     ctx->device = device;
     PBF_CUDA(nullptr, cudaSetDevice(device));
     PBF_CUDA(nullptr, cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
-    // [0]: the error word; [1]: the substep counter of the taint marks; [2]: sampled cells (pbf::DevConsts::epoch)
-    PBF_CUDA(nullptr, cudaMalloc((void**)&ctx->errWord, 3 * sizeof(int)));
-    PBF_CUDA(nullptr, cudaMemset(ctx->errWord, 0, 3 * sizeof(int)));
+    // [0]: the error word; [1] to [3]: pbf::DevConsts::epoch
+    PBF_CUDA(nullptr, cudaMalloc((void**)&ctx->errWord, 4 * sizeof(int)));
+    PBF_CUDA(nullptr, cudaMemset(ctx->errWord, 0, 4 * sizeof(int)));
     PBF_CUDA(nullptr, cudaMallocHost((void**)&ctx->errHost, sizeof(int)));
     PBF_CUDA(nullptr, cudaMalloc((void**)&ctx->tileCounters, 10 * sizeof(int)));
     PBF_CUDA(nullptr, cudaMemset(ctx->tileCounters, 0, 10 * sizeof(int)));
@@ -996,7 +996,7 @@ int pbf_init_cells(pbf_ctx* ctx) {
     PBF_CUDA(ctx, cudaMemset(ctx->meta, 0, 8 * (size_t)ctx->n));
     // taint marks are substep numbers from 1 on (the counter restarts with them); no cell start yet
     PBF_CUDA(ctx, cudaMemset(ctx->taint, 0, 4 * (size_t)ctx->n));
-    PBF_CUDA(ctx, cudaMemset(ctx->errWord + 1, 0, 2 * sizeof(int)));
+    PBF_CUDA(ctx, cudaMemset(ctx->errWord + 1, 0, 3 * sizeof(int)));
     PBF_CUDA(ctx, cudaMemset(ctx->cellStart, 0xFF, 4 * tableWords));
     apply_planes(ctx);
     ctx->cellsReady = true;

@@ -52,8 +52,9 @@ struct DevConsts {
     int quotients;               // divisions by |r| in the four neighbour passes
     int quotientPoly6q;          // the s_corr division by poly6q in the position pass
     float recipPoly6q;           // RN(1 / poly6q)
-    uint32_t* epoch;             // device words: the substep's number, counted by the predict kernel, and the cells of the
-                                 // particles that the counting sort samples (kSparseLeast)
+    uint32_t* epoch;             // device words: the substep's number, counted by the predict kernel, the runs of
+                                 // same-cell particles among those that the counting sort samples (kSparseLeast), and
+                                 // the tiles that the scan of a sparse scene has taken
     uint32_t* taint;             // per particle: the last substep that tainted it (quotients_tainted)
     int4* cellXYZ;               // per particle: the cell its friends were taken around, and the scene's first key
                                  // (NULL in relaxed mode: nothing is tainted)
@@ -106,10 +107,9 @@ constexpr int kMaxBlock = 512;
 // Particles from which on a substep that sorts by counting looks whether the scene is
 // sparse (sparse_scene): an idle launch more, and below the build by warps is no slower
 // than the two scans that it replaced (200,000 at 0.5 to a cell 207 us a substep and
-// 224; 500,000 404 and 393).  kSampleBlocks x 256 particles add kSampleOne over the
-// particles of their cell each.
+// 224; 500,000 404 and 393).  kSampleBlocks x 256 particles are asked.
 constexpr int kSparseLeast = 600000;
-constexpr uint32_t kSampleBlocks = 32, kSampleOne = 1024;
+constexpr uint32_t kSampleBlocks = 32;
 
 // Launches a kernel of the substep's chain: it may start before the kernel
 // before it on the stream has ended, and waits for that one's end itself

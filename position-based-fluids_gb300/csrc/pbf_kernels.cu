@@ -81,7 +81,7 @@ __global__ void predict_keys_kernel(DevConsts c, Batch b, const float4* pos, flo
     pred[i] = q;
     if (i == 0) {
         c.epoch[0] += 1u;  // a new substep: earlier taint marks lapse
-        c.epoch[1] = 0u;
+        c.epoch[1] = c.epoch[2] = 0u;
     }
     if (!paused) {
         const uint32_t key = base + grid_hash(__float2int_rz(q.x / c.h), __float2int_rz(q.y / c.h), __float2int_rz(q.z / c.h), c.grid);
@@ -668,17 +668,18 @@ __device__ __noinline__ uint64_t friends_in_chunks(const DevConsts& c, FriendSha
     return counts;
 }
 
-// Whether the scene's cells hold fewer than two particles on average (sample_cells):
-// a warp then takes a run for every particle or two, and the scan by threads is the faster one.  A substep of 1M random
-// particles at 0.5 / 1 / 1.5 / 2 / 3 to a cell of space takes 739 / 785 / 797 / 801 /
-// 810 us by warps and 590 / 705 / 780 / 858 / 968 by threads (4M at 0.5 / 1 / 2:
-// 3,990 / 4,100 / 3,840 and 2,815 / 3,250 / 3,710); two scans by one thread each,
-// with the passes of then, took 704 / 776 / - / 894 / 985 (3,516 / 3,703 / 3,845).
-// Dense scenes pay 4 us a substep for the question.
-// Decided for single warps it is slower: the few of a dense scene take 30 to 70 us
-// after all others have ended.
+// Whether the scene's runs have fewer than two members on average (sample_runs),
+// because cells hold few or many cells share a key: a warp then takes a run for every
+// particle or two, and the scan by threads is the faster one.  A substep of 1M random
+// particles at 0.5 / 1 / 1.5 / 2 / 3 to a cell of space takes 736 / 784 / 787 / 797 /
+// 809 us by warps and 563 / 661 / 728 by threads up to 1.5 (4M at 0.5 / 1 / 2: 3,983 /
+// 4,092 / 3,834 and 2,606 / 2,988 / 3,408); two scans by one thread each, with the
+// passes of then, took 704 / 776 / - / 894 / 985 (3,516 / 3,703 / 3,845).  The friends
+// of 3M dense particles in 2^16 keys: 8.0 ms and 6.9.  Decided for single warps it is
+// slower: the few of a dense scene take 30 to 70 us after all others have ended.
+// Dense scenes pay 3 us a substep for the question.
 __device__ __forceinline__ bool sparse_scene(const DevConsts& c) {
-    return 2u * c.epoch[1] > kSampleBlocks * 256u * kSampleOne;
+    return 2u * c.epoch[1] > kSampleBlocks * 256u;
 }
 
 // The friends of a sparse scene by one thread each, where build_friends_kernel<32>
@@ -688,9 +689,14 @@ build_friends_sparse_kernel(const __grid_constant__ DevConsts c, Batch b, const 
                             uint2* meta, int* err) {
     chain_wait();
     if (!sparse_scene(c)) return;
-#pragma unroll 1
-    for (uint32_t k = blockIdx.x * kBlock + threadIdx.x; k < (uint32_t)c.n; k += gridDim.x * kBlock) {
-        const int i = (int)k;
+    __shared__ uint32_t tile;
+    while (true) {  // tiles of particles, from a counter: they differ in cost
+        __syncthreads();
+        if (threadIdx.x == 0) tile = atomicAdd(c.epoch + 2, 1u);
+        __syncthreads();
+        if (tile * kBlock >= (uint32_t)c.n) return;
+        const int i = (int)(tile * kBlock + threadIdx.x);
+        if (i >= c.n) continue;
         const float4 pi = pred[i];
         const int cx = __float2int_rz(pi.x / c.h), cy = __float2int_rz(pi.y / c.h), cz = __float2int_rz(pi.z / c.h);
         friends_of_one(c, key_base(b, i), pred, cells, rows, meta, err, i, pi, cx, cy, cz);

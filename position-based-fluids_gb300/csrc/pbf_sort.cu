@@ -301,25 +301,19 @@ __device__ __noinline__ uint32_t smaller_in_long_cell(const uint32_t* order, uin
     return less;
 }
 
-// What a particle's cell holds, for sparse_scene: each thread draws one from its part
-// of the order and adds its share of kSampleOne.  Other cells of the same key do not
-// count.  The gather's first blocks do that and nothing else: they end long before
-// its last.
-__device__ __forceinline__ void sample_cells(int n, float perH, const uint32_t* keys, const uint32_t* starts,
-                                          const uint32_t* order, const float4* pred, uint32_t* sampled) {
+// The runs of same-cell particles, for sparse_scene: each thread draws a slot from its
+// part of the scattered order, where a warp's particles of a key lie together, and
+// counts it if the slot before holds a particle of another cell.  The gather's first
+// blocks do that and nothing else: they end long before its last.
+__device__ __forceinline__ void sample_runs(int n, float perH, const uint32_t* order, const float4* pred, uint32_t* sampled) {
     const uint32_t k = blockIdx.x * kThreads + threadIdx.x, part = (uint32_t)n / (kSampleBlocks * kThreads);
-    const uint32_t i = order[k * part + ((k * 2654435761u) >> 8) % part];
-    const float4 p = pred[i];
-    const uint32_t key = keys[i], first = starts[key], end = min(starts[key + 1], first + 16u);
-    const int cx = __float2int_rz(p.x * perH), cy = __float2int_rz(p.y * perH), cz = __float2int_rz(p.z * perH);
-    uint32_t together = 0;
-#pragma unroll 8
-    for (uint32_t q = first; q < end; ++q) {
-        const float4 o = pred[order[q]];
-        together += __float2int_rz(o.x * perH) == cx && __float2int_rz(o.y * perH) == cy && __float2int_rz(o.z * perH) == cz;
-    }
-    const uint32_t share = __reduce_add_sync(0xFFFFFFFFu, kSampleOne / max(together, 1u));
-    if ((threadIdx.x & 31) == 0) atomicAdd(sampled, share);
+    const uint32_t s = max(k * part + ((k * 2654435761u) >> 8) % part, 1u);
+    const float4 p = pred[order[s]], o = pred[order[s - 1u]];
+    const bool head = __float2int_rz(p.x * perH) != __float2int_rz(o.x * perH) ||
+                      __float2int_rz(p.y * perH) != __float2int_rz(o.y * perH) ||
+                      __float2int_rz(p.z * perH) != __float2int_rz(o.z * perH);
+    const int heads = __popc(__ballot_sync(0xFFFFFFFFu, head));
+    if ((threadIdx.x & 31) == 0) atomicAdd(sampled, (uint32_t)heads);
 }
 
 // The particle in slot s of the scattered order goes to its cell's first index
@@ -336,7 +330,7 @@ cell_gather_kernel(int n, float h, uint32_t* sampled, const uint32_t* keys, cons
                    uint32_t keyLimit, int* err) {
     chain_wait();
     if (Sample && blockIdx.x < kSampleBlocks) {
-        sample_cells(n, 1.0f / h, keys, starts, order, pred, sampled);
+        sample_runs(n, 1.0f / h, order, pred, sampled);
         return;
     }
     const int s = (blockIdx.x - (Sample ? kSampleBlocks : 0u)) * blockDim.x + threadIdx.x;

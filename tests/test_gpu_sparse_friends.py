@@ -16,7 +16,7 @@ def _spray(rng, n, per_cell, low, h):
 
 @pytest.mark.parametrize("parts", [[(600_003, 0.5)], [(600_000, 6.0)], [(250_000, 0.3), (300_000, 8.0), (50_001, 2.2)],
                                    [(599_999, 1.0)]])
-@pytest.mark.parametrize("grid", [1 << 19, 300_007])
+@pytest.mark.parametrize("grid", [1 << 19, 300_007, 1 << 14])
 def test_sparse_warps(pbf_mod, oracle_mod, cuda_device, parts, grid):
     params = pbf_mod.load_scenario("dam_break_32k")
     n = params.particleCount = sum(count for count, _ in parts)
