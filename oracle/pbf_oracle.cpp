@@ -816,9 +816,10 @@ void replay_substep(const Structure& st, const Consts<T>& c, int iters, std::vec
 // Reverse accumulation through one substep of the frozen-structure function.
 // xb, vb: adjoints of the substep's output (sorted order) on entry, of its
 // input (previous order) on exit.  cb, gb accumulate dL/d visc and dL/d g.
+// etas: the values to take for eta (NULL: summed here in T).
 template <typename T>
 void adjoint_substep(const Structure& st, const Consts<T>& c, int iters, const Tape<T>& tp, std::vector<V4<T>>& xb,
-                     std::vector<V4<T>>& vb, T& cb, T gb[3]) {
+                     std::vector<V4<T>>& vb, T& cb, T gb[3], const std::vector<V3<T>>* etas = nullptr) {
     const int N = (int)xb.size(), C = c.circles;
     const T negG = -c.gradSpiky, G = c.gradSpiky;
     const std::vector<V4<T>>& p = tp.pI;
@@ -839,6 +840,7 @@ void adjoint_substep(const Structure& st, const Consts<T>& c, int iters, const T
             eta = add(eta, scale(fast_length(xyz(tp.omega[j])), kvec(r, std::sqrt(r2), c.h)));
         }
         eta = scale(negG, eta);
+        if (etas) eta = (*etas)[i];
         T l = fast_length(eta);
         if (!(l > 0)) continue;
         V3<T> Nn = scale((T)1 / l, eta);
@@ -1217,6 +1219,94 @@ double oracle_rollout_replay_f64(void* handle, const double* g, const double* vi
                                  const double* vel0, const double* target_by_id, double* pos_by_id) {
     return replay<double>(*static_cast<RolloutRecord*>(handle), g, visc, pos0, vel0, target_by_id, pos_by_id, nullptr,
                           nullptr, nullptr);
+}
+
+// dL/dv0 (3n doubles, original order) of a rollout given dL/dx (4n doubles by
+// original index): the reverse pass in FP64 over the values that the FP32 forward
+// itself computed.  Only eta is summed in FP32, over the friends in list order
+// with fused multiply-adds, eta = fma(|omega_j|, (h - |r|)^2 (1/|r|) r, eta): where
+// it nearly cancels, its direction is that of its rounding errors.
+int oracle_rollout_grad_at(const PbfParameters* p, int n, const float* pos, const float* vel, int substeps,
+                           const double* dl_dx_by_id, double* dv0, int nthreads) {
+    if (check(p, n) || substeps < 1 || p->completeNeighbours) return -1;
+    if (nthreads > 0) omp_set_num_threads(nthreads);
+    const Consts<float> c = make_consts<float>(*p);
+    std::vector<float> at(pos, pos + 4 * (size_t)n), moves(vel, vel + 4 * (size_t)n);
+    std::vector<uint32_t> ids(n), moved(n);
+    for (int i = 0; i < n; ++i) ids[i] = (uint32_t)i;
+    std::vector<Structure> steps;
+    std::vector<Tape<double>> tapes(substeps);
+    std::vector<std::vector<V3<double>>> etas(substeps, std::vector<V3<double>>(n));
+    auto wide = [&](const std::vector<V4<float>>& a, const std::vector<float>* w) {
+        std::vector<V4<double>> o(n);
+        for (int k = 0; k < n; ++k) o[k] = {a[k].x, a[k].y, a[k].z, w ? (*w)[k] : a[k].w};
+        return o;
+    };
+    auto square = [](const V3<float>& a) { return std::fma(a.z, a.z, std::fma(a.x, a.x, a.y * a.y)); };
+    for (int step = 0; step < substeps; ++step) {
+        State<float> s;
+        s.n = n;
+        s.nKeys = int_ceil((uint32_t)n, 2048u);
+        s.pos.resize(n); s.vel.resize(n); s.pred.resize(n); s.predP.resize(n); s.omega.resize(n);
+        std::memcpy(s.pos.data(), at.data(), 16 * (size_t)n);
+        std::memcpy(s.vel.data(), moves.data(), 16 * (size_t)n);
+        s.density.assign(n, 0); s.lambda.assign(n, 0);
+        s.keys.assign(s.nKeys, 0); s.perm.assign(s.nKeys, 0);
+        s.cells.assign(2 * (size_t)p->gridBufSize, kEmpty);
+        s.friends.assign((size_t)n * c.circles * c.perCircle, 0);
+        s.fcount.assign((size_t)n * c.circles, 0);
+        std::vector<uint8_t> masks((size_t)p->simIterations * n, 0);
+        Tape<double>& tape = tapes[step];
+        predict(s, c, false);
+        sort_particles(s, c);
+        for (int k = 0; k < n; ++k) moved[k] = ids[s.perm[k]];
+        ids.swap(moved);
+        update_cells(s);
+        build_friends(s, c);
+        for (unsigned it = 0; it < p->simIterations; ++it) {
+            compute_scaling(s, c);
+            tape.q.push_back(wide(s.pred, &s.lambda));
+            compute_delta(s, c, masks.data() + (size_t)it * n);
+        }
+        update_velocities(s, c);
+        tape.pI = wide(s.pred, &s.density);
+        tape.v2 = wide(s.vel, nullptr);
+        apply_viscosity(s, c);
+        tape.omega = wide(s.omega, nullptr);
+        steps.push_back(record_structure(s, masks, c.circles));
+        const Structure& st = steps.back();
+        for (int i = 0; i < n; ++i) {
+            int kl, kd;
+            kept_circles(&st.counts[(size_t)i * c.circles], c.circles, kl, kd);
+            const int m = kept_count(&st.counts[(size_t)i * c.circles], kd);
+            V3<float> e = {0, 0, 0};
+            for (int f = 0; f < m; ++f) {
+                const int j = st.list[st.start[i] + f];
+                const V3<float> r = sub(xyz(s.pred[i]), xyz(s.pred[j]));
+                const float r2 = square(r);
+                if (!support(c, r2) || !(std::fabs(s.density[j]) > 1e-8f)) continue;
+                const float rl = std::sqrt(r2), y = 1.0f / rl, hr = c.h - rl;
+                const float ol = std::sqrt(square(xyz(s.omega[j])));
+                const V3<float> k = scale(hr * hr * y, r);
+                e = {std::fma(ol, k.x, e.x), std::fma(ol, k.y, e.y), std::fma(ol, k.z, e.z)};
+            }
+            e = scale(-c.gradSpiky, e);
+            etas[step][i] = {e.x, e.y, e.z};
+        }
+        apply_vorticity(s, c);
+        std::memcpy(at.data(), s.pos.data(), 16 * (size_t)n);
+        std::memcpy(moves.data(), s.vel.data(), 16 * (size_t)n);
+    }
+    std::vector<V4<double>> xb(n), vb(n, V4<double>{0, 0, 0, 0});
+    for (int k = 0; k < n; ++k) {
+        const double* d = dl_dx_by_id + 4 * (size_t)ids[k];
+        xb[k] = {d[0], d[1], d[2], 0};
+    }
+    double cb = 0, gb[3] = {0, 0, 0};
+    for (size_t k = steps.size(); k-- > 0;)
+        adjoint_substep(steps[k], make_consts<double>(*p), (int)p->simIterations, tapes[k], xb, vb, cb, gb, &etas[k]);
+    for (int i = 0; i < n; ++i) { dv0[3 * i] = vb[i].x; dv0[3 * i + 1] = vb[i].y; dv0[3 * i + 2] = vb[i].z; }
+    return 0;
 }
 
 // Loss and its exact gradient (FP64) with respect to the initial velocities

@@ -584,19 +584,18 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
     pbf::launch_apply_viscosity(c, b, ctx->pred[a], ctx->vel[V], ctx->vel[V ^ 1], omega, near, meta, rows, ls.viscosity,
                                 ls.balance, tiles(3), s);
     mark("applyVorticity");
-    float4* eta = tape ? tape->eta : nullptr;
     const int vortTiles = (c.n + ls.vorticity - 1) / ls.vorticity;
     if (ctx->readVel && ctx->readPos && vortTiles >= 2) {
         // the first half of the particles' velocities copy out while the second half runs
         const int half = vortTiles / 2;
         const size_t headBytes = 16 * (size_t)half * (size_t)ls.vorticity;
-        pbf::launch_apply_vorticity(c, ctx->pred[a], near, omega, ctx->vel[V ^ 1], ctx->vel[V], eta, meta, rows,
+        pbf::launch_apply_vorticity(c, ctx->pred[a], near, omega, ctx->vel[V ^ 1], ctx->vel[V], meta, rows,
                                     ls.vorticity, ls.balance, nullptr, s, 0, half);
         PBF_CUDA(ctx, cudaEventRecord(ctx->evVelHead, s));
         PBF_CUDA(ctx, cudaStreamWaitEvent(ctx->copyStream, ctx->evVelHead, 0));
         PBF_CUDA(ctx, cudaMemcpyAsync(ctx->readVel, ctx->vel[V], headBytes, cudaMemcpyDeviceToHost, ctx->copyStream));
         PBF_CUDA(ctx, cudaEventRecord(ctx->evCopyDone, ctx->copyStream));
-        pbf::launch_apply_vorticity(c, ctx->pred[a], near, omega, ctx->vel[V ^ 1], ctx->vel[V], eta, meta, rows,
+        pbf::launch_apply_vorticity(c, ctx->pred[a], near, omega, ctx->vel[V ^ 1], ctx->vel[V], meta, rows,
                                     ls.vorticity, ls.balance, nullptr, s, half, vortTiles - half);
         PBF_CUDA(ctx, cudaMemcpyAsync(reinterpret_cast<char*>(ctx->readVel) + headBytes,
                                       reinterpret_cast<const char*>(ctx->vel[V]) + headBytes, v4 - headBytes,
@@ -604,7 +603,7 @@ int enqueue_substep(pbf_ctx* ctx, StageClock* clock, const pbf::AdjointTape* tap
         velCopied = true;
         ++launched;
     } else {
-        pbf::launch_apply_vorticity(c, ctx->pred[a], near, omega, ctx->vel[V ^ 1], ctx->vel[V], eta, meta, rows,
+        pbf::launch_apply_vorticity(c, ctx->pred[a], near, omega, ctx->vel[V ^ 1], ctx->vel[V], meta, rows,
                                     ls.vorticity, ls.balance, tiles(4), s);
     }
     launched += 2;
@@ -747,7 +746,6 @@ int ensure_tape(pbf_ctx* ctx) {
             t.sums[it] = (float4*)take(v4);
             t.rho[it] = (float*)take(4 * (size_t)n);
         }
-        t.eta = (float4*)take(v4);
         t.mask = clamp ? (uint8_t*)take((size_t)iters * n) : nullptr;
         t.pI = (float4*)take(v4);
         t.v2 = (float4*)take(v4);

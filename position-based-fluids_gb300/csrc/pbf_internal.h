@@ -161,7 +161,7 @@ int launch_build_friends(const DevConsts& c, Batch b, const float4* pred, const 
 // uint4 entries per particle of the rows for `slots` friends, at least the four
 // that eight lanes read ahead (first_entry in pbf_device.cuh).
 inline size_t row_entries(int slots) { return slots > 16 ? ((size_t)slots + 3) / 4 : 4; }
-// tapeSums, tapeRho, tapeEta below: a rollout's tape (AdjointTape; NULL without).
+// tapeSums, tapeRho below: a rollout's tape (AdjointTape; NULL without).
 void launch_compute_scaling(const DevConsts& c, const float4* pred, float4* predPacked, float* density,
                             float4* tapeSums, float* tapeRho, const uint2* meta, const uint4* rows, int block, int balance, int* tileCounter,
                             cudaStream_t s);
@@ -193,7 +193,7 @@ void launch_apply_viscosity(const DevConsts& c, Batch b, const float4* pred, con
 // last vorticity pass so that the first part's velocities copy out while the
 // rest runs).
 void launch_apply_vorticity(const DevConsts& c, const float4* pred, const float4* near, const float4* omega,
-                            const float4* velIn, float4* velOut, float4* tapeEta, const uint2* meta, const uint4* rows, int block, int balance,
+                            const float4* velIn, float4* velOut, const uint2* meta, const uint4* rows, int block, int balance,
                             int* tileCounter, cudaStream_t s, int firstTile = 0, int tileCount = 0);
 
 // ---- radix sort (pbf_sort.cu) ----
@@ -260,7 +260,6 @@ struct AdjointTape {
     float4* q[64] = {};            // (p^t, lambda^t), t < iterations
     float4* sums[64] = {};         // per iteration sum g and sum |g|^2 + |sum g|^2, g the density pass' gradients
     float* rho[64] = {};           // per iteration the density
-    float4* eta = nullptr;         // the vorticity pass' eta, not normalised
     uint8_t* mask = nullptr;       // iterations x N box-clamp decisions (NULL: no clamp)
     float4* pI = nullptr;          // final predictions, w = density
     float4* v2 = nullptr;          // velocities before XSPH

@@ -1417,7 +1417,7 @@ template <bool R, bool Q, int L>
 __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const float4* near,
                                                      const float4* omega,
                                                      const float4* velIn, float4* velOut,
-                                                     float4* tapeEta, const uint4* rows, int i,
+                                                     const uint4* rows, int i,
                                                      uint4 head, const float4 pi, uint64_t mt) {
     const int n = c.n;
     float ex = 0.0f, ey = 0.0f, ez = 0.0f;
@@ -1484,7 +1484,6 @@ __device__ __forceinline__ void apply_vorticity_body(const DevConsts& c, const f
     ex = ex * c.negGradSpiky;
     ey = ey * c.negGradSpiky;
     ez = ez * c.negGradSpiky;
-    if (tapeEta) tapeEta[i] = make_float4(ex, ey, ez, 0.0f);
     if (R) {
         const float l2 = fmaf(ez, ez, fmaf(ey, ey, ex * ex));
         if (l2 > 0.0f) {
@@ -1513,7 +1512,7 @@ template <bool R, bool B, int L>
 __global__ void __maxnreg__(56)
 apply_vorticity_kernel(const __grid_constant__ DevConsts c, const float4* pred, const float4* near,
                        const float4* omega, const float4* velIn, float4* velOut,
-                       float4* tapeEta, const uint2* meta,
+                       const uint2* meta,
                        const uint4* rows, int tiles, int* tileCounter, int tileOffset) {
     chain_wait();
     for_tiles(tiles, tileCounter, [&](int tile) {
@@ -1524,8 +1523,8 @@ apply_vorticity_kernel(const __grid_constant__ DevConsts c, const float4* pred, 
         const uint4 head = first_entry<L>(rows, c.n, i);
         const uint64_t mt = load_meta(meta, i);
         // a particle that may hold a friend at an irregular position divides the IEEE way
-        if (!R && c.quotients && !quotients_tainted<L>(c, i)) apply_vorticity_body<R, true, L>(c, near, omega, velIn, velOut, tapeEta, rows, i, head, pi, mt);
-        else apply_vorticity_body<R, false, L>(c, near, omega, velIn, velOut, tapeEta, rows, i, head, pi, mt);
+        if (!R && c.quotients && !quotients_tainted<L>(c, i)) apply_vorticity_body<R, true, L>(c, near, omega, velIn, velOut, rows, i, head, pi, mt);
+        else apply_vorticity_body<R, false, L>(c, near, omega, velIn, velOut, rows, i, head, pi, mt);
     });
 }
 
@@ -1663,18 +1662,18 @@ void launch_apply_viscosity(const DevConsts& c, Batch b, const float4* pred, con
 }
 
 void launch_apply_vorticity(const DevConsts& c, const float4* pred, const float4* near, const float4* omega,
-                            const float4* velIn, float4* velOut, float4* tapeEta, const uint2* meta, const uint4* rows, int block, int balance,
+                            const float4* velIn, float4* velOut, const uint2* meta, const uint4* rows, int block, int balance,
                             int* tileCounter, cudaStream_t s, int firstTile, int tileCount) {
     const int lanes = lanes_per_particle(c, balance, tileCounter);
     auto k = c.relaxed ? (lanes > 1 ? apply_vorticity_kernel<true, false, 4> : balance ? apply_vorticity_kernel<true, true, 1> : apply_vorticity_kernel<true, false, 1>)
                        : (lanes == 8 ? apply_vorticity_kernel<false, false, 8> : lanes == 4 ? apply_vorticity_kernel<false, false, 4> : balance ? apply_vorticity_kernel<false, true, 1> : apply_vorticity_kernel<false, false, 1>);
     if (tileCount > 0) {  // tiles [firstTile, firstTile + tileCount), one block each
-        launch_chained(k, (unsigned)(tileCount * lanes), block, s, c, pred, near, omega, velIn, velOut, tapeEta, meta, rows, 0, nullptr, firstTile);
+        launch_chained(k, (unsigned)(tileCount * lanes), block, s, c, pred, near, omega, velIn, velOut, meta, rows, 0, nullptr, firstTile);
         return;
     }
     int tiles = 0;
     const unsigned grid = grid_for_tiles(k, c.n * lanes, block, tileCounter != nullptr, &tiles);
-    launch_chained(k, grid, block, s, c, pred, near, omega, velIn, velOut, tapeEta, meta, rows, tiles, tileCounter, 0);
+    launch_chained(k, grid, block, s, c, pred, near, omega, velIn, velOut, meta, rows, tiles, tileCounter, 0);
 }
 
 }  // namespace pbf
