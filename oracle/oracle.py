@@ -52,7 +52,7 @@ def lib() -> ctypes.CDLL:
         l.oracle_rollout_grad_f64.restype = c_double
         l.oracle_rollout_grad_f32.argtypes = [c_void_p] * 8
         l.oracle_rollout_grad_f32.restype = c_double
-        l.oracle_rollout_grad_at.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int]
+        l.oracle_rollout_grad_at.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int]
         l.oracle_rollout_grad_at.restype = c_int
         l.oracle_set_force_planes.argtypes = [c_void_p, c_int, c_void_p, c_int, c_int]
         l.oracle_set_force_planes.restype = c_int
@@ -295,17 +295,19 @@ def ref_sort(params, pred):
 
 
 def rollout_grad_at(params, pos, vel, substeps, dl_dx, threads=0):
-    """dL/dv0 [n,3] of a rollout given dL/dx [n,4]: the reverse pass in FP64 over
-    the FP32 forward's own values, with eta summed in FP32 in list order by fused
+    """(dL/dv0 [n,3], dL/d viscosityFactor) of a rollout given dL/dx [n,4]: the
+    reverse pass in FP64 over the FP32 forward's own values, with eta summed in FP32 in list order by fused
     multiply-adds."""
     n = int(params.particleCount)
     p = np.ascontiguousarray(pos, np.float32).reshape(n, 4)
     v = np.ascontiguousarray(vel, np.float32).reshape(n, 4)
     d = np.ascontiguousarray(dl_dx, np.float64).reshape(n, 4)
     out = np.zeros((n, 3), np.float64)
-    if lib().oracle_rollout_grad_at(ctypes.byref(params), n, _ptr(p), _ptr(v), substeps, _ptr(d), _ptr(out), threads):
+    dc = c_double(0)
+    if lib().oracle_rollout_grad_at(ctypes.byref(params), n, _ptr(p), _ptr(v), substeps, _ptr(d), _ptr(out),
+                                    ctypes.byref(dc), threads):
         raise ValueError("oracle_rollout_grad_at rejected the input")
-    return out
+    return out, dc.value
 
 
 class Rollout:

@@ -1221,13 +1221,13 @@ double oracle_rollout_replay_f64(void* handle, const double* g, const double* vi
                           nullptr, nullptr);
 }
 
-// dL/dv0 (3n doubles, original order) of a rollout given dL/dx (4n doubles by
-// original index): the reverse pass in FP64 over the values that the FP32 forward
+// dL/dv0 (3n doubles, original order) and dL/d visc of a rollout given dL/dx (4n
+// doubles by original index): the reverse pass in FP64 over the values that the FP32 forward
 // itself computed.  Only eta is summed in FP32, over the friends in list order
 // with fused multiply-adds, eta = fma(|omega_j|, (h - |r|)^2 (1/|r|) r, eta): where
 // it nearly cancels, its direction is that of its rounding errors.
 int oracle_rollout_grad_at(const PbfParameters* p, int n, const float* pos, const float* vel, int substeps,
-                           const double* dl_dx_by_id, double* dv0, int nthreads) {
+                           const double* dl_dx_by_id, double* dv0, double* dvisc, int nthreads) {
     if (check(p, n) || substeps < 1 || p->completeNeighbours) return -1;
     if (nthreads > 0) omp_set_num_threads(nthreads);
     const Consts<float> c = make_consts<float>(*p);
@@ -1306,6 +1306,7 @@ int oracle_rollout_grad_at(const PbfParameters* p, int n, const float* pos, cons
     for (size_t k = steps.size(); k-- > 0;)
         adjoint_substep(steps[k], make_consts<double>(*p), (int)p->simIterations, tapes[k], xb, vb, cb, gb, &etas[k]);
     for (int i = 0; i < n; ++i) { dv0[3 * i] = vb[i].x; dv0[3 * i + 1] = vb[i].y; dv0[3 * i + 2] = vb[i].z; }
+    *dvisc = cb;
     return 0;
 }
 

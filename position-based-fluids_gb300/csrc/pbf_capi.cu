@@ -754,7 +754,7 @@ int ensure_tape(pbf_ctx* ctx) {
     pbf::AdjointBuffers& ab = ctx->adj;
     float4** vecs[] = {&ab.xb, &ab.vb, &ab.xo, &ab.vo, &ab.pb, &ab.pbt, &ab.omb, &ab.v2b, &ab.xsb, &ctx->adjById};
     for (float4** v : vecs) *v = (float4*)take(v4);
-    ab.scalars = (float*)take(16);
+    ab.scalars = (pbf::AdjointScalars*)take(sizeof(pbf::AdjointScalars));
     cudaGetLastError();
     if (!ok) {
         free_tape(ctx);
@@ -1809,7 +1809,7 @@ int pbf_rollout_backward(pbf_ctx* ctx, const float* dL_dx, float* dL_dv0, float*
     PBF_CUDA(ctx, cudaMemcpyAsync(ctx->adjById, dL_dx, v4, cudaMemcpyHostToDevice, s));
     pbf::scatter_by_id(n, ctx->ckptEnd.ids, ctx->adjById, ab.xb, s);
     PBF_CUDA(ctx, cudaMemsetAsync(ab.vb, 0, v4, s));
-    PBF_CUDA(ctx, cudaMemsetAsync(ab.scalars, 0, 16, s));
+    PBF_CUDA(ctx, cudaMemsetAsync(ab.scalars, 0, sizeof(*ab.scalars), s));
     // the accumulators start at zero, and the adjoint kernels leave them so
     for (float4* v : {ab.pb, ab.pbt, ab.omb, ab.v2b}) PBF_CUDA(ctx, cudaMemsetAsync(v, 0, v4, s));
     ctx->launches += 1;
@@ -1830,13 +1830,13 @@ int pbf_rollout_backward(pbf_ctx* ctx, const float* dL_dx, float* dL_dv0, float*
     pbf::gather_to_id(n, ctx->ckpt[0].ids, ab.vb, ctx->adjById, s);
     ctx->launches += 1;
     if (dL_dv0) PBF_CUDA(ctx, cudaMemcpyAsync(dL_dv0, ctx->adjById, v4, cudaMemcpyDeviceToHost, s));
-    float sc[4] = {0, 0, 0, 0};
-    PBF_CUDA(ctx, cudaMemcpyAsync(sc, ab.scalars, 16, cudaMemcpyDeviceToHost, s));
+    pbf::AdjointScalars sc = {};
+    PBF_CUDA(ctx, cudaMemcpyAsync(&sc, ab.scalars, sizeof(sc), cudaMemcpyDeviceToHost, s));
     if ((rc = load_checkpoint(ctx, ctx->ckptEnd))) return rc;
     PBF_CUDA(ctx, cudaStreamSynchronize(s));
     PBF_CUDA(ctx, cudaGetLastError());
-    if (dL_dvisc) *dL_dvisc = sc[0];
-    if (dL_dg) { dL_dg[0] = sc[1]; dL_dg[1] = sc[2]; dL_dg[2] = sc[3]; }
+    if (dL_dvisc) *dL_dvisc = (float)sc.visc;
+    if (dL_dg) std::copy(sc.gravity, sc.gravity + 3, dL_dg);
     return read_error_word(ctx);
 }
 

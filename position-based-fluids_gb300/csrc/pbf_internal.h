@@ -267,9 +267,13 @@ struct AdjointTape {
 };
 // Adjoint state; xb / vb hold the adjoints of the substep's output on entry
 // and of its input on return (the pointers are swapped with xo / vo).
+struct AdjointScalars {
+    double visc;       // dL/d viscosityFactor
+    float gravity[3];  // dL/d gravity
+};
 struct AdjointBuffers {
     float4 *xb, *vb, *xo, *vo, *pb, *pbt, *omb, *v2b, *xsb;
-    float* scalars;  // [0] dL/d viscosityFactor, [1..3] dL/d gravity
+    AdjointScalars* scalars;  // on the device
 };
 // Between substeps pb, pbt, omb and v2b are zero.
 void adjoint_substep(const DevConsts& c, const AdjointTape& tp, AdjointBuffers& ab, cudaStream_t s);

@@ -28,7 +28,7 @@ def test_reverse_pass_sums_eta_in_list_order(pbf_mod, oracle_mod, cuda_device, d
     vel[:, :3] = np.cross(np.array([1.0, 0.5, 0.25]), arm).astype(np.float32)
     dldx = np.zeros((len(pos), 4), np.float32)
     dldx[:, :3] = np.random.default_rng(3).normal(0.0, 1.0, (len(pos), 3))
-    want = oracle_mod.rollout_grad_at(params, pos, vel, substeps, dldx)
+    want, _ = oracle_mod.rollout_grad_at(params, pos, vel, substeps, dldx)
     with pbf_mod.Simulation.create(params, pos, vel, device=cuda_device) as sim:
         sim.rollout_forward(substeps, substeps)
         got, _, _ = sim.rollout_backward(dldx)
